@@ -126,6 +126,16 @@ inline void mh2d_guided_chunks(int nx, int ny, int strip_w, int slots, int &h1, 
     cache[key] = std::make_tuple(h1, h2, tail);
 }
 
+struct Mh2dBand;
+
+/* The staged FP64 step (mh2d_staged.cuh).  staged_plan splits the grid's rows
+ * into bands whose workspace takes at most `budget` bytes (one row at least;
+ * `bytes` receives what it takes); the caller points every band's `ws` at
+ * that workspace. */
+void staged_plan(const Mh2dArgs<double> &a, size_t budget, std::vector<Mh2dBand> &bands, size_t &bytes);
+cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s);
+cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
+
 template <class R>
 cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s);
 template <class R>

@@ -7,9 +7,11 @@
  * operations as the reference CPU code, which never contracts a*b+c.
  */
 #include "mh2d_lim.cuh"
+#include "mh2d_staged_launch.cuh"
 
 namespace hydro {
 
 HYDRO_MH2D_INSTANTIATE(double, LIM_MINMOD, 1)
+HYDRO_STAGED_INSTANTIATE(LIM_MINMOD, 1)
 
 }  // namespace hydro

@@ -6,10 +6,12 @@
  * operations as the reference CPU code, which never contracts a*b+c.
  */
 #include "mh2d_lim.cuh"
+#include "mh2d_staged_launch.cuh"
 
 namespace hydro {
 
 HYDRO_MH2D_INSTANTIATE(double, LIM_VAN_LEER, 0)
+HYDRO_STAGED_INSTANTIATE(LIM_VAN_LEER, 0)
 template cudaError_t mh2d_launch_tape_lim<double, LIM_VAN_LEER>(const Mh2dArgs<double> &, int, cudaStream_t);
 
 }  // namespace hydro

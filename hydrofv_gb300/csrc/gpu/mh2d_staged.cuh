@@ -1,0 +1,451 @@
+/*
+ * mh2d_staged.cuh -- the FP64 2D step in three kernels per time step.
+ *
+ *   recon    per cell and direction: limited slopes and the Hancock half
+ *            step, the states at the cell's two faces
+ *            (src/integrator_muscl_hancock.c:682-755, :967-1041);
+ *   flux     per face: the HLLC flux and its update term (F dt) A
+ *            (src/riemann_solver_hllc.c:202-376);
+ *   update   per cell: the gather in the reference's order, gravity, U -> W,
+ *            the next step's CFL maxima; the last block advances the clock
+ *            and forms the next step's dt.
+ *
+ * The pointwise arithmetic is that of numerics.cuh, so the results are the
+ * bits of the reference's step (and of the fused kernel of mh2d_kernel.cuh).
+ *
+ * Why three kernels.  The fused kernel marches rows: a work item's rows are a
+ * serial chain of divides, square roots and pow with four barriers each, so a
+ * step costs at least one item (about 270 us) however small the grid is, and
+ * 16 warps per SM (128 registers) cannot hide those chains.  One thread per
+ * face or cell makes the step as long as three short chains and fills the
+ * chip from a few thousand cells on; each kernel takes only the registers of
+ * its own part, so more warps are resident.  The price is the workspace:
+ * about 530 bytes per cell-update pass through L2 or HBM, 10% of the HBM rate
+ * at 1.3 G cell-updates/s, under the arithmetic.  Time per step, fused ->
+ * staged: 64^2 276 -> 47 us, 122^2 with gravity 282 -> 58, 401 x 250 van Leer
+ * 308 -> 113, 1024^2 blast 0.86 -> 0.65 ms, 2048^2 3.25 -> 3.07 ms.
+ *
+ * Kernels follow one another by programmatic dependent launch: the next
+ * kernel's blocks become resident while this one drains and wait for its
+ * results (pdl_begin), which hides the launch gaps of small grids.
+ */
+#ifndef HYDRO_GPU_MH2D_STAGED_CUH
+#define HYDRO_GPU_MH2D_STAGED_CUH
+
+#include "mh2d_kernel.cuh"
+
+#ifndef MH2D_RECON_CTAS
+#define MH2D_RECON_CTAS 6
+#endif
+#ifndef MH2D_FLUX_CTAS
+#define MH2D_FLUX_CTAS 5
+#endif
+#ifndef MH2D_UPDATE_CTAS
+#define MH2D_UPDATE_CTAS 6
+#endif
+
+namespace hydro {
+
+/* Threads per block: 128, or one warp where the grid has too few cells to
+ * give every scheduler a warp otherwise. */
+constexpr int kStagedThreads = 128;
+constexpr int kStagedSmall = 32;
+constexpr unsigned kStagedSmallItems = 152 * 4 * 2 * 32;   /* two warps for each of the 608 schedulers */
+constexpr unsigned kStagedUpdateGrid = 152 * MH2D_UPDATE_CTAS;
+
+/* Fields of the workspace: the low and high face states of each cell in x
+ * and y.  The flux kernel leaves a face's update term where its left (lower)
+ * state was. */
+enum : int { WS_XLO = 0, WS_XHI = 4, WS_YLO = 8, WS_YHI = 12, WS_FIELDS = 16 };
+
+/* The rows of a step are processed in one band as long as its workspace stays
+ * below a fixed size (1 GiB in runtime2d.cu).  Bands small enough for the L2
+ * cache lost: 2048^2 3.07 ms with one band, 3.16 / 3.22 / 3.35 / 3.70 ms with
+ * 160 / 96 / 48 / 24 MB (the launches' tails cost more than the traffic).
+ *
+ * Rows [r0, r1) (padded indices) of one grid and the workspace they use: a
+ * plane holds rows r0 - 1 .. r1 with the grid's pitch. */
+struct Mh2dBand {
+    int r0, r1;
+    unsigned update_blocks;   /* update blocks of the whole step of this grid (all bands) */
+    long long plane;          /* doubles per workspace field */
+    double *ws;
+};
+
+inline __host__ __device__ unsigned staged_recon_items(int nx, int rows) { return (unsigned) rows * (nx + 2) + (unsigned) (rows + 2) * nx; }
+inline __host__ __device__ unsigned staged_face_items(int nx, int rows) { return (unsigned) rows * (nx + 1) + (unsigned) (rows + 1) * nx; }
+
+/* Programmatic dependent launch: let the next kernel's blocks start (they
+ * wait below), and wait for the previous kernel's results. */
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+/* The dt of step n, which starts at time t with the maxima smax[n % 3], and
+ * the ratios dt A / V (src/integrator_muscl_hancock.c:533-549, src/utils.c:55-95).
+ * One converged warp; the two directions' quotients run in two lanes. */
+__device__ __forceinline__ void arm_dt(const Mh2dArgs<double> &a, HydroStepControl *ctrl, long long n, double t,
+                                       double tf)
+{
+    const int lane = threadIdx.x & 31;
+    const bool y = lane & 1;
+    const double S = from_ordered_bits(*(volatile unsigned long long *) &ctrl->smax[n % 3][y]);
+    const double q = dv(S, y ? a.dy : a.dx);
+    const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
+    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
+    double dt = dv(cfl, qx + qy);
+    if (t + dt > tf) dt = tf - t;
+    const double w = dv(dt * (y ? a.area_y : a.area_x), a.vol);
+    if (lane == 0) ctrl->step_dt = dt;
+    if (lane < 2) ctrl->step_dtA[lane] = w;
+}
+
+/* Face states of item k of the band: first the x items (rows r0 .. r1-1,
+ * columns g-1 .. g+nx), then the y items (rows r0-1 .. r1, columns g ..
+ * g+nx-1). */
+template <int LIM, int FIRST_ORDER>
+__device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned k, int buf, bool raw,
+                                             const double dtA[2])
+{
+    const unsigned nx = (unsigned) a.nx, nX = (unsigned) (b.r1 - b.r0) * (nx + 2);
+    const bool y = k >= nX;
+    int r, c;
+    if (!y) {
+        const unsigned q = k / (nx + 2);
+        r = b.r0 + (int) q;
+        c = a.g - 1 + (int) (k - q * (nx + 2));
+    } else {
+        const unsigned j = k - nX, q = j / nx;
+        r = b.r0 - 1 + (int) q;
+        c = a.g + (int) (j - q * nx);
+    }
+    const double *const *W = a.W[buf];
+    const double *const *U = a.U[buf];
+    double w[5];
+    fetch_w(a, W, U, raw, r, c, w);
+    const double n = y ? w[2] : w[1], t = y ? w[1] : w[2];
+    double lo[4], hi[4];
+    if (FIRST_ORDER) {
+        lo[0] = hi[0] = w[0]; lo[1] = hi[1] = n; lo[2] = hi[2] = t; lo[3] = hi[3] = w[3];
+    } else {
+        double wm[5], wp[5];
+        fetch_w(a, W, U, raw, y ? r - 1 : r, y ? c : c - 1, wm);
+        fetch_w(a, W, U, raw, y ? r + 1 : r, y ? c : c + 1, wp);
+        double s[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] = limit_slope<LIM>(w[q] - wm[q], wp[q] - w[q]);
+        const double h = y ? dtA[1] : dtA[0];
+        const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
+        hancock_2d(h, dv(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
+    }
+    double *o = b.ws + (long long) (r - b.r0 + 1) * a.pitch + c + (y ? WS_YLO : WS_XLO) * b.plane;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        o[q * b.plane] = lo[q];
+        o[(4 + q) * b.plane] = hi[q];
+    }
+}
+
+template <int NT>
+struct FluxShared {
+    double rho[2][NT], u[2][NT], p[2][NT], a[2][NT];   /* both states of each face */
+    double pg[NT];                                     /* star-pressure guess */
+    short listT[NT], listS[NT];
+    int nT, nS;
+};
+
+/* The flux of one block's faces: face k of the band for thread k0 + tid.
+ * Faces are classified, the expensive guesses run on compacted lists, and
+ * each thread finishes its own face from registers. */
+template <int NT, bool TAPE>
+__device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared<NT> &sm, unsigned k,
+                                            unsigned total, double dt)
+{
+    const int tid = threadIdx.x;
+    const bool on = k < total;
+    const unsigned nx = (unsigned) a.nx, nX = (unsigned) (b.r1 - b.r0) * (nx + 1);
+    const bool y = k >= nX;
+    long long at = 0, tape_at = 0;
+    double L[4], R[4], aL = 0, aR = 0, pg = 0;
+    int reg = PREG_PVRS;
+    if (tid == 0) { sm.nT = 0; sm.nS = 0; }
+    __syncthreads();
+    if (on) {
+        int r, c;
+        if (!y) {
+            const unsigned q = k / (nx + 1);
+            r = b.r0 + (int) q;
+            c = a.g - 1 + (int) (k - q * (nx + 1));
+        } else {
+            const unsigned j = k - nX, q = j / nx;
+            r = b.r0 - 1 + (int) q;
+            c = a.g + (int) (j - q * nx);
+        }
+        at = (long long) (r - b.r0 + 1) * a.pitch + c;
+        tape_at = (long long) r * a.pitch + c;
+        const double *l = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
+        const double *h = b.ws + (y ? WS_YLO : WS_XLO) * b.plane + at + (y ? a.pitch : 1);
+#pragma unroll
+        for (int q = 0; q < 4; q++) { L[q] = l[q * b.plane]; R[q] = h[q * b.plane]; }
+        reg = hllc_classify(a.gas, L[0], L[1], L[3], R[0], R[1], R[3], aL, aR, pg);
+        if (reg == PREG_TRRS || reg == PREG_TSRS) {
+            sm.rho[0][tid] = L[0]; sm.u[0][tid] = L[1]; sm.p[0][tid] = L[3]; sm.a[0][tid] = aL;
+            sm.rho[1][tid] = R[0]; sm.u[1][tid] = R[1]; sm.p[1][tid] = R[3]; sm.a[1][tid] = aR;
+            sm.pg[tid] = pg;
+            if (reg == PREG_TRRS) sm.listT[atomicAdd(&sm.nT, 1)] = (short) tid;
+            else sm.listS[atomicAdd(&sm.nS, 1)] = (short) tid;
+        }
+    }
+    __syncthreads();
+    double z0 = 0, z1 = 0;
+    const int nT = sm.nT, nS = sm.nS;
+    for (int i = tid; i < nT + nS; i += NT) {
+        if (i < nT) {
+            const int f = sm.listT[i];
+            sm.pg[f] = guess_p_trrs_z(a.gas, sm.u[0][f], sm.p[0][f], sm.a[0][f], sm.u[1][f], sm.p[1][f], sm.a[1][f], z0, z1);
+            if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
+        } else {
+            const int f = sm.listS[i - nT];
+            sm.pg[f] = guess_p_tsrs_g(a.gas, sm.rho[0][f], sm.u[0][f], sm.p[0][f], sm.rho[1][f], sm.u[1][f], sm.p[1][f],
+                                      sm.pg[f], z0, z1);
+            if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
+        }
+    }
+    __syncthreads();
+    if (!on) return;
+    double F[4];
+    double wave[3] = { 0.0, 0.0, 0.0 };
+    const bool guessed = reg == PREG_TRRS || reg == PREG_TSRS;
+    if (guessed) pg = sm.pg[tid];
+    if (reg == PREG_VACUUM) {
+        vacuum_flux_dev(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, F);
+    } else {
+        const int rc = hllc_finish(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, pg, F,
+                                   TAPE ? wave : nullptr);
+        if (rc) record_error(a.ctrl, rc, (int) blockIdx.x);
+    }
+    if constexpr (TAPE) {
+        double *t = a.tape + (y ? MH2D_TAPE_FIELDS : 0) * a.tape_plane + tape_at;
+        const double v[MH2D_TAPE_FIELDS] = { L[0], L[1], L[2], L[3], R[0], R[1], R[2], R[3], aL, aR, pg,
+                                             guessed ? sm.rho[0][tid] : 0.0, guessed ? sm.rho[1][tid] : 0.0,
+                                             (double) reg, wave[0], wave[1], wave[2] };
+#pragma unroll
+        for (int q = 0; q < MH2D_TAPE_FIELDS; q++) t[q * a.tape_plane] = v[q];
+    }
+    const double A = y ? a.area_y : a.area_x;
+    double *o = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
+#pragma unroll
+    for (int q = 0; q < 4; q++) o[q * b.plane] = (F[q] * dt) * A;
+}
+
+/* Cell k of the band: update, gravity, U -> W; mx receives a + |u|, a + |v|. */
+template <bool GRAV>
+__device__ __forceinline__ void staged_update(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned k, int buf, double dt,
+                                              double &mx_x, double &mx_y)
+{
+    const int ymap[4] = { 0, 2, 1, 3 };   /* y fluxes come back as (mass, mom_y, mom_x, energy) */
+    const unsigned nx = (unsigned) a.nx, q0 = k / nx;
+    const int r = b.r0 + (int) q0, c = a.g + (int) (k - q0 * nx);
+    const long long idx = (long long) r * a.pitch + c;
+    const double *fx = b.ws + WS_XHI * b.plane + (long long) (r - b.r0 + 1) * a.pitch + c;
+    const double *fy = b.ws + WS_YHI * b.plane + (long long) (r - b.r0 + 1) * a.pitch + c;
+    const double *const *Uin = a.U[buf];
+    double *const *Uout = a.U[buf ^ 1];
+    double *const *Wout = a.W[buf ^ 1];
+    double Un[4], fl[4], fh[4], gl[4], gh[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        fl[q] = fx[q * b.plane - 1];
+        fh[q] = fx[q * b.plane];
+        gl[q] = fy[ymap[q] * b.plane - a.pitch];
+        gh[q] = fy[ymap[q] * b.plane];
+        Un[q] = Uin[q][idx];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        double v = Un[q];
+        v = v + fl[q];
+        v = v - fh[q];
+        v = v + gl[q];
+        v = v - gh[q];
+        Un[q] = v;
+    }
+    if constexpr (GRAV) gravity_kick(-dt * a.gravity, Un[0], Un[2], Un[3]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) Uout[q][idx] = Un[q];
+    double w[4];
+    cons_to_prim_2d(a.gas, a.vol, Un[0], Un[1], Un[2], Un[3], w);
+    const double as = sound_speed(a.gas, w[0], w[3]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) Wout[q][idx] = w[q];
+    Wout[4][idx] = as;
+    const double sx = as + fabs(w[1]), sy = as + fabs(w[2]);
+    if (lt(mx_x, sx)) mx_x = sx;
+    if (lt(mx_y, sy)) mx_y = sy;
+    /* the first ghost layer receives its one-sided update */
+    if (c == a.g) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx - 1] = Uin[q][idx - 1] - fl[q];
+    }
+    if (c == a.g + a.nx - 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx + 1] = Uin[q][idx + 1] + fh[q];
+    }
+    if (r == a.g) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx - a.pitch] = Uin[q][idx - a.pitch] - gl[q];
+    }
+    if (r == a.g + a.ny - 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx + a.pitch] = Uin[q][idx + a.pitch] + gh[q];
+    }
+}
+
+template <int NT>
+struct UpdateShared {
+    double red[2][NT / 32];
+    int am_last;
+};
+
+/* End of an update block: fold its maxima into the next step's words; the
+ * last block of the grid advances the clock (src/integrator_muscl_hancock.c:
+ * 1143-1154) and forms the next dt. */
+template <int NT>
+__device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateShared<NT> &sm, unsigned blocks, long long n,
+                                              double dt, double mx_x, double mx_y)
+{
+    const int tid = threadIdx.x;
+    HydroStepControl *ctrl = a.ctrl;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ox = __shfl_xor_sync(0xffffffffu, mx_x, o);
+        const double oy = __shfl_xor_sync(0xffffffffu, mx_y, o);
+        if (lt(mx_x, ox)) mx_x = ox;
+        if (lt(mx_y, oy)) mx_y = oy;
+    }
+    if constexpr (NT > 32) {
+        if ((tid & 31) == 0) {
+            sm.red[0][tid >> 5] = mx_x;
+            sm.red[1][tid >> 5] = mx_y;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        if constexpr (NT > 32) {
+            for (int w = 1; w < NT / 32; w++) {
+                if (lt(mx_x, sm.red[0][w])) mx_x = sm.red[0][w];
+                if (lt(mx_y, sm.red[1][w])) mx_y = sm.red[1][w];
+            }
+        }
+        unsigned long long *word = ctrl->smax[(n + 1) % 3];
+        const unsigned long long bx = ordered_bits(mx_x), by = ordered_bits(mx_y);
+        if (bx > *(volatile unsigned long long *) &word[0]) atomicMax(&word[0], bx);
+        if (by > *(volatile unsigned long long *) &word[1]) atomicMax(&word[1], by);
+        __threadfence();
+        sm.am_last = atomicAdd(&ctrl->blocks_done, 1u) == blocks - 1;
+    }
+    __syncthreads();
+    if (!sm.am_last || tid >= 32) return;
+    __threadfence();
+    volatile HydroStepControl *vc = ctrl;
+    const bool failed = vc->error_code != 0;
+    const double tn = vc->t + dt, tf = vc->tf;
+    const long long nn = n + 1, most = vc->max_steps;
+    const int stored = vc->store_count;
+    if (!failed) arm_dt(a, ctrl, nn, tn, tf);
+    __syncwarp();
+    if (tid != 0) return;
+    ctrl->dt = dt;
+    ctrl->blocks_done = 0;
+    if (failed) {
+        ctrl->active = 0;
+        return;
+    }
+    ctrl->t = tn;
+    ctrl->num_steps = nn;
+    const int nn2 = (int) ((n + 2) % 3);
+    ctrl->smax[nn2][0] = ordered_bits(-CUDART_INF);
+    ctrl->smax[nn2][1] = ordered_bits(-CUDART_INF);
+    int act = (tn < tf) && (most < 0 || nn < most);
+    if (a.sp.is_storing && tn >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
+        ctrl->snapshot_due = 1;
+        act = 0;
+    }
+    ctrl->active = act;
+}
+
+/* The step's n and dt, or false when nothing is to be done (not active, or
+ * dt is zero, which the recon kernel records). */
+__device__ __forceinline__ bool staged_step(HydroStepControl *ctrl, long long &n, double &dt)
+{
+    if (!*(volatile int *) &ctrl->active) return false;
+    n = ctrl->num_steps;
+    dt = ctrl->step_dt;
+    return dt != 0.0;
+}
+
+/* ------------------------------------------------------- one grid, one band */
+
+template <int LIM, int FIRST_ORDER, int NT>
+__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_RECON_CTAS)
+staged_recon_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
+{
+    pdl_begin();
+    long long n;
+    double dt;
+    HydroStepControl *ctrl = a.ctrl;
+    if (!staged_step(ctrl, n, dt)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0 && ctrl->active && ctrl->error_code == 0) {
+            ctrl->dt = 0.0;
+            record_error(ctrl, DEV_ERR_DT_ZERO, -1);
+            ctrl->active = 0;
+        }
+        return;
+    }
+    const unsigned k = blockIdx.x * NT + threadIdx.x;
+    if (k >= staged_recon_items(a.nx, b.r1 - b.r0)) return;
+    const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
+    staged_recon<LIM, FIRST_ORDER>(a, b, k, (int) (n & 1), n == 0, dtA);
+}
+
+template <int NT, bool TAPE>
+__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_FLUX_CTAS)
+staged_flux_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
+{
+    __shared__ FluxShared<NT> sm;
+    pdl_begin();
+    long long n;
+    double dt;
+    if (!staged_step(a.ctrl, n, dt)) return;
+    staged_flux<NT, TAPE>(a, b, sm, blockIdx.x * NT + threadIdx.x, staged_face_items(a.nx, b.r1 - b.r0), dt);
+}
+
+template <int NT, bool GRAV>
+__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_UPDATE_CTAS)
+staged_update_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
+{
+    __shared__ UpdateShared<NT> sm;
+    pdl_begin();
+    long long n;
+    double dt;
+    if (!staged_step(a.ctrl, n, dt)) return;
+    double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
+    const unsigned cells = (unsigned) (b.r1 - b.r0) * a.nx;
+    for (unsigned k = blockIdx.x * NT + threadIdx.x; k < cells; k += gridDim.x * NT)
+        staged_update<GRAV>(a, b, k, (int) (n & 1), dt, mx_x, mx_y);
+    staged_finish<NT>(a, sm, b.update_blocks, n, dt, mx_x, mx_y);
+}
+
+/* The first step's dt after the maxima of the state are known, and again
+ * when the stopping time moves. */
+static __global__ void staged_arm_kernel(const Mh2dArgs<double> a)
+{
+    const HydroStepControl *c = a.ctrl;
+    arm_dt(a, a.ctrl, c->num_steps, c->t, c->tf);
+}
+
+}  // namespace hydro
+
+#endif

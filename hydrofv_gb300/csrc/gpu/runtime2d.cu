@@ -32,12 +32,18 @@
 
 #include "gpu_bridge.h"
 #include "gpu_internal.h"
+#include "mh2d_staged.cuh"
 
 using namespace hydro;
 
 namespace {
 
 constexpr int kGraphSteps = 32;
+/* Most bytes of the staged FP64 step's workspace (16 fields of a band's rows). */
+#ifndef MH2D_WORKSPACE_MB
+#define MH2D_WORKSPACE_MB 1024
+#endif
+constexpr size_t kWorkspaceBytes = (size_t) MH2D_WORKSPACE_MB << 20;
 
 void set_cuda_error(HydroRunOutcome *oc, cudaError_t e, const char *what)
 {
@@ -79,6 +85,8 @@ struct HydroRun2D {
     HydroStepControl *ctrl_h = nullptr;   /* pinned */
     Mh2dArgs<double> args{};
     Mh2dArgs<float> args32{};
+    void *ws = nullptr;               /* FP64: workspace of the staged step, shared by its bands */
+    std::vector<Mh2dBand> bands;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[6] = {};
     /* asynchronous snapshots: D2H on a side stream, the writer on a host thread */
@@ -155,8 +163,19 @@ static void setup_args(HydroRun2D *run, Mh2dArgs<R> &a, const HydroGrid2D *grid,
 static cudaError_t launch_step(HydroRun2D *run)
 {
     return run->fp32 ? mh2d_launch_step<float>(run->args32, run->grid.limiter, run->stream)
-                     : mh2d_launch_step<double>(run->args, run->grid.limiter, run->stream);
+                     : staged_launch_step(run->args, run->grid.limiter, run->bands, run->stream);
 }
+
+/* After the maxima of the state at hand are known: the first dt. */
+static cudaError_t launch_prepare(HydroRun2D *run)
+{
+    if (run->fp32) return mh2d_launch_prepare<float>(run->args32, run->stream);
+    const cudaError_t e = mh2d_launch_prepare<double>(run->args, run->stream);
+    return e != cudaSuccess ? e : staged_launch_arm(run->args, run->stream);
+}
+
+/* Kernels that launch_step launches. */
+static int launches_per_step(const HydroRun2D *run) { return run->fp32 ? 1 : 3 * (int) run->bands.size(); }
 
 /* The FP64 step's work-item plan for an nx x ny grid on `slots` resident CTAs
  * (guided row chunks), and each item's strip and padded rows as the kernel
@@ -321,6 +340,26 @@ extern "C" int hydro_gpu_trim_device_memory(int device)
     return 0;
 }
 
+/* The staged step's workspace: as much as kWorkspaceBytes, less where the
+ * device has no room for it (more and shorter bands). */
+static int alloc_workspace(HydroRun2D *run, HydroRunOutcome *oc)
+{
+    size_t budget = kWorkspaceBytes;
+    for (;;) {
+        size_t bytes = 0;
+        staged_plan(run->args, budget, run->bands, bytes);
+        const cudaError_t e = pool_alloc(run, &run->ws, bytes);
+        if (e == cudaSuccess) break;
+        const int h = run->bands[0].r1 - run->bands[0].r0;
+        if (e != cudaErrorMemoryAllocation || h == 1) CK(e, "cudaMallocFromPoolAsync(workspace)");
+        cudaGetLastError();
+        run->ws = nullptr;
+        budget = bytes / 2;
+    }
+    for (auto &b : run->bands) b.ws = static_cast<double *>(run->ws);
+    return 0;
+}
+
 extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions *opt,
                                   HydroRun2D **out, HydroRunOutcome *oc)
 {
@@ -383,6 +422,7 @@ extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     } else {
         carve<double>(run, run->args);
         setup_args<double>(run, run->args, grid, opt);
+        if (alloc_workspace(run, oc)) return -1;
     }
     return 0;
 }
@@ -586,8 +626,7 @@ static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome 
             for (int k = 0; k < 3; k++) c->smax[k][0] = c->smax[k][1] = ninf;
             c->active = 1;
             CK(cudaMemcpyAsync(run->ctrl_d, c, sizeof *c, cudaMemcpyHostToDevice, run->stream), "H2D control");
-            CK(run->fp32 ? mh2d_launch_prepare<float>(run->args32, run->stream)
-                         : mh2d_launch_prepare<double>(run->args, run->stream), "prepare kernel");
+            CK(launch_prepare(run), "prepare kernel");
             CK(launch_step(run), "step kernel");
             CK(cudaEventRecord(run->ev[2], run->stream), "cudaEventRecord");
             CK(launch_step(run), "step kernel");
@@ -625,7 +664,7 @@ extern "C" int hydro_run2d_begin(HydroRun2D *run, const HydroStepParams *sp, dou
     CK(cudaSetDevice(run->device), "cudaSetDevice");
     run->args.sp = *sp;
     run->args32.sp = *sp;
-    if (run->opt.autotune && autotune(run, sp, oc)) return -1;
+    if (run->opt.autotune && run->fp32 && autotune(run, sp, oc)) return -1;
     HydroStepControl *c = run->ctrl_h;
     memset(c, 0, sizeof *c);
     c->tf = tf;
@@ -635,9 +674,8 @@ extern "C" int hydro_run2d_begin(HydroRun2D *run, const HydroStepParams *sp, dou
     for (int k = 0; k < 3; k++) c->smax[k][0] = c->smax[k][1] = ninf;
     c->active = recompute_active(c);
     if (push_control(run, oc)) return -1;
-    CK(run->fp32 ? mh2d_launch_prepare<float>(run->args32, run->stream)
-                 : mh2d_launch_prepare<double>(run->args, run->stream), "prepare kernel");
-    run->kernel_launches++;
+    CK(launch_prepare(run), "prepare kernel");
+    run->kernel_launches += run->fp32 ? 1 : 2;
     CK(cudaStreamSynchronize(run->stream), "prepare");
     /* The kernel arguments changed: any recorded graph is stale. */
     if (run->graph) {
@@ -659,6 +697,11 @@ extern "C" int hydro_run2d_set_limits(HydroRun2D *run, double tf, int64 max_step
     c->max_steps = max_steps;
     c->active = recompute_active(c);
     if (push_control(run, oc)) return -1;
+    if (!run->fp32) {
+        /* the next dt is clipped to the stopping time */
+        CK(staged_launch_arm(run->args, run->stream), "dt kernel");
+        run->kernel_launches++;
+    }
     CK(cudaStreamSynchronize(run->stream), "set limits");
     fill_outcome(run, oc);
     return 0;
@@ -762,12 +805,12 @@ static int enqueue_steps(HydroRun2D *run, long long k, HydroRunOutcome *oc)
             CK(cudaGraphLaunch(run->graph, run->stream), "graph launch");
             k -= kGraphSteps;
             run->step_launches += kGraphSteps;
-            run->kernel_launches += kGraphSteps;
+            run->kernel_launches += kGraphSteps * launches_per_step(run);
         } else {
             CK(launch_step(run), "step kernel");
             k -= 1;
             run->step_launches += 1;
-            run->kernel_launches += 1;
+            run->kernel_launches += launches_per_step(run);
         }
     }
     return 0;
@@ -1032,7 +1075,7 @@ extern "C" void hydro_run2d_destroy(HydroRun2D *run)
     bool idle = false;
     if (run->stream) {
         /* back to the pool, in stream order (the stream is idle here) */
-        for (void *m : { run->slab, run->init_slab, static_cast<void *>(run->stage_d) }) {
+        for (void *m : { run->slab, run->init_slab, static_cast<void *>(run->stage_d), run->ws }) {
             if (!m) continue;
             if (run->pooled) cudaFreeAsync(m, run->stream);
             else cudaFree(m);
