@@ -16,6 +16,7 @@
 #include "pow_int.cuh"
 #include "numerics.cuh"
 #include "quad_exact.cuh"
+#include "staged_math.cuh"
 #include "hydro_gpu.h"
 
 using namespace hydro;
@@ -233,3 +234,55 @@ int hydro_gpu_pointwise_eval(int device, int op, long long n, const double *gamm
 }
 
 }  // extern "C"
+
+/* The staged step's face (staged_math.cuh) and the template of numerics.cuh
+ * on the same state pairs: five values each, the flux and the guess regime. */
+extern "C" void hydro_fx_staged_face_host(double gamma, double tol, long long n, const double *L, const double *R,
+                                          double *out, int *rc, double *ref, int *rc_ref)
+{
+    const GasConst<double> c = make_gas_const<double>(gamma, tol);
+    const Fm f = make_fm();
+    for (long long k = 0; k < n; k++) {
+        const double *l = L + 4 * k, *r = R + 4 * k;
+        double a_L, a_R, pg, z0, z1, wave[3], *F = out + 5 * k;
+        bool plain;
+        const int reg = face_classify(f, c, l[0], l[1], l[3], r[0], r[1], r[3], a_L, a_R, pg, plain);
+        rc[k] = DEV_OK;
+        for (int q = 0; q < 4; q++) F[q] = ref[5 * k + q] = 0.0;
+        F[4] = reg;
+        if (reg == PREG_VACUUM) {
+            hllc_vacuum_flux(c, l[0], l[1], l[2], l[3], a_L, r[0], r[1], r[2], r[3], a_R, F);
+        } else {
+            if (reg == PREG_TRRS) pg = face_trrs(f, c, l[1], l[3], a_L, r[1], r[3], a_R, z0, z1);
+            else if (reg == PREG_TSRS) pg = face_tsrs(f, c, l[0], l[1], l[3], r[0], r[1], r[3], pg, z0, z1);
+            rc[k] = face_finish(f, c, plain, l[0], l[1], l[2], l[3], a_L, r[0], r[1], r[2], r[3], a_R, pg, F, wave);
+        }
+        ref[5 * k + 4] = hllc_classify(c, l[0], l[1], l[3], r[0], r[1], r[3], a_L, a_R, pg);
+        rc_ref[k] = hllc_flux_2d(c, l[0], l[1], l[2], l[3], r[0], r[1], r[2], r[3], ref + 5 * k);
+    }
+}
+
+/* The staged step's slopes, predictor and conversion beside the templates:
+ * per cell 12 values each: low and high face states, then U -> W of
+ * (w0, with w0[0] as the mass and w0[3] as the energy). */
+extern "C" void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long n, const double *wm,
+                                          const double *w0, const double *wp, double *out, double *ref)
+{
+    const GasConst<double> c = make_gas_const<double>(gamma, 1e-6);
+    const Fm f = make_fm();
+    for (long long k = 0; k < n; k++) {
+        const double *a = wm + 4 * k, *b = w0 + 4 * k, *e = wp + 4 * k;
+        double d[4], g[4], *o = out + 12 * k, *r = ref + 12 * k;
+        for (int q = 0; q < 4; q++) {
+            const double x = f.sub(b[q], a[q]), y = f.sub(e[q], b[q]);
+            d[q] = limiter == LIM_MINMOD ? slope<LIM_MINMOD>(f, x, y)
+                 : limiter == LIM_VAN_LEER ? slope<LIM_VAN_LEER>(f, x, y) : slope<LIM_MC>(f, x, y);
+            g[q] = limit_slope_rt(limiter, b[q] - a[q], e[q] - b[q]);
+        }
+        const double s = sound_speed(c, b[0], b[3]);
+        predict(f, dtA, dv(dtA, b[0]), b[0], b[1], b[2], b[3], s, d, d[1], o, o + 4);
+        hancock_2d(dtA, dv(dtA, b[0]), b[0], b[1], b[2], b[3], s, g, g[1], r, r + 4);
+        to_primitive(f, c, 0.37, b[0], b[1], b[2], b[3], o + 8);
+        cons_to_prim_2d(c, 0.37, b[0], b[1], b[2], b[3], r + 8);
+    }
+}

@@ -126,7 +126,19 @@ inline void mh2d_guided_chunks(int nx, int ny, int strip_w, int slots, int &h1, 
     cache[key] = std::make_tuple(h1, h2, tail);
 }
 
-struct Mh2dBand;
+/* The rows of a step are processed in one band as long as its workspace stays
+ * below a fixed size (1 GiB in runtime2d.cu).  Bands small enough for the L2
+ * cache lost: 2048^2 3.07 ms with one band, 3.16 / 3.22 / 3.35 / 3.70 ms with
+ * 160 / 96 / 48 / 24 MB (the launches' tails cost more than the traffic).
+ *
+ * Rows [r0, r1) (padded indices) of one grid and the workspace they use: a
+ * plane holds rows r0 - 1 .. r1 with the grid's pitch. */
+struct Mh2dBand {
+    int r0, r1;
+    unsigned update_blocks;   /* update blocks of the whole step of this grid (all bands) */
+    long long plane;          /* doubles per workspace field */
+    double *ws;
+};
 
 /* The staged FP64 step (mh2d_staged.cuh).  staged_plan splits the grid's rows
  * into bands whose workspace takes at most `budget` bytes (one row at least;

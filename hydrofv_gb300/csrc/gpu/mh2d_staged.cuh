@@ -32,7 +32,8 @@
 #ifndef HYDRO_GPU_MH2D_STAGED_CUH
 #define HYDRO_GPU_MH2D_STAGED_CUH
 
-#include "mh2d_kernel.cuh"
+#include "gpu_internal.h"
+#include "staged_math.cuh"
 
 #ifndef MH2D_RECON_CTAS
 #define MH2D_RECON_CTAS 6
@@ -57,20 +58,6 @@ constexpr unsigned kStagedUpdateGrid = 152 * MH2D_UPDATE_CTAS;
  * and y.  The flux kernel leaves a face's update term where its left (lower)
  * state was. */
 enum : int { WS_XLO = 0, WS_XHI = 4, WS_YLO = 8, WS_YHI = 12, WS_FIELDS = 16 };
-
-/* The rows of a step are processed in one band as long as its workspace stays
- * below a fixed size (1 GiB in runtime2d.cu).  Bands small enough for the L2
- * cache lost: 2048^2 3.07 ms with one band, 3.16 / 3.22 / 3.35 / 3.70 ms with
- * 160 / 96 / 48 / 24 MB (the launches' tails cost more than the traffic).
- *
- * Rows [r0, r1) (padded indices) of one grid and the workspace they use: a
- * plane holds rows r0 - 1 .. r1 with the grid's pitch. */
-struct Mh2dBand {
-    int r0, r1;
-    unsigned update_blocks;   /* update blocks of the whole step of this grid (all bands) */
-    long long plane;          /* doubles per workspace field */
-    double *ws;
-};
 
 inline __host__ __device__ unsigned staged_recon_items(int nx, int rows) { return (unsigned) rows * (nx + 2) + (unsigned) (rows + 2) * nx; }
 inline __host__ __device__ unsigned staged_face_items(int nx, int rows) { return (unsigned) rows * (nx + 1) + (unsigned) (rows + 1) * nx; }
@@ -133,12 +120,13 @@ __device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh
         double wm[5], wp[5];
         fetch_w(a, W, U, raw, y ? r - 1 : r, y ? c : c - 1, wm);
         fetch_w(a, W, U, raw, y ? r + 1 : r, y ? c : c + 1, wp);
+        const Fm f = make_fm();
         double s[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) s[q] = limit_slope<LIM>(w[q] - wm[q], wp[q] - w[q]);
+        for (int q = 0; q < 4; q++) s[q] = slope<LIM>(f, f.sub(w[q], wm[q]), f.sub(wp[q], w[q]));
         const double h = y ? dtA[1] : dtA[0];
         const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
-        hancock_2d(h, dv(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
+        predict(f, h, dv(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
     }
     double *o = b.ws + (long long) (r - b.r0 + 1) * a.pitch + c + (y ? WS_YLO : WS_XLO) * b.plane;
 #pragma unroll
@@ -165,6 +153,8 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
 {
     const int tid = threadIdx.x;
     const bool on = k < total;
+    const Fm fm = make_fm();
+    bool plain = true;
     const unsigned nx = (unsigned) a.nx, nX = (unsigned) (b.r1 - b.r0) * (nx + 1);
     const bool y = k >= nX;
     long long at = 0, tape_at = 0;
@@ -189,7 +179,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
         const double *h = b.ws + (y ? WS_YLO : WS_XLO) * b.plane + at + (y ? a.pitch : 1);
 #pragma unroll
         for (int q = 0; q < 4; q++) { L[q] = l[q * b.plane]; R[q] = h[q * b.plane]; }
-        reg = hllc_classify(a.gas, L[0], L[1], L[3], R[0], R[1], R[3], aL, aR, pg);
+        reg = face_classify(fm, a.gas, L[0], L[1], L[3], R[0], R[1], R[3], aL, aR, pg, plain);
         if (reg == PREG_TRRS || reg == PREG_TSRS) {
             sm.rho[0][tid] = L[0]; sm.u[0][tid] = L[1]; sm.p[0][tid] = L[3]; sm.a[0][tid] = aL;
             sm.rho[1][tid] = R[0]; sm.u[1][tid] = R[1]; sm.p[1][tid] = R[3]; sm.a[1][tid] = aR;
@@ -204,11 +194,11 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     for (int i = tid; i < nT + nS; i += NT) {
         if (i < nT) {
             const int f = sm.listT[i];
-            sm.pg[f] = guess_p_trrs_z(a.gas, sm.u[0][f], sm.p[0][f], sm.a[0][f], sm.u[1][f], sm.p[1][f], sm.a[1][f], z0, z1);
+            sm.pg[f] = face_trrs(fm, a.gas, sm.u[0][f], sm.p[0][f], sm.a[0][f], sm.u[1][f], sm.p[1][f], sm.a[1][f], z0, z1);
             if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
         } else {
             const int f = sm.listS[i - nT];
-            sm.pg[f] = guess_p_tsrs_g(a.gas, sm.rho[0][f], sm.u[0][f], sm.p[0][f], sm.rho[1][f], sm.u[1][f], sm.p[1][f],
+            sm.pg[f] = face_tsrs(fm, a.gas, sm.rho[0][f], sm.u[0][f], sm.p[0][f], sm.rho[1][f], sm.u[1][f], sm.p[1][f],
                                       sm.pg[f], z0, z1);
             if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
         }
@@ -222,8 +212,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     if (reg == PREG_VACUUM) {
         vacuum_flux_dev(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, F);
     } else {
-        const int rc = hllc_finish(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, pg, F,
-                                   TAPE ? wave : nullptr);
+        const int rc = face_finish(fm, a.gas, plain, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, pg, F, wave);
         if (rc) record_error(a.ctrl, rc, (int) blockIdx.x);
     }
     if constexpr (TAPE) {
@@ -237,12 +226,12 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     const double A = y ? a.area_y : a.area_x;
     double *o = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
 #pragma unroll
-    for (int q = 0; q < 4; q++) o[q * b.plane] = (F[q] * dt) * A;
+    for (int q = 0; q < 4; q++) o[q * b.plane] = fm.mul(fm.mul(F[q], dt), A);
 }
 
 /* Cell k of the band: update, gravity, U -> W; mx receives a + |u|, a + |v|. */
 template <bool GRAV>
-__device__ __forceinline__ void staged_update(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned k, int buf, double dt,
+__device__ __forceinline__ void staged_update(const Fm &f, const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned k, int buf, double dt,
                                               double &mx_x, double &mx_y)
 {
     const int ymap[4] = { 0, 2, 1, 3 };   /* y fluxes come back as (mass, mom_y, mom_x, energy) */
@@ -265,23 +254,18 @@ __device__ __forceinline__ void staged_update(const Mh2dArgs<double> &a, const M
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        double v = Un[q];
-        v = v + fl[q];
-        v = v - fh[q];
-        v = v + gl[q];
-        v = v - gh[q];
-        Un[q] = v;
+        Un[q] = f.sub(f.add(f.sub(f.add(Un[q], fl[q]), fh[q]), gl[q]), gh[q]);
     }
     if constexpr (GRAV) gravity_kick(-dt * a.gravity, Un[0], Un[2], Un[3]);
 #pragma unroll
     for (int q = 0; q < 4; q++) Uout[q][idx] = Un[q];
     double w[4];
-    cons_to_prim_2d(a.gas, a.vol, Un[0], Un[1], Un[2], Un[3], w);
-    const double as = sound_speed(a.gas, w[0], w[3]);
+    to_primitive(f, a.gas, a.vol, Un[0], Un[1], Un[2], Un[3], w);
+    const double as = sq(dv(f.mul(a.gas.gamma, w[3]), w[0]));
 #pragma unroll
     for (int q = 0; q < 4; q++) Wout[q][idx] = w[q];
     Wout[4][idx] = as;
-    const double sx = as + fabs(w[1]), sy = as + fabs(w[2]);
+    const double sx = f.add(as, fabs(w[1])), sy = f.add(as, fabs(w[2]));
     if (lt(mx_x, sx)) mx_x = sx;
     if (lt(mx_y, sy)) mx_y = sy;
     /* the first ghost layer receives its one-sided update */
@@ -431,10 +415,11 @@ staged_update_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     long long n;
     double dt;
     if (!staged_step(a.ctrl, n, dt)) return;
+    const Fm f = make_fm();
     double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
     const unsigned cells = (unsigned) (b.r1 - b.r0) * a.nx;
     for (unsigned k = blockIdx.x * NT + threadIdx.x; k < cells; k += gridDim.x * NT)
-        staged_update<GRAV>(a, b, k, (int) (n & 1), dt, mx_x, mx_y);
+        staged_update<GRAV>(f, a, b, k, (int) (n & 1), dt, mx_x, mx_y);
     staged_finish<NT>(a, sm, b.update_blocks, n, dt, mx_x, mx_y);
 }
 

@@ -32,7 +32,6 @@
 
 #include "gpu_bridge.h"
 #include "gpu_internal.h"
-#include "mh2d_staged.cuh"
 
 using namespace hydro;
 

@@ -378,6 +378,15 @@ void hydro_fx_ratio_below_host(long long n, const double *x, const double *y, co
 void hydro_fx_quot_le_host(long long n, const double *x, const double *y, const double *z,
                            unsigned char *out, unsigned char *decided);
 
+/* The FP64 step's face and cell arithmetic beside the general templates it
+ * must equal bit for bit (host build, for tests): per state pair the flux and
+ * the guess regime (5 values) with its return code; per cell triple the low
+ * and high face states and a U -> W conversion (12 values). */
+void hydro_fx_staged_face_host(double gamma, double tol, long long n, const double *L, const double *R, double *out,
+                               int *rc, double *ref, int *rc_ref);
+void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long n, const double *wm, const double *w0,
+                               const double *wp, double *out, double *ref);
+
 /* Device build of the exported pointwise numerics over n state pairs:
  * L[4k..4k+3], R[4k..4k+3] = (rho, u, v, p) (the 1D forms read rho, u, p),
  * gas constants from gamma[k] and tol.
