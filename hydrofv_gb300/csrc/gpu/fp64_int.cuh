@@ -9,36 +9,37 @@
  * integer multiplies (IMAD) and one FP32 MUFU seed, leaving the FP64 pipe to
  * the additions and multiplications of the scheme.
  *
- * Division a / b of normal operands (mantissas ma, mb in [2^52, 2^53)):
- *   1. y0 ~ 1/mb from the FP32 reciprocal of mb's leading 24 bits
- *      (relative error ~2^-22), as a 32-bit fixed-point Y0 ~ 2^84/mb;
- *   2. one Newton step in integer arithmetic, Y1 = Y0 (1 + e0) with the
- *      exact residual e0 = 1 - mb Y0 2^-84; Y1 <= 2^116/mb and its relative
- *      error is ~e0^2 ~ 2^-44;
- *   3. the quotient Q = floor(ma 2^(52+s) / mb) (s = [ma < mb], so Q has 53
- *      bits) by a multiply-high with Y1, one correction by the remainder
- *      times Y1, and one single-step fix, which make Q exact whenever the
- *      seed's residual is small (|e0| < 3 2^61, checked; the bounds are in
- *      div_fast);
- *   4. round-to-nearest-even on the remainder (2R against mb).
- * This is the reciprocal-multiply-and-correct form of long division
- * (Knuth, TAOCP vol. 2, 4.3.1; Moller & Granlund, "Improved division by
- * invariant integers", IEEE TC 2011) applied to the 53-bit mantissas.
+ * Division a / b of normal operands (mantissas ma, mb in [2^52, 2^53)), with
+ * B = mb 2^8 and A = ma 2^(7 + s) (s = [ma < mb], so A / B is in [1/2, 1)):
+ *   1. Y ~ 2^92 / B to 32 bits: the FP32 reciprocal of mb's leading 24 bits
+ *      (relative error ~2^-22) and one integer Newton step Y0 (1 + e) with
+ *      the residual e = 1 - B Y0 2^-92, kept below the exact value;
+ *   2. the quotient in two digits, each a 32-bit high product with Y and the
+ *      exact remainder modulo 2^64: 31 bits, then 22 bits that come out exact
+ *      or one too large;
+ *   3. the rounding from the signed remainder: up above B / 2, down below
+ *      -B / 2 (a quotient of two 53-bit integers is never a midpoint).
+ * This is long division with a reciprocal of one digit (Knuth, TAOCP vol. 2,
+ * 4.3.1; Moller & Granlund, "Improved division by invariant integers", IEEE
+ * TC 2011).  The bounds beside the code hold for every seed with |e| < 2^-21,
+ * which is checked.
  *
- * Square root of a normal positive x (mantissa m, M = m or 2m so that the
- * exponent left over is even, M in [2^52, 2^54)):
- *   1. y0 ~ 1/sqrt(M 2^-52) from the FP32 reciprocal square root, Y0 = y0 2^32;
- *   2. one integer Newton step for the reciprocal square root,
- *      Y1 = Y0 (1 + e0/2), e0 = 1 - M 2^-52 y0^2, which stays below the exact
- *      value (1/sqrt(1-e) >= 1 + e/2);
- *   3. S1 = M Y1 2^-64 <= sqrt(M 2^52), one Heron correction with the exact
- *      integer residual M 2^52 - S1^2, at most two single-step fixes;
- *   4. an exact 128-bit check that 0 <= M 2^52 - S^2 <= 2S, then rounding
- *      up where the residual exceeds S (a square root is never a midpoint).
+ * Square root of a normal positive x (mantissa M = m 2^52, m in [1, 4), the
+ * exponent left over even):
+ *   1. Y ~ 2^32 / sqrt(m): the FP32 reciprocal square root and one integer
+ *      Newton step (checked like the divide's);
+ *   2. 31 bits of the root, s1 = m Y; the exact remainder M 2^8 - s1^2 and Y
+ *      give 22 more;
+ *   3. the exact remainder R of that root S decides the rounding: up where
+ *      R > S, down where R <= -S (a square root is never a midpoint).
  *
- * Correctness does not rest on the seed's accuracy: the divide checks the
- * seed's exact residual, the square root verifies its result exactly, and
- * every operand or result outside the fast path
+ * Cost on one SM with 24 resident warps: an inlined divide 27.4 cycles per
+ * warp (33.8 with 53-bit quotients from a 64 x 64 high product), out of line
+ * 36.8 (46.7), a square root out of line 29.9 (50.1, which checked its result
+ * with a 128-bit product); latency out of line 282 (448) and 298 (496) cycles.
+ *
+ * Correctness does not rest on the seed's accuracy: both check the seed's
+ * residual, and every operand or result outside the fast path
  * (zero, subnormal, infinite, NaN, negative for sqrt, quotients that
  * overflow the normal range before rounding or underflow) or a failed check
  * takes the hardware operation.  The results are therefore bit-identical to
@@ -124,15 +125,6 @@ FXHD float from_fbits(unsigned b)
 #endif
 }
 
-FXHD u64 mulhi(u64 a, u64 b)
-{
-#if defined(__CUDA_ARCH__)
-    return __umul64hi(a, b);
-#else
-    return (u64) (((unsigned __int128) a * b) >> 64);
-#endif
-}
-
 /* FP32 seeds: reciprocal and reciprocal square root of x in [1, 4). */
 FXHD float rcp_seed(float x)
 {
@@ -156,65 +148,92 @@ FXHD float rsqrt_seed(float x)
 #endif
 }
 
-/* y in [0.5, 1] (an FP32 seed) as a 32-bit fixed-point value y 2^32,
- * saturated at 2^32 - 1.  Seeds outside [0.5, 1] give a poor estimate,
- * which the exact check turns into the fallback. */
-FXHD unsigned seed_fixed(float y)
-{
-    const unsigned fy = fbits(y);
-    return (fy >= 0x3f800000u) ? 0xffffffffu : (((fy & 0x7fffffu) | 0x800000u) << 8);
-}
-
 static const u64 FRAC = 0x000fffffffffffffull;
 static const u64 HIDDEN = 0x0010000000000000ull;
 static const u64 SIGN = 0x8000000000000000ull;
 
-/* RN(a / b) when `ok` comes back true (see the header comment).
- * seed_scale multiplies the FP32 reciprocal seed: 1 in the kernels; the
- * tests perturb it to exercise the seed check. */
+/* 32-bit high products. */
+FXHD unsigned mulhi32(unsigned a, unsigned b)
+{
+#if defined(__CUDA_ARCH__)
+    return __umulhi(a, b);
+#else
+    return (unsigned) (((u64) a * b) >> 32);
+#endif
+}
+
+FXHD int mulhi32s(int a, int b)
+{
+#if defined(__CUDA_ARCH__)
+    return __mulhi(a, b);
+#else
+    return (int) (((i64) a * b) >> 32);
+#endif
+}
+
+/* A divisor's reciprocal, for one or several quotients: B = mb 2^8 (61
+ * bits), Y = 2^92 / B - d with 1 <= d < 3.2 (32 bits), and its sign and
+ * exponent word. */
+struct Recip {
+    u64 B;
+    unsigned Y, hb;
+    bool ok;      /* normal divisor, seed within its bound */
+};
+
+/* seed_scale multiplies the FP32 seed: 1 in the kernels; the tests perturb
+ * it to exercise the check. */
+FXHD Recip recip(double b, float seed_scale = 1.0f)
+{
+    const u64 ub = bits(b);
+    Recip r;
+    r.hb = (unsigned) (ub >> 32);
+    r.B = ((ub & FRAC) | HIDDEN) << 8;
+    /* the seed, kept below 1 so that its fixed-point form is a shift */
+    const float y = fminf(rcp_seed(from_fbits(0x3f800000u | ((unsigned) (ub >> 29) & 0x7fffffu))) * seed_scale, 0x1.fffffep-1f);
+    const unsigned Y0 = (fbits(y) << 8) | 0x80000000u;
+    /* e = 1 - B Y0 2^-92 to 60 bits; one Newton step Y0 (1 + e) needs
+     * |e| < 2^-21 (then e^2 is below the last place of Y) */
+    const u64 p = (r.B >> 32) * Y0 + mulhi32((unsigned) r.B, Y0);
+    const i64 e = (i64) ((1ull << 60) - p);
+    const unsigned eh = (unsigned) ((u64) e >> 32);
+    r.ok = eh + 0x80u < 0x100u && ((r.hb >> 20) & 0x7ffu) - 1u < 2046u;
+    r.Y = Y0 + (unsigned) (mulhi32s((int) (unsigned) ((u64) e >> 8), (int) (Y0 >> 1)) >> 19) - 1u;
+    return r;
+}
+
+/* RN(a / b) with b's reciprocal when `ok` comes back true (see the header
+ * comment). */
+FXHD double div_recip(double a, const Recip &r, bool &ok)
+{
+    const u64 ua = bits(a);
+    const unsigned ha = (unsigned) (ua >> 32);
+    const u64 ma = (ua & FRAC) | HIDDEN;
+    const int s = (ma << 8) < r.B ? 1 : 0;
+    /* 31 quotient bits, at most 5.2 low; the remainder is below 6.2 B < 2^64 */
+    const unsigned q1 = mulhi32((unsigned) ((ma << (10 + s)) >> 32), r.Y);
+    const u64 R1 = ((u64) ((unsigned) ma << (6 + s)) << 32) - (u64) q1 * r.B;
+    /* 22 more: the product is at most 4.7 / 64 low, so with 5 / 64 added they
+     * are exact or one too large and the remainder lies in (-B, B) */
+    const unsigned q2 = (mulhi32((unsigned) (R1 >> 32), r.Y) + 5u) >> 6;
+    const i64 R2 = (i64) ((R1 << 22) - (u64) q2 * r.B);
+    const i64 half = (i64) (r.B >> 1);
+    u64 Q = (u64) q1 * (1u << 22) + q2;
+    /* nearest: a quotient of two 53-bit integers is never a midpoint */
+    Q += (R2 > half) ? 1ull : 0ull;
+    Q -= (R2 < -half) ? 1ull : 0ull;
+    const unsigned ea = (ha >> 20) & 0x7ffu, eb = (r.hb >> 20) & 0x7ffu;
+    const unsigned e = ea - eb + 1022u - (unsigned) s;       /* biased exponent of the quotient - 1 */
+    const unsigned sign = (ha ^ r.hb) & 0x80000000u;
+    const bool a_zero = (ua << 1) == 0ull;
+    ok = r.ok && (a_zero || (ea - 1u < 2046u && e < 2046u));
+    const u64 res = Q + ((u64) (sign + (e << 20)) << 32);
+    return from_bits(a_zero ? (u64) sign << 32 : res);
+}
+
+/* RN(a / b) when `ok` comes back true. */
 FXHD double div_fast(double a, double b, bool &ok, float seed_scale = 1.0f)
 {
-    const u64 ua = bits(a), ub = bits(b);
-    const unsigned ea = (unsigned) (ua >> 52) & 0x7ffu, eb = (unsigned) (ub >> 52) & 0x7ffu;
-    const u64 sign = (ua ^ ub) & SIGN;
-    const u64 ma = (ua & FRAC) | HIDDEN, mb = (ub & FRAC) | HIDDEN;
-    const int s = ma < mb ? 1 : 0;
-    const int e = (int) ea - (int) eb + 1023 - s;          /* biased exponent of the quotient */
-
-    const unsigned Y0 = seed_fixed(rcp_seed(from_fbits(0x3f800000u | (unsigned) ((mb >> 29) & 0x7fffffu))) * seed_scale);
-    /* mb Y0 (85 bits) from two 32 x 32 products.  Its low 64 bits, negated,
-     * are the residual e0 = 2^84 - mb Y0 exactly when the high bits are
-     * 2^20 - 1 with e0 > 0, or 2^20 with e0 <= 0 (so |2^84 - mb Y0| < 2^63) */
-    const u64 t = (u64) (unsigned) mb * Y0;
-    const u64 hm = (u64) (unsigned) (mb >> 32) * Y0 + (t >> 32);
-    const i64 e0 = (i64) (0ull - ((hm << 32) | (t & 0xffffffffull)));
-    const unsigned top = (unsigned) (hm >> 32);
-    /* the seed is good enough when |e0| < 3 2^61 (relative error < 2^-21.4):
-     * then Y1 <= 2^116 / mb with relative error < 2^-42.8, the first
-     * remainder R lies in [0, 2^64), the correction leaves it in [0, 2 mb)
-     * and one step finishes the exact quotient (a seed outside the bound
-     * takes the hardware divide) */
-    const bool seed_ok = (top == (1u << 20) - 1u ? e0 > 0 : (top == (1u << 20) && e0 <= 0))
-                      && e0 < 3 * (1ll << 61) && e0 > -3 * (1ll << 61);
-    const i64 d = ((i64) (int) (e0 >> 32) * (i64) Y0) >> 20; /* Y0 e0 2^-52 */
-    const u64 Y1 = ((u64) Y0 << 32) + (u64) d;               /* ~2^116 / mb, from below */
-
-    const u64 A_lo = ma << (52 + s);
-    u64 Q = mulhi(ma << s, Y1);                              /* <= floor(A / mb), A = ma 2^(52+s) */
-    u64 R = A_lo - Q * mb;
-    const u64 dq = ((R >> 32) * (Y1 >> 32)) >> 52;
-    Q += dq;
-    R -= dq * mb;
-    if (R >= mb) { Q += 1; R -= mb; }
-    const bool exact = seed_ok;
-    const u64 r2 = R << 1;
-    Q += (r2 > mb || (r2 == mb && (Q & 1ull))) ? 1ull : 0ull;
-    const u64 res = sign | (((u64) (unsigned) (e - 1) << 52) + Q);
-
-    const bool b_normal = eb - 1u < 2046u;
-    const bool a_zero = (ua << 1) == 0ull;
-    ok = b_normal && (a_zero || (ea - 1u < 2046u && (unsigned) (e - 1) < 2046u && exact));
-    return from_bits(a_zero ? sign : res);
+    return div_recip(a, recip(b, seed_scale), ok);
 }
 
 /* RN(sqrt(x)) when `ok` comes back true. */
@@ -222,34 +241,32 @@ FXHD double sqrt_fast(double x, bool &ok)
 {
     const u64 ux = bits(x);
     const unsigned ex = (unsigned) (ux >> 52);                /* sign bit included */
-    const int odd = (ex & 1u) ? 0 : 1;                        /* unbiased exponent - 52 is odd */
-    const u64 M = ((ux & FRAC) | HIDDEN) << odd;              /* [2^52, 2^54) */
+    const unsigned odd = (ex & 1u) ^ 1u;                      /* unbiased exponent - 52 is odd */
+    const u64 M = ((ux & FRAC) | HIDDEN) << odd;              /* m 2^52, m in [1, 4) */
+    const unsigned M30 = (unsigned) (M >> 22);                /* m 2^30 */
 
-    const float fm = from_fbits(((127u + (unsigned) odd) << 23) | (unsigned) ((ux >> 29) & 0x7fffffu));
-    const unsigned Y0 = seed_fixed(rsqrt_seed(fm));
-    const u64 Y0sq = (u64) Y0 * Y0;                           /* y0^2 2^64 */
-    const i64 e0 = (i64) ((1ull << 62) - mulhi(M << 10, Y0sq));   /* (1 - M 2^-52 y0^2) 2^62 */
-    const i64 d = ((i64) (int) (e0 >> 11) * (i64) Y0) >> 20;      /* Y0 e0 2^-31 */
-    const u64 Y1 = ((u64) Y0 << 32) + (u64) d - 2ull;             /* ~2^64 / sqrt(M 2^-52), from below */
-
-    const u64 X_lo = M << 52, X_hi = M >> 12;                 /* X = M 2^52 */
-    u64 S = mulhi(M, Y1);
-    const u64 R1 = X_lo - S * S;
-    S += ((R1 >> 32) * (Y1 >> 32)) >> 53;
-    i64 R = (i64) (X_lo - S * S);
-    if (R < 0) { S -= 1; R += (i64) (2 * S + 1); }
-    if (R > (i64) (2 * S)) { R -= (i64) (2 * S + 1); S += 1; }
-    if (R > (i64) (2 * S)) { R -= (i64) (2 * S + 1); S += 1; }
-
-    const u64 P_lo = S * S, P_hi = mulhi(S, S);
-    const bool exact = (X_hi - P_hi - (X_lo < P_lo ? 1ull : 0ull)) == 0ull
-                    && R >= 0 && (u64) R <= 2 * S;
-    S += ((u64) R > S) ? 1ull : 0ull;
-    const int t = ((int) ex - 1075 - odd) >> 1;               /* exponent left over, halved */
-    const u64 res = ((u64) (unsigned) (t + 1048) << 52) + S;
-
-    ok = ex - 1u < 2046u && exact;
-    return from_bits(res);
+    const float fm = from_fbits(((127u + odd) << 23) | ((unsigned) (ux >> 29) & 0x7fffffu));
+    const float y = fminf(rsqrt_seed(fm), 0x1.fffffep-1f);
+    const unsigned Y0 = (fbits(y) << 8) | 0x80000000u;        /* y 2^32, y in (1/2, 1) */
+    /* e = 1 - m y^2 to 2^-29; the Newton step Y0 (1 + e / 2) needs |e| < 2^-20 */
+    const i64 e = (i64) ((1ull << 62) - (u64) M30 * mulhi32(Y0, Y0));
+    const unsigned eh = (unsigned) ((u64) e >> 32);
+    const bool seed_ok = eh + 0x400u < 0x800u;
+    const unsigned Y = Y0 + (unsigned) (mulhi32s((int) (unsigned) ((u64) e >> 11), (int) (Y0 >> 1)) >> 19);
+    /* 31 bits of the root S = sqrt(m) 2^52, then 22 more from the remainder
+     * of either sign; S comes out within one of the rounded root */
+    const unsigned s1 = mulhi32(M30, Y);
+    const i64 r1 = (i64) ((M << 8) - (u64) s1 * s1);
+    const int s2 = mulhi32s((int) (r1 >> 6), (int) (Y >> 1)) >> 2;
+    const u64 T = ((u64) s1 << 23) + (u64) (i64) s2;          /* 2 S - s2 */
+    i64 S = (i64) ((u64) s1 << 22) + s2;
+    const i64 R2 = (i64) (((u64) r1 << 44) - T * (u64) (i64) s2);   /* S_exact^2 - S^2 */
+    /* nearest: (S +- 1/2)^2 = S^2 +- S + 1/4 */
+    const i64 d = (R2 > S ? 1 : 0) - (R2 <= -S ? 1 : 0);
+    S += d;
+    const int t = ((int) ex - 1075 - (int) odd) >> 1;         /* exponent left over, halved */
+    ok = ex - 1u < 2046u && seed_ok;
+    return from_bits(((u64) (unsigned) (t + 1048) << 52) + (u64) S);
 }
 
 /*
