@@ -11,10 +11,9 @@
 
 namespace hydro {
 
-/* Launch with programmatic stream serialization: the kernel's blocks may
- * become resident while the kernel before it in the stream drains; every
- * staged kernel waits for that kernel's completion before it reads or
- * writes (pdl_begin). */
+/* Launch with programmatic stream serialization: the launch is processed
+ * while the kernel before it in the stream runs; every staged kernel waits
+ * for that kernel's completion before it reads or writes (pdl_wait). */
 template <class... P, class... A>
 cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, const A &...args)
 {
