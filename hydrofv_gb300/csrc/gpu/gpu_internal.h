@@ -147,6 +147,11 @@ struct Mh2dBand {
 void staged_plan(const Mh2dArgs<double> &a, size_t budget, std::vector<Mh2dBand> &bands, size_t &bytes);
 cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s);
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
+/* Small grids: blocks of the many-step kernel (0: the grid steps with three
+ * launches), and up to `steps` steps in one launch of it. */
+unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, int device);
+cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh2dBand &band, unsigned grid, int steps,
+                                cudaStream_t s);
 
 template <class R>
 cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s);

@@ -22,23 +22,25 @@ template cudaError_t mh2d_launch_ghost_sound_speed<double>(const Mh2dArgs<double
 
 /* ------------------------------------------------------ the staged step */
 
-extern template cudaError_t staged_launch_recon<LIM_MINMOD, 0>(const Mh2dArgs<double> &, const Mh2dBand &, bool, cudaStream_t);
-extern template cudaError_t staged_launch_recon<LIM_MINMOD, 1>(const Mh2dArgs<double> &, const Mh2dBand &, bool, cudaStream_t);
-extern template cudaError_t staged_launch_recon<LIM_VAN_LEER, 0>(const Mh2dArgs<double> &, const Mh2dBand &, bool, cudaStream_t);
-extern template cudaError_t staged_launch_recon<LIM_MC, 0>(const Mh2dArgs<double> &, const Mh2dBand &, bool, cudaStream_t);
+#define HYDRO_STAGED_EXTERN(LIM, FO)                                                                                      \
+    extern template cudaError_t staged_launch_recon<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, cudaStream_t); \
+    extern template int staged_loop_resident<LIM, FO>(bool, int);                                                       \
+    extern template cudaError_t staged_launch_loop<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, unsigned, int, cudaStream_t);
+HYDRO_STAGED_EXTERN(LIM_MINMOD, 0)
+HYDRO_STAGED_EXTERN(LIM_MINMOD, 1)
+HYDRO_STAGED_EXTERN(LIM_VAN_LEER, 0)
+HYDRO_STAGED_EXTERN(LIM_MC, 0)
 
-/* Whether a band's kernels run as one-warp blocks: with fewer items than
- * this the 128-thread blocks would leave schedulers without a warp. */
-static bool staged_small(const Mh2dArgs<double> &a, const Mh2dBand &b)
-{
-    return staged_recon_items(a.nx, b.r1 - b.r0) <= kStagedSmallItems;
-}
+/* f<LIM, FIRST_ORDER>(...) of a run. */
+#define STAGED_DISPATCH(f, ...)                                          \
+    (a.first_order             ? f<LIM_MINMOD, 1>(__VA_ARGS__)           \
+     : limiter == LIM_MINMOD   ? f<LIM_MINMOD, 0>(__VA_ARGS__)           \
+     : limiter == LIM_VAN_LEER ? f<LIM_VAN_LEER, 0>(__VA_ARGS__)         \
+                               : f<LIM_MC, 0>(__VA_ARGS__))
 
 static unsigned update_grid(const Mh2dArgs<double> &a, const Mh2dBand &b)
 {
-    const unsigned cells = (unsigned) (b.r1 - b.r0) * a.nx;
-    if (staged_small(a, b)) return staged_blocks(cells, kStagedSmall);
-    const unsigned n = staged_blocks(cells, kStagedThreads);
+    const unsigned n = staged_blocks((unsigned) (b.r1 - b.r0) * a.nx);
     return n < kStagedUpdateGrid ? n : kStagedUpdateGrid;
 }
 
@@ -72,35 +74,35 @@ cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-template <int NT, bool TAPE>
-static cudaError_t launch_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, cudaStream_t s)
-{
-    return launch_pdl(staged_flux_kernel<NT, TAPE>, staged_blocks(staged_face_items(a.nx, b.r1 - b.r0), NT), NT, s, a, b);
-}
-
-template <int NT>
-static cudaError_t launch_update(const Mh2dArgs<double> &a, const Mh2dBand &b, cudaStream_t s)
-{
-    if (a.gravity != 0.0) return launch_pdl(staged_update_kernel<NT, true>, update_grid(a, b), NT, s, a, b);
-    return launch_pdl(staged_update_kernel<NT, false>, update_grid(a, b), NT, s, a, b);
-}
-
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s)
 {
     for (const Mh2dBand &b : bands) {
-        const bool small = staged_small(a, b);
-        cudaError_t e = a.first_order             ? staged_launch_recon<LIM_MINMOD, 1>(a, b, small, s)
-                        : limiter == LIM_MINMOD   ? staged_launch_recon<LIM_MINMOD, 0>(a, b, small, s)
-                        : limiter == LIM_VAN_LEER ? staged_launch_recon<LIM_VAN_LEER, 0>(a, b, small, s)
-                                                  : staged_launch_recon<LIM_MC, 0>(a, b, small, s);
+        cudaError_t e = STAGED_DISPATCH(staged_launch_recon, a, b, s);
         if (e != cudaSuccess) return e;
-        if (a.tape) e = small ? launch_flux<kStagedSmall, true>(a, b, s) : launch_flux<kStagedThreads, true>(a, b, s);
-        else e = small ? launch_flux<kStagedSmall, false>(a, b, s) : launch_flux<kStagedThreads, false>(a, b, s);
+        const unsigned faces = staged_blocks(staged_face_items(a.nx, b.r1 - b.r0));
+        e = a.tape ? launch_pdl(staged_flux_kernel<true>, faces, s, a, b) : launch_pdl(staged_flux_kernel<false>, faces, s, a, b);
         if (e != cudaSuccess) return e;
-        e = small ? launch_update<kStagedSmall>(a, b, s) : launch_update<kStagedThreads>(a, b, s);
+        e = a.gravity != 0.0 ? launch_pdl(staged_update_kernel<true>, update_grid(a, b), s, a, b)
+                             : launch_pdl(staged_update_kernel<false>, update_grid(a, b), s, a, b);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, int device)
+{
+    if (bands.size() != 1) return 0;
+    const unsigned items = staged_recon_items(a.nx, a.ny);
+    if (items > kStagedLoopItems) return 0;
+    const int resident = STAGED_DISPATCH(staged_loop_resident, a.gravity != 0.0, device);
+    const unsigned blocks = staged_blocks(items);
+    return resident <= 0 ? 0 : (blocks < (unsigned) resident ? blocks : (unsigned) resident);
+}
+
+cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh2dBand &band, unsigned grid, int steps,
+                                cudaStream_t s)
+{
+    return STAGED_DISPATCH(staged_launch_loop, a, band, grid, steps, s);
 }
 
 }  // namespace hydro

@@ -40,14 +40,24 @@
 #ifndef MH2D_UPDATE_CTAS
 #define MH2D_UPDATE_CTAS 6
 #endif
+#ifndef MH2D_LOOP_CTAS
+#define MH2D_LOOP_CTAS 4
+#endif
 
 namespace hydro {
 
-/* Threads per block: 128, or one warp where the grid has too few cells to
- * give every scheduler a warp otherwise. */
 constexpr int kStagedThreads = 128;
-constexpr int kStagedSmall = 32;
-constexpr unsigned kStagedSmallItems = 152 * 4 * 2 * 32;   /* two warps for each of the 608 schedulers */
+
+/* Largest number of recon items (about two per cell) that steps in the
+ * many-step kernel.  Time per step, three launches replayed from a graph
+ * against the many-step kernel: 64^2 26.2 / 24.7 us, 128^2 29.1 / 29.8, 192^2
+ * 40.4 / 40.3, 256^2 63.8 / 60.2, 320^2 86.6 / 84.9, 384^2 106.7 / 109.3,
+ * 512^2 167 / 176; without a graph (short runs) the three launches take at
+ * least 34 us of host time. */
+#ifndef MH2D_LOOP_ITEMS
+#define MH2D_LOOP_ITEMS 200000
+#endif
+constexpr unsigned kStagedLoopItems = MH2D_LOOP_ITEMS;
 constexpr unsigned kStagedUpdateGrid = 152 * MH2D_UPDATE_CTAS;
 
 /* Fields of the workspace: the low and high face states of each cell in x
@@ -68,20 +78,28 @@ __device__ __forceinline__ void pdl_wait()
 }
 
 /* The dt of step n, which starts at time t with the maxima smax[n % 3], and
- * the ratios dt A / V (src/integrator_muscl_hancock.c:533-549, src/utils.c:55-95).
- * One converged warp; the two directions' quotients run in two lanes. */
+ * in lanes 0 and 1 the ratios dt A / V of the x and y faces
+ * (src/integrator_muscl_hancock.c:533-549, src/utils.c:55-95).  One converged
+ * warp; the two directions' quotients run in two lanes. */
+__device__ __forceinline__ void next_dt(const Mh2dArgs<double> &a, const HydroStepControl *ctrl, long long n, double t,
+                                        double tf, double &dt, double &dtA)
+{
+    const bool y = threadIdx.x & 1;
+    const double S = from_ordered_bits(*(const volatile unsigned long long *) &ctrl->smax[n % 3][y]);
+    const double q = dv(S, y ? a.dy : a.dx);
+    const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
+    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
+    dt = dv(cfl, qx + qy);
+    if (t + dt > tf) dt = tf - t;
+    dtA = dv(dt * (y ? a.area_y : a.area_x), a.vol);
+}
+
 __device__ __forceinline__ void arm_dt(const Mh2dArgs<double> &a, HydroStepControl *ctrl, long long n, double t,
                                        double tf)
 {
     const int lane = threadIdx.x & 31;
-    const bool y = lane & 1;
-    const double S = from_ordered_bits(*(volatile unsigned long long *) &ctrl->smax[n % 3][y]);
-    const double q = dv(S, y ? a.dy : a.dx);
-    const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
-    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
-    double dt = dv(cfl, qx + qy);
-    if (t + dt > tf) dt = tf - t;
-    const double w = dv(dt * (y ? a.area_y : a.area_x), a.vol);
+    double dt, w;
+    next_dt(a, ctrl, n, t, tf, dt, w);
     if (lane == 0) ctrl->step_dt = dt;
     if (lane < 2) ctrl->step_dtA[lane] = w;
 }
@@ -133,8 +151,8 @@ __device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh
     }
 }
 
-template <int NT>
 struct FluxShared {
+    static constexpr int NT = kStagedThreads;
     double rho[2][NT], u[2][NT], p[2][NT], a[2][NT];   /* both states of each face */
     double pg[NT];                                     /* star-pressure guess */
     short listT[NT], listS[NT];
@@ -144,8 +162,8 @@ struct FluxShared {
 /* The flux of one block's faces: face k of the band for thread k0 + tid.
  * Faces are classified, the expensive guesses run on compacted lists, and
  * each thread finishes its own face from registers. */
-template <int NT, bool TAPE>
-__device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared<NT> &sm, unsigned k,
+template <bool TAPE>
+__device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared &sm, unsigned k,
                                             unsigned total, double dt)
 {
     const int tid = threadIdx.x;
@@ -188,7 +206,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     __syncthreads();
     double z0 = 0, z1 = 0;
     const int nT = sm.nT, nS = sm.nS;
-    for (int i = tid; i < nT + nS; i += NT) {
+    for (int i = tid; i < nT + nS; i += kStagedThreads) {
         if (i < nT) {
             const int f = sm.listT[i];
             sm.pg[f] = face_trrs(fm, a.gas, sm.u[0][f], sm.p[0][f], sm.a[0][f], sm.u[1][f], sm.p[1][f], sm.a[1][f], z0, z1);
@@ -284,21 +302,16 @@ __device__ __forceinline__ void staged_update(const Fm &f, const Mh2dArgs<double
     }
 }
 
-template <int NT>
 struct UpdateShared {
-    double red[2][NT / 32];
+    double red[2][kStagedThreads / 32];
     int am_last;
 };
 
-/* End of an update block: fold its maxima into the next step's words; the
- * last block of the grid advances the clock (src/integrator_muscl_hancock.c:
- * 1143-1154) and forms the next dt. */
-template <int NT>
-__device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateShared<NT> &sm, unsigned blocks, long long n,
-                                              double dt, double mx_x, double mx_y)
+/* Fold a block's maxima into the next step's words (thread 0 writes them). */
+__device__ __forceinline__ void block_maxima(HydroStepControl *ctrl, double (*red)[kStagedThreads / 32], long long n, double mx_x,
+                                             double mx_y)
 {
     const int tid = threadIdx.x;
-    HydroStepControl *ctrl = a.ctrl;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const double ox = __shfl_xor_sync(0xffffffffu, mx_x, o);
@@ -306,24 +319,33 @@ __device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateS
         if (lt(mx_x, ox)) mx_x = ox;
         if (lt(mx_y, oy)) mx_y = oy;
     }
-    if constexpr (NT > 32) {
-        if ((tid & 31) == 0) {
-            sm.red[0][tid >> 5] = mx_x;
-            sm.red[1][tid >> 5] = mx_y;
-        }
-        __syncthreads();
+    if ((tid & 31) == 0) {
+        red[0][tid >> 5] = mx_x;
+        red[1][tid >> 5] = mx_y;
     }
+    __syncthreads();
     if (tid == 0) {
-        if constexpr (NT > 32) {
-            for (int w = 1; w < NT / 32; w++) {
-                if (lt(mx_x, sm.red[0][w])) mx_x = sm.red[0][w];
-                if (lt(mx_y, sm.red[1][w])) mx_y = sm.red[1][w];
-            }
+        for (int w = 1; w < kStagedThreads / 32; w++) {
+            if (lt(mx_x, red[0][w])) mx_x = red[0][w];
+            if (lt(mx_y, red[1][w])) mx_y = red[1][w];
         }
         unsigned long long *word = ctrl->smax[(n + 1) % 3];
         const unsigned long long bx = ordered_bits(mx_x), by = ordered_bits(mx_y);
         if (bx > *(volatile unsigned long long *) &word[0]) atomicMax(&word[0], bx);
         if (by > *(volatile unsigned long long *) &word[1]) atomicMax(&word[1], by);
+    }
+}
+
+/* End of an update block: fold its maxima into the next step's words; the
+ * last block of the grid advances the clock (src/integrator_muscl_hancock.c:
+ * 1143-1154) and forms the next dt. */
+__device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateShared &sm, unsigned blocks, long long n,
+                                              double dt, double mx_x, double mx_y)
+{
+    const int tid = threadIdx.x;
+    HydroStepControl *ctrl = a.ctrl;
+    block_maxima(ctrl, sm.red, n, mx_x, mx_y);
+    if (tid == 0) {
         __threadfence();
         sm.am_last = atomicAdd(&ctrl->blocks_done, 1u) == blocks - 1;
     }
@@ -369,8 +391,8 @@ __device__ __forceinline__ bool staged_step(HydroStepControl *ctrl, long long &n
 
 /* ------------------------------------------------------- one grid, one band */
 
-template <int LIM, int FIRST_ORDER, int NT>
-__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_RECON_CTAS)
+template <int LIM, int FIRST_ORDER>
+__global__ void __launch_bounds__(kStagedThreads, MH2D_RECON_CTAS)
 staged_recon_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
 {
     pdl_wait();
@@ -385,29 +407,29 @@ staged_recon_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
         }
         return;
     }
-    const unsigned k = blockIdx.x * NT + threadIdx.x;
+    const unsigned k = blockIdx.x * kStagedThreads + threadIdx.x;
     if (k >= staged_recon_items(a.nx, b.r1 - b.r0)) return;
     const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
     staged_recon<LIM, FIRST_ORDER>(a, b, k, (int) (n & 1), n == 0, dtA);
 }
 
-template <int NT, bool TAPE>
-__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_FLUX_CTAS)
+template <bool TAPE>
+__global__ void __launch_bounds__(kStagedThreads, MH2D_FLUX_CTAS)
 staged_flux_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
 {
-    __shared__ FluxShared<NT> sm;
+    __shared__ FluxShared sm;
     pdl_wait();
     long long n;
     double dt;
     if (!staged_step(a.ctrl, n, dt)) return;
-    staged_flux<NT, TAPE>(a, b, sm, blockIdx.x * NT + threadIdx.x, staged_face_items(a.nx, b.r1 - b.r0), dt);
+    staged_flux<TAPE>(a, b, sm, blockIdx.x * kStagedThreads + threadIdx.x, staged_face_items(a.nx, b.r1 - b.r0), dt);
 }
 
-template <int NT, bool GRAV>
-__global__ void __launch_bounds__(NT, NT == 32 ? 16 : MH2D_UPDATE_CTAS)
+template <bool GRAV>
+__global__ void __launch_bounds__(kStagedThreads, MH2D_UPDATE_CTAS)
 staged_update_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
 {
-    __shared__ UpdateShared<NT> sm;
+    __shared__ UpdateShared sm;
     pdl_wait();
     long long n;
     double dt;
@@ -415,9 +437,136 @@ staged_update_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     const Fm f = make_fm();
     double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
     const unsigned cells = (unsigned) (b.r1 - b.r0) * a.nx;
-    for (unsigned k = blockIdx.x * NT + threadIdx.x; k < cells; k += gridDim.x * NT)
+    for (unsigned k = blockIdx.x * kStagedThreads + threadIdx.x; k < cells; k += gridDim.x * kStagedThreads)
         staged_update<GRAV>(f, a, b, k, (int) (n & 1), dt, mx_x, mx_y);
-    staged_finish<NT>(a, sm, b.update_blocks, n, dt, mx_x, mx_y);
+    staged_finish(a, sm, b.update_blocks, n, dt, mx_x, mx_y);
+}
+
+/* ------------------------------------------------ small grids: many steps */
+
+/*
+ * The same three stages, many steps in one cooperative launch, for grids
+ * whose step is a few microseconds of work: grid barriers between the stages
+ * instead of kernel boundaries.  A step has three barriers (about 1.5 us
+ * each); the three launches it replaces cost about 4 us each in gaps, ramps
+ * and control-block reads, and 11 us of host time where no graph is
+ * recorded.  Every block forms the next dt itself after the third barrier.
+ *
+ * grid_barrier: each block counts itself in on a counter that only grows and
+ * waits until it has reached `target`.  All blocks are resident (cooperative
+ * launch), so every wait ends; a limit on the polls guards against an error in
+ * that, after which the block records DEV_ERR_SPIN_LIMIT and leaves (and so do
+ * the others).
+ */
+constexpr int kBarrierPolls = 1 << 22;
+
+__device__ __forceinline__ bool grid_barrier(HydroStepControl *ctrl, unsigned &target, int *ok)
+{
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        int left = kBarrierPolls;
+        if (atomicAdd(&ctrl->barrier_count, 1u) + 1u != target)
+            while (*(volatile unsigned *) &ctrl->barrier_count - target > 0x7fffffffu && --left > 0) { }
+        __threadfence();
+        if (left == 0) record_error(ctrl, DEV_ERR_SPIN_LIMIT, -1);
+        *ok = left > 0;
+    }
+    __syncthreads();
+    return *ok != 0;
+}
+
+template <int LIM, int FIRST_ORDER, bool GRAV>
+__global__ void __launch_bounds__(kStagedThreads, MH2D_LOOP_CTAS)
+staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
+{
+    constexpr int NT = kStagedThreads;
+    __shared__ FluxShared sm;
+    __shared__ double red[2][NT / 32], s_dt, s_dtA[2];
+    __shared__ int ok, failed;
+    HydroStepControl *ctrl = a.ctrl;
+    volatile HydroStepControl *vc = ctrl;
+    const int tid = threadIdx.x;
+    const bool leader = blockIdx.x == 0 && tid == 0;
+    if (!vc->active) return;
+    long long n = vc->num_steps;
+    double t = vc->t, dt = vc->step_dt, dtA[2] = { vc->step_dtA[0], vc->step_dtA[1] };
+    const double tf = vc->tf;
+    const long long last = vc->max_steps;
+    const int stored = vc->store_count;
+    const int rows = b.r1 - b.r0;
+    const unsigned recon = staged_recon_items(a.nx, rows), faces = staged_face_items(a.nx, rows);
+    const unsigned cells = (unsigned) rows * a.nx;
+    const Fm f = make_fm();
+    /* where the counter stood when the launch began: the leader moves the
+     * base on its way out, past the launch's last barrier */
+    unsigned target = vc->barrier_base;
+
+    for (int it = 0; it < most; it++) {
+        const int buf = (int) (n & 1);
+        if (dt == 0.0) {
+            if (leader) {
+                ctrl->dt = dt;
+                record_error(ctrl, DEV_ERR_DT_ZERO, -1);
+                ctrl->active = 0;
+            }
+            return;
+        }
+        for (unsigned k = blockIdx.x * NT + tid; k < recon; k += gridDim.x * NT)
+            staged_recon<LIM, FIRST_ORDER>(a, b, k, buf, n == 0, dtA);
+        if (!grid_barrier(ctrl, target, &ok)) return;
+        for (unsigned k = blockIdx.x * NT; k < faces; k += gridDim.x * NT)
+            staged_flux<false>(a, b, sm, k + tid, faces, dt);
+        if (!grid_barrier(ctrl, target, &ok)) return;
+        double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
+        for (unsigned k = blockIdx.x * NT + tid; k < cells; k += gridDim.x * NT)
+            staged_update<GRAV>(f, a, b, k, buf, dt, mx_x, mx_y);
+        block_maxima(ctrl, red, n, mx_x, mx_y);
+        if (!grid_barrier(ctrl, target, &ok)) return;
+        /* every block: the next dt; block 0 publishes the clock */
+        if (tid < 32) {
+            const bool bad = vc->error_code != 0;
+            const double tn = t + dt;
+            double next, w;
+            next_dt(a, ctrl, n + 1, tn, tf, next, w);
+            if (tid == 0) { failed = bad; s_dt = next; }
+            if (tid < 2) s_dtA[tid] = w;
+        }
+        __syncthreads();
+        if (failed) {
+            if (leader) {
+                ctrl->barrier_base = target;
+                ctrl->dt = dt;
+                ctrl->active = 0;
+            }
+            return;
+        }
+        n += 1;
+        t = t + dt;
+        bool act = (t < tf) && (last < 0 || n < last), due = false;
+        if (a.sp.is_storing && t >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
+            due = true;
+            act = false;
+        }
+        if (leader) {
+            ctrl->dt = dt;
+            ctrl->t = t;
+            ctrl->num_steps = n;
+            ctrl->step_dt = s_dt;
+            ctrl->step_dtA[0] = s_dtA[0];
+            ctrl->step_dtA[1] = s_dtA[1];
+            ctrl->barrier_base = target;
+            ctrl->smax[(n + 1) % 3][0] = ordered_bits(-CUDART_INF);
+            ctrl->smax[(n + 1) % 3][1] = ordered_bits(-CUDART_INF);
+            if (due) ctrl->snapshot_due = 1;
+            if (!act) ctrl->active = 0;
+        }
+        if (!act) return;
+        dt = s_dt;
+        dtA[0] = s_dtA[0];
+        dtA[1] = s_dtA[1];
+    }
 }
 
 /* The first step's dt after the maxima of the state are known, and again

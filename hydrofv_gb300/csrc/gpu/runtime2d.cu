@@ -42,6 +42,9 @@ constexpr int kGraphSteps = 32;
 #ifndef MH2D_WORKSPACE_MB
 #define MH2D_WORKSPACE_MB 1024
 #endif
+/* Most steps of one launch of the many-step kernel (a launch of up to a few
+ * tens of milliseconds). */
+constexpr int kLoopSteps = 1024;
 constexpr size_t kWorkspaceBytes = (size_t) MH2D_WORKSPACE_MB << 20;
 
 void set_cuda_error(HydroRunOutcome *oc, cudaError_t e, const char *what)
@@ -86,6 +89,7 @@ struct HydroRun2D {
     Mh2dArgs<float> args32{};
     void *ws = nullptr;               /* FP64: workspace of the staged step, shared by its bands */
     std::vector<Mh2dBand> bands;
+    unsigned loop_grid = 0;           /* small FP64 grids: blocks of the many-step kernel */
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[6] = {};
     /* asynchronous snapshots: D2H on a side stream, the writer on a host thread */
@@ -422,6 +426,7 @@ extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions
         carve<double>(run, run->args);
         setup_args<double>(run, run->args, grid, opt);
         if (alloc_workspace(run, oc)) return -1;
+        run->loop_grid = staged_loop_grid(run->args, grid->limiter, run->bands, run->device);
     }
     return 0;
 }
@@ -797,6 +802,17 @@ static int apply_host_bc(HydroRun2D *run, HydroRunOutcome *oc)
 /* Enqueue `k` step kernels. */
 static int enqueue_steps(HydroRun2D *run, long long k, HydroRunOutcome *oc)
 {
+    if (run->loop_grid) {
+        while (k > 0) {
+            const int steps = (int) (k < kLoopSteps ? k : kLoopSteps);
+            CK(staged_launch_steps(run->args, run->grid.limiter, run->bands[0], run->loop_grid, steps, run->stream),
+               "step kernel");
+            k -= steps;
+            run->step_launches += 1;
+            run->kernel_launches += 1;
+        }
+        return 0;
+    }
     const bool graphs = run->opt.use_graph && k >= kGraphSteps;
     if (graphs && !run->graph && record_graph(run, oc)) return -1;
     while (k > 0) {

@@ -31,6 +31,8 @@ typedef struct HydroStepControl {
     double tf;                     /* stop once t >= tf (the dt is clipped to it) */
     double step_dt;                /* FP64 2D: dt of the next step, formed when the step before it ends */
     double step_dtA[2];            /* and dt A / V of its x and y faces */
+    unsigned int barrier_count;    /* grid barrier of the many-step kernel: blocks that have arrived */
+    unsigned int barrier_base;     /* and the count when its launch began */
     long long max_steps;           /* stop once num_steps reaches it; < 0: no limit */
     /* smax[k % 3] = ordered-bit maxima of (a+|u|, a+|v|) over the interior of
      * the state that step k starts from. */

@@ -1,7 +1,7 @@
-"""The FP64 step in three kernels (recon, flux, update) where its launch shape
-changes: one-warp or 128-thread blocks, ragged last blocks, first-order
-faces, gravity, and a grid whose workspace holds only part of its rows (two
-bands).  Parity with the oracle, at the tolerance of the other parity tests."""
+"""The FP64 step in three stages (recon, flux, update) where its launch shape
+changes: many steps in one cooperative launch or three launches a step, ragged
+last blocks, first-order faces, gravity, stopping times and snapshots inside a
+launch, and a grid whose workspace holds only part of its rows (two bands).  Parity with the oracle, at the tolerance of the other parity tests."""
 import numpy as np
 import pytest
 
@@ -10,11 +10,11 @@ from test_gpu_parity_2d import assert_parity, run_gpu
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny", [(2, 2), (31, 1024), (137, 139), (138, 138), (139, 139), (1025, 33)])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (31, 1024), (137, 139), (315, 315), (316, 316), (1025, 33)])
 def test_block_shapes(gpu_available, oracle_mod, nx, ny):
-    """Around the size where the blocks change from one warp to four
-    (138^2 has 38640 recon items, 139^2 has 39198; the rule's limit is
-    38912), the smallest grid, and long thin ones."""
+    """The smallest grid, long thin ones, and around the largest that steps in
+    the many-step kernel (315^2 has 199710 recon items, 316^2 has 200976; the
+    rule's limit is 200000)."""
     O = oracle_mod
     p = O.random_problem_2d(nx, ny, nx + ny, ("reflective", "none", "transmissive", "reflective"),
                             "monotonized_central", 6, smooth=True)
@@ -28,6 +28,26 @@ def test_gravity_and_first_order(gpu_available, oracle_mod, n, integrator):
     p = O.rayleigh_taylor(n, n + 3, g=2, steps=10)
     p.integrator = integrator
     assert_parity(p, run_gpu(p), O.load("oracle").run_2d(p))
+
+
+@pytest.mark.parametrize("n", [40, 330])
+def test_stopping_time(gpu_available, oracle_mod, n):
+    """A run to tf (the last dt is clipped, the steps past it are not taken)
+    in either form, and a session whose stopping time moves between calls."""
+    import hydrofv_gb300 as H
+    O = oracle_mod
+    p = O.random_problem_2d(n, n, 3, ("periodic",) * 4, "minmod", -1, smooth=True)
+    p.tf = 0.012
+    ref = O.load("oracle").run_2d(p)
+    assert_parity(p, run_gpu(p), ref)
+    with H.Solver2D(p.nx, p.ny, p.g, (p.x_min, p.x_max, p.y_min, p.y_max), p.gamma, p.W, p.U, bc=p.bc,
+                    slope_limiter=p.slope_limiter, cfl=p.cfl) as s:
+        st, _ = s.advance(3)
+        assert st.num_steps == 3
+        st, _ = s.advance(1000, tf=p.tf)
+        assert st.num_steps == ref.num_steps and st.t == ref.t and st.dt == ref.dt
+        W, U = s.download()
+    assert np.all(O.rel_l1(U, ref.U, p.g) <= 1e-12)
 
 
 def test_two_bands(gpu_available, oracle_mod):
