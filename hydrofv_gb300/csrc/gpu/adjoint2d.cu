@@ -781,6 +781,7 @@ struct HydroAdj2D {
     bool have_codes = false;
     int *err_d = nullptr;
     Mh2dArgs<double> pargs{};
+    std::vector<Mh2dBand> bands;       /* the staged step's bands and workspace */
     /* face-parallel stepper (double): replay and the reverse sweep's faces */
     StateP<double> gen[2]{};
     FacesP<double> faces{};
@@ -890,7 +891,7 @@ int copy_state(HydroAdj2D *a, const StateP<double> &src, const StateP<double> &d
     return 0;
 }
 
-/* One production step n from `in` to `out`. */
+/* One production step n from `in` to `out` (three launches per band). */
 int prod_step(HydroAdj2D *a, long long n, const StateP<double> &in, const StateP<double> &out,
               double *tape, HydroRunOutcome *oc)
 {
@@ -898,14 +899,10 @@ int prod_step(HydroAdj2D *a, long long n, const StateP<double> &in, const StateP
     const int b = (int) (n & 1);
     for (int i = 0; i < 4; i++) { args.U[b][i] = in.U[i]; args.U[b ^ 1][i] = out.U[i]; }
     for (int i = 0; i < 5; i++) { args.W[b][i] = in.W[i]; args.W[b ^ 1][i] = out.W[i]; }
-    if (tape) {
-        args.tape = tape;
-        args.tape_plane = (long long) a->ncell;
-        CK(mh2d_launch_step_tape<double>(args, a->grid.limiter, a->stream), "step kernel (tape)");
-    } else {
-        CK(mh2d_launch_step<double>(args, a->grid.limiter, a->stream), "step kernel");
-    }
-    a->launches++;
+    args.tape = tape;
+    args.tape_plane = (long long) a->ncell;
+    CK(staged_launch_step(args, a->grid.limiter, a->bands, a->stream), tape ? "step kernels (tape)" : "step kernels");
+    a->launches += 3 * (long long) a->bands.size();
     return 0;
 }
 
@@ -1113,7 +1110,6 @@ extern "C" int hydro_adj2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     pa.ny = grid->ny;
     pa.g = grid->g;
     pa.pitch = tx;
-    pa.strip_w = mh2d_threads<double>() - 2;
     for (int s = 0; s < 4; s++) pa.bc[s] = grid->bc[s];
     pa.dx = grid->dx;
     pa.dy = grid->dy;
@@ -1121,9 +1117,14 @@ extern "C" int hydro_adj2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     pa.area_y = grid->area_y;
     pa.vol = grid->vol;
     pa.first_order = 0;
-    pa.grid_ctas = mh2d_resident_ctas<double>(grid->limiter, 0, a->device);
-    pa.chunk_h = opt->chunk_rows > 0 ? opt->chunk_rows
-                                     : mh2d_default_chunk(pa.nx, pa.ny, pa.strip_w, pa.grid_ctas);
+    CK(staged_alloc(pa, a->bands, [&](void **w, size_t bytes) {
+           const cudaError_t e = cudaMalloc(w, bytes);
+           if (e == cudaSuccess) {
+               a->allocs.push_back(*w);
+               a->device_bytes += (long long) bytes;
+           }
+           return e;
+       }), "cudaMalloc(adjoint)");
 
     /* initial state: interior W0, ghosts from the boundary rules, U0 = W->U(W0) */
     StateP<double> s0 = a->ckpt[0];
@@ -1155,7 +1156,8 @@ extern "C" int hydro_adj2d_forward(HydroAdj2D *a, double *const W[4], double *co
     Mh2dArgs<double> args = a->pargs;
     for (int i = 0; i < 5; i++) args.W[0][i] = a->ckpt[0].W[i];
     CK(mh2d_launch_prepare<double>(args, a->stream), "prepare kernel");
-    a->launches++;
+    CK(staged_launch_arm(args, a->stream), "dt kernel");
+    a->launches += 2;
     CK(cudaMemcpyAsync(&a->ckpt_ctrl_d[0], a->ctrl_d, sizeof *c, cudaMemcpyDeviceToDevice, a->stream), "D2D control");
     const StateP<double> *in = &a->ckpt[0];
     for (long long n = 0; n < a->nsteps; n++) {

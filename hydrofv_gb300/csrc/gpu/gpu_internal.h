@@ -140,11 +140,39 @@ struct Mh2dBand {
     double *ws;
 };
 
+/* Most bytes of the staged FP64 step's workspace (16 fields of a band's rows). */
+#ifndef MH2D_WORKSPACE_MB
+#define MH2D_WORKSPACE_MB 1024
+#endif
+constexpr size_t kStagedWorkspaceBytes = (size_t) MH2D_WORKSPACE_MB << 20;
+
 /* The staged FP64 step (mh2d_staged.cuh).  staged_plan splits the grid's rows
  * into bands whose workspace takes at most `budget` bytes (one row at least;
  * `bytes` receives what it takes); the caller points every band's `ws` at
  * that workspace. */
 void staged_plan(const Mh2dArgs<double> &a, size_t budget, std::vector<Mh2dBand> &bands, size_t &bytes);
+/* The same with the workspace: `alloc(&p, bytes)` is asked for
+ * kStagedWorkspaceBytes at most, and for less where the device has no room
+ * (more and shorter bands, down to single rows). */
+template <class Alloc>
+cudaError_t staged_alloc(const Mh2dArgs<double> &a, std::vector<Mh2dBand> &bands, Alloc alloc)
+{
+    size_t budget = kStagedWorkspaceBytes;
+    for (;;) {
+        size_t bytes = 0;
+        void *p = nullptr;
+        staged_plan(a, budget, bands, bytes);
+        const cudaError_t e = alloc(&p, bytes);
+        if (e == cudaSuccess) {
+            for (auto &b : bands) b.ws = static_cast<double *>(p);
+            return e;
+        }
+        if (e != cudaErrorMemoryAllocation || bands[0].r1 - bands[0].r0 == 1) return e;
+        cudaGetLastError();
+        budget = bytes / 2;
+    }
+}
+
 cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s);
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
 /* Small grids: blocks of the many-step kernel (0: the grid steps with three
@@ -155,8 +183,6 @@ cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh
 
 template <class R>
 cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s);
-template <class R>
-cudaError_t mh2d_launch_step_tape(const Mh2dArgs<R> &a, int limiter, cudaStream_t s);
 template <class R>
 int mh2d_resident_ctas(int limiter, int first_order, int device);
 template <class R>

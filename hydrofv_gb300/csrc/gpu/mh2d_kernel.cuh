@@ -93,7 +93,7 @@ struct Mh2dArgs {
     int first_order;         /* 1: Godunov first order (face states = cell states) */
     int grid_ctas;           /* persistent CTAs per step launch (0: one per work item) */
     double gravity;          /* System.gravity (kernels built with GRAV only) */
-    R *tape;                 /* adjoint tape of this step (kernels built with TAPE only) */
+    R *tape;                 /* adjoint tape of this step (staged flux kernel; null: none) */
     long long tape_plane;    /* elements per tape field (padded cells) */
 };
 
@@ -134,8 +134,8 @@ __host__ __device__ inline void mh2d_item_rows(const Mh2dArgs<R> &a, int item, i
 }
 
 /*
- * Adjoint tape of one step (written by the TAPE build of the step kernel,
- * read by the reverse sweep).  Per face, at the padded index of its left
+ * Adjoint tape of one step (written by the TAPE build of the staged flux
+ * kernel, read by the reverse sweep).  Per face, at the padded index of its left
  * (x faces) or lower (y faces) cell, MH2D_TAPE_FIELDS fields per direction
  * (x fields first, then y): the face states (4 + 4, normal velocity in
  * slot 1), both sound speeds, the star-pressure guess before the floor, the
@@ -147,23 +147,6 @@ __host__ __device__ inline void mh2d_item_rows(const Mh2dArgs<R> &a, int item, i
 enum : int {
     TAPE_L = 0, TAPE_R = 4, TAPE_AL = 8, TAPE_AR = 9, TAPE_PG = 10, TAPE_Z0 = 11, TAPE_Z1 = 12,
     TAPE_REG = 13, TAPE_QL = 14, TAPE_QR = 15, TAPE_SS = 16,
-};
-
-/* Where solve_faces writes the tape of a batch: faces [0, nxf) are x faces
- * of row row_x with left cells c0-1+f; the rest are y faces between row_y
- * and row_y+1 in columns c0+(f-nxf). */
-template <class R>
-struct TapeCtx {
-    R *tape;
-    long long plane;
-    int pitch, nxf, row_x, row_y, c0;
-    __device__ __forceinline__ R *field(int f, int q) const
-    {
-        const bool x = f < nxf;
-        const long long idx = x ? (long long) row_x * pitch + c0 - 1 + f
-                                : (long long) row_y * pitch + c0 + (f - nxf);
-        return tape + ((x ? 0 : MH2D_TAPE_FIELDS) + q) * plane + idx;
-    }
 };
 
 /* Where W at padded (r, c) comes from: the stored cell (rr, cc), with the
@@ -309,14 +292,13 @@ __device__ __noinline__ void vacuum_flux_dev(const GasConst<R> &c, R rl, R ul, R
  * build (contraction allowed) fuses; the point blast at 8192^2 needs that
  * accuracy near its vacuum.  Ends with a barrier.
  */
-template <class R, int NT, bool TAPE = false>
+template <class R, int NT>
 __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst<R> &gas, int nF,
-                                           int nXf, R dtr, R Ax, R Ay,
-                                           const TapeCtx<R> &tc = TapeCtx<R>{})
+                                           int nXf, R dtr, R Ax, R Ay)
 {
     const int tid = threadIdx.x;
     int err = DEV_OK;
-    if constexpr (sizeof(R) == 4 && !TAPE) {
+    if constexpr (sizeof(R) == 4) {
         for (int f = tid; f < nF; f += NT) {
             R F[4];
             const int rc = hllc_flux_2d(gas, sm.FL[0][f], sm.FL[1][f], sm.FL[2][f], sm.FL[3][f],
@@ -342,21 +324,7 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
         __syncthreads();
         const int nT = sm.nT, nS = sm.nS;
         for (int i = tid; i < nT + nS; i += NT) {
-            if constexpr (TAPE) {
-                R z0, z1;
-                int f;
-                if (i < nT) {
-                    f = sm.listT[i];
-                    sm.pg[f] = guess_p_trrs_z(gas, sm.FL[1][f], sm.FL[3][f], sm.aL[f],
-                                              sm.FR[1][f], sm.FR[3][f], sm.aR[f], z0, z1);
-                } else {
-                    f = sm.listS[i - nT];
-                    sm.pg[f] = guess_p_tsrs_g(gas, sm.FL[0][f], sm.FL[1][f], sm.FL[3][f],
-                                              sm.FR[0][f], sm.FR[1][f], sm.FR[3][f], sm.pg[f], z0, z1);
-                }
-                *tc.field(f, TAPE_Z0) = z0;
-                *tc.field(f, TAPE_Z1) = z1;
-            } else if (i < nT) {
+            if (i < nT) {
                 const int f = sm.listT[i];
                 sm.pg[f] = guess_p_trrs(gas, sm.FL[1][f], sm.FL[3][f], sm.aL[f],
                                         sm.FR[1][f], sm.FR[3][f], sm.aR[f]);
@@ -371,27 +339,8 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
             R F[4];
             const R rl = sm.FL[0][f], ul = sm.FL[1][f], vl = sm.FL[2][f], pl = sm.FL[3][f];
             const R rr = sm.FR[0][f], ur = sm.FR[1][f], vr = sm.FR[2][f], pr = sm.FR[3][f];
-            if constexpr (TAPE) {
-                const R v[11] = { rl, ul, vl, pl, rr, ur, vr, pr, sm.aL[f], sm.aR[f], sm.pg[f] };
-#pragma unroll
-                for (int q = 0; q < 11; q++) *tc.field(f, q) = v[q];
-                *tc.field(f, TAPE_REG) = (R) sm.reg[f];
-            }
             if (sm.reg[f] == PREG_VACUUM) {
                 vacuum_flux_dev(gas, rl, ul, vl, pl, sm.aL[f], rr, ur, vr, pr, sm.aR[f], F);
-                if constexpr (TAPE) {
-                    *tc.field(f, TAPE_QL) = R(0);
-                    *tc.field(f, TAPE_QR) = R(0);
-                    *tc.field(f, TAPE_SS) = R(0);
-                }
-            } else if constexpr (TAPE) {
-                R wave[3];
-                const int rc = hllc_finish(gas, rl, ul, vl, pl, sm.aL[f], rr, ur, vr, pr, sm.aR[f],
-                                           sm.pg[f], F, wave);
-                if (rc) err = rc;
-                *tc.field(f, TAPE_QL) = wave[0];
-                *tc.field(f, TAPE_QR) = wave[1];
-                *tc.field(f, TAPE_SS) = wave[2];
             } else {
                 const int rc = hllc_finish(gas, rl, ul, vl, pl, sm.aL[f], rr, ur, vr, pr, sm.aR[f],
                                            sm.pg[f], F);
@@ -416,7 +365,7 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
  * rows) of step n with time step dt.  Shared by the single-grid and the
  * batched kernels; the caller reduces mx_x / mx_y and handles errors.
  */
-template <class R, int LIM, int NT, int FIRST_ORDER, bool TAPE = false, bool GRAV = false>
+template <class R, int LIM, int NT, int FIRST_ORDER, bool GRAV = false>
 __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT> &sm, int item,
                                           long long n, double dt, double &mx_x, double &mx_y,
                                           int &err)
@@ -562,7 +511,7 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
      * cell itself, from the two states it holds in registers, so y faces
      * never pass through shared memory; only the x faces, whose states come
      * from two threads, are batched there */
-    constexpr bool YREG = sizeof(R) == 4 && !TAPE;
+    constexpr bool YREG = sizeof(R) == 4;
     R ytop[4], gbot[4];         /* FP32 */
     R tmp_lo[4], prev_hi[4];
     if (inner) recon_y(r_begin - 1, tmp_lo, prev_hi);
@@ -593,12 +542,7 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
         __syncthreads();
         {
             int rc;
-            if constexpr (TAPE) {
-                const TapeCtx<R> tc{ a.tape, a.tape_plane, a.pitch, 0, -1, r_begin - 1, c0 };
-                rc = solve_faces<R, NT, true>(sm, a.gas, sw, 0, dtr, Ax, Ay, tc);
-            } else {
-                rc = solve_faces<R, NT>(sm, a.gas, sw, 0, dtr, Ax, Ay);
-            }
+            rc = solve_faces<R, NT>(sm, a.gas, sw, 0, dtr, Ax, Ay);
             if (rc) err = rc;
         }
         if (inner) {
@@ -681,12 +625,7 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
         __syncthreads();
         {
             int rc;
-            if constexpr (TAPE) {
-                const TapeCtx<R> tc{ a.tape, a.tape_plane, a.pitch, nX, r, r, c0 };
-                rc = solve_faces<R, NT, true>(sm, a.gas, nX + sw, nX, dtr, Ax, Ay, tc);
-            } else {
-                rc = solve_faces<R, NT>(sm, a.gas, YREG ? nX : nX + sw, nX, dtr, Ax, Ay);
-            }
+            rc = solve_faces<R, NT>(sm, a.gas, YREG ? nX : nX + sw, nX, dtr, Ax, Ay);
             if (rc) err = rc;
         }
 
@@ -790,7 +729,7 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
  * SMs that finish early take more work (the FP64 pipe of an SM is shared by
  * its CTAs).
  */
-template <class R, int LIM, int NT, int FIRST_ORDER, bool TAPE = false, bool GRAV = false>
+template <class R, int LIM, int NT, int FIRST_ORDER, bool GRAV = false>
 __global__ void __launch_bounds__(NT, (sizeof(R) == 4 ? MH2D_CTAS_FP32 : MH2D_CTAS_FP64))
 mh2d_step_kernel(const Mh2dArgs<R> a)
 {
@@ -828,7 +767,7 @@ mh2d_step_kernel(const Mh2dArgs<R> a)
         const int item = sm.item;
         __syncthreads();
         if (item >= n_items) break;
-        mh2d_item<R, LIM, NT, FIRST_ORDER, TAPE, GRAV>(a, sm, item, n, dt, mx_x, mx_y, err);
+        mh2d_item<R, LIM, NT, FIRST_ORDER, GRAV>(a, sm, item, n, dt, mx_x, mx_y, err);
     }
 
     if (err) record_error(ctrl, err, (int) blockIdx.x);

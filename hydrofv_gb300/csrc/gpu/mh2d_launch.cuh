@@ -138,8 +138,6 @@ __global__ void mh2d_ghost_sound_speed_kernel(const Mh2dArgs<R> a, int buf, int 
  */
 template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_step_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s);
-template <class R, int LIM>
-cudaError_t mh2d_launch_tape_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s);
 template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_batch_lim(const Mh2dBatchArgs<R> &b, int grid, cudaStream_t s);
 template <class R, int LIM, int FIRST_ORDER>
@@ -155,19 +153,6 @@ cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s)
     case LIM_MINMOD: return mh2d_launch_step_lim<R, LIM_MINMOD, 0>(a, grid, s);
     case LIM_VAN_LEER: return mh2d_launch_step_lim<R, LIM_VAN_LEER, 0>(a, grid, s);
     default: return mh2d_launch_step_lim<R, LIM_MC, 0>(a, grid, s);
-    }
-}
-
-/* The step kernel that also writes the adjoint tape (a.tape, FP64 MUSCL-Hancock). */
-template <class R>
-cudaError_t mh2d_launch_step_tape(const Mh2dArgs<R> &a, int limiter, cudaStream_t s)
-{
-    const int n_items = mh2d_n_items(a);
-    const int grid = (a.grid_ctas > 0 && a.grid_ctas < n_items) ? a.grid_ctas : n_items;
-    switch (limiter) {
-    case LIM_MINMOD: return mh2d_launch_tape_lim<R, LIM_MINMOD>(a, grid, s);
-    case LIM_VAN_LEER: return mh2d_launch_tape_lim<R, LIM_VAN_LEER>(a, grid, s);
-    default: return mh2d_launch_tape_lim<R, LIM_MC>(a, grid, s);
     }
 }
 

@@ -15,16 +15,9 @@ template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_step_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s)
 {
     if (a.gravity != 0.0)
-        mh2d_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER, false, true><<<grid, mh2d_threads<R>(), 0, s>>>(a);
+        mh2d_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER, true><<<grid, mh2d_threads<R>(), 0, s>>>(a);
     else
         mh2d_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER><<<grid, mh2d_threads<R>(), 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <class R, int LIM>
-cudaError_t mh2d_launch_tape_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s)
-{
-    mh2d_step_kernel<R, LIM, mh2d_threads<R>(), 0, true><<<grid, mh2d_threads<R>(), 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -12,6 +12,5 @@ namespace hydro {
 
 HYDRO_MH2D_INSTANTIATE(double, LIM_VAN_LEER, 0)
 HYDRO_STAGED_INSTANTIATE(LIM_VAN_LEER, 0)
-template cudaError_t mh2d_launch_tape_lim<double, LIM_VAN_LEER>(const Mh2dArgs<double> &, int, cudaStream_t);
 
 }  // namespace hydro

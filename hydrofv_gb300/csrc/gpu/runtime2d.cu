@@ -38,14 +38,9 @@ using namespace hydro;
 namespace {
 
 constexpr int kGraphSteps = 32;
-/* Most bytes of the staged FP64 step's workspace (16 fields of a band's rows). */
-#ifndef MH2D_WORKSPACE_MB
-#define MH2D_WORKSPACE_MB 1024
-#endif
 /* Most steps of one launch of the many-step kernel (a launch of up to a few
  * tens of milliseconds). */
 constexpr int kLoopSteps = 1024;
-constexpr size_t kWorkspaceBytes = (size_t) MH2D_WORKSPACE_MB << 20;
 
 void set_cuda_error(HydroRunOutcome *oc, cudaError_t e, const char *what)
 {
@@ -343,26 +338,6 @@ extern "C" int hydro_gpu_trim_device_memory(int device)
     return 0;
 }
 
-/* The staged step's workspace: as much as kWorkspaceBytes, less where the
- * device has no room for it (more and shorter bands). */
-static int alloc_workspace(HydroRun2D *run, HydroRunOutcome *oc)
-{
-    size_t budget = kWorkspaceBytes;
-    for (;;) {
-        size_t bytes = 0;
-        staged_plan(run->args, budget, run->bands, bytes);
-        const cudaError_t e = pool_alloc(run, &run->ws, bytes);
-        if (e == cudaSuccess) break;
-        const int h = run->bands[0].r1 - run->bands[0].r0;
-        if (e != cudaErrorMemoryAllocation || h == 1) CK(e, "cudaMallocFromPoolAsync(workspace)");
-        cudaGetLastError();
-        run->ws = nullptr;
-        budget = bytes / 2;
-    }
-    for (auto &b : run->bands) b.ws = static_cast<double *>(run->ws);
-    return 0;
-}
-
 extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions *opt,
                                   HydroRun2D **out, HydroRunOutcome *oc)
 {
@@ -425,7 +400,11 @@ extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     } else {
         carve<double>(run, run->args);
         setup_args<double>(run, run->args, grid, opt);
-        if (alloc_workspace(run, oc)) return -1;
+        CK(staged_alloc(run->args, run->bands, [&](void **p, size_t bytes) {
+               const cudaError_t e = pool_alloc(run, p, bytes);
+               run->ws = *p;
+               return e;
+           }), "cudaMallocFromPoolAsync(workspace)");
         run->loop_grid = staged_loop_grid(run->args, grid->limiter, run->bands, run->device);
     }
     return 0;

@@ -204,7 +204,8 @@ FXHD int face_classify(const Fm &f, const GasConst<double> &c, double rho_L, dou
     return (bp <= up && up <= lo + (fx::i64) fx::HIDDEN) ? PREG_PVRS : PREG_TSRS;
 }
 
-/* guess_p_trrs_z and guess_p_tsrs_g (numerics.cuh). */
+/* guess_p_trrs and guess_p_tsrs (numerics.cuh); they also hand back their
+ * factors (p^((g-1)/2g) and g_K of each side), which the adjoint's tape keeps. */
 FXHD double face_trrs(const Fm &f, const GasConst<double> &c, double u_L, double p_L, double a_L, double u_R, double p_R,
                       double a_R, double &zL, double &zR)
 {
