@@ -175,6 +175,32 @@ cudaError_t staged_alloc(const Mh2dArgs<double> &a, std::vector<Mh2dBand> &bands
 
 cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s);
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
+/* Batches: band `band` of instance `inst`; its blocks of the recon, flux and
+ * update launches start at first[0], first[1], first[2] of the group's. */
+struct StagedBatchBand {
+    Mh2dBand band;
+    int inst;
+    unsigned first[3], update_grid;
+};
+
+/* Bands that share the workspace: one launch per stage.  map[s][k] is the
+ * band (index into `bands`) of block k of stage s (device memory). */
+struct StagedBatchGroup {
+    const int *map[3];
+    unsigned blocks[3];
+};
+
+struct StagedBatchArgs {
+    const Mh2dArgs<double> *inst;     /* device memory, one per instance */
+    const StagedBatchBand *bands;     /* device memory */
+};
+
+/* Blocks of a band's stages. */
+void staged_band_blocks(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned blocks[3]);
+cudaError_t staged_launch_batch(const StagedBatchArgs &b, const std::vector<StagedBatchGroup> &groups, int limiter,
+                                int first_order, cudaStream_t s);
+cudaError_t staged_launch_batch_arm(const StagedBatchArgs &b, int n, cudaStream_t s);
+
 /* Small grids: blocks of the many-step kernel (0: the grid steps with three
  * launches), and up to `steps` steps in one launch of it. */
 unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, int device);

@@ -10,7 +10,6 @@
 namespace hydro {
 
 template int mh2d_resident_ctas<double>(int, int, int);
-template cudaError_t mh2d_launch_batch_step<double>(const Mh2dBatchArgs<double> &, int, int, int, cudaStream_t);
 template cudaError_t mh2d_launch_step<double>(const Mh2dArgs<double> &, int, cudaStream_t);
 template cudaError_t mh2d_launch_prepare<double>(const Mh2dArgs<double> &, cudaStream_t);
 template cudaError_t mh2d_launch_materialize<double>(const Mh2dArgs<double> &, int,
@@ -23,6 +22,7 @@ template cudaError_t mh2d_launch_ghost_sound_speed<double>(const Mh2dArgs<double
 
 #define HYDRO_STAGED_EXTERN(LIM, FO)                                                                                      \
     extern template cudaError_t staged_launch_recon<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, cudaStream_t); \
+    extern template cudaError_t staged_launch_batch_recon<LIM, FO>(const StagedBatchArgs &, const StagedBatchGroup &, cudaStream_t); \
     extern template int staged_loop_resident<LIM, FO>(bool, int);                                                       \
     extern template cudaError_t staged_launch_loop<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, unsigned, int, cudaStream_t);
 HYDRO_STAGED_EXTERN(LIM_MINMOD, 0)
@@ -30,9 +30,9 @@ HYDRO_STAGED_EXTERN(LIM_MINMOD, 1)
 HYDRO_STAGED_EXTERN(LIM_VAN_LEER, 0)
 HYDRO_STAGED_EXTERN(LIM_MC, 0)
 
-/* f<LIM, FIRST_ORDER>(...) of a run. */
+/* f<LIM, FIRST_ORDER>(...) for `limiter` and `first_order`. */
 #define STAGED_DISPATCH(f, ...)                                          \
-    (a.first_order             ? f<LIM_MINMOD, 1>(__VA_ARGS__)           \
+    (first_order               ? f<LIM_MINMOD, 1>(__VA_ARGS__)           \
      : limiter == LIM_MINMOD   ? f<LIM_MINMOD, 0>(__VA_ARGS__)           \
      : limiter == LIM_VAN_LEER ? f<LIM_VAN_LEER, 0>(__VA_ARGS__)         \
                                : f<LIM_MC, 0>(__VA_ARGS__))
@@ -75,6 +75,7 @@ cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s)
 
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s)
 {
+    const int first_order = a.first_order;
     for (const Mh2dBand &b : bands) {
         cudaError_t e = STAGED_DISPATCH(staged_launch_recon, a, b, s);
         if (e != cudaSuccess) return e;
@@ -88,8 +89,36 @@ cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std
     return cudaSuccess;
 }
 
+void staged_band_blocks(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned blocks[3])
+{
+    blocks[0] = staged_blocks(staged_recon_items(a.nx, b.r1 - b.r0));
+    blocks[1] = staged_blocks(staged_face_items(a.nx, b.r1 - b.r0));
+    blocks[2] = update_grid(a, b);
+}
+
+cudaError_t staged_launch_batch(const StagedBatchArgs &b, const std::vector<StagedBatchGroup> &groups, int limiter,
+                                int first_order, cudaStream_t s)
+{
+    for (const StagedBatchGroup &g : groups) {
+        cudaError_t e = STAGED_DISPATCH(staged_launch_batch_recon, b, g, s);
+        if (e != cudaSuccess) return e;
+        e = launch_pdl(staged_batch_flux_kernel, g.blocks[1], s, b, g.map[1]);
+        if (e != cudaSuccess) return e;
+        e = launch_pdl(staged_batch_update_kernel, g.blocks[2], s, b, g.map[2]);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t staged_launch_batch_arm(const StagedBatchArgs &b, int n, cudaStream_t s)
+{
+    staged_batch_arm_kernel<<<n, 32, 0, s>>>(b);
+    return cudaGetLastError();
+}
+
 unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, int device)
 {
+    const int first_order = a.first_order;
     if (bands.size() != 1) return 0;
     const unsigned items = staged_recon_items(a.nx, a.ny);
     if (items > kStagedLoopItems) return 0;
@@ -101,6 +130,7 @@ unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vec
 cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh2dBand &band, unsigned grid, int steps,
                                 cudaStream_t s)
 {
+    const int first_order = a.first_order;
     return STAGED_DISPATCH(staged_launch_loop, a, band, grid, steps, s);
 }
 

@@ -72,9 +72,6 @@ namespace hydro {
 template <class R>
 constexpr int mh2d_threads() { return sizeof(R) == 8 ? MH2D_THREADS_FP64 : MH2D_THREADS_FP32; }
 
-/* The same, for host code that holds the precision as a flag. */
-inline int mh2d_threads_for(bool fp32) { return fp32 ? MH2D_THREADS_FP32 : MH2D_THREADS_FP64; }
-
 template <class R>
 struct Mh2dArgs {
     R *U[2][4];              /* [buffer][mass, mom_x, mom_y, energy] */

@@ -37,10 +37,13 @@ cudaError_t mh2d_step_occupancy(int *per_sm)
 
 }  // namespace hydro
 
-/* Everything one (precision, limiter, first-order) combination launches. */
-#define HYDRO_MH2D_INSTANTIATE(R, LIM, FO)                                                                 \
+/* Everything one (precision, limiter, first-order) combination launches:
+ * the single grid, and (FP32) the batch. */
+#define HYDRO_MH2D_INSTANTIATE_GRID(R, LIM, FO)                                                            \
     template cudaError_t mh2d_launch_step_lim<R, LIM, FO>(const Mh2dArgs<R> &, int, cudaStream_t);        \
-    template cudaError_t mh2d_launch_batch_lim<R, LIM, FO>(const Mh2dBatchArgs<R> &, int, cudaStream_t);  \
     template cudaError_t mh2d_step_occupancy<R, LIM, FO>(int *);
+#define HYDRO_MH2D_INSTANTIATE(R, LIM, FO)                                                                 \
+    HYDRO_MH2D_INSTANTIATE_GRID(R, LIM, FO)                                                               \
+    template cudaError_t mh2d_launch_batch_lim<R, LIM, FO>(const Mh2dBatchArgs<R> &, int, cudaStream_t);
 
 #endif

@@ -11,7 +11,7 @@
 
 namespace hydro {
 
-HYDRO_MH2D_INSTANTIATE(double, LIM_MINMOD, 1)
+HYDRO_MH2D_INSTANTIATE_GRID(double, LIM_MINMOD, 1)
 HYDRO_STAGED_INSTANTIATE(LIM_MINMOD, 1)
 
 }  // namespace hydro

@@ -389,6 +389,15 @@ __device__ __forceinline__ bool staged_step(HydroStepControl *ctrl, long long &n
     return dt != 0.0;
 }
 
+/* A step that was due but has a zero dt. */
+__device__ __forceinline__ void record_zero_dt(HydroStepControl *ctrl)
+{
+    if (!ctrl->active || ctrl->error_code != 0) return;
+    ctrl->dt = 0.0;
+    record_error(ctrl, DEV_ERR_DT_ZERO, -1);
+    ctrl->active = 0;
+}
+
 /* ------------------------------------------------------- one grid, one band */
 
 template <int LIM, int FIRST_ORDER>
@@ -400,11 +409,7 @@ staged_recon_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     double dt;
     HydroStepControl *ctrl = a.ctrl;
     if (!staged_step(ctrl, n, dt)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0 && ctrl->active && ctrl->error_code == 0) {
-            ctrl->dt = 0.0;
-            record_error(ctrl, DEV_ERR_DT_ZERO, -1);
-            ctrl->active = 0;
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) record_zero_dt(ctrl);
         return;
     }
     const unsigned k = blockIdx.x * kStagedThreads + threadIdx.x;
@@ -440,6 +445,89 @@ staged_update_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     for (unsigned k = blockIdx.x * kStagedThreads + threadIdx.x; k < cells; k += gridDim.x * kStagedThreads)
         staged_update<GRAV>(f, a, b, k, (int) (n & 1), dt, mx_x, mx_y);
     staged_finish(a, sm, b.update_blocks, n, dt, mx_x, mx_y);
+}
+
+/* ------------------------------------------------------------- many grids */
+
+/*
+ * The stages of a batch: one launch per stage over the blocks of all
+ * instances (bands) of a group.  A block finds its band in a map, copies the
+ * instance's arguments to shared memory and runs the single grid's code, so
+ * each instance has the single grid's bits.  Instances keep their own clock;
+ * one that has stopped leaves at once.
+ */
+struct BatchBlock {
+    Mh2dArgs<double> a;
+    StagedBatchBand b;
+    long long n;
+    double dt, dtA[2];
+    int go;
+};
+
+__device__ __forceinline__ bool batch_block(const StagedBatchArgs &g, const int *map, BatchBlock &sm)
+{
+    pdl_wait();
+    const StagedBatchBand *band = g.bands + map[blockIdx.x];
+    const Mh2dArgs<double> *inst = g.inst + band->inst;
+    const int tid = threadIdx.x;
+    static_assert(sizeof(Mh2dArgs<double>) % 8 == 0 && sizeof(StagedBatchBand) % 8 == 0, "copied as 8-byte words");
+    for (int k = tid; k < (int) (sizeof(Mh2dArgs<double>) / 8); k += kStagedThreads)
+        ((unsigned long long *) &sm.a)[k] = ((const unsigned long long *) inst)[k];
+    for (int k = tid; k < (int) (sizeof(StagedBatchBand) / 8); k += kStagedThreads)
+        ((unsigned long long *) &sm.b)[k] = ((const unsigned long long *) band)[k];
+    if (tid == 0) {
+        HydroStepControl *ctrl = inst->ctrl;
+        sm.go = staged_step(ctrl, sm.n, sm.dt);
+        sm.dtA[0] = ctrl->step_dtA[0];
+        sm.dtA[1] = ctrl->step_dtA[1];
+    }
+    __syncthreads();
+    return sm.go != 0;
+}
+
+template <int LIM, int FIRST_ORDER>
+__global__ void __launch_bounds__(kStagedThreads, MH2D_RECON_CTAS)
+staged_batch_recon_kernel(const StagedBatchArgs g, const int *map)
+{
+    __shared__ BatchBlock sm;
+    if (!batch_block(g, map, sm)) {
+        if (threadIdx.x == 0 && blockIdx.x == sm.b.first[0] && sm.b.band.r0 == sm.a.g) record_zero_dt(sm.a.ctrl);
+        return;
+    }
+    const unsigned k = (blockIdx.x - sm.b.first[0]) * kStagedThreads + threadIdx.x;
+    if (k >= staged_recon_items(sm.a.nx, sm.b.band.r1 - sm.b.band.r0)) return;
+    staged_recon<LIM, FIRST_ORDER>(sm.a, sm.b.band, k, (int) (sm.n & 1), sm.n == 0, sm.dtA);
+}
+
+static __global__ void __launch_bounds__(kStagedThreads, MH2D_FLUX_CTAS)
+staged_batch_flux_kernel(const StagedBatchArgs g, const int *map)
+{
+    __shared__ BatchBlock sm;
+    __shared__ FluxShared fs;
+    if (!batch_block(g, map, sm)) return;
+    staged_flux<false>(sm.a, sm.b.band, fs, (blockIdx.x - sm.b.first[1]) * kStagedThreads + threadIdx.x,
+                       staged_face_items(sm.a.nx, sm.b.band.r1 - sm.b.band.r0), sm.dt);
+}
+
+static __global__ void __launch_bounds__(kStagedThreads, MH2D_UPDATE_CTAS)
+staged_batch_update_kernel(const StagedBatchArgs g, const int *map)
+{
+    __shared__ BatchBlock sm;
+    __shared__ UpdateShared us;
+    if (!batch_block(g, map, sm)) return;
+    const Fm f = make_fm();
+    double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
+    const unsigned cells = (unsigned) (sm.b.band.r1 - sm.b.band.r0) * sm.a.nx;
+    for (unsigned k = (blockIdx.x - sm.b.first[2]) * kStagedThreads + threadIdx.x; k < cells;
+         k += sm.b.update_grid * kStagedThreads)
+        staged_update<false>(f, sm.a, sm.b.band, k, (int) (sm.n & 1), sm.dt, mx_x, mx_y);
+    staged_finish(sm.a, us, sm.b.band.update_blocks, sm.n, sm.dt, mx_x, mx_y);
+}
+
+static __global__ void staged_batch_arm_kernel(const StagedBatchArgs g)
+{
+    const Mh2dArgs<double> &a = g.inst[blockIdx.x];
+    arm_dt(a, a.ctrl, a.ctrl->num_steps, a.ctrl->t, a.ctrl->tf);
 }
 
 /* ------------------------------------------------ small grids: many steps */

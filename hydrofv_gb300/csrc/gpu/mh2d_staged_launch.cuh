@@ -37,6 +37,12 @@ cudaError_t staged_launch_recon(const Mh2dArgs<double> &a, const Mh2dBand &b, cu
     return launch_pdl(staged_recon_kernel<LIM, FIRST_ORDER>, staged_blocks(staged_recon_items(a.nx, b.r1 - b.r0)), s, a, b);
 }
 
+template <int LIM, int FIRST_ORDER>
+cudaError_t staged_launch_batch_recon(const StagedBatchArgs &b, const StagedBatchGroup &g, cudaStream_t s)
+{
+    return launch_pdl(staged_batch_recon_kernel<LIM, FIRST_ORDER>, g.blocks[0], s, b, g.map[0]);
+}
+
 /* Blocks of the many-step kernel that are resident at once (0: it cannot be
  * launched), and its cooperative launch. */
 template <int LIM, int FIRST_ORDER>
@@ -74,6 +80,7 @@ cudaError_t staged_launch_loop(const Mh2dArgs<double> &a, const Mh2dBand &b, uns
 
 #define HYDRO_STAGED_INSTANTIATE(LIM, FO) \
     template cudaError_t staged_launch_recon<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, cudaStream_t); \
+    template cudaError_t staged_launch_batch_recon<LIM, FO>(const StagedBatchArgs &, const StagedBatchGroup &, cudaStream_t); \
     template int staged_loop_resident<LIM, FO>(bool, int);                                                           \
     template cudaError_t staged_launch_loop<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, unsigned, int, cudaStream_t);
 

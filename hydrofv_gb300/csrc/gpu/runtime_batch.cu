@@ -73,6 +73,10 @@ struct HydroBatch2D {
     int *item_off_d = nullptr;
     void *args_d = nullptr;                 /* Mh2dArgs<R>[n] */
     std::vector<Mh2dArgs<double>> a64;
+    /* FP64: the staged step's bands and groups, and its device memory */
+    std::vector<StagedBatchGroup> groups;
+    StagedBatchArgs staged{};
+    void *ws = nullptr, *plan_d = nullptr;
     std::vector<Mh2dArgs<float>> a32;
     int grid_ctas = 0;
     bool tuned = false;
@@ -102,7 +106,7 @@ static void build_args(HydroBatch2D *b, std::vector<Mh2dArgs<R>> &av)
         a.ny = g.ny;
         a.g = g.g;
         a.pitch = g.nx + 2 * g.g;
-        a.strip_w = mh2d_threads<R>() - 2;
+        a.strip_w = mh2d_threads<R>() - 2;   /* FP32: work items */
         a.chunk_h = b->opt.chunk_rows > 0 ? b->opt.chunk_rows : 32;
         for (int s = 0; s < 4; s++) a.bc[s] = g.bc[s];
         a.dx = g.dx;
@@ -118,6 +122,90 @@ template <class R>
 static R *snap_field(HydroBatch2D *b, int k, int q)
 {
     return static_cast<R *>(b->slab) + b->off[k] + (18 + q) * b->ncell[k];
+}
+
+/*
+ * FP64: bands of the instances and the groups that share the workspace.
+ * Instances go into a group, in storage order, until its workspace is used up
+ * (an instance that alone needs more is split into bands); the workspace
+ * takes what staged_plan's limit allows, and less where the device has no
+ * room.
+ */
+static int staged_setup(HydroBatch2D *b, HydroRunOutcome *oc)
+{
+    std::vector<StagedBatchBand> bands;
+    std::vector<int> group_of;
+    size_t budget = kStagedWorkspaceBytes, most = 0;
+    for (;;) {
+        bands.clear();
+        group_of.clear();
+        std::vector<size_t> off;
+        size_t used = 0;
+        int group = 0;
+        bool rows_left = false;
+        most = 0;
+        for (int k = 0; k < b->n; k++) {
+            std::vector<Mh2dBand> own;
+            size_t bytes = 0;
+            staged_plan(b->a64[k], budget, own, bytes);
+            rows_left = rows_left || own[0].r1 - own[0].r0 > 1;
+            for (const Mh2dBand &w : own) {
+                if (used > 0 && used + bytes > budget) {
+                    used = 0;
+                    group++;
+                }
+                StagedBatchBand e{};
+                e.band = w;
+                e.inst = k;
+                bands.push_back(e);
+                off.push_back(used);
+                group_of.push_back(group);
+                used += bytes;
+                most = std::max(most, used);
+            }
+        }
+        const cudaError_t e = cudaMalloc(&b->ws, most);
+        if (e == cudaSuccess) {
+            for (size_t i = 0; i < bands.size(); i++)
+                bands[i].band.ws = reinterpret_cast<double *>(static_cast<char *>(b->ws) + off[i]);
+            break;
+        }
+        if (e != cudaErrorMemoryAllocation || !rows_left) BK(e, "cudaMalloc(workspace)");
+        cudaGetLastError();
+        b->ws = nullptr;
+        budget = most / 2;
+    }
+    std::vector<int> map[3];
+    const int ng = group_of.back() + 1;
+    std::vector<size_t> start[3];
+    b->groups.assign(ng, StagedBatchGroup());
+    for (int s = 0; s < 3; s++) start[s].assign(ng, 0);
+    for (size_t i = 0; i < bands.size(); i++) {
+        StagedBatchGroup &g = b->groups[group_of[i]];
+        if (i == 0 || group_of[i] != group_of[i - 1])
+            for (int s = 0; s < 3; s++) start[s][group_of[i]] = map[s].size();
+        unsigned blocks[3];
+        staged_band_blocks(b->a64[bands[i].inst], bands[i].band, blocks);
+        for (int s = 0; s < 3; s++) {
+            bands[i].first[s] = g.blocks[s];
+            g.blocks[s] += blocks[s];
+            map[s].insert(map[s].end(), blocks[s], (int) i);
+        }
+        bands[i].update_grid = blocks[2];
+    }
+    const size_t band_bytes = bands.size() * sizeof(StagedBatchBand);
+    const size_t ints = map[0].size() + map[1].size() + map[2].size();
+    BK(cudaMalloc(&b->plan_d, band_bytes + ints * sizeof(int)), "cudaMalloc(plan)");
+    BK(cudaMemcpy(b->plan_d, bands.data(), band_bytes, cudaMemcpyHostToDevice), "H2D plan");
+    int *p = reinterpret_cast<int *>(static_cast<char *>(b->plan_d) + band_bytes);
+    for (int s = 0; s < 3; s++) {
+        BK(cudaMemcpy(p, map[s].data(), map[s].size() * sizeof(int), cudaMemcpyHostToDevice), "H2D plan");
+        for (int g = 0; g < ng; g++) b->groups[g].map[s] = p + start[s][g];
+        p += map[s].size();
+    }
+    b->staged.inst = static_cast<const Mh2dArgs<double> *>(b->args_d);
+    b->staged.bands = static_cast<const StagedBatchBand *>(b->plan_d);
+    return 0;
 }
 
 extern "C" int hydro_batch2d_create(const HydroGrid2D *grids, int n, const HydroGpuOptions *opt,
@@ -174,7 +262,7 @@ extern "C" int hydro_batch2d_create(const HydroGrid2D *grids, int n, const Hydro
         b->off[k] = total;
         total += 22 * b->ncell[k];
         max_cells = std::max(max_cells, b->ncell[k]);
-        const int nt = mh2d_threads_for(b->fp32);
+        const int nt = mh2d_threads<float>();
         const int items = ((g.nx + nt - 3) / (nt - 2)) * ((g.ny + chunk_h - 1) / chunk_h);
         b->item_off[k + 1] = b->item_off[k] + items;
     }
@@ -207,7 +295,7 @@ extern "C" int hydro_batch2d_create(const HydroGrid2D *grids, int n, const Hydro
     } else {
         build_args<double>(b, b->a64);
         BK(cudaMalloc(&b->args_d, n * sizeof(Mh2dArgs<double>)), "cudaMalloc(args)");
-        b->grid_ctas = mh2d_resident_ctas<double>(b->limiter, b->first_order, b->device);
+        if (staged_setup(b, oc)) return -1;
     }
     if (b->grid_ctas <= 0 || b->grid_ctas > b->item_off[n]) b->grid_ctas = b->item_off[n];
     BK(cudaStreamSynchronize(b->stream), "batch create");
@@ -304,35 +392,25 @@ static cudaError_t launch_batch(HydroBatch2D *b)
         a.bctrl = b->bctrl_d;
         return mh2d_launch_batch_step<float>(a, b->limiter, b->first_order, b->grid_ctas, b->stream);
     }
-    Mh2dBatchArgs<double> a;
-    a.inst = static_cast<const Mh2dArgs<double> *>(b->args_d);
-    a.item_off = b->item_off_d;
-    a.n_inst = b->n;
-    a.total_items = b->item_off[b->n];
-    a.bctrl = b->bctrl_d;
-    return mh2d_launch_batch_step<double>(a, b->limiter, b->first_order, b->grid_ctas, b->stream);
+    return staged_launch_batch(b->staged, b->groups, b->limiter, b->first_order, b->stream);
 }
 
-/* Rows per work item for every instance: item table and arguments. */
+/* Kernels that launch_batch launches. */
+static int launches_per_step(const HydroBatch2D *b) { return b->fp32 ? 1 : 3 * (int) b->groups.size(); }
+
+/* FP32: rows per work item for every instance: item table and arguments. */
 static int set_chunk(HydroBatch2D *b, int chunk, int ctas, HydroRunOutcome *oc)
 {
     b->item_off[0] = 0;
     for (int k = 0; k < b->n; k++) {
-        const int nx = b->fp32 ? b->a32[k].nx : b->a64[k].nx;
-        const int ny = b->fp32 ? b->a32[k].ny : b->a64[k].ny;
-        const int nt = mh2d_threads_for(b->fp32);
+        const int nx = b->a32[k].nx, ny = b->a32[k].ny, nt = mh2d_threads<float>();
         b->item_off[k + 1] = b->item_off[k] + ((nx + nt - 3) / (nt - 2)) * ((ny + chunk - 1) / chunk);
-        if (b->fp32) b->a32[k].chunk_h = chunk;
-        else b->a64[k].chunk_h = chunk;
+        b->a32[k].chunk_h = chunk;
     }
     BK(cudaMemcpyAsync(b->item_off_d, b->item_off.data(), (b->n + 1) * sizeof(int), cudaMemcpyHostToDevice,
                        b->stream), "H2D items");
-    if (b->fp32)
-        BK(cudaMemcpyAsync(b->args_d, b->a32.data(), b->n * sizeof(Mh2dArgs<float>), cudaMemcpyHostToDevice,
-                           b->stream), "H2D args");
-    else
-        BK(cudaMemcpyAsync(b->args_d, b->a64.data(), b->n * sizeof(Mh2dArgs<double>), cudaMemcpyHostToDevice,
-                           b->stream), "H2D args");
+    BK(cudaMemcpyAsync(b->args_d, b->a32.data(), b->n * sizeof(Mh2dArgs<float>), cudaMemcpyHostToDevice,
+                       b->stream), "H2D args");
     b->grid_ctas = std::min(ctas, b->item_off[b->n]);
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -344,12 +422,11 @@ static int set_chunk(HydroBatch2D *b, int chunk, int ctas, HydroRunOutcome *oc)
 
 static int batch_prepare_all(HydroBatch2D *b, double tf, int64 max_steps, HydroRunOutcome *oc);
 
-/* Time candidate (rows per item, persistent CTAs) pairs on the batch's own
+/* FP32: time candidate (rows per item, persistent CTAs) pairs on the batch's own
  * initial state, keep the fastest, rewind (see runtime2d.cu). */
 static int batch_autotune(HydroBatch2D *b, HydroRunOutcome *oc)
 {
-    int resident = b->fp32 ? mh2d_resident_ctas<float>(b->limiter, b->first_order, b->device)
-                           : mh2d_resident_ctas<double>(b->limiter, b->first_order, b->device);
+    int resident = mh2d_resident_ctas<float>(b->limiter, b->first_order, b->device);
     if (resident <= 0) resident = b->grid_ctas;
     const int chunks[] = { 8, 16, 32, 64 };
     int best_chunk = 32, best_ctas = resident;
@@ -395,6 +472,8 @@ static int batch_prepare_all(HydroBatch2D *b, double tf, int64 max_steps, HydroR
         for (auto &a : b->a32) BK(mh2d_launch_prepare<float>(a, b->stream), "prepare kernel");
     } else {
         for (auto &a : b->a64) BK(mh2d_launch_prepare<double>(a, b->stream), "prepare kernel");
+        BK(staged_launch_batch_arm(b->staged, b->n, b->stream), "dt kernel");
+        b->launches++;
     }
     b->launches += b->n;
     BK(cudaStreamSynchronize(b->stream), "prepare");
@@ -417,7 +496,7 @@ extern "C" int hydro_batch2d_begin(HydroBatch2D *b, const HydroStepParams *sp, d
         BK(cudaMemcpyAsync(b->args_d, b->a64.data(), b->n * sizeof(Mh2dArgs<double>), cudaMemcpyHostToDevice,
                            b->stream), "H2D args");
     }
-    if (b->opt.autotune && !b->tuned) {
+    if (b->opt.autotune && b->fp32 && !b->tuned) {
         if (batch_autotune(b, oc)) return -1;
         b->tuned = true;
     }
@@ -436,6 +515,11 @@ extern "C" int hydro_batch2d_set_limits(HydroBatch2D *b, double tf, int64 max_st
         c.active = active(c);
     }
     if (push(b, oc)) return -1;
+    if (!b->fp32) {
+        /* the next dt is clipped to the stopping time */
+        BK(staged_launch_batch_arm(b->staged, b->n, b->stream), "dt kernel");
+        b->launches++;
+    }
     BK(cudaStreamSynchronize(b->stream), "set limits");
     return 0;
 }
@@ -482,11 +566,11 @@ extern "C" int hydro_batch2d_advance(HydroBatch2D *b, HydroRunOutcome *oc, doubl
             if (b->graph && k >= kGraphSteps) {
                 BK(cudaGraphLaunch(b->graph, b->stream), "graph launch");
                 k -= kGraphSteps;
-                b->launches += kGraphSteps;
+                b->launches += kGraphSteps * launches_per_step(b);
             } else {
                 BK(launch_batch(b), "batch step kernel");
                 k -= 1;
-                b->launches += 1;
+                b->launches += launches_per_step(b);
             }
         }
         BK(cudaEventRecord(b->ev[1], b->stream), "cudaEventRecord");
@@ -584,6 +668,8 @@ extern "C" void hydro_batch2d_destroy(HydroBatch2D *b)
     cudaFree(b->bctrl_d);
     cudaFree(b->item_off_d);
     cudaFree(b->args_d);
+    cudaFree(b->ws);
+    cudaFree(b->plan_d);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }

@@ -59,3 +59,34 @@ def test_two_bands(gpu_available, oracle_mod):
                             "van_leer", 3, smooth=True)
     gpu, ref = run_gpu(p), O.load("oracle").run_2d(p)
     assert_parity(p, gpu, ref)
+
+
+def _batch_equals_single(probs, steps):
+    import hydrofv_gb300 as H
+    with H.Batch2D(probs) as b:
+        st, _ = b.advance(steps)
+        outs = b.download()
+    for p, (W, U), s in zip(probs, outs, st):
+        r = run_gpu(p)
+        assert r.code == 0 and s == (r.num_steps, r.t, r.dt)
+        assert np.array_equal(U, r.U, equal_nan=True) and np.array_equal(W, r.W, equal_nan=True)
+
+
+@pytest.mark.parametrize("integrator", ["muscl_hancock_2d", "godunov_first_order_2d"])
+def test_batch_equals_single_grids(gpu_available, oracle_mod, integrator):
+    """Instances of one to many blocks in the batch's launches against the
+    single grids (the many-step kernel and the three launches)."""
+    O = oracle_mod
+    probs = [O.random_problem_2d(nx, ny, 7 + nx, ("reflective", "transmissive", "none", "reflective"), "van_leer", 9,
+                                 smooth=True, integrator=integrator) for nx, ny in [(2, 3), (9, 11), (400, 300), (65, 130)]]
+    for p in probs:
+        p.cfl = 0.5
+    _batch_equals_single(probs, 9)
+
+
+def test_batch_groups(gpu_available, oracle_mod):
+    """Three instances of 0.44 GB of workspace each: two share the 1 GB, the
+    third is stepped by launches of its own."""
+    O = oracle_mod
+    probs = [O.random_problem_2d(2000, 1700, k, ("periodic",) * 4, "minmod", 3, smooth=True) for k in range(3)]
+    _batch_equals_single(probs, 3)
