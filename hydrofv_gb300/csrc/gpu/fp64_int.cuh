@@ -360,6 +360,32 @@ FXHD double dv(double a, double b)
 #endif
 }
 
+/* The same with the integer form inlined, for kernels with few divides: the
+ * staged step's recon and update kernels and the flux kernel's classification
+ * (2048^2 2.274 -> 2.243 ms per step; with the flux kernel's finish inlined
+ * too it is 2.31 - 2.34). */
+FXHD double dvi(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+    bool ok;
+    const double q = fx::div_fast(a, b, ok);
+    return ok ? q : fx::div_hw(a, b);
+#else
+    return a / b;
+#endif
+}
+
+FXHD double sqi(double x)
+{
+#if defined(__CUDA_ARCH__)
+    bool ok;
+    const double r = fx::sqrt_fast(x, ok);
+    return ok ? r : fx::sqrt_hw(x);
+#else
+    return sqrt(x);
+#endif
+}
+
 FXHD double sq(double x)
 {
 #if defined(__CUDA_ARCH__)

@@ -141,7 +141,7 @@ __device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh
         for (int q = 0; q < 4; q++) s[q] = slope<LIM>(f, f.sub(w[q], wm[q]), f.sub(wp[q], w[q]));
         const double h = y ? dtA[1] : dtA[0];
         const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
-        predict(f, h, dv(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
+        predict(f, h, dvi(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
     }
     double *o = b.ws + (long long) (r - b.r0 + 1) * a.pitch + c + (y ? WS_YLO : WS_XLO) * b.plane;
 #pragma unroll
@@ -276,7 +276,7 @@ __device__ __forceinline__ void staged_update(const Fm &f, const Mh2dArgs<double
     for (int q = 0; q < 4; q++) Uout[q][idx] = Un[q];
     double w[4];
     to_primitive(f, a.gas, a.vol, Un[0], Un[1], Un[2], Un[3], w);
-    const double as = sq(dv(f.mul(a.gas.gamma, w[3]), w[0]));
+    const double as = sqi(dvi(f.mul(a.gas.gamma, w[3]), w[0]));
 #pragma unroll
     for (int q = 0; q < 4; q++) Wout[q][idx] = w[q];
     Wout[4][idx] = as;

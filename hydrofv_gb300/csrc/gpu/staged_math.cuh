@@ -183,8 +183,8 @@ FXHD int face_classify(const Fm &f, const GasConst<double> &c, double rho_L, dou
 {
     plain = fx::moderate(rho_L) && fx::moderate(rho_R) && fx::moderate(p_L) && fx::moderate(p_R);
     if (!plain) return classify_slow(c, rho_L, u_L, p_L, rho_R, u_R, p_R, a_L, a_R, ppv);
-    a_L = sq(dv(f.mul(c.gamma, p_L), rho_L));
-    a_R = sq(dv(f.mul(c.gamma, p_R), rho_R));
+    a_L = sqi(dvi(f.mul(c.gamma, p_L), rho_L));
+    a_R = sqi(dvi(f.mul(c.gamma, p_R), rho_R));
     const double as = f.add(a_L, a_R), du = f.sub(u_R, u_L);
     /* 2 (a_L + a_R) / (gamma + 1) lies in [2^(d-1), 2^(d+1)] (quot_le_fast):
      * a negative u_R - u_L, or one below 2^(d-1), is not above it */
@@ -287,11 +287,11 @@ FXHD void to_primitive(const Fm &f, const GasConst<double> &c, double vol, doubl
         to_primitive_slow(c, vol, m, mx, my, E, w);
         return;
     }
-    w[0] = dv(m, vol);
-    w[1] = dv(mx, m);
-    w[2] = dv(my, m);
+    w[0] = dvi(m, vol);
+    w[1] = dvi(mx, m);
+    w[2] = dvi(my, m);
     const double ke = f.mul(fx::halve(m), f.add(f.mul(w[1], w[1]), f.mul(w[2], w[2])));
-    w[3] = dv(f.mul(c.gm1, f.sub(E, ke)), vol);
+    w[3] = dvi(f.mul(c.gm1, f.sub(E, ke)), vol);
 }
 
 }  // namespace hydro
