@@ -1156,7 +1156,7 @@ extern "C" int hydro_adj2d_forward(HydroAdj2D *a, double *const W[4], double *co
     Mh2dArgs<double> args = a->pargs;
     for (int i = 0; i < 5; i++) args.W[0][i] = a->ckpt[0].W[i];
     CK(mh2d_launch_prepare<double>(args, a->stream), "prepare kernel");
-    CK(staged_launch_arm(args, a->stream), "dt kernel");
+    CK(mh2d_launch_arm<double>(args, a->stream), "dt kernel");
     a->launches += 2;
     CK(cudaMemcpyAsync(&a->ckpt_ctrl_d[0], a->ctrl_d, sizeof *c, cudaMemcpyDeviceToDevice, a->stream), "D2D control");
     const StateP<double> *in = &a->ckpt[0];

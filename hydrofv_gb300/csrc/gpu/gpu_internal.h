@@ -19,24 +19,58 @@
 namespace hydro {
 
 /*
- * Rows per work item when the caller sets none.  The step's CTAs are
- * persistent (one per resident slot) and take (strip, row chunk) items from
- * a queue, so a last partial round of items leaves slots idle.  The choice
- * maximises the filled fraction of whole rounds, less the extra y
- * reconstruction an item adds below its first row (about 0.4 of a row's
- * work).  Measured on the FP64 shear layer (608 resident CTAs): 1024^2
- * takes 16 rows (1117 M cell-updates/s against 792 M at 32), 2048^2 takes
- * 12 (1249 M against 1226 M).
+ * Rows per work item of the FP32 step when the caller sets none.  The step's
+ * CTAs are persistent (one per resident slot) and take (strip, row chunk)
+ * items from a queue.  An item of c rows also reconstructs the rows below it
+ * (0.95 of a row's work: 2048^2 takes 317 / 244 / 182 us a step with 1 / 2 /
+ * 12 rows), and the last items run while other slots are already idle.  In
+ * units of a row's work with all slots busy (5.0 us) a step is modelled as
+ *     items (c + 0.95) / slots + 1.2 + 0.24 c,
+ * and as no less than an item alone, 2.1 + 0.48 c.  `items` gives the number
+ * of items for a height.
+ * Measured on 1064 slots, this choice / the best of 1 .. 64 rows / 32 rows, us
+ * a step: 64^2 12.8 (1 row) / 12.8 / 85, 301 x 200 15.2 (1) / 15.2 / 93, 512^2
+ * 26.5 (3) / 26.5 / 94, 700 x 900 44.8 (4) / 40.4 / 100, 1024^2 64.0 (6) / 63.9
+ * / 103, 2048^2 181 (12) / 181 / 212, 4096^2 603 (24) / 594 / 594; 28 grids of
+ * side 128 to 640 258 (12) / 258 / 298, 60 of side 500 to 900 1257 (24) / 1253
+ * / 1253.
+ */
+template <class Items>
+int mh2d_fp32_chunk(int slots, Items items)
+{
+    static const int cand[] = { 1, 2, 3, 4, 6, 8, 12, 16, 20, 24, 32, 40, 48, 64 };
+    if (slots <= 0) return 32;
+    int best = 32;
+    double best_t = 1e300;
+    for (int c : cand) {
+        const double full = (double) items(c) * (c + 0.95) / slots + 1.2 + 0.24 * c, one = 2.1 + 0.48 * c;
+        const double t = full > one ? full : one;
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    return best;
+}
+
+/* Work items of c rows of an nx x ny grid. */
+inline long long mh2d_item_count(int nx, int ny, int strip_w, int c)
+{
+    return (long long) ((nx + strip_w - 1) / strip_w) * ((ny + c - 1) / c);
+}
+
+/*
+ * The single height that the guided plan below starts from: the same model
+ * with the fused FP64 kernel's prologue (0.4 of a row).
  */
 inline int mh2d_default_chunk(int nx, int ny, int strip_w, int slots)
 {
     static const int cand[] = { 8, 12, 16, 20, 24, 32, 40, 48, 64 };
     if (slots <= 0 || strip_w <= 0) return 32;
-    const long long strips = (nx + strip_w - 1) / strip_w;
     int best = 32;
     double best_eff = -1.0;
     for (int c : cand) {
-        const long long items = strips * ((ny + c - 1) / c);
+        const long long items = mh2d_item_count(nx, ny, strip_w, c);
         const long long rounds = (items + slots - 1) / slots;
         const double eff = (double) items / (double) (rounds * slots) * (1.0 - 0.4 / c);
         if (eff > best_eff + 1e-9) {
@@ -173,7 +207,6 @@ cudaError_t staged_alloc(const Mh2dArgs<double> &a, std::vector<Mh2dBand> &bands
     }
 }
 
-cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s);
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
 /* Batches: band `band` of instance `inst`; its blocks of the recon, flux and
  * update launches start at first[0], first[1], first[2] of the group's. */
@@ -199,7 +232,6 @@ struct StagedBatchArgs {
 void staged_band_blocks(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned blocks[3]);
 cudaError_t staged_launch_batch(const StagedBatchArgs &b, const std::vector<StagedBatchGroup> &groups, int limiter,
                                 int first_order, cudaStream_t s);
-cudaError_t staged_launch_batch_arm(const StagedBatchArgs &b, int n, cudaStream_t s);
 
 /* Small grids: blocks of the many-step kernel (0: the grid steps with three
  * launches), and up to `steps` steps in one launch of it. */
@@ -216,6 +248,12 @@ cudaError_t mh2d_launch_batch_step(const Mh2dBatchArgs<R> &b, int limiter, int f
                                    cudaStream_t s);
 template <class R>
 cudaError_t mh2d_launch_prepare(const Mh2dArgs<R> &a, cudaStream_t s);
+/* The first dt after the maxima of the state are known (prepare), and again
+ * when the stopping time moves: one grid, and n instances in device memory. */
+template <class R>
+cudaError_t mh2d_launch_arm(const Mh2dArgs<R> &a, cudaStream_t s);
+template <class R>
+cudaError_t mh2d_launch_batch_arm(const Mh2dArgs<R> *inst, int n, cudaStream_t s);
 template <class R>
 cudaError_t mh2d_launch_materialize(const Mh2dArgs<R> &a, int buf, R *const out[4], cudaStream_t s);
 template <class R>

@@ -12,6 +12,8 @@ namespace hydro {
 template int mh2d_resident_ctas<double>(int, int, int);
 template cudaError_t mh2d_launch_step<double>(const Mh2dArgs<double> &, int, cudaStream_t);
 template cudaError_t mh2d_launch_prepare<double>(const Mh2dArgs<double> &, cudaStream_t);
+template cudaError_t mh2d_launch_arm<double>(const Mh2dArgs<double> &, cudaStream_t);
+template cudaError_t mh2d_launch_batch_arm<double>(const Mh2dArgs<double> *, int, cudaStream_t);
 template cudaError_t mh2d_launch_materialize<double>(const Mh2dArgs<double> &, int,
                                                      double *const[4], cudaStream_t);
 template cudaError_t mh2d_launch_totals<double>(const Mh2dArgs<double> &, int, double *, cudaStream_t);
@@ -67,12 +69,6 @@ void staged_plan(const Mh2dArgs<double> &a, size_t budget, std::vector<Mh2dBand>
     bytes = (size_t) (h + 2) * row;
 }
 
-cudaError_t staged_launch_arm(const Mh2dArgs<double> &a, cudaStream_t s)
-{
-    staged_arm_kernel<<<1, 32, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s)
 {
     const int first_order = a.first_order;
@@ -108,12 +104,6 @@ cudaError_t staged_launch_batch(const StagedBatchArgs &b, const std::vector<Stag
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
-}
-
-cudaError_t staged_launch_batch_arm(const StagedBatchArgs &b, int n, cudaStream_t s)
-{
-    staged_batch_arm_kernel<<<n, 32, 0, s>>>(b);
-    return cudaGetLastError();
 }
 
 unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, int device)

@@ -44,16 +44,17 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include "fast32.cuh"
 #include "numerics.cuh"
 #include "step_control.h"
 
 /* Threads per 2D step CTA (a strip of threads - 2 interior columns) and the
  * CTAs per SM each state precision is compiled for (launch bounds).  FP64:
  * 4 CTAs of 128 threads (128 registers); FP32: 7 CTAs of 128 (72
- * registers).  Measured with the one-pass FP32 face solve (2048^2 shear
- * layer / 8192^2 point blast / 256-grid ensemble, G cell-updates/s): 8 CTAs
- * 15.05 / 27.5 / 20.1, 7 CTAs 15.19 / 28.6 / 21.35, 6 CTAs 15.7 / 27.7 /
- * 20.4. */
+ * registers).  Measured (2048^2 shear layer / 4096^2 point blast / 28 grids of
+ * side 128 to 640, G cell-updates/s): 8 CTAs 23.6 / 29.4 / 17.4, 7 CTAs 23.1 /
+ * 29.4 / 18.6, 6 CTAs 22.0 / 28.3 / 17.8; 10 CTAs of 96 threads 22.9 / 27.7 /
+ * 17.7; 5 of 192 22.9 / 28.5 / 17.0. */
 #ifndef MH2D_THREADS_FP64
 #define MH2D_THREADS_FP64 128
 #endif
@@ -92,6 +93,7 @@ struct Mh2dArgs {
     double gravity;          /* System.gravity (kernels built with GRAV only) */
     R *tape;                 /* adjoint tape of this step (staged flux kernel; null: none) */
     long long tape_plane;    /* elements per tape field (padded cells) */
+    double *dt_log;          /* receives the dt of step n at [n] (null: none) */
 };
 
 /* Work items of one step: (strip, row chunk) pairs, chunk-major, so the
@@ -145,6 +147,35 @@ enum : int {
     TAPE_L = 0, TAPE_R = 4, TAPE_AL = 8, TAPE_AR = 9, TAPE_PG = 10, TAPE_Z0 = 11, TAPE_Z1 = 12,
     TAPE_REG = 13, TAPE_QL = 14, TAPE_QR = 15, TAPE_SS = 16,
 };
+
+/* The dt of step n, which starts at time t with the maxima smax[n % 3], and
+ * in lanes 0 and 1 the ratios dt A / V of the x and y faces
+ * (src/integrator_muscl_hancock.c:533-549, src/utils.c:55-95).  One converged
+ * warp; the two directions' quotients run in two lanes. */
+template <class R>
+__device__ __forceinline__ void next_dt(const Mh2dArgs<R> &a, const HydroStepControl *ctrl, long long n, double t,
+                                        double tf, double &dt, double &dtA)
+{
+    const bool y = threadIdx.x & 1;
+    const double S = from_ordered_bits(*(const volatile unsigned long long *) &ctrl->smax[n % 3][y]);
+    const double q = dv(S, y ? a.dy : a.dx);
+    const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
+    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
+    dt = dv(cfl, qx + qy);
+    if (t + dt > tf) dt = tf - t;
+    dtA = dv(dt * (y ? a.area_y : a.area_x), a.vol);
+}
+
+template <class R>
+__device__ __forceinline__ void arm_dt(const Mh2dArgs<R> &a, HydroStepControl *ctrl, long long n, double t,
+                                       double tf)
+{
+    const int lane = threadIdx.x & 31;
+    double dt, w;
+    next_dt(a, ctrl, n, t, tf, dt, w);
+    if (lane == 0) ctrl->step_dt = dt;
+    if (lane < 2) ctrl->step_dtA[lane] = w;
+}
 
 /* Where W at padded (r, c) comes from: the stored cell (rr, cc), with the
  * sign of u (neg = 1) or v (neg = 2) flipped, or (cons) converted from the
@@ -298,8 +329,9 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
     if constexpr (sizeof(R) == 4) {
         for (int f = tid; f < nF; f += NT) {
             R F[4];
-            const int rc = hllc_flux_2d(gas, sm.FL[0][f], sm.FL[1][f], sm.FL[2][f], sm.FL[3][f],
-                                        sm.FR[0][f], sm.FR[1][f], sm.FR[2][f], sm.FR[3][f], F);
+            const R L[4] = { sm.FL[0][f], sm.FL[1][f], sm.FL[2][f], sm.FL[3][f] };
+            const R Rt[4] = { sm.FR[0][f], sm.FR[1][f], sm.FR[2][f], sm.FR[3][f] };
+            const int rc = fast_flux(gas, L, Rt, F);
             if (rc) err = rc;
 #pragma unroll
             for (int q = 0; q < 4; q++) sm.FL[q][f] = F[q];
@@ -357,6 +389,11 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
     }
 }
 
+template <int LIM>
+__device__ __forceinline__ float step_slope(float a, float b) { return fast_slope<LIM>(a, b); }
+template <int LIM>
+__device__ __forceinline__ double step_slope(double a, double b) { return limit_slope<LIM>(a, b); }
+
 /*
  * Process one work item (one strip of NT-2 columns x one chunk of chunk_h
  * rows) of step n with time step dt.  Shared by the single-grid and the
@@ -364,7 +401,7 @@ __device__ __forceinline__ int solve_faces(Mh2dShared<R, NT> &sm, const GasConst
  */
 template <class R, int LIM, int NT, int FIRST_ORDER, bool GRAV = false>
 __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT> &sm, int item,
-                                          long long n, double dt, double &mx_x, double &mx_y,
+                                          long long n, double dt, const double dtA[2], double &mx_x, double &mx_y,
                                           int &err)
 {
     const R dtr = (R) dt;
@@ -374,9 +411,8 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
         if constexpr (sizeof(R) == 8) return v;
         else return (v * dtr) * area;
     };
-    const R dtA_x = (R) (dt * a.area_x / a.vol);
-    const R dtA_y = (R) (dt * a.area_y / a.vol);
-    const R Ax = (R) a.area_x, Ay = (R) a.area_y;
+    const R dtA_x = (R) dtA[0], dtA_y = (R) dtA[1];
+    const R Ax = (R) a.area_x, Ay = (R) a.area_y, vol = (R) a.vol;
     const int buf = (int) (n & 1);
     const bool raw = (n == 0);
     const R *const *Uin = a.U[buf];
@@ -465,11 +501,11 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
             return;
         }
         R d[4];
-        d[0] = limit_slope<LIM>(rho - sm.ring[sb][0][u], sm.ring[st][0][u] - rho);
-        const R dvx = limit_slope<LIM>(vx - sm.ring[sb][1][u], sm.ring[st][1][u] - vx);
-        d[1] = limit_slope<LIM>(vy - sm.ring[sb][2][u], sm.ring[st][2][u] - vy);
+        d[0] = step_slope<LIM>(rho - sm.ring[sb][0][u], sm.ring[st][0][u] - rho);
+        const R dvx = step_slope<LIM>(vx - sm.ring[sb][1][u], sm.ring[st][1][u] - vx);
+        d[1] = step_slope<LIM>(vy - sm.ring[sb][2][u], sm.ring[st][2][u] - vy);
         d[2] = dvx;
-        d[3] = limit_slope<LIM>(p - sm.ring[sb][3][u], sm.ring[st][3][u] - p);
+        d[3] = step_slope<LIM>(p - sm.ring[sb][3][u], sm.ring[st][3][u] - p);
         hancock_2d(dtA_y, dv(dtA_y, rho), rho, vy, vx, p, as, d, dvx, lo, hi);
     };
 
@@ -483,17 +519,26 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
             return;
         }
         R d[4];
-        d[0] = limit_slope<LIM>(rho - sm.ring[s][0][u - 1], sm.ring[s][0][u + 1] - rho);
-        d[1] = limit_slope<LIM>(vx - sm.ring[s][1][u - 1], sm.ring[s][1][u + 1] - vx);
-        d[2] = limit_slope<LIM>(vy - sm.ring[s][2][u - 1], sm.ring[s][2][u + 1] - vy);
-        d[3] = limit_slope<LIM>(p - sm.ring[s][3][u - 1], sm.ring[s][3][u + 1] - p);
+        d[0] = step_slope<LIM>(rho - sm.ring[s][0][u - 1], sm.ring[s][0][u + 1] - rho);
+        d[1] = step_slope<LIM>(vx - sm.ring[s][1][u - 1], sm.ring[s][1][u + 1] - vx);
+        d[2] = step_slope<LIM>(vy - sm.ring[s][2][u - 1], sm.ring[s][2][u + 1] - vy);
+        d[3] = step_slope<LIM>(p - sm.ring[s][3][u - 1], sm.ring[s][3][u + 1] - p);
         hancock_2d(dtA_x, dv(dtA_x, rho), rho, vx, vy, p, as, d, d[1], lo, hi);
     };
 
     /* ---- prologue: the faces below r_begin ---- */
-    load_row(r_begin - 2);
-    load_row(r_begin - 1);
-    load_row(r_begin);
+    if constexpr (RING == 4) {
+        /* all four rows in flight together: one memory latency */
+        load_row_async(r_begin - 2);
+        load_row_async(r_begin - 1);
+        load_row_async(r_begin);
+        load_row_async(r_begin + 1);
+        cp_async_wait<0>();
+    } else {
+        load_row(r_begin - 2);
+        load_row(r_begin - 1);
+        load_row(r_begin);
+    }
     __syncthreads();
     /* What a thread carries up its column from row to row: ytop, the low
      * state of the y face above its cell (from the reconstruction one row
@@ -513,16 +558,17 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
     R tmp_lo[4], prev_hi[4];
     if (inner) recon_y(r_begin - 1, tmp_lo, prev_hi);
     __syncthreads();
-    load_row(r_begin + 1);
     if constexpr (RING == 4) load_row_async(r_begin + 2);
-    if (tid == 0) { sm.nT = 0; sm.nS = 0; }
-    __syncthreads();
+    else load_row(r_begin + 1);
+    if constexpr (!YREG) {
+        if (tid == 0) { sm.nT = 0; sm.nS = 0; }
+        __syncthreads();
+    }
     if constexpr (YREG) {
         /* FP32: the face below the chunk is solved by its column's thread */
         if (inner) {
             recon_y(r_begin, tmp_lo, ytop);
-            const int rc = hllc_flux_2d(a.gas, prev_hi[0], prev_hi[1], prev_hi[2], prev_hi[3],
-                                        tmp_lo[0], tmp_lo[1], tmp_lo[2], tmp_lo[3], gbot);
+            const int rc = fast_flux(a.gas, prev_hi, tmp_lo, gbot);
             if (rc) err = rc;
         }
         __syncthreads();
@@ -590,8 +636,7 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
              * state from the cell above, whose own high state is carried to
              * the next row (FP64: now; FP32: after the update) */
             if constexpr (YREG) {
-                const int rc = hllc_flux_2d(a.gas, ytop[0], ytop[1], ytop[2], ytop[3],
-                                            nlo[0], nlo[1], nlo[2], nlo[3], gy);
+                const int rc = fast_flux(a.gas, ytop, nlo, gy);
                 if (rc) err = rc;
             } else {
                 const int f = nX + tid - 1;
@@ -658,12 +703,16 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
 #pragma unroll
                 for (int q = 0; q < 4; q++) Uout[q][idx] = Un[q];
             }
-            R w[4];
-            cons_to_prim_2d_guarded(a.gas, (R) a.vol, Un[0], Un[1], Un[2], Un[3], w);
-            const R as = sound_speed(a.gas, w[0], w[3]);
+            R w[5];
+            if constexpr (sizeof(R) == 4) {
+                fast_primitive(a.gas, vol, Un[0], Un[1], Un[2], Un[3], w);
+            } else {
+                cons_to_prim_2d(a.gas, vol, Un[0], Un[1], Un[2], Un[3], w);
+                w[4] = sound_speed(a.gas, w[0], w[3]);
+            }
+            const R as = w[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) Wout[q][idx] = w[q];
-            Wout[4][idx] = as;
+            for (int q = 0; q < 5; q++) Wout[q][idx] = w[q];
             const R sx = as + fabs(w[1]);
             const R sy = as + fabs(w[2]);
             if constexpr (sizeof(R) == 4) {
@@ -720,6 +769,40 @@ __device__ __forceinline__ void mh2d_item(const Mh2dArgs<R> &a, Mh2dShared<R, NT
     }
 }
 
+/* End of step n (time t, dt): the clock, the stop flags and the next dt.  One
+ * converged warp, after every block's maxima and errors are visible. */
+template <class R>
+__device__ __forceinline__ void advance_clock(const Mh2dArgs<R> &a, HydroStepControl *ctrl, long long n, double t, double tf,
+                                              double dt)
+{
+    volatile HydroStepControl *vc = ctrl;
+    const bool failed = vc->error_code != 0;
+    const double tn = t + dt;
+    const long long nn = n + 1, most = vc->max_steps;
+    const int stored = vc->store_count;
+    if (!failed) arm_dt(a, ctrl, nn, tn, tf);
+    __syncwarp();
+    if ((threadIdx.x & 31) != 0) return;
+    ctrl->dt = dt;
+    ctrl->blocks_done = 0;
+    if (failed) {
+        ctrl->active = 0;
+        return;
+    }
+    if (a.dt_log) a.dt_log[n] = dt;
+    ctrl->t = tn;
+    ctrl->num_steps = nn;
+    const int nn2 = (int) ((n + 2) % 3);
+    ctrl->smax[nn2][0] = ordered_bits(-CUDART_INF);
+    ctrl->smax[nn2][1] = ordered_bits(-CUDART_INF);
+    int act = (tn < tf) && (most < 0 || nn < most);
+    if (a.sp.is_storing && tn >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
+        ctrl->snapshot_due = 1;
+        act = 0;
+    }
+    ctrl->active = act;
+}
+
 /*
  * One time step of one grid.  The grid is persistent: each CTA takes
  * (strip, row chunk) items from a device counter until none are left, so
@@ -734,15 +817,9 @@ mh2d_step_kernel(const Mh2dArgs<R> a)
     HydroStepControl *ctrl = a.ctrl;
     if (!*(volatile int *) &ctrl->active) return;
 
-    /* ---- dt for this step (src/integrator_muscl_hancock.c:533-549) ---- */
     const long long n = ctrl->num_steps;
-    const double t_now = ctrl->t;
-    const double Sx = from_ordered_bits(ctrl->smax[n % 3][0]);
-    const double Sy = from_ordered_bits(ctrl->smax[n % 3][1]);
-    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
-    double dt = cfl / (Sx / a.dx + Sy / a.dy);
-    const double tf = ctrl->tf;
-    if (t_now + dt > tf) dt = tf - t_now;
+    const double t_now = ctrl->t, tf = ctrl->tf, dt = ctrl->step_dt;
+    const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
     if (dt == 0.0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             ctrl->dt = dt;
@@ -764,7 +841,7 @@ mh2d_step_kernel(const Mh2dArgs<R> a)
         const int item = sm.item;
         __syncthreads();
         if (item >= n_items) break;
-        mh2d_item<R, LIM, NT, FIRST_ORDER, GRAV>(a, sm, item, n, dt, mx_x, mx_y, err);
+        mh2d_item<R, LIM, NT, FIRST_ORDER, GRAV>(a, sm, item, n, dt, dtA, mx_x, mx_y, err);
     }
 
     if (err) record_error(ctrl, err, (int) blockIdx.x);
@@ -796,32 +873,12 @@ mh2d_step_kernel(const Mh2dArgs<R> a)
     }
     __syncthreads();
 
-    /* ---- last CTA: advance the clock (src/integrator_muscl_hancock.c:1143-1154) ---- */
-    if (sm.am_last && tid == 0) {
+    /* ---- last CTA: advance the clock (src/integrator_muscl_hancock.c:1143-1154)
+     * and form the next dt ---- */
+    if (sm.am_last && tid < 32) {
         __threadfence();
-        volatile HydroStepControl *vc = ctrl;
-        ctrl->dt = dt;
-        ctrl->work_next = 0;
-        if (vc->error_code != 0) {
-            ctrl->active = 0;
-        } else {
-            const double tn = t_now + dt;
-            const long long nn = n + 1;
-            ctrl->t = tn;
-            ctrl->num_steps = nn;
-            const int nn2 = (int) ((n + 2) % 3);
-            ctrl->smax[nn2][0] = ordered_bits(-CUDART_INF);
-            ctrl->smax[nn2][1] = ordered_bits(-CUDART_INF);
-            int act = (tn < tf) && (vc->max_steps < 0 || nn < vc->max_steps);
-            if (a.sp.is_storing &&
-                tn >= a.sp.storing_interval *
-                          (double) (vc->store_count - a.sp.store_initial_offset + 1)) {
-                ctrl->snapshot_due = 1;
-                act = 0;
-            }
-            ctrl->active = act;
-        }
-        ctrl->blocks_done = 0;
+        if (tid == 0) ctrl->work_next = 0;
+        advance_clock(a, ctrl, n, t_now, tf, dt);
     }
 }
 
@@ -844,57 +901,6 @@ struct Mh2dBatchArgs {
     HydroBatchControl *bctrl;
 };
 
-/* dt of instance `a` for its current step, or 0 when it must not step
- * (inactive; on dt == 0 the error is recorded as the single-grid kernel does). */
-template <class R>
-__device__ double instance_dt(const Mh2dArgs<R> &a, long long &n)
-{
-    HydroStepControl *ctrl = a.ctrl;
-    if (!*(volatile int *) &ctrl->active) return 0.0;
-    n = ctrl->num_steps;
-    const double t_now = ctrl->t;
-    const double Sx = from_ordered_bits(ctrl->smax[n % 3][0]);
-    const double Sy = from_ordered_bits(ctrl->smax[n % 3][1]);
-    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
-    double dt = cfl / (Sx / a.dx + Sy / a.dy);
-    const double tf = ctrl->tf;
-    if (t_now + dt > tf) dt = tf - t_now;
-    if (dt == 0.0) {
-        ctrl->dt = dt;
-        record_error(ctrl, DEV_ERR_DT_ZERO, -1);
-        ctrl->active = 0;
-    }
-    return dt;
-}
-
-/* Clock advance of one instance by the last of its items (the single-grid
- * kernel's last-CTA block, per instance). */
-__device__ __forceinline__ void instance_bookkeeping(HydroStepControl *ctrl, const HydroStepParams &sp,
-                                                     long long n, double dt)
-{
-    volatile HydroStepControl *vc = ctrl;
-    ctrl->dt = dt;
-    if (vc->error_code != 0) {
-        ctrl->active = 0;
-    } else {
-        const double tn = vc->t + dt;
-        const long long nn = n + 1;
-        ctrl->t = tn;
-        ctrl->num_steps = nn;
-        const int nn2 = (int) ((n + 2) % 3);
-        ctrl->smax[nn2][0] = ordered_bits(-CUDART_INF);
-        ctrl->smax[nn2][1] = ordered_bits(-CUDART_INF);
-        int act = (tn < vc->tf) && (vc->max_steps < 0 || nn < vc->max_steps);
-        if (sp.is_storing &&
-            tn >= sp.storing_interval * (double) (vc->store_count - sp.store_initial_offset + 1)) {
-            ctrl->snapshot_due = 1;
-            act = 0;
-        }
-        ctrl->active = act;
-    }
-    ctrl->blocks_done = 0;
-}
-
 /*
  * One time step of every active instance of a batch.  Persistent CTAs take
  * global items from one queue; an item belongs to one instance (found by
@@ -912,7 +918,7 @@ mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
     __shared__ Mh2dShared<R, NT> sm;
     __shared__ int s_inst, s_local, s_go, s_last;
     __shared__ long long s_n;
-    __shared__ double s_dt;
+    __shared__ double s_dt, s_dtA[2];
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) {
@@ -928,24 +934,32 @@ mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
                 }
                 s_inst = lo;
                 s_local = gi - b.item_off[lo];
-                long long n = 0;
-                const double dt = instance_dt(b.inst[lo], n);
-                s_dt = dt;
-                s_n = n;
-                s_go = (dt != 0.0);
+                HydroStepControl *ctrl = b.inst[lo].ctrl;
+                if (*(volatile int *) &ctrl->active) {
+                    s_n = ctrl->num_steps;
+                    s_dt = ctrl->step_dt;
+                    s_dtA[0] = ctrl->step_dtA[0];
+                    s_dtA[1] = ctrl->step_dtA[1];
+                    s_go = (s_dt != 0.0);
+                    if (!s_go) {
+                        ctrl->dt = 0.0;
+                        record_error(ctrl, DEV_ERR_DT_ZERO, -1);
+                        ctrl->active = 0;
+                    }
+                }
             }
         }
         __syncthreads();
         if (sm.item >= b.total_items) break;
         const int go = s_go, inst = s_inst, local = s_local;
         const long long n = s_n;
-        const double dt = s_dt;
+        const double dt = s_dt, dtA[2] = { s_dtA[0], s_dtA[1] };
         __syncthreads();
         if (!go) continue;
         const Mh2dArgs<R> &a = b.inst[inst];
         double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
         int err = DEV_OK;
-        mh2d_item<R, LIM, NT, FIRST_ORDER>(a, sm, local, n, dt, mx_x, mx_y, err);
+        mh2d_item<R, LIM, NT, FIRST_ORDER>(a, sm, local, n, dt, dtA, mx_x, mx_y, err);
         if (err) record_error(a.ctrl, err, inst);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -972,10 +986,12 @@ mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
             __threadfence();
             const int n_items = b.item_off[inst + 1] - b.item_off[inst];
             s_last = (atomicAdd(&ctrl->blocks_done, 1u) == (unsigned) (n_items - 1));
-            if (s_last) {
-                __threadfence();
-                instance_bookkeeping(ctrl, a.sp, n, dt);
-            }
+        }
+        __syncthreads();
+        if (s_last && tid < 32) {
+            __threadfence();
+            volatile HydroStepControl *vc = a.ctrl;
+            advance_clock(a, a.ctrl, n, vc->t, vc->tf, dt);
         }
         __syncthreads();
     }
@@ -986,6 +1002,23 @@ mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
             b.bctrl->ctas_done = 0;
         }
     }
+}
+
+/* The first step's dt after the maxima of the state are known, and again
+ * when the stopping time moves. */
+template <class R>
+__global__ void mh2d_arm_kernel(const Mh2dArgs<R> a)
+{
+    const HydroStepControl *c = a.ctrl;
+    arm_dt(a, a.ctrl, c->num_steps, c->t, c->tf);
+}
+
+/* The same for every instance of a batch. */
+template <class R>
+__global__ void mh2d_batch_arm_kernel(const Mh2dArgs<R> *inst)
+{
+    const Mh2dArgs<R> &a = inst[blockIdx.x];
+    arm_dt(a, a.ctrl, a.ctrl->num_steps, a.ctrl->t, a.ctrl->tf);
 }
 
 }  // namespace hydro

@@ -164,6 +164,20 @@ cudaError_t mh2d_launch_prepare(const Mh2dArgs<R> &a, cudaStream_t s)
 }
 
 template <class R>
+cudaError_t mh2d_launch_arm(const Mh2dArgs<R> &a, cudaStream_t s)
+{
+    mh2d_arm_kernel<R><<<1, 32, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+template <class R>
+cudaError_t mh2d_launch_batch_arm(const Mh2dArgs<R> *inst, int n, cudaStream_t s)
+{
+    mh2d_batch_arm_kernel<R><<<n, 32, 0, s>>>(inst);
+    return cudaGetLastError();
+}
+
+template <class R>
 cudaError_t mh2d_launch_convert_all(const Mh2dArgs<R> &a, int buf, R *const out[4], cudaStream_t s)
 {
     mh2d_convert_all_kernel<R><<<1024, 256, 0, s>>>(a, buf, out[0], out[1], out[2], out[3]);

@@ -77,33 +77,6 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-/* The dt of step n, which starts at time t with the maxima smax[n % 3], and
- * in lanes 0 and 1 the ratios dt A / V of the x and y faces
- * (src/integrator_muscl_hancock.c:533-549, src/utils.c:55-95).  One converged
- * warp; the two directions' quotients run in two lanes. */
-__device__ __forceinline__ void next_dt(const Mh2dArgs<double> &a, const HydroStepControl *ctrl, long long n, double t,
-                                        double tf, double &dt, double &dtA)
-{
-    const bool y = threadIdx.x & 1;
-    const double S = from_ordered_bits(*(const volatile unsigned long long *) &ctrl->smax[n % 3][y]);
-    const double q = dv(S, y ? a.dy : a.dx);
-    const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
-    const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
-    dt = dv(cfl, qx + qy);
-    if (t + dt > tf) dt = tf - t;
-    dtA = dv(dt * (y ? a.area_y : a.area_x), a.vol);
-}
-
-__device__ __forceinline__ void arm_dt(const Mh2dArgs<double> &a, HydroStepControl *ctrl, long long n, double t,
-                                       double tf)
-{
-    const int lane = threadIdx.x & 31;
-    double dt, w;
-    next_dt(a, ctrl, n, t, tf, dt, w);
-    if (lane == 0) ctrl->step_dt = dt;
-    if (lane < 2) ctrl->step_dtA[lane] = w;
-}
-
 /* Face states of item k of the band: first the x items (rows r0 .. r1-1,
  * columns g-1 .. g+nx), then the y items (rows r0-1 .. r1, columns g ..
  * g+nx-1). */
@@ -352,31 +325,7 @@ __device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateS
     __syncthreads();
     if (!sm.am_last || tid >= 32) return;
     __threadfence();
-    volatile HydroStepControl *vc = ctrl;
-    const bool failed = vc->error_code != 0;
-    const double tn = vc->t + dt, tf = vc->tf;
-    const long long nn = n + 1, most = vc->max_steps;
-    const int stored = vc->store_count;
-    if (!failed) arm_dt(a, ctrl, nn, tn, tf);
-    __syncwarp();
-    if (tid != 0) return;
-    ctrl->dt = dt;
-    ctrl->blocks_done = 0;
-    if (failed) {
-        ctrl->active = 0;
-        return;
-    }
-    ctrl->t = tn;
-    ctrl->num_steps = nn;
-    const int nn2 = (int) ((n + 2) % 3);
-    ctrl->smax[nn2][0] = ordered_bits(-CUDART_INF);
-    ctrl->smax[nn2][1] = ordered_bits(-CUDART_INF);
-    int act = (tn < tf) && (most < 0 || nn < most);
-    if (a.sp.is_storing && tn >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
-        ctrl->snapshot_due = 1;
-        act = 0;
-    }
-    ctrl->active = act;
+    advance_clock(a, ctrl, n, ((volatile HydroStepControl *) ctrl)->t, ((volatile HydroStepControl *) ctrl)->tf, dt);
 }
 
 /* The step's n and dt, or false when nothing is to be done (not active, or
@@ -524,12 +473,6 @@ staged_batch_update_kernel(const StagedBatchArgs g, const int *map)
     staged_finish(sm.a, us, sm.b.band.update_blocks, sm.n, sm.dt, mx_x, mx_y);
 }
 
-static __global__ void staged_batch_arm_kernel(const StagedBatchArgs g)
-{
-    const Mh2dArgs<double> &a = g.inst[blockIdx.x];
-    arm_dt(a, a.ctrl, a.ctrl->num_steps, a.ctrl->t, a.ctrl->tf);
-}
-
 /* ------------------------------------------------ small grids: many steps */
 
 /*
@@ -638,6 +581,7 @@ staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
             act = false;
         }
         if (leader) {
+            if (a.dt_log) a.dt_log[n - 1] = dt;
             ctrl->dt = dt;
             ctrl->t = t;
             ctrl->num_steps = n;
@@ -655,14 +599,6 @@ staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
         dtA[0] = s_dtA[0];
         dtA[1] = s_dtA[1];
     }
-}
-
-/* The first step's dt after the maxima of the state are known, and again
- * when the stopping time moves. */
-static __global__ void staged_arm_kernel(const Mh2dArgs<double> a)
-{
-    const HydroStepControl *c = a.ctrl;
-    arm_dt(a, a.ctrl, c->num_steps, c->t, c->tf);
 }
 
 }  // namespace hydro

@@ -222,6 +222,7 @@ extern "C" int hydro_gpu_muscl_hancock_2d_noalloc(
     c.active = (c.t < c.tf) && (max_steps < 0 || max_steps > 0);
     NA_CK(cudaMemcpy(ctrl_d, &c, sizeof c, cudaMemcpyHostToDevice), "upload control");
     NA_CK(mh2d_launch_prepare<double>(a, 0), "prepare kernel");
+    NA_CK(mh2d_launch_arm<double>(a, 0), "dt kernel");
 
     /* ---- step until the device reports a stop ---- */
     while (c.active) {

@@ -423,6 +423,9 @@ HD void hllc_vacuum_flux(const GasConst<R> &c, R rho_L, R u_L, R v_L, R p_L, R a
     F[3] = s[1] * (E + s[3]);
 }
 
+template <class R>
+HD R prod(R a, R b) { return a * b; }
+
 /* From the (unfloored) star-pressure guess to the flux.  Returns DEV_OK or
  * DEV_ERR_HLLC_WAVE_SPEED.  wave (may be null) receives q_L, q_R and S*, the
  * intermediates the adjoint's tape keeps. */
@@ -454,7 +457,7 @@ HD int hllc_finish(const GasConst<R> &c, R rho_L, R u_L, R v_L, R p_L, R a_L,
     F[0] = fm;
     F[1] = fm * u + p;
     F[2] = fm * v;
-    F[3] = u * (E + p);
+    F[3] = prod(u, E + p);
     if (region == 1 || region == 2) {
         const R S = left ? S_L : S_R;
         const R rs = dv(rho * (S - u), S - S_s);

@@ -143,17 +143,12 @@ static void setup_args(HydroRun2D *run, Mh2dArgs<R> &a, const HydroGrid2D *grid,
     a.area_y = grid->area_y;
     a.vol = grid->vol;
     a.first_order = (grid->integrator == INTEGRATOR_GODUNOV_FIRST_ORDER_2D) ? 1 : 0;
-    a.grid_ctas = mh2d_resident_ctas<R>(grid->limiter, a.first_order, run->device);
-    /* FP64: guided row chunks (measured on the 2048^2 shear layer: 1287 M
-     * against 1257 M with one height).  FP32, at 8 CTAs per SM sharing an SM,
-     * does not fit the model's equal workers (10.8 G against 11.1 G): one
-     * height from the fill model. */
-    if (opt->chunk_rows > 0) {
-        a.chunk_h = opt->chunk_rows;
-    } else if (sizeof(R) == 8) {
-        mh2d_guided_chunks(a.nx, a.ny, a.strip_w, a.grid_ctas, a.chunk_h, a.tail_h, a.tail_rows);
-    } else {
-        a.chunk_h = mh2d_default_chunk(a.nx, a.ny, a.strip_w, a.grid_ctas);
+    if (sizeof(R) == 4) {
+        a.grid_ctas = mh2d_resident_ctas<R>(grid->limiter, a.first_order, run->device);
+        a.chunk_h = opt->chunk_rows > 0 ? opt->chunk_rows
+                                        : mh2d_fp32_chunk(a.grid_ctas, [&](int c) {
+                                              return mh2d_item_count(a.nx, a.ny, a.strip_w, c);
+                                          });
     }
     a.gravity = grid->gravity;
 }
@@ -164,20 +159,25 @@ static cudaError_t launch_step(HydroRun2D *run)
                      : staged_launch_step(run->args, run->grid.limiter, run->bands, run->stream);
 }
 
-/* After the maxima of the state at hand are known: the first dt. */
+static cudaError_t launch_arm(HydroRun2D *run)
+{
+    return run->fp32 ? mh2d_launch_arm<float>(run->args32, run->stream) : mh2d_launch_arm<double>(run->args, run->stream);
+}
+
+/* The maxima of the state at hand and the first dt. */
 static cudaError_t launch_prepare(HydroRun2D *run)
 {
-    if (run->fp32) return mh2d_launch_prepare<float>(run->args32, run->stream);
-    const cudaError_t e = mh2d_launch_prepare<double>(run->args, run->stream);
-    return e != cudaSuccess ? e : staged_launch_arm(run->args, run->stream);
+    const cudaError_t e = run->fp32 ? mh2d_launch_prepare<float>(run->args32, run->stream)
+                                    : mh2d_launch_prepare<double>(run->args, run->stream);
+    return e != cudaSuccess ? e : launch_arm(run);
 }
 
 /* Kernels that launch_step launches. */
 static int launches_per_step(const HydroRun2D *run) { return run->fp32 ? 1 : 3 * (int) run->bands.size(); }
 
-/* The FP64 step's work-item plan for an nx x ny grid on `slots` resident CTAs
- * (guided row chunks), and each item's strip and padded rows as the kernel
- * decodes them (rows: 3 ints per item, or NULL).  Host only; for tests. */
+/* The row-marching FP64 kernel's work-item plan for an nx x ny grid on `slots`
+ * resident CTAs (guided row chunks), and each item's strip and padded rows as
+ * the kernel decodes them (rows: 3 ints per item, or NULL).  Host only. */
 extern "C" int hydro_gpu_chunk_plan(int nx, int ny, int g, int slots, int *h1, int *h2, int *tail,
                                     int *rows, int max_items)
 {
@@ -594,12 +594,12 @@ static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome 
     const int resident = run->fp32 ? run->args32.grid_ctas : run->args.grid_ctas;
     const int storing = run->args.sp.is_storing;
     run->args.sp.is_storing = run->args32.sp.is_storing = 0;
-    const int chunks[] = { 8, 16, 32, 64 };
+    const int chunks[] = { run->args32.chunk_h, 8, 16, 32, 64 };   /* the model's choice first */
     int best_chunk = 32, best_ctas = resident;
     float best_ms = 1e30f;
     HydroStepControl *c = run->ctrl_h;
     const unsigned long long ninf = ordered_bits(-INFINITY);
-    for (int ci = 0; ci < 4; ci++) {
+    for (int ci = 0; ci < 5; ci++) {
         for (int half = 0; half < 2; half++) {
             const int ctas = half ? (resident / 2 > 0 ? resident / 2 : 1) : resident;
             set_shape(run, chunks[ci], ctas);
@@ -616,7 +616,7 @@ static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome 
             CK(launch_step(run), "step kernel");
             CK(cudaEventRecord(run->ev[3], run->stream), "cudaEventRecord");
             CK(cudaEventSynchronize(run->ev[3]), "autotune");
-            run->kernel_launches += 4;
+            run->kernel_launches += 5;
             float ms = 0;
             CK(cudaEventElapsedTime(&ms, run->ev[2], run->ev[3]), "cudaEventElapsedTime");
             if (ms < best_ms) {
@@ -658,7 +658,7 @@ extern "C" int hydro_run2d_begin(HydroRun2D *run, const HydroStepParams *sp, dou
     c->active = recompute_active(c);
     if (push_control(run, oc)) return -1;
     CK(launch_prepare(run), "prepare kernel");
-    run->kernel_launches += run->fp32 ? 1 : 2;
+    run->kernel_launches += 2;
     CK(cudaStreamSynchronize(run->stream), "prepare");
     /* The kernel arguments changed: any recorded graph is stale. */
     if (run->graph) {
@@ -680,11 +680,8 @@ extern "C" int hydro_run2d_set_limits(HydroRun2D *run, double tf, int64 max_step
     c->max_steps = max_steps;
     c->active = recompute_active(c);
     if (push_control(run, oc)) return -1;
-    if (!run->fp32) {
-        /* the next dt is clipped to the stopping time */
-        CK(staged_launch_arm(run->args, run->stream), "dt kernel");
-        run->kernel_launches++;
-    }
+    CK(launch_arm(run), "dt kernel");   /* the next dt is clipped to the stopping time */
+    run->kernel_launches++;
     CK(cudaStreamSynchronize(run->stream), "set limits");
     fill_outcome(run, oc);
     return 0;
@@ -853,7 +850,7 @@ static int snapshot_async(HydroRun2D *run, HydroSnapshotFn snap, void *ctx, Hydr
             CK(convert_f32_to_f64(out[q], st, (long long) run->ncell, run->stream), "convert");
             src[q] = st;
         }
-        run->kernel_launches += 4;
+        run->kernel_launches += 5;
     } else {
         double *out[4];
         for (int q = 0; q < 4; q++) out[q] = static_cast<double *>(run->snap_d[q]);

@@ -79,6 +79,7 @@ struct HydroBatch2D {
     void *ws = nullptr, *plan_d = nullptr;
     std::vector<Mh2dArgs<float>> a32;
     int grid_ctas = 0;
+    int chunk_h = 32;                       /* FP32: rows per work item */
     bool tuned = false;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[2] = {};
@@ -107,7 +108,7 @@ static void build_args(HydroBatch2D *b, std::vector<Mh2dArgs<R>> &av)
         a.g = g.g;
         a.pitch = g.nx + 2 * g.g;
         a.strip_w = mh2d_threads<R>() - 2;   /* FP32: work items */
-        a.chunk_h = b->opt.chunk_rows > 0 ? b->opt.chunk_rows : 32;
+        a.chunk_h = b->chunk_h;
         for (int s = 0; s < 4; s++) a.bc[s] = g.bc[s];
         a.dx = g.dx;
         a.dy = g.dy;
@@ -255,16 +256,30 @@ extern "C" int hydro_batch2d_create(const HydroGrid2D *grids, int n, const Hydro
     b->off.resize(n);
     b->item_off.assign(n + 1, 0);
     size_t total = 0, max_cells = 0;
-    const int chunk_h = opt->chunk_rows > 0 ? opt->chunk_rows : 32;
     for (int k = 0; k < n; k++) {
         const HydroGrid2D &g = grids[order[k]];
         b->ncell[k] = cells(order[k]);
         b->off[k] = total;
         total += 22 * b->ncell[k];
         max_cells = std::max(max_cells, b->ncell[k]);
-        const int nt = mh2d_threads<float>();
-        const int items = ((g.nx + nt - 3) / (nt - 2)) * ((g.ny + chunk_h - 1) / chunk_h);
-        b->item_off[k + 1] = b->item_off[k] + items;
+    }
+    /* FP32: rows per work item of every instance, and the items' offsets */
+    int resident = 0;
+    if (b->fp32) {
+        BK(cudaSetDevice(b->device), "cudaSetDevice");
+        resident = mh2d_resident_ctas<float>(b->limiter, b->first_order, b->device);
+    }
+    const int strip_w = mh2d_threads<float>() - 2;
+    auto items = [&](int k, int c) { return mh2d_item_count(grids[order[k]].nx, grids[order[k]].ny, strip_w, c); };
+    b->chunk_h = opt->chunk_rows > 0 ? opt->chunk_rows : mh2d_fp32_chunk(resident, [&](int c) {
+        long long all = 0;
+        for (int k = 0; k < n; k++) all += items(k, c);
+        return all;
+    });
+    long long all = 0;
+    for (int k = 0; k < n; k++) {
+        all = std::min(all + items(k, b->chunk_h), (long long) INT_MAX);
+        b->item_off[k + 1] = (int) all;
     }
     if (b->item_off[n] <= 0 || (long long) b->item_off[n] > INT_MAX / 2) {
         oc->kind = HYDRO_RUN_UNSUPPORTED;
@@ -291,7 +306,7 @@ extern "C" int hydro_batch2d_create(const HydroGrid2D *grids, int n, const Hydro
     if (b->fp32) {
         build_args<float>(b, b->a32);
         BK(cudaMalloc(&b->args_d, n * sizeof(Mh2dArgs<float>)), "cudaMalloc(args)");
-        b->grid_ctas = mh2d_resident_ctas<float>(b->limiter, b->first_order, b->device);
+        b->grid_ctas = resident;
     } else {
         build_args<double>(b, b->a64);
         BK(cudaMalloc(&b->args_d, n * sizeof(Mh2dArgs<double>)), "cudaMalloc(args)");
@@ -395,6 +410,13 @@ static cudaError_t launch_batch(HydroBatch2D *b)
     return staged_launch_batch(b->staged, b->groups, b->limiter, b->first_order, b->stream);
 }
 
+/* Every instance's next dt. */
+static cudaError_t launch_arm(HydroBatch2D *b)
+{
+    return b->fp32 ? mh2d_launch_batch_arm<float>(static_cast<const Mh2dArgs<float> *>(b->args_d), b->n, b->stream)
+                   : mh2d_launch_batch_arm<double>(static_cast<const Mh2dArgs<double> *>(b->args_d), b->n, b->stream);
+}
+
 /* Kernels that launch_batch launches. */
 static int launches_per_step(const HydroBatch2D *b) { return b->fp32 ? 1 : 3 * (int) b->groups.size(); }
 
@@ -428,10 +450,10 @@ static int batch_autotune(HydroBatch2D *b, HydroRunOutcome *oc)
 {
     int resident = mh2d_resident_ctas<float>(b->limiter, b->first_order, b->device);
     if (resident <= 0) resident = b->grid_ctas;
-    const int chunks[] = { 8, 16, 32, 64 };
+    const int chunks[] = { b->chunk_h, 8, 16, 32, 64 };   /* the model's choice first */
     int best_chunk = 32, best_ctas = resident;
     float best_ms = 1e30f;
-    for (int ci = 0; ci < 4; ci++) {
+    for (int ci = 0; ci < 5; ci++) {
         for (int half = 0; half < 2; half++) {
             const int ctas = half ? std::max(1, resident / 2) : resident;
             if (set_chunk(b, chunks[ci], ctas, oc)) return -1;
@@ -472,10 +494,9 @@ static int batch_prepare_all(HydroBatch2D *b, double tf, int64 max_steps, HydroR
         for (auto &a : b->a32) BK(mh2d_launch_prepare<float>(a, b->stream), "prepare kernel");
     } else {
         for (auto &a : b->a64) BK(mh2d_launch_prepare<double>(a, b->stream), "prepare kernel");
-        BK(staged_launch_batch_arm(b->staged, b->n, b->stream), "dt kernel");
-        b->launches++;
     }
-    b->launches += b->n;
+    BK(launch_arm(b), "dt kernel");
+    b->launches += b->n + 1;
     BK(cudaStreamSynchronize(b->stream), "prepare");
     return 0;
 }
@@ -515,11 +536,8 @@ extern "C" int hydro_batch2d_set_limits(HydroBatch2D *b, double tf, int64 max_st
         c.active = active(c);
     }
     if (push(b, oc)) return -1;
-    if (!b->fp32) {
-        /* the next dt is clipped to the stopping time */
-        BK(staged_launch_batch_arm(b->staged, b->n, b->stream), "dt kernel");
-        b->launches++;
-    }
+    BK(launch_arm(b), "dt kernel");   /* the next dt is clipped to the stopping time */
+    b->launches++;
     BK(cudaStreamSynchronize(b->stream), "set limits");
     return 0;
 }
