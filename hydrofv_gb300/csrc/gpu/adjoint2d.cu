@@ -12,16 +12,16 @@
  * values of the pass being differentiated, so the derivative is that of the
  * smooth piece the forward pass lies on.
  *
- * Forward pass.  The production step kernel (mh2d_step_kernel) runs the N
- * steps with its own CFL dt; after each step a one-thread kernel logs dt.
- * Every K steps the state (U, W incl. sound speed) and the step-control
- * block are copied aside: a checkpoint.
+ * Forward pass.  The production step (three staged kernels) runs the N steps
+ * with its own CFL dt and logs each step's dt.  Every K steps the state (U, W
+ * incl. sound speed) and the step-control block are copied aside: a
+ * checkpoint.
  *
  * Backward pass.  Segments are processed last to first.  A segment is
- * recomputed from its checkpoint with the production kernel (each step
- * writes its own slab, so all K states stay resident; the recomputed dt is
- * checked against the log and the segment's last state against the next
- * checkpoint, both bit for bit), then swept in reverse:
+ * recomputed from its checkpoint with the production step (each step writes
+ * its own slab, so all K states stay resident; the recomputed dt are checked
+ * against the log and the segment's last state against the next checkpoint,
+ * both bit for bit), then swept in reverse:
  *
  *   ad_recon_kernel      face states of step k (x and y, per cell);
  *   ad_flux_vjp_kernel   per face: Fbar from the adjoints of the two cells it
@@ -65,6 +65,11 @@ using namespace hydro;
 namespace {
 
 constexpr int kThreads = 256;
+/* Up to this many padded cells the reverse HLLC runs without binning its
+ * faces by regime: two launches fewer per step are worth more there than warps
+ * of one regime (40 steps of the reverse sweep, binned against not: 64^2 2.12 /
+ * 1.90 ms, 192^2 2.62 / 2.50, 256^2 4.08 / 4.07, 384^2 6.97 / 7.36). */
+constexpr long long kUnbinnedCells = 60000;
 
 struct AdGeom {
     int nx, ny, g, tx, ty;      /* tx is the row pitch */
@@ -426,21 +431,20 @@ __global__ void ad_copy_interior_kernel(const AdGeom q, F4<double> src, F4<doubl
 
 /* ------------------------------------------------------ stepping control */
 
-__global__ void ad_log_dt_kernel(const HydroStepControl *ctrl, double *dt_log, long long n)
+/* Recomputed dt that differ from the forward pass's. */
+__global__ void ad_check_dt_kernel(const double *dt_log, const double *dt_re, long long n, unsigned long long *mismatch)
 {
-    dt_log[n] = ctrl->dt;
+    GRID_STRIDE(k, n) {
+        if (dt_log[k] != dt_re[k]) atomicAdd(mismatch, 1ull);
+    }
 }
 
-__global__ void ad_check_dt_kernel(const HydroStepControl *ctrl, const double *dt_log, long long n,
-                                   unsigned long long *mismatch)
+/* Interior cells whose recomputed U differs (bitwise) from the stored one,
+ * and one more if the recomputation ended in an error. */
+__global__ void ad_compare_kernel(const AdGeom q, StateP<double> a, StateP<double> b, const HydroStepControl *ctrl,
+                                  unsigned long long *mismatch)
 {
-    if (ctrl->dt != dt_log[n] || ctrl->error_code != 0) atomicAdd(mismatch, 1ull);
-}
-
-/* Interior cells whose recomputed U differs (bitwise) from the stored one. */
-__global__ void ad_compare_kernel(const AdGeom q, StateP<double> a, StateP<double> b, unsigned long long *mismatch)
-{
-    unsigned long long n = 0;
+    unsigned long long n = blockIdx.x == 0 && threadIdx.x == 0 && ctrl->error_code != 0;
     GRID_STRIDE(k, (long long) q.tx * q.ty) {
         int r, c;
         row_col(q, k, r, c);
@@ -580,27 +584,52 @@ __device__ __forceinline__ bool owns_face(const AdGeom &q, int r, int c, int dir
  * PVRS, two-rarefaction, two-shock), so that the reverse HLLC runs warps of
  * one regime (the regimes' reverse code differs; mixed warps serialise
  * over it).  A face is 2k + dir; bins[b * cap + i], counts[b].  Appends are
- * aggregated per warp and regime. */
-__global__ void ad_face_bins_kernel(const AdGeom q, const double *tape, long long plane, unsigned *bins,
-                                    unsigned *counts, long long cap)
+ * counted per block in shared memory, so the four global counters see one
+ * atomic per block and regime (per warp, their serialisation took 47 us of a
+ * 1024^2 step). */
+__global__ void __launch_bounds__(kThreads) ad_face_bins_kernel(const AdGeom q, const double *tape, long long plane,
+                                                                unsigned *bins, unsigned *counts, long long cap)
 {
-    GRID_STRIDE(k, (long long) q.tx * q.ty) {
+    __shared__ unsigned n[4], base[4];
+    const long long cells = (long long) q.tx * q.ty;
+    for (long long k0 = blockIdx.x * (long long) kThreads; k0 < cells; k0 += (long long) gridDim.x * kThreads) {
+        const long long k = k0 + threadIdx.x;
+        if (threadIdx.x < 4) n[threadIdx.x] = 0;
+        __syncthreads();
+        int b[2] = { -1, -1 };
+        unsigned pos[2] = { 0, 0 };
+        if (k < cells) {
+            int r, c;
+            row_col(q, k, r, c);
+#pragma unroll
+            for (int dir = 0; dir < 2; dir++) {
+                if (!owns_face(q, r, c, dir)) continue;
+                b[dir] = (int) tape[(long long) (dir * MH2D_TAPE_FIELDS + TAPE_REG) * plane + k] & 3;
+                pos[dir] = atomicAdd(&n[b[dir]], 1u);
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) base[threadIdx.x] = atomicAdd(&counts[threadIdx.x], n[threadIdx.x]);
+        __syncthreads();
+#pragma unroll
+        for (int dir = 0; dir < 2; dir++)
+            if (b[dir] >= 0) bins[(long long) b[dir] * cap + base[b[dir]] + pos[dir]] = (unsigned) (2 * k + dir);
+        __syncthreads();
+    }
+}
+
+/* Small grids: the reverse HLLC of every face without bins. */
+__global__ void __launch_bounds__(kThreads, 2) ad_flux_vjp_tape_kernel(const AdGeom q, const GasConst<double> gas,
+                                                                     const double *tape, long long plane,
+                                                                     FacesP<double> fb, F4<double> Ub, double cx,
+                                                                     double cy, int *err)
+{
+    GRID_STRIDE(i, 2 * (long long) q.tx * q.ty) {
+        const int dir = i >= (long long) q.tx * q.ty;
+        const long long k = i - dir * (long long) q.tx * q.ty;
         int r, c;
         row_col(q, k, r, c);
-#pragma unroll
-        for (int dir = 0; dir < 2; dir++) {
-            if (!owns_face(q, r, c, dir)) continue;
-            const int b = (int) tape[(long long) (dir * MH2D_TAPE_FIELDS + TAPE_REG) * plane + k] & 3;
-            const unsigned mask = __activemask();
-            const unsigned peers = __match_any_sync(mask, b);
-            const int lane = threadIdx.x & 31;
-            const int leader = __ffs(peers) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(&counts[b], (unsigned) __popc(peers));
-            base = __shfl_sync(peers, base, leader);
-            const unsigned pos = base + (unsigned) __popc(peers & ((1u << lane) - 1u));
-            bins[(long long) b * cap + pos] = (unsigned) (2 * k + dir);
-        }
+        if (owns_face(q, r, c, dir)) flux_vjp_tape_face(q, gas, tape, plane, fb, Ub, cx, cy, err, k, dir);
     }
 }
 
@@ -773,7 +802,7 @@ struct HydroAdj2D {
     HydroStepControl *ctrl_d = nullptr;
     HydroStepControl *ckpt_ctrl_d = nullptr;
     HydroStepControl *ctrl_h = nullptr;
-    double *dt_log_d = nullptr;
+    double *dt_log_d = nullptr, *dt_re_d = nullptr;   /* dt of the forward pass and of the recomputation */
     std::vector<double> dt_h;
     unsigned long long *counters_d = nullptr;  /* [0] recompute mismatches, [1] dt mismatches */
     unsigned long long *sig_d = nullptr;       /* branch signature per replayed step */
@@ -893,12 +922,13 @@ int copy_state(HydroAdj2D *a, const StateP<double> &src, const StateP<double> &d
 
 /* One production step n from `in` to `out` (three launches per band). */
 int prod_step(HydroAdj2D *a, long long n, const StateP<double> &in, const StateP<double> &out,
-              double *tape, HydroRunOutcome *oc)
+              double *tape, double *dt_log, HydroRunOutcome *oc)
 {
     Mh2dArgs<double> args = a->pargs;
     const int b = (int) (n & 1);
     for (int i = 0; i < 4; i++) { args.U[b][i] = in.U[i]; args.U[b ^ 1][i] = out.U[i]; }
     for (int i = 0; i < 5; i++) { args.W[b][i] = in.W[i]; args.W[b ^ 1][i] = out.W[i]; }
+    args.dt_log = dt_log;
     args.tape = tape;
     args.tape_plane = (long long) a->ncell;
     CK(staged_launch_step(args, a->grid.limiter, a->bands, a->stream), tape ? "step kernels (tape)" : "step kernels");
@@ -1093,6 +1123,8 @@ extern "C" int hydro_adj2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     a->ckpt_ctrl_d = static_cast<HydroStepControl *>(p);
     if (dalloc(a, (size_t) num_steps * sizeof(double), &p, oc)) return -1;
     a->dt_log_d = static_cast<double *>(p);
+    if (dalloc(a, (size_t) num_steps * sizeof(double), &p, oc)) return -1;
+    a->dt_re_d = static_cast<double *>(p);
     if (dalloc(a, 4 * sizeof(unsigned long long), &p, oc)) return -1;
     a->counters_d = static_cast<unsigned long long *>(p);
     if (dalloc(a, (size_t) num_steps * sizeof(unsigned long long), &p, oc)) return -1;
@@ -1162,10 +1194,7 @@ extern "C" int hydro_adj2d_forward(HydroAdj2D *a, double *const W[4], double *co
     const StateP<double> *in = &a->ckpt[0];
     for (long long n = 0; n < a->nsteps; n++) {
         const StateP<double> &o = a->fwd[(n + 1) & 1];
-        if (prod_step(a, n, *in, o, nullptr, oc)) return -1;
-        ad_log_dt_kernel<<<1, 1, 0, a->stream>>>(a->ctrl_d, a->dt_log_d, n);
-        CK(cudaGetLastError(), "dt log kernel");
-        a->launches++;
+        if (prod_step(a, n, *in, o, nullptr, a->dt_log_d, oc)) return -1;
         const long long nn = n + 1;
         if (nn < a->nsteps && nn % a->K == 0) {
             const int ci = (int) (nn / a->K);
@@ -1238,6 +1267,8 @@ extern "C" int hydro_adj2d_backward(HydroAdj2D *a, double *const seed[4], double
     const double vol = a->grid.vol;
     CK(cudaMemsetAsync(a->err_d, 0, sizeof(int), a->stream), "memset");
     CK(cudaMemsetAsync(a->counters_d, 0, 4 * sizeof(unsigned long long), a->stream), "memset");
+    /* NaN: a step that is not recomputed does not pass the check */
+    CK(cudaMemsetAsync(a->dt_re_d, 0xff, (size_t) a->nsteps * sizeof(double), a->stream), "memset");
     double *sd[4] = { a->stage[0], a->stage[1], a->stage[2], a->stage[3] };
     if (upload4(a, seed, sd, oc)) return -1;
     ad_seed_kernel<<<nb, kThreads, 0, a->stream>>>(q, gas, vol, a->fin, f4(sd), f4(a->Ub));
@@ -1272,13 +1303,10 @@ extern "C" int hydro_adj2d_backward(HydroAdj2D *a, double *const seed[4], double
             return tape_base ? tape_base + (size_t) (k - k0) * 2 * MH2D_TAPE_FIELDS * a->ncell : nullptr;
         };
         for (long long n = k0; n < k1; n++) {
-            if (prod_step(a, n, slab(n), slab(n + 1), tape_of(n), oc)) return -1;
-            ad_check_dt_kernel<<<1, 1, 0, a->stream>>>(a->ctrl_d, a->dt_log_d, n, a->counters_d + 1);
-            CK(cudaGetLastError(), "dt check kernel");
-            a->launches++;
+            if (prod_step(a, n, slab(n), slab(n + 1), tape_of(n), a->dt_re_d, oc)) return -1;
         }
         const StateP<double> &ref = (k1 == a->nsteps) ? a->fin : a->ckpt[(size_t) (s + 1)];
-        ad_compare_kernel<<<nb, kThreads, 0, a->stream>>>(q, slab(k1), ref, a->counters_d);
+        ad_compare_kernel<<<nb, kThreads, 0, a->stream>>>(q, slab(k1), ref, a->ctrl_d, a->counters_d);
         CK(cudaGetLastError(), "compare kernel");
         a->launches++;
         CK(cudaEventRecord(a->ev[1], a->stream), "cudaEventRecord");
@@ -1286,7 +1314,12 @@ extern "C" int hydro_adj2d_backward(HydroAdj2D *a, double *const seed[4], double
         for (long long k = k1 - 1; k >= k0; k--) {
             const StateP<double> &st = slab(k);
             const double dt = a->dt_h[(size_t) k];
-            if (tape_base) {
+            if (tape_base && a->ncell <= (size_t) kUnbinnedCells) {
+                ad_flux_vjp_tape_kernel<<<grid_for(2 * (long long) a->ncell), kThreads, 0, a->stream>>>(
+                    q, gas, tape_of(k), (long long) a->ncell, a->faces_b, f4(a->Ub), dt * a->grid.area_x,
+                    dt * a->grid.area_y, a->err_d);
+                CK(cudaGetLastError(), "flux vjp kernel");
+            } else if (tape_base) {
                 const long long cap = 2 * (long long) a->ncell;
                 CK(cudaMemsetAsync(a->bin_counts_d, 0, 4 * sizeof(unsigned), a->stream), "cudaMemset(bins)");
                 ad_face_bins_kernel<<<nb, kThreads, 0, a->stream>>>(q, tape_of(k), (long long) a->ncell, a->bins_d,
@@ -1327,6 +1360,9 @@ extern "C" int hydro_adj2d_backward(HydroAdj2D *a, double *const seed[4], double
         a->recompute_ms += elapsed(a, 0, 1);
         a->vjp_ms += elapsed(a, 1, 2);
     }
+    ad_check_dt_kernel<<<grid_for(a->nsteps), kThreads, 0, a->stream>>>(a->dt_log_d, a->dt_re_d, a->nsteps, a->counters_d + 1);
+    CK(cudaGetLastError(), "dt check kernel");
+    a->launches++;
     unsigned long long cnt[2] = { 0, 0 };
     CK(cudaMemcpyAsync(cnt, a->counters_d, sizeof cnt, cudaMemcpyDeviceToHost, a->stream), "D2H counters");
     if (check_err(a, oc)) return -1;

@@ -22,7 +22,7 @@
 #ifndef HYDRO_GPU_ADJOINT_NUMERICS_CUH
 #define HYDRO_GPU_ADJOINT_NUMERICS_CUH
 
-#include "numerics.cuh"
+#include "staged_math.cuh"
 
 /* `#pragma unroll` for the device compiler only (the host compiler builds
  * these functions too, and does not know the pragma) */
@@ -34,6 +34,67 @@
 
 namespace hydro {
 
+/* ------------------------------------------------------ contracted reals */
+
+/*
+ * A double whose sums with products contract into fused multiply-adds.  The
+ * reverse sweep is bound by the FP64 pipe and its arithmetic is derivatives
+ * only (nothing of it decides a branch of the forward pass), so
+ * x y + z is one instruction and one rounding instead of two.  The
+ * contraction is written here, not left to the compiler: every kernel (and
+ * the host build) forms the same values, so the gradient does not depend on
+ * the tape or on the checkpoints.
+ */
+struct Fd;
+struct FdProd {
+    double a, b;                              /* a b, not yet rounded */
+};
+
+/* Plain sums and products as register-only FMAs (staged_math.cuh); the
+ * constants are read from memory once per thread. */
+HD double fd_add(double x, double y)
+{
+#if defined(__CUDA_ARCH__)
+    return fma(x, d_fma_const[0], y);
+#else
+    return x + y;
+#endif
+}
+
+HD double fd_mul(double x, double y)
+{
+#if defined(__CUDA_ARCH__)
+    return fma(x, y, d_fma_const[1]);
+#else
+    return x * y;
+#endif
+}
+
+struct Fd {
+    double v;
+    Fd() = default;
+    HD Fd(double x) : v(x) {}
+    HD Fd(const FdProd &p) : v(fd_mul(p.a, p.b)) {}
+    HD Fd &operator+=(const Fd &x) { v = fd_add(v, x.v); return *this; }
+    HD Fd &operator-=(const Fd &x) { v = fd_add(-x.v, v); return *this; }
+    HD Fd &operator+=(const FdProd &p) { v = fma(p.a, p.b, v); return *this; }
+    HD Fd &operator-=(const FdProd &p) { v = fma(-p.a, p.b, v); return *this; }
+};
+HD FdProd operator*(const Fd &x, const Fd &y) { return FdProd{ x.v, y.v }; }
+HD FdProd operator*(const FdProd &p, const Fd &y) { return FdProd{ fd_mul(p.a, p.b), y.v }; }
+HD FdProd operator*(const Fd &x, const FdProd &p) { return FdProd{ x.v, fd_mul(p.a, p.b) }; }
+HD FdProd operator*(const FdProd &p, const FdProd &q) { return FdProd{ fd_mul(p.a, p.b), fd_mul(q.a, q.b) }; }
+HD Fd operator+(const Fd &x, const Fd &y) { return Fd(fd_add(x.v, y.v)); }
+HD Fd operator-(const Fd &x, const Fd &y) { return Fd(fd_add(-y.v, x.v)); }
+HD Fd operator+(const FdProd &p, const Fd &y) { return Fd(fma(p.a, p.b, y.v)); }
+HD Fd operator+(const Fd &x, const FdProd &p) { return Fd(fma(p.a, p.b, x.v)); }
+HD Fd operator-(const FdProd &p, const Fd &y) { return Fd(fma(p.a, p.b, -y.v)); }
+HD Fd operator-(const Fd &x, const FdProd &p) { return Fd(fma(-p.a, p.b, x.v)); }
+HD Fd operator+(const FdProd &p, const FdProd &q) { return Fd(fma(p.a, p.b, fd_mul(q.a, q.b))); }
+HD Fd operator-(const FdProd &p, const FdProd &q) { return Fd(fma(p.a, p.b, -fd_mul(q.a, q.b))); }
+HD Fd operator-(const Fd &x) { return Fd(-x.v); }
+HD FdProd operator-(const FdProd &p) { return FdProd{ -p.a, p.b }; }
+
 /* ---------------------------------------------------------------- limiter */
 
 /* Slope d = L(a, b) with its partial derivatives and a branch code:
@@ -44,30 +105,33 @@ template <int LIM>
 HD double limit_slope_partials(double a, double b, double &da, double &db, int &code)
 {
 #if defined(__CUDA_ARCH__)
-    /* the branch decided on the bits, as the forward limiter decides it
-     * (fx::product_nonpositive; minima of positive doubles on their bit
-     * patterns); operands it does not decide take the code below */
-    {
+    /* the branch decided on the bits, with the forward limiter's ranges and
+     * exact scalings (slope, staged_math.cuh); other operands take the code
+     * below */
+    if (LIM != LIM_VAN_LEER) {
         const fx::u64 ua = fx::bits(a), ub = fx::bits(b);
-        const int t = fx::product_nonpositive(ua, ub);
-        if (t > 0) { da = 0.0; db = 0.0; code = 0; return 0.0; }
-        if (t == 0 && LIM != LIM_VAN_LEER) {
-            const fx::u64 aa = ua & ~fx::SIGN, ab = ub & ~fx::SIGN;
+        const fx::u64 aa = ua & ~fx::SIGN, ab = ub & ~fx::SIGN;
+        const unsigned ha = (unsigned) (aa >> 32), hb = (unsigned) (ab >> 32);
+        const unsigned lo = 2u << 20, span = 2042u << 20;
+        const bool in = ha - lo < span && hb - lo < span && ha + hb >= (975u << 20);
+        const bool zero = (aa == 0ull && hb < 0x7ff00000u) || (ab == 0ull && ha < 0x7ff00000u);
+        if (zero || (in && ((ua ^ ub) >> 63))) { da = 0.0; db = 0.0; code = 0; return 0.0; }
+        if (in) {
+            const bool take_b = ab < aa;
             if (LIM == LIM_MINMOD) {
                 if (aa < ab) { da = 1.0; db = 0.0; code = 1; return a; }
                 da = 0.0; db = 1.0; code = 2; return b;
             }
-            const bool take_b = ab < aa;
-            const double two = 2.0 * fx::from_bits(take_b ? ab : aa);
-            const double avg = ((ua >> 63) ? -0.5 : 0.5) * (a + b);
-            const fx::u64 ut = fx::bits(two), uv = fx::bits(avg);
-            if (ut < uv) {
-                if (take_b) { da = 0.0; db = 2.0; code = 3; }
-                else { da = 2.0; db = 0.0; code = 2; }
-                return fx::from_bits(ut | (ua & fx::SIGN));
+            const fx::u64 two = (take_b ? ab : aa) + fx::HIDDEN;
+            const fx::u64 avg = (fx::bits(fd_add(a, b)) & ~fx::SIGN) - fx::HIDDEN;
+            if (two < avg) {
+                da = take_b ? 0.0 : 2.0;
+                db = take_b ? 2.0 : 0.0;
+                code = take_b ? 3 : 2;
+                return fx::from_bits(two | (ua & fx::SIGN));
             }
             da = 0.5; db = 0.5; code = 1;
-            return fx::from_bits(uv | (ua & fx::SIGN));
+            return fx::from_bits(avg | (ua & fx::SIGN));
         }
     }
 #endif
@@ -115,40 +179,43 @@ HD void sound_speed_vjp(double rho, double p, double a, double ab, double &rhob,
 /*
  * Reverse of hancock_2d.  Inputs are those of the forward call (with
  * dtA_rho = dtA / rho); lob / hib are the adjoints of the extrapolated
- * states.  Accumulates into rhob, nb, tb, pb, ab, the slope adjoints db[4]
- * and d_rho_velb (the slope that feeds the density row).
+ * states.  Writes rhob, nb, tb, pb, ab, the slope adjoints db[4] and
+ * d_rho_velb (the slope that feeds the density row).
  */
-HD void hancock_2d_vjp(double dtA, double dtA_rho, double rho, double inv_rho, double n, double a,
-                       const double d[4], double d_rho_vel, const double lob[4],
-                       const double hib[4], double &rhob, double &nb, double &tb, double &pb,
-                       double &ab, double db[4], double &d_rho_velb)
+HD void hancock_2d_vjp(double dtA_, double dtA_rho_, double rho_, double inv_rho_, double n_, double a_,
+                       const double d_[4], double d_rho_vel_, const double lob_[4],
+                       const double hib_[4], Fd &rhob, Fd &nb, Fd &tb, Fd &pb,
+                       Fd &ab, Fd db[4], Fd &d_rho_velb)
 {
-    const double up = 1.0 + dtA * n;
-    const double um = 1.0 - dtA * n;
-    const double dr = dtA * rho;
-    rhob += lob[0] + hib[0];
-    nb += lob[1] + hib[1];
-    tb += lob[2] + hib[2];
-    pb += lob[3] + hib[3];
-    const double upb = -0.5 * (lob[0] * d[0] + lob[1] * d[1] + lob[2] * d[2] + lob[3] * d[3]);
-    const double umb = 0.5 * (hib[0] * d[0] + hib[1] * d[1] + hib[2] * d[2] + hib[3] * d[3]);
-    nb += dtA * (upb - umb);
-    const double s0 = lob[0] + hib[0];
-    double drb = -0.5 * s0 * d_rho_vel;
-    d_rho_velb += -0.5 * dr * s0;
-    const double drab = -0.5 * (lob[3] + hib[3]);          /* adjoint of dr*a*a*d[1] */
-    drb += drab * a * a * d[1];
-    ab += drab * 2.0 * dr * a * d[1];
-    db[1] += drab * dr * a * a;
-    const double s1 = lob[1] + hib[1];
-    const double dtA_rhob = -0.5 * d[3] * s1;
-    db[3] += -0.5 * dtA_rho * s1;
-    rhob += -dtA_rhob * dtA_rho * inv_rho;                 /* d(dtA/rho)/drho */
+    const Fd dtA = dtA_, dtA_rho = dtA_rho_, rho = rho_, inv_rho = inv_rho_, n = n_, a = a_, d_rho_vel = d_rho_vel_;
+    Fd d[4], lob[4], hib[4], s[4];
+HYDRO_UNROLL
+    for (int q = 0; q < 4; q++) {
+        d[q] = d_[q];
+        lob[q] = lob_[q];
+        hib[q] = hib_[q];
+        s[q] = lob[q] + hib[q];
+    }
+    const Fd hn = Fd(0.5) * (dtA * n);
+    const Fd up = Fd(-0.5) - hn, um = Fd(0.5) - hn;        /* -(1 + dtA n) / 2, (1 - dtA n) / 2 */
+    const Fd dr = dtA * rho;
+    tb = s[2];
+    pb = s[3];
+    /* nb = s1 + dtA (up_bar - um_bar), up_bar = -lob . d / 2, um_bar = hib . d / 2 */
+    nb = s[1] + (dtA * Fd(-0.5)) * (s[0] * d[0] + (s[1] * d[1] + (s[2] * d[2] + s[3] * d[3])));
+    const Fd h0 = Fd(-0.5) * s[0], h3 = Fd(-0.5) * s[3];   /* h3: adjoint of dr a a d[1] */
+    d_rho_velb = dr * h0;
+    const Fd aa = a * a, h3d = h3 * d[1];
+    const Fd drb = h0 * d_rho_vel + h3d * aa;
+    ab = (Fd(2.0) * h3d) * (dr * a);
+    const Fd h1 = Fd(-0.5) * s[1];
+    const Fd dtA_rhob = h1 * d[3];
+    rhob = s[0] - dtA_rhob * (dtA_rho * inv_rho);          /* d(dtA/rho)/drho */
     rhob += drb * dtA;
-    db[0] += -0.5 * up * lob[0] + 0.5 * um * hib[0];
-    db[1] += -0.5 * up * lob[1] + 0.5 * um * hib[1];
-    db[2] += -0.5 * up * lob[2] + 0.5 * um * hib[2];
-    db[3] += -0.5 * up * lob[3] + 0.5 * um * hib[3];
+HYDRO_UNROLL
+    for (int q = 0; q < 4; q++) db[q] = up * lob[q] + um * hib[q];
+    db[1] += h3 * (dr * aa);
+    db[3] += h1 * dtA_rho;
 }
 
 /* ------------------------------------------------------------------ HLLC */
@@ -350,170 +417,165 @@ void hllc_vacuum_vjp(const GasConst<double> &c, const double L[4], const double 
  * instead of recomputed.  Writes Lb, Rb.
  */
 HD void hllc_vjp_core(const GasConst<double> &c, const double L[4], const double Rs[4], const HllcFwd &s,
-                      bool have_z, double z0, double z1, const double Fb[4], double Lb[4], double Rb[4])
+                      bool have_z, double z0, double z1, const double Fb_[4], double Lb[4], double Rb[4])
 {
     if (s.reg == PREG_VACUUM) {
-        hllc_vacuum_vjp(c, L, Rs, s.aL, s.aR, Fb, Lb, Rb);
+        hllc_vacuum_vjp(c, L, Rs, s.aL, s.aR, Fb_, Lb, Rb);
         return;
     }
     /* Only the forward intermediates in s decide branches; the reverse below
      * is derivatives only, so a quotient that appears several times is
      * formed once as a reciprocal (a derivative, not a bit-parity value). */
-    const double rl = L[0], ul = L[1], vl = L[2], pl = L[3];
-    const double rr = Rs[0], ur = Rs[1], vr = Rs[2], pr = Rs[3];
-    const double inv_rl = rv(rl), inv_rr = rv(rr), inv_pl = rv(pl), inv_pr = rv(pr);
-    const double inv_gm1 = c.inv_gm1;
-    double rLb = 0, uLb = 0, vLb = 0, pLb = 0, rRb = 0, uRb = 0, vRb = 0, pRb = 0;
-    double aLb = 0, aRb = 0;
+    const Fd rl = L[0], ul = L[1], pl = L[3], rr = Rs[0], ur = Rs[1], pr = Rs[3];
+    const Fd F0 = Fb_[0], F1 = Fb_[1], F2 = Fb_[2], F3 = Fb_[3];
+    const Fd inv_rl = rv(L[0]), inv_rr = rv(Rs[0]), inv_pl = rv(L[3]), inv_pr = rv(Rs[3]);
+    const Fd inv_gm1 = c.inv_gm1;
+    Fd rLb = 0.0, uLb = 0.0, pLb = 0.0, rRb = 0.0, uRb = 0.0, pRb = 0.0;
     /* ---- region flux of the selected side K ---- */
     const bool left = s.region <= 1;
-    const double rho = left ? rl : rr, u = left ? ul : ur, v = left ? vl : vr, p = left ? pl : pr;
-    const double inv_rho = left ? inv_rl : inv_rr;
-    const double E = 0.5 * rho * (u * u + v * v) + p * inv_gm1;
-    const double fm = rho * u;
-    double rhob = 0, ub = 0, vb = 0, pb = 0;
-    double fmb = Fb[0] + Fb[1] * u + Fb[2] * v;
-    ub += Fb[1] * fm + Fb[3] * (E + p);
-    vb += Fb[2] * fm;
-    pb += Fb[1] + Fb[3] * u;
-    double Eb = Fb[3] * u;
-    double SLb = 0, SRb = 0, Ssb = 0;
-    if (s.region == 1 || s.region == 2) {
-        const double S = left ? s.SL : s.SR;
-        const double Ss = s.Ss;
-        const double Smu = S - u, SmS = S - Ss;
-        const double inv_SmS = rv(SmS);
-        const double D = rho * Smu;
-        const double inv_D = rv(D);
-        const double rs = D * inv_SmS;
-        const double pD = p * inv_D;
-        const double Z = Ss + pD;
-        const double Er = E * inv_rho;
-        const double Y = Er + (Ss - u) * Z;
-        const double es = rs * Y;
-        double Sb = Fb[0] * (rs - rho) + Fb[1] * (rs * Ss - rho * u) + Fb[2] * (rs * v - rho * v)
-                  + Fb[3] * (es - E);
-        double rsb = S * (Fb[0] + Fb[1] * Ss + Fb[2] * v);
-        Ssb += Fb[1] * S * rs;
-        const double esb = Fb[3] * S;
-        Eb += -Fb[3] * S;
-        rhob += -S * (Fb[0] + Fb[1] * u + Fb[2] * v);
-        ub += -Fb[1] * S * rho;
-        vb += Fb[2] * S * (rs - rho);
-        rsb += esb * Y;
-        const double Yb = esb * rs;
-        Eb += Yb * inv_rho;
-        rhob += -Yb * Er * inv_rho;
-        Ssb += Yb * Z;
-        ub += -Yb * Z;
-        const double Zb = Yb * (Ss - u);
-        Ssb += Zb;
-        pb += Zb * inv_D;
-        const double Db = -Zb * pD * inv_D;
-        /* rs = N / M, N = D = rho (S - u), M = S - Ss */
-        const double Nb = rsb * inv_SmS + Db;
-        const double Mb = -rsb * rs * inv_SmS;
-        rhob += Nb * Smu;
-        Sb += Nb * rho;
-        ub += -Nb * rho;
-        Sb += Mb;
-        Ssb += -Mb;
-        if (left) SLb += Sb;
-        else SRb += Sb;
-    }
-    rhob += fmb * u;
+    const Fd rho = left ? rl : rr, u = left ? ul : ur, v = left ? L[2] : Rs[2], p = left ? pl : pr;
+    const Fd inv_rho = left ? inv_rl : inv_rr;
+    const Fd K2 = Fd(0.5) * (u * u + v * v);
+    const Fd E = rho * K2 + p * inv_gm1;
+    const Fd fm = rho * u;
+    const Fd fmb = F0 + (F1 * u + F2 * v);
+    Fd ub = F1 * fm + F3 * (E + p), vb = F2 * fm, pb = F3 * u + F1, Eb = F3 * u;
+    Fd rhob = fmb * u;
     ub += fmb * rho;
-    rhob += Eb * 0.5 * (u * u + v * v);
-    ub += Eb * rho * u;
-    vb += Eb * rho * v;
+    Fd SLb = 0.0, SRb = 0.0, Ssb = 0.0;
+    if (s.region == 1 || s.region == 2) {
+        const Fd S = left ? s.SL : s.SR, Ss = s.Ss;
+        const Fd Smu = S - u, D = rho * Smu;
+        const Fd inv_SmS = rv((S - Ss).v), inv_D = rv(D.v);
+        const Fd rs = D * inv_SmS;
+        const Fd pD = p * inv_D;
+        const Fd Z = Ss + pD, dS = Ss - u;
+        const Fd Er = E * inv_rho;
+        const Fd Y = dS * Z + Er;
+        const Fd drs = rs - rho;
+        /* F += S (rs - rho, rs Ss - rho u, (rs - rho) v, es - E), es = rs Y */
+        Fd Sb = (F0 + F2 * v) * drs + (F1 * (rs * Ss - fm) + F3 * (rs * Y - E));
+        const Fd SF1 = S * F1, SF3 = S * F3, SF02 = S * (F0 + F2 * v);
+        Ssb += SF1 * rs;
+        const Fd rsb = SF02 + (SF1 * Ss + SF3 * Y);
+        rhob -= SF02 + SF1 * u;
+        ub -= SF1 * rho;
+        vb += (S * F2) * drs;
+        const Fd Yb = SF3 * rs;
+        Eb += Yb * inv_rho - SF3;
+        rhob -= Yb * (Er * inv_rho);
+        const Fd YZ = Yb * Z, Zb = Yb * dS;
+        Ssb += YZ + Zb;
+        ub -= YZ;
+        const Fd ZD = Zb * inv_D;
+        pb += ZD;
+        /* rs = N / M, N = D = rho (S - u), M = S - Ss */
+        const Fd rM = rsb * inv_SmS;
+        const Fd Nb = rM - ZD * pD;
+        const Fd Mb = -(rM * rs);
+        rhob += Nb * Smu;
+        const Fd Nr = Nb * rho;
+        ub -= Nr;
+        Sb += Nr + Mb;
+        Ssb -= Mb;
+        if (left) SLb = Sb;
+        else SRb = Sb;
+    }
+    rhob += Eb * K2;
+    const Fd Er_ = Eb * rho;
+    ub += Er_ * u;
+    vb += Er_ * v;
     pb += Eb * inv_gm1;
-    if (left) { rLb += rhob; uLb += ub; vLb += vb; pLb += pb; }
-    else { rRb += rhob; uRb += ub; vRb += vb; pRb += pb; }
+    if (left) { rLb = rhob; uLb = ub; pLb = pb; }
+    else { rRb = rhob; uRb = ub; pRb = pb; }
 
     /* ---- S* ---- */
-    if (!eq_zero(Ssb)) {
-        const double dL = s.SL - ul, dR = s.SR - ur;
-        const double Dd = rl * dL - rr * dR;
-        const double Nnb = dv(Ssb, Dd);
-        const double Ddb = -Nnb * s.Ss;
+    if (!eq_zero(Ssb.v)) {
+        const Fd dL = Fd(s.SL) - ul, dR = Fd(s.SR) - ur;
+        const Fd Dd = rl * dL - rr * dR;
+        const Fd Nnb = dv(Ssb.v, Dd.v);
+        const Fd Ddb = -(Nnb * s.Ss);
         pRb += Nnb;
         pLb -= Nnb;
-        rLb += Nnb * ul * dL + Ddb * dL;
-        uLb += Nnb * rl * (dL - ul) - Ddb * rl;
-        SLb += (Nnb * ul + Ddb) * rl;
-        rRb -= Nnb * ur * dR + Ddb * dR;
-        uRb -= Nnb * rr * (dR - ur) - Ddb * rr;
-        SRb -= (Nnb * ur + Ddb) * rr;
+        const Fd kL = Nnb * ul + Ddb, kR = Nnb * ur + Ddb;
+        rLb += kL * dL;
+        uLb += rl * (Nnb * (dL - ul) - Ddb);
+        SLb += kL * rl;
+        rRb -= kR * dR;
+        uRb -= rr * (Nnb * (dR - ur) - Ddb);
+        SRb -= kR * rr;
     }
 
     /* ---- wave speeds ---- */
+    const Fd aL = s.aL, aR = s.aR, ps = s.ps;
     uLb += SLb;
-    aLb -= SLb * s.qL;
-    const double qLb = -SLb * s.aL;
+    Fd aLb = -(SLb * s.qL);
     uRb += SRb;
-    aRb += SRb * s.qR;
-    const double qRb = SRb * s.aR;
-    double psb = 0.0;
-    if (lt(pl, s.ps)) {
-        const double t = dv(qLb * (0.5 * c.q_coef), s.qL) * inv_pl;
+    Fd aRb = SRb * s.qR;
+    Fd psb = 0.0;
+    const double hq = 0.5 * c.q_coef;
+    if (lt(L[3], s.ps)) {
+        const Fd qb = (SLb * aL) * Fd(-hq);
+        const Fd t = Fd(dv(qb.v, s.qL)) * inv_pl;
         psb += t;
-        pLb -= t * s.ps * inv_pl;
+        pLb -= t * (ps * inv_pl);
     }
-    if (lt(pr, s.ps)) {
-        const double t = dv(qRb * (0.5 * c.q_coef), s.qR) * inv_pr;
+    if (lt(Rs[3], s.ps)) {
+        const Fd qb = (SRb * aR) * Fd(hq);
+        const Fd t = Fd(dv(qb.v, s.qR)) * inv_pr;
         psb += t;
-        pRb -= t * s.ps * inv_pr;
+        pRb -= t * (ps * inv_pr);
     }
-    const double pgb = lt(s.pg, c.tol) ? 0.0 : psb;
+    const Fd pgb = lt(s.pg, c.tol) ? Fd(0.0) : psb;
 
     /* ---- star-pressure guess ---- */
-    double ppvb = 0.0;
+    Fd ppvb = 0.0;
     if (s.reg == PREG_PVRS) {
-        ppvb += pgb;
+        ppvb = pgb;
     } else if (s.reg == PREG_TRRS) {
-        const double zL = have_z ? z0 : pw(pl, c.half_gm1_g);
-        const double zR = have_z ? z1 : pw(pr, c.half_gm1_g);
-        const double izL = rv(zL), izR = rv(zR);
-        const double num = s.aL + s.aR - c.half_gm1 * (ur - ul);
-        const double den = s.aL * izL + s.aR * izR;
+        const Fd izL = rv(have_z ? z0 : pw(L[3], c.half_gm1_g)), izR = rv(have_z ? z1 : pw(Rs[3], c.half_gm1_g));
+        const Fd hg = c.half_gm1;
+        const Fd num = (aL + aR) - hg * (ur - ul);
+        const Fd wL = aL * izL, wR = aR * izR;
+        const Fd den = wL + wR;
         /* pg = (num / den)^(1/hg): d pg = (pg / hg) (d num / num - d den / den) */
-        const double k = pgb * c.g_half_gm1 * s.pg;
-        const double numb = dv(k, num);
-        const double denb = dv(-k, den);
-        aLb += numb + denb * izL;
-        aRb += numb + denb * izR;
-        uRb -= numb * c.half_gm1;
-        uLb += numb * c.half_gm1;
+        const Fd k = pgb * (Fd(c.g_half_gm1) * s.pg);
+        const Fd numb = dv(k.v, num.v), denb = dv(-k.v, den.v);
+        aLb += denb * izL + numb;
+        aRb += denb * izR + numb;
+        uRb -= numb * hg;
+        uLb += numb * hg;
         /* den = aL zL^-1 + aR zR^-1, zK = pK^hg: d den / d pK = -aK hg zK^-1 / pK */
-        pLb -= denb * s.aL * izL * c.half_gm1_g * inv_pl;
-        pRb -= denb * s.aR * izR * c.half_gm1_g * inv_pr;
+        const Fd dh = denb * c.half_gm1_g;
+        pLb -= dh * (wL * inv_pl);
+        pRb -= dh * (wR * inv_pr);
     } else {
-        const double BL = s.ppv + pl * c.gm1_gp1, BR = s.ppv + pr * c.gm1_gp1;
-        const double gL = have_z ? z0 : sq(dv(dv(2.0, c.gp1 * rl), BL));
-        const double gR = have_z ? z1 : sq(dv(dv(2.0, c.gp1 * rr), BR));
-        const double Nnb = dv(pgb, gL + gR);
-        const double Ddb = -Nnb * s.pg;
-        const double gLb = Nnb * pl + Ddb, gRb = Nnb * pr + Ddb;
+        /* not contracted: g_K is the forward pass's, as the tape keeps it */
+        const double BL = s.ppv + L[3] * c.gm1_gp1, BR = s.ppv + Rs[3] * c.gm1_gp1;
+        const Fd gL = have_z ? z0 : sq(dv(dv(2.0, c.gp1 * L[0]), BL));
+        const Fd gR = have_z ? z1 : sq(dv(dv(2.0, c.gp1 * Rs[0]), BR));
+        const Fd Nnb = dv(pgb.v, (gL + gR).v);
+        const Fd Ddb = -(Nnb * s.pg);
+        const Fd gLb = Nnb * pl + Ddb, gRb = Nnb * pr + Ddb;
         pLb += Nnb * gL;
         pRb += Nnb * gR;
         uRb -= Nnb;
         uLb += Nnb;
-        const double hL = 0.5 * gLb * gL, hR = 0.5 * gRb * gR;
+        const Fd hL = (Fd(0.5) * gLb) * gL, hR = (Fd(0.5) * gRb) * gR;
         rLb -= hL * inv_rl;
         rRb -= hR * inv_rr;
-        const double BLb = dv(-hL, BL), BRb = dv(-hR, BR);
-        ppvb += BLb + BRb;
+        const Fd BLb = dv(-hL.v, BL), BRb = dv(-hR.v, BR);
+        ppvb = BLb + BRb;
         pLb += BLb * c.gm1_gp1;
         pRb += BRb * c.gm1_gp1;
     }
-    if (!eq_zero(ppvb)) {
-        pLb += 0.5 * ppvb;
-        pRb += 0.5 * ppvb;
-        const double du = ur - ul, sr = rl + rr, sa = s.aL + s.aR;
-        const double w = -0.125 * ppvb;
-        const double dub = w * sr * sa;
-        const double srb = w * du * sa;
-        const double sab = w * du * sr;
+    if (!eq_zero(ppvb.v)) {
+        pLb += Fd(0.5) * ppvb;
+        pRb += Fd(0.5) * ppvb;
+        const Fd du = ur - ul, sr = rl + rr, sa = aL + aR;
+        const Fd w = Fd(-0.125) * ppvb;
+        const Fd wd = w * du, dub = (w * sr) * sa;
+        const Fd srb = wd * sa, sab = wd * sr;
         uRb += dub;
         uLb -= dub;
         rLb += srb;
@@ -522,13 +584,13 @@ HD void hllc_vjp_core(const GasConst<double> &c, const double L[4], const double
         aRb += sab;
     }
     /* a = sqrt(gamma p / rho): da = a/2 (dp/p - drho/rho) */
-    const double hL = 0.5 * aLb * s.aL, hR = 0.5 * aRb * s.aR;
+    const Fd hL = (Fd(0.5) * aLb) * aL, hR = (Fd(0.5) * aRb) * aR;
     rLb -= hL * inv_rl;
     pLb += hL * inv_pl;
     rRb -= hR * inv_rr;
     pRb += hR * inv_pr;
-    Lb[0] = rLb; Lb[1] = uLb; Lb[2] = vLb; Lb[3] = pLb;
-    Rb[0] = rRb; Rb[1] = uRb; Rb[2] = vRb; Rb[3] = pRb;
+    Lb[0] = rLb.v; Lb[1] = uLb.v; Lb[2] = left ? vb.v : 0.0; Lb[3] = pLb.v;
+    Rb[0] = rRb.v; Rb[1] = uRb.v; Rb[2] = left ? 0.0 : vb.v; Rb[3] = pRb.v;
 }
 
 /* Reverse of hllc_flux_2d from the face states alone (forward intermediates
@@ -607,7 +669,7 @@ HD void recon_cell_vjp(int dir, double dtA, const double wm[4], const double w0[
     double pa[4], pb[4], d[4];
     int code;
 HYDRO_UNROLL
-    for (int q = 0; q < 4; q++) d[q] = limit_slope_partials<LIM>(w0[q] - wm[q], wp[q] - w0[q], pa[q], pb[q], code);
+    for (int q = 0; q < 4; q++) d[q] = limit_slope_partials<LIM>(fd_add(-wm[q], w0[q]), fd_add(-w0[q], wp[q]), pa[q], pb[q], code);
     const int in_ = (dir == 0) ? 1 : 2;    /* storage index of the normal velocity */
     const int it_ = (dir == 0) ? 2 : 1;    /* storage index of the tangential velocity */
     double ds[4];                          /* slopes in sweep order */
@@ -615,29 +677,27 @@ HYDRO_UNROLL
     ds[1] = d[in_];
     ds[2] = d[it_];
     ds[3] = d[3];
-    double rhob = 0, nb = 0, tb = 0, pbb = 0, ab = 0, dvxb = 0;
-    double dsb[4] = { 0, 0, 0, 0 };
+    Fd rhob, nb, tb, pbb, ab, dvxb, dsb[4];
     hancock_2d_vjp(dtA, dtA * inv_rho, w0[0], inv_rho, w0[in_], a0, ds, d[1], lob, hib, rhob, nb, tb, pbb,
                    ab, dsb, dvxb);
-    double db[4];                          /* slope adjoints, storage order */
+    Fd db[4], ow[4];                       /* slope adjoints, storage order */
     db[0] = dsb[0];
     db[in_] = dsb[1];
     db[it_] = dsb[2];
     db[3] = dsb[3];
     db[1] += dvxb;
-    own[0] = rhob;
-    own[in_] = nb;
-    own[it_] = tb;
-    own[3] = pbb;
     /* a = sqrt(gamma p / rho): da = a/2 (dp/p - drho/rho) */
-    const double h = 0.5 * ab * a0;
-    own[0] -= h * inv_rho;
-    own[3] += h * inv_p;
+    const Fd h = (Fd(0.5) * ab) * Fd(a0);
+    ow[0] = rhob - h * Fd(inv_rho);
+    ow[in_] = nb;
+    ow[it_] = tb;
+    ow[3] = pbb + h * Fd(inv_p);
 HYDRO_UNROLL
     for (int q = 0; q < 4; q++) {
-        A[q] = db[q] * pa[q];
-        B[q] = db[q] * pb[q];
-        own[q] += A[q] - B[q];
+        const Fd x = db[q] * Fd(pa[q]), y = db[q] * Fd(pb[q]);
+        A[q] = x.v;
+        B[q] = y.v;
+        own[q] = (ow[q] + db[q] * Fd(pa[q] - pb[q])).v;
     }
 }
 
@@ -756,17 +816,19 @@ HD void hllc_flux_2d_forced(const GasConst<double> &c, double rl, double ul, dou
 HD void cons_to_prim_2d_vjp(const GasConst<double> &c, double vol, double m, double mx, double my,
                             const double wb[4], double Ub[4])
 {
-    const double w1 = dv(mx, m), w2 = dv(my, m);
-    const double K = w1 * w1 + w2 * w2;
-    const double Pb = dv(wb[3] * c.gm1, vol);
-    Ub[3] += Pb;
-    double mb = -0.5 * K * Pb + dv(wb[0], vol);
-    const double w1b = wb[1] - m * w1 * Pb;
-    const double w2b = wb[2] - m * w2 * Pb;
-    Ub[1] += dv(w1b, m);
-    Ub[2] += dv(w2b, m);
-    mb += dv(-(w1b * w1 + w2b * w2), m);
-    Ub[0] += mb;
+    const Fd im = rv(m), iv = rv(vol);
+    const Fd w1 = Fd(mx) * im, w2 = Fd(my) * im;
+    const Fd Pb = (Fd(wb[3]) * c.gm1) * iv, mP = Fd(m) * Pb;
+    Fd U0 = Ub[0], U1 = Ub[1], U2 = Ub[2];
+    const Fd w1b = Fd(wb[1]) - mP * w1, w2b = Fd(wb[2]) - mP * w2;
+    U1 += w1b * im;
+    U2 += w2b * im;
+    U0 += Fd(wb[0]) * iv - (Fd(0.5) * Pb) * (w1 * w1 + w2 * w2);
+    U0 -= (w1b * w1 + w2b * w2) * im;
+    Ub[0] = U0.v;
+    Ub[1] = U1.v;
+    Ub[2] = U2.v;
+    Ub[3] += Pb.v;
 }
 
 /* Reverse of the 2D primitive -> conserved conversion (src/system.c:884-905):
