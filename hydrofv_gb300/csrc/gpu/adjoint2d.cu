@@ -513,10 +513,10 @@ __global__ void __launch_bounds__(kThreads, 2) ad_flux_vjp_kernel(const AdGeom q
                 Rs[e] = f.ylo[e][kn];
             }
             /* y flux components are (mass, mom_y, mom_x, energy) */
-            Fb[0] = cy * (Ub.p[0][kn] - Ub.p[0][k]);
-            Fb[1] = cy * (Ub.p[2][kn] - Ub.p[2][k]);
-            Fb[2] = cy * (Ub.p[1][kn] - Ub.p[1][k]);
-            Fb[3] = cy * (Ub.p[3][kn] - Ub.p[3][k]);
+            Fb[0] = fd_mul(cy, fd_add(Ub.p[0][kn], -Ub.p[0][k]));
+            Fb[1] = fd_mul(cy, fd_add(Ub.p[2][kn], -Ub.p[2][k]));
+            Fb[2] = fd_mul(cy, fd_add(Ub.p[1][kn], -Ub.p[1][k]));
+            Fb[3] = fd_mul(cy, fd_add(Ub.p[3][kn], -Ub.p[3][k]));
             const int rc = hllc_vjp(gas, L, Rs, Fb, Lb, Rb, nullptr);
             if (rc) record(err, rc);
 #pragma unroll
@@ -544,13 +544,13 @@ __device__ __forceinline__ void flux_vjp_tape_face(const AdGeom &q, const GasCon
     }
     if (dir == 0) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) Fb[e] = cx * (Ub.p[e][kn] - Ub.p[e][k]);
+        for (int e = 0; e < 4; e++) Fb[e] = fd_mul(cx, fd_add(Ub.p[e][kn], -Ub.p[e][k]));
     } else {
         /* y flux components are (mass, mom_y, mom_x, energy) */
-        Fb[0] = cy * (Ub.p[0][kn] - Ub.p[0][k]);
-        Fb[1] = cy * (Ub.p[2][kn] - Ub.p[2][k]);
-        Fb[2] = cy * (Ub.p[1][kn] - Ub.p[1][k]);
-        Fb[3] = cy * (Ub.p[3][kn] - Ub.p[3][k]);
+        Fb[0] = fd_mul(cy, fd_add(Ub.p[0][kn], -Ub.p[0][k]));
+        Fb[1] = fd_mul(cy, fd_add(Ub.p[2][kn], -Ub.p[2][k]));
+        Fb[2] = fd_mul(cy, fd_add(Ub.p[1][kn], -Ub.p[1][k]));
+        Fb[3] = fd_mul(cy, fd_add(Ub.p[3][kn], -Ub.p[3][k]));
     }
     HllcFwd st;
     const int rc = hllc_fwd_from_tape(gas, L[0], L[1], L[3], Rs[0], Rs[1], Rs[3], T[TAPE_AL * plane],
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kThreads) ad_recon_vjp_kernel(const AdGeom q, 
             for (int e = 0; e < 4; e++) { lob[e] = fb.xlo[e][k]; hib[e] = fb.xhi[e][k]; }
             recon_cell_vjp<LIM>(0, dtA_x, wm, w0, wp, a0, inv_rho, inv_p, lob, hib, ox, A, B);
 #pragma unroll
-            for (int e = 0; e < 4; e++) { o[e] += ox[e]; sh.Ax[e][k] = A[e]; sh.Bx[e][k] = B[e]; }
+            for (int e = 0; e < 4; e++) { o[e] = ox[e]; sh.Ax[e][k] = A[e]; sh.Bx[e][k] = B[e]; }
         }
         if (ny_) {
             double wm[4], wp[4], lob[4], hib[4], oy[4], A[4], B[4];
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kThreads) ad_recon_vjp_kernel(const AdGeom q, 
             for (int e = 0; e < 4; e++) { lob[e] = fb.ylo[e][k]; hib[e] = fb.yhi[e][k]; }
             recon_cell_vjp<LIM>(1, dtA_y, wm, w0, wp, a0, inv_rho, inv_p, lob, hib, oy, A, B);
 #pragma unroll
-            for (int e = 0; e < 4; e++) { o[e] += oy[e]; sh.Ay[e][k] = A[e]; sh.By[e][k] = B[e]; }
+            for (int e = 0; e < 4; e++) { o[e] = nx_ ? fd_add(o[e], oy[e]) : oy[e]; sh.Ay[e][k] = A[e]; sh.By[e][k] = B[e]; }
         }
 #pragma unroll
         for (int e = 0; e < 4; e++) sh.own[e][k] = o[e];
@@ -712,10 +712,10 @@ __device__ __forceinline__ void gather_cell(const AdGeom &q, const SharesP &sh, 
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         double v = self ? sh.own[e][k] : 0.0;
-        if (xp) v -= sh.Ax[e][k + 1];
-        if (xm) v += sh.Bx[e][k - 1];
-        if (yp) v -= sh.Ay[e][k + q.tx];
-        if (ym) v += sh.By[e][k - q.tx];
+        if (xp) v = fd_add(-sh.Ax[e][k + 1], v);
+        if (xm) v = fd_add(sh.Bx[e][k - 1], v);
+        if (yp) v = fd_add(-sh.Ay[e][k + q.tx], v);
+        if (ym) v = fd_add(sh.By[e][k - q.tx], v);
         o[e] = v;
     }
 }

@@ -164,6 +164,23 @@ HD double limit_slope_partials(double a, double b, double &da, double &db, int &
     return d;
 }
 
+/* The same for a = w0 - wm, b = wp - w0; minmod and MC of close neighbours on
+ * the integer pipes (near_slope). */
+template <int LIM>
+HD double slope_partials(double wm, double w0, double wp, double &da, double &db, int &code)
+{
+#if defined(__CUDA_ARCH__)
+    double s;
+    if (LIM != LIM_VAN_LEER && near_slope<LIM>(wm, w0, wp, s, code)) {
+        const double one = LIM == LIM_MINMOD ? 1.0 : code == 1 ? 0.5 : 2.0;
+        da = (LIM == LIM_MINMOD ? code == 1 : code == 1 || code == 2) ? one : 0.0;
+        db = (LIM == LIM_MINMOD ? code == 2 : code == 1 || code == 3) ? one : 0.0;
+        return s;
+    }
+#endif
+    return limit_slope_partials<LIM>(fd_add(-wm, w0), fd_add(-w0, wp), da, db, code);
+}
+
 /* ------------------------------------------------------------ sound speed */
 
 /* a = sqrt(gamma p / rho): rho_b += -a/(2 rho) a_b, p_b += a/(2 p) a_b. */
@@ -264,15 +281,15 @@ HD int hllc_fwd_from_tape(const GasConst<double> &c, double rl, double ul, doubl
     s.aR = aR;
     s.reg = reg;
     s.region = -1;
-    s.ppv = 0.5 * (pl + pr) - 0.125 * (ur - ul) * (rl + rr) * (aL + aR);
+    s.ppv = reg == PREG_TSRS ? 0.5 * (pl + pr) - 0.125 * (ur - ul) * (rl + rr) * (aL + aR) : 0.0;   /* used there alone */
     s.pg = pg;
     s.ps = s.qL = s.qR = s.SL = s.SR = s.Ss = 0.0;
     if (reg == PREG_VACUUM) return DEV_OK;
     s.ps = lt(s.pg, c.tol) ? c.tol : s.pg;
     s.qL = qL;
     s.qR = qR;
-    s.SL = ul - s.aL * s.qL;
-    s.SR = ur + s.aR * s.qR;
+    s.SL = fd_add(ul, -fd_mul(s.aL, s.qL));
+    s.SR = fd_add(ur, fd_mul(s.aR, s.qR));
     s.Ss = Ss;
     if (le(0.0, s.SL)) s.region = 0;
     else if (le(s.SL, 0.0) && le(0.0, s.Ss)) s.region = 1;
@@ -528,9 +545,11 @@ HD void hllc_vjp_core(const GasConst<double> &c, const double L[4], const double
     }
     const Fd pgb = lt(s.pg, c.tol) ? Fd(0.0) : psb;
 
-    /* ---- star-pressure guess ---- */
+    /* ---- star-pressure guess (both q are 1 up to the smaller pressure) ---- */
     Fd ppvb = 0.0;
-    if (s.reg == PREG_PVRS) {
+    if (!lt(L[3], s.ps) && !lt(Rs[3], s.ps)) {
+        ppvb = 0.0;
+    } else if (s.reg == PREG_PVRS) {
         ppvb = pgb;
     } else if (s.reg == PREG_TRRS) {
         const Fd izL = rv(have_z ? z0 : pw(L[3], c.half_gm1_g)), izR = rv(have_z ? z1 : pw(Rs[3], c.half_gm1_g));
@@ -669,7 +688,7 @@ HD void recon_cell_vjp(int dir, double dtA, const double wm[4], const double w0[
     double pa[4], pb[4], d[4];
     int code;
 HYDRO_UNROLL
-    for (int q = 0; q < 4; q++) d[q] = limit_slope_partials<LIM>(fd_add(-wm[q], w0[q]), fd_add(-w0[q], wp[q]), pa[q], pb[q], code);
+    for (int q = 0; q < 4; q++) d[q] = slope_partials<LIM>(wm[q], w0[q], wp[q], pa[q], pb[q], code);
     const int in_ = (dir == 0) ? 1 : 2;    /* storage index of the normal velocity */
     const int it_ = (dir == 0) ? 2 : 1;    /* storage index of the tangential velocity */
     double ds[4];                          /* slopes in sweep order */
@@ -694,10 +713,19 @@ HYDRO_UNROLL
     ow[3] = pbb + h * Fd(inv_p);
 HYDRO_UNROLL
     for (int q = 0; q < 4; q++) {
-        const Fd x = db[q] * Fd(pa[q]), y = db[q] * Fd(pb[q]);
-        A[q] = x.v;
-        B[q] = y.v;
-        own[q] = (ow[q] + db[q] * Fd(pa[q] - pb[q])).v;
+        if (LIM == LIM_VAN_LEER) {
+            const Fd x = db[q] * Fd(pa[q]), y = db[q] * Fd(pb[q]);
+            A[q] = x.v;
+            B[q] = y.v;
+            own[q] = (ow[q] + db[q] * Fd(pa[q] - pb[q])).v;
+        } else {
+            /* pa and pb are equal, or one of them is zero */
+            const bool a = fx::bits(pa[q]) != 0ull, b = fx::bits(pb[q]) != 0ull;
+            const Fd t = db[q] * Fd(a ? pa[q] : pb[q]);
+            A[q] = a ? t.v : 0.0;
+            B[q] = b ? t.v : 0.0;
+            own[q] = (ow[q] + t * Fd(a == b ? 0.0 : a ? 1.0 : -1.0)).v;
+        }
     }
 }
 

@@ -253,7 +253,9 @@ extern "C" void hydro_fx_staged_face_host(double gamma, double tol, long long n,
         if (reg == PREG_VACUUM) {
             hllc_vacuum_flux(c, l[0], l[1], l[2], l[3], a_L, r[0], r[1], r[2], r[3], a_R, F);
         } else {
-            if (reg == PREG_TRRS) pg = face_trrs(f, c, l[1], l[3], a_L, r[1], r[3], a_R, z0, z1);
+            double p_min;
+            if (reg == PREG_TRRS && plain && both_rarefactions(f, c, l[1], l[3], a_L, r[1], r[3], a_R, p_min)) pg = p_min;
+            else if (reg == PREG_TRRS) pg = face_trrs(f, c, l[1], l[3], a_L, r[1], r[3], a_R, z0, z1);
             else if (reg == PREG_TSRS) pg = face_tsrs(f, c, l[0], l[1], l[3], r[0], r[1], r[3], pg, z0, z1);
             rc[k] = face_finish(f, c, plain, l[0], l[1], l[2], l[3], a_L, r[0], r[1], r[2], r[3], a_R, pg, F, wave);
         }
@@ -274,13 +276,17 @@ extern "C" void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA,
         const double *a = wm + 4 * k, *b = w0 + 4 * k, *e = wp + 4 * k;
         double d[4], g[4], *o = out + 12 * k, *r = ref + 12 * k;
         for (int q = 0; q < 4; q++) {
-            const double x = f.sub(b[q], a[q]), y = f.sub(e[q], b[q]);
-            d[q] = limiter == LIM_MINMOD ? slope<LIM_MINMOD>(f, x, y)
-                 : limiter == LIM_VAN_LEER ? slope<LIM_VAN_LEER>(f, x, y) : slope<LIM_MC>(f, x, y);
+            d[q] = limiter == LIM_MINMOD ? slope_of<LIM_MINMOD>(f, a[q], b[q], e[q])
+                 : limiter == LIM_VAN_LEER ? slope_of<LIM_VAN_LEER>(f, a[q], b[q], e[q])
+                                           : slope_of<LIM_MC>(f, a[q], b[q], e[q]);
             g[q] = limit_slope_rt(limiter, b[q] - a[q], e[q] - b[q]);
         }
         const double s = sound_speed(c, b[0], b[3]);
-        predict(f, dtA, dv(dtA, b[0]), b[0], b[1], b[2], b[3], s, d, d[1], o, o + 4);
+        if (flat(d, b[0], b[1], b[2], b[3]) && fx::moderate(dtA)) {
+            for (int q = 0; q < 4; q++) o[q] = o[4 + q] = b[q];
+        } else {
+            predict(f, dtA, dv(dtA, b[0]), b[0], b[1], b[2], b[3], s, d, d[1], o, o + 4);
+        }
         hancock_2d(dtA, dv(dtA, b[0]), b[0], b[1], b[2], b[3], s, g, g[1], r, r + 4);
         to_primitive(f, c, 0.37, b[0], b[1], b[2], b[3], o + 8);
         cons_to_prim_2d(c, 0.37, b[0], b[1], b[2], b[3], r + 8);

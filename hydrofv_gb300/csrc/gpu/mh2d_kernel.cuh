@@ -140,7 +140,10 @@ __host__ __device__ inline void mh2d_item_rows(const Mh2dArgs<R> &a, int item, i
  * slot 1), both sound speeds, the star-pressure guess before the floor, the
  * guess's factors (p^((g-1)/2g) of each side for the two-rarefaction guess,
  * g_K of each side for the two-shock guess), the regime, and the wave-speed
- * factors q_L, q_R and S* of the finish (zero for vacuum faces).
+ * factors q_L, q_R and S* of the finish (zero for vacuum faces).  A face with
+ * two sure rarefactions (both_rarefactions) has the smaller pressure as its
+ * guess and no factors: q_L = q_R = 1 and nothing flows back through the
+ * guess.
  */
 #define MH2D_TAPE_FIELDS 17
 enum : int {

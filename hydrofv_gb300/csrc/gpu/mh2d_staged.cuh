@@ -20,10 +20,15 @@
  * face or cell makes the step as long as three short chains and fills the
  * chip from a few thousand cells on; each kernel takes only the registers of
  * its own part, so more warps are resident.  The price is the workspace:
- * about 530 bytes per cell-update pass through L2 or HBM, 10% of the HBM rate
- * at 1.3 G cell-updates/s, under the arithmetic.  Time per step, fused ->
- * staged: 64^2 276 -> 47 us, 122^2 with gravity 282 -> 58, 401 x 250 van Leer
- * 308 -> 113, 1024^2 blast 0.86 -> 0.65 ms, 2048^2 3.25 -> 3.07 ms.
+ * about 530 bytes per cell-update pass through L2 or HBM, 17% of the HBM rate
+ * at 2.2 G cell-updates/s, under the arithmetic.  Time per step, fused ->
+ * staged with the fused kernel's arithmetic: 64^2 276 -> 47 us, 122^2 with
+ * gravity 282 -> 58, 401 x 250 van Leer 308 -> 113, 1024^2 blast 0.86 -> 0.65
+ * ms, 2048^2 3.25 -> 3.07 ms.
+ *
+ * Blocks per SM (registers): flux 5 / 6 / 7 (96 / 80 / 72) takes 1.99 / 1.95 /
+ * 2.00 ms a step at 2048^2; recon is the same with 5 to 8; update 5 / 6 / 8
+ * takes 2.25 / 2.27 / 2.26.
  */
 #ifndef HYDRO_GPU_MH2D_STAGED_CUH
 #define HYDRO_GPU_MH2D_STAGED_CUH
@@ -35,10 +40,10 @@
 #define MH2D_RECON_CTAS 6
 #endif
 #ifndef MH2D_FLUX_CTAS
-#define MH2D_FLUX_CTAS 5
+#define MH2D_FLUX_CTAS 6
 #endif
 #ifndef MH2D_UPDATE_CTAS
-#define MH2D_UPDATE_CTAS 6
+#define MH2D_UPDATE_CTAS 5
 #endif
 #ifndef MH2D_LOOP_CTAS
 #define MH2D_LOOP_CTAS 4
@@ -50,10 +55,10 @@ constexpr int kStagedThreads = 128;
 
 /* Largest number of recon items (about two per cell) that steps in the
  * many-step kernel.  Time per step, three launches replayed from a graph
- * against the many-step kernel: 64^2 26.2 / 24.7 us, 128^2 29.1 / 29.8, 192^2
- * 40.4 / 40.3, 256^2 63.8 / 60.2, 320^2 86.6 / 84.9, 384^2 106.7 / 109.3,
- * 512^2 167 / 176; without a graph (short runs) the three launches take at
- * least 34 us of host time. */
+ * against the many-step kernel: 64^2 25.7 / 23.7 us, 128^2 29.9 / 28.4, 192^2
+ * 38.2 / 36.2, 256^2 55.2 / 52.8, 320^2 71.5 / 73.5, 384^2 89.0 / 92.9, 512^2
+ * 139 / 149; without a graph (short runs) the three launches take at least 34
+ * us of host time. */
 #ifndef MH2D_LOOP_ITEMS
 #define MH2D_LOOP_ITEMS 200000
 #endif
@@ -111,10 +116,14 @@ __device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh
         const Fm f = make_fm();
         double s[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) s[q] = slope<LIM>(f, f.sub(w[q], wm[q]), f.sub(wp[q], w[q]));
+        for (int q = 0; q < 4; q++) s[q] = slope_of<LIM>(f, wm[q], w[q], wp[q]);
         const double h = y ? dtA[1] : dtA[0];
-        const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
-        predict(f, h, dvi(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
+        if (flat(s, w[0], n, t, w[3]) && fx::moderate(h)) {
+            lo[0] = hi[0] = w[0]; lo[1] = hi[1] = n; lo[2] = hi[2] = t; lo[3] = hi[3] = w[3];
+        } else {
+            const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
+            predict(f, h, dvi(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], lo, hi);
+        }
     }
     double *o = b.ws + (long long) (r - b.r0 + 1) * a.pitch + c + (y ? WS_YLO : WS_XLO) * b.plane;
 #pragma unroll
@@ -148,6 +157,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     long long at = 0, tape_at = 0;
     double L[4], R[4], aL = 0, aR = 0, pg = 0;
     int reg = PREG_PVRS;
+    bool guessed = false;
     if (tid == 0) { sm.nT = 0; sm.nS = 0; }
     __syncthreads();
     if (on) {
@@ -168,7 +178,10 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
 #pragma unroll
         for (int q = 0; q < 4; q++) { L[q] = l[q * b.plane]; R[q] = h[q * b.plane]; }
         reg = face_classify(fm, a.gas, L[0], L[1], L[3], R[0], R[1], R[3], aL, aR, pg, plain);
-        if (reg == PREG_TRRS || reg == PREG_TSRS) {
+        double p_min;
+        if (reg == PREG_TRRS && plain && both_rarefactions(fm, a.gas, L[1], L[3], aL, R[1], R[3], aR, p_min)) pg = p_min;
+        else guessed = reg == PREG_TRRS || reg == PREG_TSRS;
+        if (guessed) {
             sm.rho[0][tid] = L[0]; sm.u[0][tid] = L[1]; sm.p[0][tid] = L[3]; sm.a[0][tid] = aL;
             sm.rho[1][tid] = R[0]; sm.u[1][tid] = R[1]; sm.p[1][tid] = R[3]; sm.a[1][tid] = aR;
             sm.pg[tid] = pg;
@@ -195,7 +208,6 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     if (!on) return;
     double F[4];
     double wave[3] = { 0.0, 0.0, 0.0 };
-    const bool guessed = reg == PREG_TRRS || reg == PREG_TSRS;
     if (guessed) pg = sm.pg[tid];
     if (reg == PREG_VACUUM) {
         vacuum_flux_dev(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, F);
