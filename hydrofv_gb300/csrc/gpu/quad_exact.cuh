@@ -8,7 +8,7 @@
 #ifndef HYDRO_GPU_QUAD_EXACT_CUH
 #define HYDRO_GPU_QUAD_EXACT_CUH
 
-#include "numerics.cuh"
+#include "staged_math.cuh"
 
 namespace hydro {
 
@@ -62,15 +62,17 @@ static __device__ void quad_fdf(const Quad &Q, const GasConst<double> &c, const 
     const bool d = Q.q >= 2;
     const double p = side ? S.p_R : S.p_L;
     const double a = side ? S.a_R : S.a_L;
-    double x, r = 0.0;
-    if (ps > p) {
-        const double A = side ? S.A_R : S.A_L;
-        const double B = p * c.gm1_gp1;
-        if (d) x = sample ? 0.0 : (1.0 - dv(0.5 * (ps - p), B - ps)) * sq(dv(A, B + ps));
-        else x = (ps - p) * sq(dv(A, ps + B));
-    } else {
-        r = pw(dv(ps, p), d ? (sample ? c.inv_g : c.neg_gp1_2g) : c.gm1_2g);
-        x = d ? (sample ? r : dv(r, p * a)) : dv(2.0 * a * (r - 1.0), c.gm1);
+    /* the four forms of fK and dfK share their quotients, so that a warp of
+     * unlike problems takes two divides, a root and a power, not six */
+    const bool shock = ps > p;
+    const double B = p * c.gm1_gp1;
+    const double t = dv(shock ? (side ? S.A_R : S.A_L) : ps, shock ? B + ps : p);
+    const double r = shock ? 0.0 : pw(t, d ? (sample ? c.inv_g : c.neg_gp1_2g) : c.gm1_2g);
+    const double s = shock ? sq(t) : 0.0;
+    double x = shock ? (ps - p) * s : r;
+    if (d ? !sample : !shock) {
+        const double y = dv(shock ? 0.5 * (ps - p) : d ? r : 2.0 * a * (r - 1.0), shock ? B - ps : d ? p * a : c.gm1);
+        x = shock ? (1.0 - y) * s : y;
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) v[k] = __shfl_sync(Q.mask, x, Q.base + k);
@@ -89,12 +91,34 @@ __device__ __forceinline__ double quad_f(const Quad &Q, const GasConst<double> &
     return v[0] + v[1] + S.du;
 }
 
-/* exact_p_star (numerics.cuh) with the function evaluations shared by the quad. */
-static __device__ int quad_p_star(const Quad &Q, const GasConst<double> &c, const Sides &S, double rho_L, double u_L,
-                           double p_L, double a_L, double rho_R, double u_R, double p_R, double a_R, double *out,
-                           unsigned int *marks)
+/* guess_p (numerics.cuh) with the two sides' terms in two lanes. */
+static __device__ double quad_guess_p(const Quad &Q, const GasConst<double> &c, const Sides &S, double rho_L, double rho_R)
 {
-    const double pg = guess_p(c, rho_L, u_L, p_L, a_L, rho_R, u_R, p_R, a_R);
+    const double p_min = (S.p_L > S.p_R) ? S.p_R : S.p_L, p_max = (S.p_L > S.p_R) ? S.p_L : S.p_R;
+    const double ppv = 0.5 * (S.p_L + S.p_R) - 0.125 * S.du * (rho_L + rho_R) * (S.a_L + S.a_R);
+    const bool right = Q.q & 1;
+    const double p = right ? S.p_R : S.p_L;
+    double pg;
+    if (ratio_at_most_two(p_max, p_min) && (p_min <= ppv && ppv <= p_max)) {
+        pg = ppv;
+    } else if (ppv < p_min) {
+        const double w = dv(right ? S.a_R : S.a_L, pw(p, c.half_gm1_g));
+        const double w_L = __shfl_sync(Q.mask, w, Q.base), w_R = __shfl_sync(Q.mask, w, Q.base + 1);
+        pg = pw(dv(S.a_L + S.a_R - c.half_gm1 * S.du, w_L + w_R), c.g_half_gm1);
+    } else {
+        const double g = sq(dv(right ? S.A_R : S.A_L, ppv + p * c.gm1_gp1)), gp = g * p;
+        const double g_L = __shfl_sync(Q.mask, g, Q.base), g_R = __shfl_sync(Q.mask, g, Q.base + 1);
+        const double gp_L = __shfl_sync(Q.mask, gp, Q.base), gp_R = __shfl_sync(Q.mask, gp, Q.base + 1);
+        pg = dv(gp_L + gp_R - S.du, g_L + g_R);
+    }
+    return pg < c.tol ? c.tol : pg;
+}
+
+/* exact_p_star (numerics.cuh) with the function evaluations shared by the quad. */
+static __device__ int quad_p_star(const Quad &Q, const GasConst<double> &c, const Sides &S, double rho_L, double rho_R,
+                           double *out, unsigned int *marks)
+{
+    const double pg = quad_guess_p(Q, c, S, rho_L, rho_R);
     bool bracket = false;
     double p_hi = pg;
     /* f(p_hi) and, for the first Newton step at p0 = p_hi, f'(p_hi) */
@@ -233,7 +257,7 @@ static __device__ int quad_exact_solve(const Quad &Q, const GasConst<double> &c,
     }
     const Sides Sd{ rho_L, p_L, a_L, rho_R, p_R, a_R, u_R - u_L, A_L, A_R };
     double ps = 0.0;
-    const int rc = quad_p_star(Q, c, Sd, rho_L, u_L, p_L, a_L, rho_R, u_R, p_R, a_R, &ps, marks);
+    const int rc = quad_p_star(Q, c, Sd, rho_L, rho_R, &ps, marks);
     if (rc != DEV_OK) { o[0] = o[1] = o[2] = 0.0; return rc; }
     double v[4], pre[4];
     quad_fdf(Q, c, Sd, ps, v, true, pre);
@@ -242,12 +266,23 @@ static __device__ int quad_exact_solve(const Quad &Q, const GasConst<double> &c,
     return DEV_OK;
 }
 
+/* Equal states on both sides, for which the solver's result is that state:
+ * the guess is p, f(p) is zero and so is the first Newton step, every power is
+ * 1 and the star velocity u (but for the sign of a zero u). */
+static __device__ __forceinline__ bool same_state(const GasConst<double> &c, double rho_L, double u_L, double p_L, double rho_R,
+                                                  double u_R, double p_R)
+{
+    return fx::bits(rho_L) == fx::bits(rho_R) && fx::bits(u_L) == fx::bits(u_R) && fx::bits(p_L) == fx::bits(p_R) &&
+           fx::moderate(rho_L) && fx::moderate(p_L) && fx::bits(u_L) != fx::SIGN && fabs(u_L) < 1e100 &&
+           fx::moderate(c.tol) && p_L >= c.tol;
+}
+
 /* exact_flux_1d (numerics.cuh) on a quad, at x/t = 0. */
 static __device__ int quad_exact_flux(const Quad &Q, const GasConst<double> &c, double rl, double ul, double pl,
                                double rr, double ur, double pr, double F[3], unsigned int *marks = nullptr)
 {
-    double s[3];
-    const int rc = quad_exact_solve(Q, c, rl, ul, pl, rr, ur, pr, 0.0, s, marks);
+    double s[3] = { rl, ul, pl };
+    const int rc = same_state(c, rl, ul, pl, rr, ur, pr) ? DEV_OK : quad_exact_solve(Q, c, rl, ul, pl, rr, ur, pr, 0.0, s, marks);
     F[0] = s[0] * s[1];
     F[1] = s[0] * s[1] * s[1] + s[2];
     F[2] = (s[2] * c.g_gm1 + 0.5 * s[0] * s[1] * s[1]) * s[1];

@@ -23,7 +23,19 @@
  * CTA would put every face's exact Riemann solve (Newton iterations, pow)
  * on one SM's FP64 pipe, about as fast as one host core; the cluster spreads
  * the faces over 16 SMs, and four lanes share each exact Riemann solve
- * (quad_exact_solve, quad_exact.cuh).  Per step a cluster-wide max (partials exchanged
+ * (quad_exact_solve, quad_exact.cuh).
+ *
+ * A step is bound by the latency of its slowest face: of the 42 thousand
+ * cycles of a Sod step (1000 cells, exact solver) 32 thousand are the warp
+ * whose faces take every branch of the solver, and of the 40 thousand of a
+ * spherical Sedov step (508 cells, HLLC) 14 are the flux, 16 the update with
+ * its RK4 source, 8 the predictor.  Hence quotients in line where several are
+ * independent, no powers that do not matter, no solve between equal states,
+ * warps dealt to the CTAs in turn and two or three barriers a step: Sod 1000
+ * to t = 0.2 12.5 -> 10.5 ms, 400 Sedov steps 16.2 -> 8.4 ms (the plain
+ * divides before that: 15.9 and 19.0).
+ *
+ * Per step a cluster-wide max (partials exchanged
  * through distributed shared memory) gives dt, every face flux is computed
  * into a global scratch array, and after a barrier each cell gathers its two
  * faces in the reference's order (+F_left, then -F_right, each (F*dt)*A)
@@ -106,27 +118,32 @@ __device__ double van_der_corput(long long n)
     return result;
 }
 
-/* The cluster's threads: a global index and count for the cell and face loops. */
+/* The cluster's threads: a global index and count for the cell and face loops.
+ * Warps are dealt to the CTAs in turn, so a few hundred cells or faces, and a
+ * wave that covers part of the tube, load every SM's FP64 pipe alike (an FP64
+ * instruction takes 72 cycles with two warps on an SM, 166 with eight). */
 struct Lanes {
     int gt, GT;
 };
 
-/* The CTA's maximum of v, written to *part (this CTA's shared memory). */
-__device__ void block_partial_max(double v, double *red, double *part)
+/* The warp's maximum of an ordered encoding (ordered_bits). */
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long b)
 {
-    for (int o = 16; o > 0; o >>= 1) {
-        const double w = __shfl_xor_sync(0xffffffffu, v, o);
-        if (w > v) v = w;
-    }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0u);
+    return ((unsigned long long) hi << 32) | lo;
+}
+
+/* The CTA's maximum of v (not NaN), encoded, written to *part (this CTA's
+ * shared memory). */
+__device__ void block_partial_max(double v, unsigned long long *red, unsigned long long *part)
+{
+    const unsigned long long b = warp_max(ordered_bits(v));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;
     __syncthreads();
     if (threadIdx.x < 32) {
-        v = (threadIdx.x < kThreads / 32) ? red[threadIdx.x] : -CUDART_INF;
-        for (int o = 16; o > 0; o >>= 1) {
-            const double w = __shfl_xor_sync(0xffffffffu, v, o);
-            if (w > v) v = w;
-        }
-        if (threadIdx.x == 0) *part = v;
+        const unsigned long long m = warp_max((threadIdx.x < kThreads / 32) ? red[threadIdx.x] : 0ull);
+        if (threadIdx.x == 0) *part = m;
     }
 }
 
@@ -134,19 +151,15 @@ __device__ void block_partial_max(double v, double *red, double *part)
  * the partials through distributed shared memory.  Callers alternate two
  * `part` slots between steps, so no CTA overwrites a slot another may still
  * be reading; a cluster barrier separates the reads from any exit. */
-__device__ double cluster_gather_max(double *part, double *red, cg::cluster_group &cl)
+__device__ double cluster_gather_max(unsigned long long *part, unsigned long long *red, cg::cluster_group &cl)
 {
     cl.sync();
     if (threadIdx.x < 32) {
-        double v = (threadIdx.x < (int) cl.num_blocks()) ? *cl.map_shared_rank(part, threadIdx.x) : -CUDART_INF;
-        for (int o = 16; o > 0; o >>= 1) {
-            const double w = __shfl_xor_sync(0xffffffffu, v, o);
-            if (w > v) v = w;
-        }
-        if (threadIdx.x == 0) red[0] = v;
+        const unsigned long long m = warp_max((threadIdx.x < (int) cl.num_blocks()) ? *cl.map_shared_rank(part, threadIdx.x) : 0ull);
+        if (threadIdx.x == 0) red[0] = m;
     }
     __syncthreads();
-    const double r = red[0];
+    const double r = from_ordered_bits(red[0]);
     __syncthreads();
     return r;
 }
@@ -166,6 +179,56 @@ __device__ int cluster_error(int *err, int *bcast, cg::cluster_group &cl)
     const int r = *bcast;
     __syncthreads();
     return r;
+}
+
+__device__ __forceinline__ double quotient(double a, const fx::Recip &b, bool &ok)
+{
+    bool o;
+    const double q = fx::div_recip(a, b, o);
+    ok = ok && o;
+    return q;
+}
+
+__device__ __forceinline__ void source_rates(double pf, double gm1, double rho_, double sm, double se, double &dm,
+                                             double &dmom, double &de, bool &ok)
+{
+    const fx::Recip rho = fx::recip(rho_);
+    const double p = gm1 * (se - quotient(0.5 * sm * sm, rho, ok));
+    dm = pf * sm;
+    dmom = quotient(pf * sm * sm, rho, ok);
+    de = quotient(pf * sm * (se + p), rho, ok);
+}
+
+/* geometry_source_rk4 (numerics.cuh) with one reciprocal each of vol, each
+ * stage's rho and 6, and the quotients in line, so that independent ones overlap; one warp is
+ * alone on its scheduler here and waits for its own chain (the update phase of
+ * a spherical Sedov step took 22 thousand cycles with calls). */
+__device__ void source_rk4(double pf, double gm1, double vol, double dt, double rho, double &m, double &mom, double &E)
+{
+    bool ok = true;
+    const fx::Recip rv = fx::recip(vol), r6 = fx::recip(6.0);
+    double k1m, k1p, k1e, k2m, k2p, k2e, k3m, k3p, k3e, k4m, k4p, k4e;
+    source_rates(pf, gm1, rho, quotient(mom, rv, ok), quotient(E, rv, ok), k1m, k1p, k1e, ok);
+    double tm = m + 0.5 * dt * k1m, tp = mom + 0.5 * dt * k1p, te = E + 0.5 * dt * k1e;
+    source_rates(pf, gm1, quotient(tm, rv, ok), quotient(tp, rv, ok), quotient(te, rv, ok), k2m, k2p, k2e, ok);
+    tm = m + 0.5 * dt * k2m;
+    tp = mom + 0.5 * dt * k2p;
+    te = E + 0.5 * dt * k2e;
+    source_rates(pf, gm1, quotient(tm, rv, ok), quotient(tp, rv, ok), quotient(te, rv, ok), k3m, k3p, k3e, ok);
+    tm = m + dt * k3m;
+    tp = mom + dt * k3p;
+    te = E + dt * k3e;
+    source_rates(pf, gm1, quotient(tm, rv, ok), quotient(tp, rv, ok), quotient(te, rv, ok), k4m, k4p, k4e, ok);
+    const double dm = quotient(dt * (k1m + 2.0 * k2m + 2.0 * k3m + k4m), r6, ok);
+    const double dp = quotient(dt * (k1p + 2.0 * k2p + 2.0 * k3p + k4p), r6, ok);
+    const double de = quotient(dt * (k1e + 2.0 * k2e + 2.0 * k3e + k4e), r6, ok);
+    if (!ok) {
+        geometry_source_rk4(pf, gm1, vol, dt, rho, m, mom, E);
+        return;
+    }
+    m = m + dm;
+    mom = mom + dp;
+    E = E + de;
 }
 
 /* All-cell U -> W (src/system.c:735-761). */
@@ -203,18 +266,80 @@ __device__ void ghost_fill(const Run1dArgs &a, double *const *W, int g, int n, L
     }
 }
 
+__device__ __forceinline__ double wave_factor(const GasConst<double> &c, double p, double ps)
+{
+    return ps <= p ? 1.0 : sqi(1.0 + c.q_coef * (dvi(ps, p) - 1.0));
+}
+
+/* The end of hllc_flux_1d (numerics.cuh): one side selected, the quotients in line. */
+__device__ int hllc_star(const GasConst<double> &c, double rho_L, double u_L, double p_L, double a_L, double rho_R, double u_R,
+                         double p_R, double a_R, double ps, double F[3])
+{
+    const double q_L = wave_factor(c, p_L, ps), q_R = wave_factor(c, p_R, ps);
+    const double S_L = u_L - a_L * q_L, S_R = u_R + a_R * q_R;
+    const double m_L = rho_L * u_L, m_R = rho_R * u_R, d_L = S_L - u_L, d_R = S_R - u_R;
+    const double rd_L = rho_L * d_L, rd_R = rho_R * d_R;
+    const double S_s = dvi(p_R - p_L + m_L * d_L - m_R * d_R, rd_L - rd_R);
+    int region;
+    if (0.0 <= S_L) region = 0;
+    else if (S_L <= 0.0 && 0.0 <= S_s) region = 1;
+    else if (S_s <= 0.0 && 0.0 <= S_R) region = 2;
+    else if (S_R <= 0.0) region = 3;
+    else return DEV_ERR_HLLC_WAVE_SPEED;
+    const bool left = region <= 1;
+    const double rho = left ? rho_L : rho_R, u = left ? u_L : u_R, p = left ? p_L : p_R;
+    const double fm = left ? m_L : m_R, S = left ? S_L : S_R, rd = left ? rd_L : rd_R;
+    const double E = rho * (0.5 * u * u + dvi(p, rho * c.gm1));
+    F[0] = fm;
+    F[1] = fm * u + p;
+    F[2] = u * (E + p);
+    if (region == 1 || region == 2) {
+        const double rs = dvi(rd, S - S_s);
+        const double es = rs * (dvi(E, rho) + (S_s - u) * (S_s + dvi(p, rd)));
+        F[0] = fm + S * (rs - rho);
+        F[1] = F[1] + S * (rs * S_s - fm);
+        F[2] = F[2] + S * (es - E);
+    }
+    return DEV_OK;
+}
+
+/* hllc_flux_1d (numerics.cuh) with the staged step's classification and
+ * guesses (staged_math.cuh): no powers at a face with two sure rarefactions. */
+__device__ int hllc_face(const Fm &f, const GasConst<double> &c, double rl, double ul, double pl, double rr, double ur, double pr,
+                         double F[3])
+{
+    double aL, aR, ps, p_min, z0, z1;
+    bool plain;
+    const int reg = face_classify(f, c, rl, ul, pl, rr, ur, pr, aL, aR, ps, plain);
+    if (!plain || reg == PREG_VACUUM) return hllc_flux_1d(c, rl, ul, pl, rr, ur, pr, F);
+    if (reg == PREG_TRRS) ps = both_rarefactions(f, c, ul, pl, aL, ur, pr, aR, p_min) ? p_min : face_trrs(f, c, ul, pl, aL, ur, pr, aR, z0, z1);
+    else if (reg == PREG_TSRS) ps = face_tsrs(f, c, rl, ul, pl, rr, ur, pr, ps, z0, z1);
+    if (ps < c.tol) ps = c.tol;
+    return hllc_star(c, rl, ul, pl, aL, rr, ur, pr, aR, ps, F);
+}
+
+/* limit_slope_rt (numerics.cuh) of the differences of three neighbours. */
+__device__ __forceinline__ double slope_1d(const Fm &f, int limiter, double wm, double w, double wp)
+{
+    if (limiter == LIM_MINMOD) return slope_of<LIM_MINMOD>(f, wm, w, wp);
+    if (limiter == LIM_VAN_LEER) return slope_of<LIM_VAN_LEER>(f, wm, w, wp);
+    return slope_of<LIM_MC>(f, wm, w, wp);
+}
+
 /* Every phase boundary is a cluster barrier: it orders the phase's global
  * writes (release) before the next phase's reads on any SM of the cluster
  * (acquire).  Every exit is taken by all CTAs at the same point, after a
  * cluster barrier that follows the last distributed-shared-memory read. */
 __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
 {
-    __shared__ double red[kThreads / 32];
-    __shared__ double part[2];
+    __shared__ unsigned long long red[kThreads / 32];
+    __shared__ unsigned long long part[2];
     __shared__ int errs[2];
     __shared__ int s_err;
     cg::cluster_group cl = cg::this_cluster();
-    const Lanes L{ (int) cl.block_rank() * kThreads + (int) threadIdx.x, (int) cl.num_blocks() * kThreads };
+    const Lanes L{ (int) ((threadIdx.x & ~31u) * cl.num_blocks() + cl.block_rank() * 32 + (threadIdx.x & 31u)),
+                   (int) cl.num_blocks() * kThreads };
+    const Fm fm = make_fm();
     const bool leader = cl.block_rank() == 0 && threadIdx.x == 0;
     const Quad Q = make_quad();
     volatile HydroStepControl *ctrl = a.ctrl;
@@ -233,11 +358,11 @@ __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
     const int store_count = ctrl->store_count;
     long long ns = ctrl->num_steps;
     double t = ctrl->t;
-    /* Godunov or MUSCL-Hancock on a Cartesian grid: the final per-cell loop
-     * also writes the ghost cells (each from its source cell, by the thread
-     * that converts that cell) and the next step's partial maximum of
-     * a + |u|, so a step needs two cluster barriers */
-    const bool fused = a.scheme != 2 && a.alpha == 0.0;
+    /* Godunov or MUSCL-Hancock: the final per-cell loop also takes the geometry
+     * source, writes the ghost cells (each from its source cell, by the thread
+     * that converts that cell) and forms the next step's partial maximum of
+     * a + |u|, so a step needs two cluster barriers (MUSCL-Hancock three) */
+    const bool fused = a.scheme != 2;
     const bool periodic = a.bc[1] == BC_PERIODIC;
     const bool ghost_l = periodic || (a.bc[0] != BC_NONE && a.bc[0] != BC_PERIODIC);
     const bool ghost_r = a.bc[1] != BC_NONE;
@@ -275,12 +400,16 @@ __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
         if (a.scheme == 1) {
             for (int i = L.gt; i < n + 2; i += L.GT) {
                 const int k = g + i - 1;
-                const double dtA = dv(dt * a.area[k], a.vol[k]);
-                const double rho = W[0][k], u = W[1][k], p = W[2][k];
-                const double as = sound_speed(a.gas, rho, p);
-                double d[3];
+                double w[3][3], d[3];
+#pragma unroll
                 for (int q = 0; q < 3; q++)
-                    d[q] = limit_slope_rt(a.limiter, W[q][k] - W[q][k - 1], W[q][k + 1] - W[q][k]);
+#pragma unroll
+                    for (int e = 0; e < 3; e++) w[q][e] = W[q][k - 1 + e];
+                const double dtA = dvi(dt * a.area[k], a.vol[k]);
+                const double rho = w[0][1], u = w[1][1], p = w[2][1];
+                const double as = sqi(dvi(a.gas.gamma * p, rho));
+#pragma unroll
+                for (int q = 0; q < 3; q++) d[q] = slope_1d(fm, a.limiter, w[q][0], w[q][1], w[q][2]);
                 double lo[3], hi[3];
                 hancock_1d(dtA, rho, u, p, as, d, lo, hi);
                 /* cell k's low face is face g+i-1 (its right state); high face is g+i (left state) */
@@ -357,7 +486,7 @@ __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
                 const double rr = sr[0][i], ur = sr[1][i], pr = sr[2][i];
                 const int rc = quad ? quad_exact_flux(Q, a.gas, rl, ul, pl, rr, ur, pr, F, a.ctrl->bisect_marks)
                              : a.solver == 1 ? exact_flux_1d(a.gas, rl, ul, pl, rr, ur, pr, 0.0, F, a.ctrl->bisect_marks)
-                                             : hllc_flux_1d(a.gas, rl, ul, pl, rr, ur, pr, F);
+                                             : hllc_face(fm, a.gas, rl, ul, pl, rr, ur, pr, F);
                 if (!quad || Q.q == 0) {
                     if (rc != DEV_OK && a.scheme == 0) atomicCAS(&errs[buf], 0, rc);
                     for (int q = 0; q < 3; q++) a.F[q][i] = F[q];
@@ -389,16 +518,23 @@ __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
                     }
                 }
                 /* a ghost cell that the boundary routine fills keeps only its U */
-                if (fused && ((c < g && ghost_l) || (c >= g + n && ghost_r))) continue;
-                const double m = U[0][c];
+                if ((c < g && ghost_l) || (c >= g + n && ghost_r)) continue;
                 const double vol = a.vol[c];
-                const double rho = dv(m, vol);
-                const double u = dv(U[1][c], m);
-                const double p = dv(a.gas.gm1 * (U[2][c] - 0.5 * m * u * u), vol);
+                double m = U[0][c], mom = U[1][c], E = U[2][c];
+                /* cylindrical / spherical source, RK4 (src/source_term.c:45-183) */
+                if (a.alpha != 0.0 && c >= g && c < g + n) {
+                    source_rk4(dvi(-a.alpha * vol, a.mid[c]), a.gas.gm1, vol, dt, dvi(m, vol), m, mom, E);
+                    U[0][c] = m;
+                    U[1][c] = mom;
+                    U[2][c] = E;
+                }
+                const double rho = dvi(m, vol);
+                const double u = dvi(mom, m);
+                const double p = dvi(a.gas.gm1 * (E - 0.5 * m * u * u), vol);
                 W[0][c] = rho;
                 W[1][c] = u;
                 W[2][c] = p;
-                if (fused && c >= g && c < g + n) {
+                if (c >= g && c < g + n) {
                     /* the ghost cells filled from this cell (src/boundary.c:411-511:
                      * the left side mirrors cell g + k into g - 1 - k, the right
                      * side cell g + n - 1 - k into g + n + k; a periodic right
@@ -422,30 +558,22 @@ __global__ void __launch_bounds__(kThreads) run1d_kernel(const Run1dArgs a)
                             W[2][g + n + kr] = p;
                         }
                     }
-                    const double s = sound_speed(a.gas, rho, p) + fabs(u);
+                    const double s = sqi(dvi(a.gas.gamma * p, rho)) + fabs(u);
                     if (s > snext) snext = s;
                 }
             }
-            if (fused) {
-                block_partial_max(snext, red, &part[buf ^ 1]);
-            } else {
-                cl.sync();
-                ghost_fill(a, W, g, n, L);
-                cl.sync();
-            }
+            block_partial_max(snext, red, &part[buf ^ 1]);
         }
 
-        /* ---- cylindrical / spherical source, RK4 (src/source_term.c:45-183) ---- */
-        if (a.alpha != 0.0) {
-            const double gm1 = a.gas.gm1;
+        /* ---- random choice: cylindrical / spherical source, RK4 ---- */
+        if (a.scheme == 2 && a.alpha != 0.0) {
             for (int i = g + L.gt; i < g + n; i += L.GT) {
                 const double vol = a.vol[i];
-                const double m = U[0][i], mom = U[1][i], E = U[2][i], rho = W[0][i];
-                double mm = m, mp = mom, me = E;
-                geometry_source_rk4(dv(-a.alpha * vol, a.mid[i]), gm1, vol, dt, rho, mm, mp, me);
-                U[0][i] = mm;
-                U[1][i] = mp;
-                U[2][i] = me;
+                double m = U[0][i], mom = U[1][i], E = U[2][i];
+                geometry_source_rk4(dv(-a.alpha * vol, a.mid[i]), a.gas.gm1, vol, dt, W[0][i], m, mom, E);
+                U[0][i] = m;
+                U[1][i] = mom;
+                U[2][i] = E;
             }
             cl.sync();
             convert_all(a, U, W, ntot, L);
