@@ -25,7 +25,7 @@ template cudaError_t mh2d_launch_ghost_sound_speed<double>(const Mh2dArgs<double
 #define HYDRO_STAGED_EXTERN(LIM, FO)                                                                                      \
     extern template cudaError_t staged_launch_recon<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, cudaStream_t); \
     extern template cudaError_t staged_launch_batch_recon<LIM, FO>(const StagedBatchArgs &, const StagedBatchGroup &, cudaStream_t); \
-    extern template int staged_loop_resident<LIM, FO>(bool, int);                                                       \
+    extern template unsigned staged_loop_blocks<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, int);              \
     extern template cudaError_t staged_launch_loop<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, unsigned, int, cudaStream_t);
 HYDRO_STAGED_EXTERN(LIM_MINMOD, 0)
 HYDRO_STAGED_EXTERN(LIM_MINMOD, 1)
@@ -110,11 +110,8 @@ unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vec
 {
     const int first_order = a.first_order;
     if (bands.size() != 1) return 0;
-    const unsigned items = staged_recon_items(a.nx, a.ny);
-    if (items > kStagedLoopItems) return 0;
-    const int resident = STAGED_DISPATCH(staged_loop_resident, a.gravity != 0.0, device);
-    const unsigned blocks = staged_blocks(items);
-    return resident <= 0 ? 0 : (blocks < (unsigned) resident ? blocks : (unsigned) resident);
+    if (staged_recon_items(a.nx, a.ny) > kStagedLoopItems) return 0;
+    return STAGED_DISPATCH(staged_loop_blocks, a, bands[0], device);
 }
 
 cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh2dBand &band, unsigned grid, int steps,

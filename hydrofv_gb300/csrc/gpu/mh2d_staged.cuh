@@ -55,14 +55,25 @@ constexpr int kStagedThreads = 128;
 
 /* Largest number of recon items (about two per cell) that steps in the
  * many-step kernel.  Time per step, three launches replayed from a graph
- * against the many-step kernel: 64^2 25.7 / 23.7 us, 128^2 29.9 / 28.4, 192^2
- * 38.2 / 36.2, 256^2 55.2 / 52.8, 320^2 71.5 / 73.5, 384^2 89.0 / 92.9, 512^2
- * 139 / 149; without a graph (short runs) the three launches take at least 34
+ * against the many-step kernel: 64^2 25.7 / 20.1 us, 128^2 29.9 / 26.1, 192^2
+ * 38.2 / 34.2, 256^2 55.2 / 50.0, 320^2 71.5 / 71.1, 384^2 89.0 / 88.8, 512^2
+ * 139 / 139; without a graph (short runs) the three launches take at least 34
  * us of host time. */
 #ifndef MH2D_LOOP_ITEMS
 #define MH2D_LOOP_ITEMS 200000
 #endif
 constexpr unsigned kStagedLoopItems = MH2D_LOOP_ITEMS;
+
+/* Largest number of faces that the many-step kernel solves with their states
+ * in one phase (staged_recon_flux): a grid barrier and a pass through the
+ * workspace less, two threads a face, as long as that is one round of the
+ * resident blocks (608 of 64 faces).  Time per step, two phases / one: 32^2
+ * 22.1 / 20.0 us, 64^2 22.1 / 20.1, 96^2 23.3 / 22.8, 128^2 27.1 / 26.1, 160^2
+ * 29.8 / 37.3. */
+#ifndef MH2D_FUSED_FACES
+#define MH2D_FUSED_FACES 35000
+#endif
+constexpr unsigned kStagedFusedFaces = MH2D_FUSED_FACES;
 constexpr unsigned kStagedUpdateGrid = 152 * MH2D_UPDATE_CTAS;
 
 /* Fields of the workspace: the low and high face states of each cell in x
@@ -133,6 +144,29 @@ __device__ __forceinline__ void staged_recon(const Mh2dArgs<double> &a, const Mh
     }
 }
 
+/* The state at the high or low face of cell (r, c) in y or x (staged_recon). */
+template <int LIM, int FIRST_ORDER>
+__device__ __forceinline__ void face_side(const Fm &f, const Mh2dArgs<double> &a, bool y, int r, int c, bool high, int buf, bool raw,
+                                          const double dtA[2], double o[4])
+{
+    const double *const *W = a.W[buf];
+    const double *const *U = a.U[buf];
+    double w[5];
+    fetch_w(a, W, U, raw, r, c, w);
+    const double n = y ? w[2] : w[1], t = y ? w[1] : w[2];
+    o[0] = w[0]; o[1] = n; o[2] = t; o[3] = w[3];
+    if (FIRST_ORDER) return;
+    double wm[5], wp[5], s[4];
+    fetch_w(a, W, U, raw, y ? r - 1 : r, y ? c : c - 1, wm);
+    fetch_w(a, W, U, raw, y ? r + 1 : r, y ? c : c + 1, wp);
+#pragma unroll
+    for (int q = 0; q < 4; q++) s[q] = slope_of<LIM>(f, wm[q], w[q], wp[q]);
+    const double h = y ? dtA[1] : dtA[0];
+    if (flat(s, w[0], n, t, w[3]) && fx::moderate(h)) return;
+    const double d[4] = { s[0], y ? s[2] : s[1], y ? s[1] : s[2], s[3] };
+    predict_side(f, high, h, dvi(h, w[0]), w[0], n, t, w[3], w[4], d, s[1], o);
+}
+
 struct FluxShared {
     static constexpr int NT = kStagedThreads;
     double rho[2][NT], u[2][NT], p[2][NT], a[2][NT];   /* both states of each face */
@@ -141,42 +175,41 @@ struct FluxShared {
     int nT, nS;
 };
 
-/* The flux of one block's faces: face k of the band for thread k0 + tid.
- * Faces are classified, the expensive guesses run on compacted lists, and
- * each thread finishes its own face from registers. */
-template <bool TAPE>
-__device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared &sm, unsigned k,
-                                            unsigned total, double dt)
+/* Where face k of the band lies: x faces first (row-major, nx + 1 a row), then
+ * y faces; (r, c) is its left or lower cell. */
+__device__ __forceinline__ bool face_at(const Mh2dArgs<double> &a, const Mh2dBand &b, unsigned k, int &r, int &c)
 {
-    const int tid = threadIdx.x;
-    const bool on = k < total;
-    const Fm fm = make_fm();
-    bool plain = true;
     const unsigned nx = (unsigned) a.nx, nX = (unsigned) (b.r1 - b.r0) * (nx + 1);
     const bool y = k >= nX;
-    long long at = 0, tape_at = 0;
-    double L[4], R[4], aL = 0, aR = 0, pg = 0;
+    if (!y) {
+        const unsigned q = k / (nx + 1);
+        r = b.r0 + (int) q;
+        c = a.g - 1 + (int) (k - q * (nx + 1));
+    } else {
+        const unsigned j = k - nX, q = j / nx;
+        r = b.r0 - 1 + (int) q;
+        c = a.g + (int) (j - q * nx);
+    }
+    return y;
+}
+
+/* The flux of one block's faces, one per thread with `on`: at (r, c), in y or
+ * x, with the states L and R.  Faces are classified, the expensive guesses run
+ * on compacted lists, and each thread finishes its own face from registers.
+ * INL: the finish's quotients in line (staged_math.cuh). */
+template <bool TAPE, bool INL>
+__device__ __forceinline__ void face_flux(const Fm &fm, const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared &sm, bool on, bool y,
+                                          int r, int c, const double L[4], const double R[4], double dt)
+{
+    const int tid = threadIdx.x;
+    bool plain = true;
+    const long long at = (long long) (r - b.r0 + 1) * a.pitch + c, tape_at = (long long) r * a.pitch + c;
+    double aL = 0, aR = 0, pg = 0;
     int reg = PREG_PVRS;
     bool guessed = false;
     if (tid == 0) { sm.nT = 0; sm.nS = 0; }
     __syncthreads();
     if (on) {
-        int r, c;
-        if (!y) {
-            const unsigned q = k / (nx + 1);
-            r = b.r0 + (int) q;
-            c = a.g - 1 + (int) (k - q * (nx + 1));
-        } else {
-            const unsigned j = k - nX, q = j / nx;
-            r = b.r0 - 1 + (int) q;
-            c = a.g + (int) (j - q * nx);
-        }
-        at = (long long) (r - b.r0 + 1) * a.pitch + c;
-        tape_at = (long long) r * a.pitch + c;
-        const double *l = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
-        const double *h = b.ws + (y ? WS_YLO : WS_XLO) * b.plane + at + (y ? a.pitch : 1);
-#pragma unroll
-        for (int q = 0; q < 4; q++) { L[q] = l[q * b.plane]; R[q] = h[q * b.plane]; }
         reg = face_classify(fm, a.gas, L[0], L[1], L[3], R[0], R[1], R[3], aL, aR, pg, plain);
         double p_min;
         if (reg == PREG_TRRS && plain && both_rarefactions(fm, a.gas, L[1], L[3], aL, R[1], R[3], aR, p_min)) pg = p_min;
@@ -199,7 +232,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
             if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
         } else {
             const int f = sm.listS[i - nT];
-            sm.pg[f] = face_tsrs(fm, a.gas, sm.rho[0][f], sm.u[0][f], sm.p[0][f], sm.rho[1][f], sm.u[1][f], sm.p[1][f],
+            sm.pg[f] = face_tsrs<INL>(fm, a.gas, sm.rho[0][f], sm.u[0][f], sm.p[0][f], sm.rho[1][f], sm.u[1][f], sm.p[1][f],
                                       sm.pg[f], z0, z1);
             if constexpr (TAPE) { sm.rho[0][f] = z0; sm.rho[1][f] = z1; }
         }
@@ -212,7 +245,7 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     if (reg == PREG_VACUUM) {
         vacuum_flux_dev(a.gas, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, F);
     } else {
-        const int rc = face_finish(fm, a.gas, plain, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, pg, F, wave);
+        const int rc = face_finish<INL>(fm, a.gas, plain, L[0], L[1], L[2], L[3], aL, R[0], R[1], R[2], R[3], aR, pg, F, wave);
         if (rc) record_error(a.ctrl, rc, (int) blockIdx.x);
     }
     if constexpr (TAPE) {
@@ -227,6 +260,52 @@ __device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2
     double *o = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
 #pragma unroll
     for (int q = 0; q < 4; q++) o[q * b.plane] = fm.mul(fm.mul(F[q], dt), A);
+}
+
+/* Faces k0 .. of one block from the workspace's states. */
+template <bool TAPE, bool INL>
+__device__ __forceinline__ void staged_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared &sm, unsigned k,
+                                            unsigned total, double dt)
+{
+    const Fm fm = make_fm();
+    const bool on = k < total;
+    bool y = false;
+    int r = b.r0, c = a.g;
+    double L[4], R[4];
+    if (on) {
+        y = face_at(a, b, k, r, c);
+        const long long at = (long long) (r - b.r0 + 1) * a.pitch + c;
+        const double *l = b.ws + (y ? WS_YHI : WS_XHI) * b.plane + at;
+        const double *h = b.ws + (y ? WS_YLO : WS_XLO) * b.plane + at + (y ? a.pitch : 1);
+#pragma unroll
+        for (int q = 0; q < 4; q++) { L[q] = l[q * b.plane]; R[q] = h[q * b.plane]; }
+    }
+    face_flux<TAPE, INL>(fm, a, b, sm, on, y, r, c, L, R, dt);
+}
+
+/* Faces k0 .. of one block, half as many as threads: each thread forms one
+ * side's state, then the first half solves the faces.  Every cell's slopes are
+ * formed by both of its faces, but the states pass through shared memory
+ * instead of the workspace and a grid barrier. */
+template <int LIM, int FIRST_ORDER>
+__device__ __forceinline__ void staged_recon_flux(const Mh2dArgs<double> &a, const Mh2dBand &b, FluxShared &sm, double (*v)[kStagedThreads / 2],
+                                                  unsigned k0, unsigned total, double dt, int buf, bool raw, const double dtA[2])
+{
+    constexpr int half = kStagedThreads / 2;
+    const Fm fm = make_fm();
+    const int right = threadIdx.x >= half, f = threadIdx.x - right * half;
+    const bool on = k0 + f < total;
+    bool y = false;
+    int r = b.r0, c = a.g;
+    double L[4], R[4];
+    if (on) {
+        y = face_at(a, b, k0 + f, r, c);
+        face_side<LIM, FIRST_ORDER>(fm, a, y, y ? r + right : r, y ? c : c + right, !right, buf, raw, dtA, L);
+        if (right) { sm.rho[1][f] = L[0]; sm.u[1][f] = L[1]; v[0][f] = L[2]; sm.p[1][f] = L[3]; }
+    }
+    __syncthreads();
+    if (on && !right) { R[0] = sm.rho[1][f]; R[1] = sm.u[1][f]; R[2] = v[0][f]; R[3] = sm.p[1][f]; }
+    face_flux<false, true>(fm, a, b, sm, on && !right, y, r, c, L, R, dt);
 }
 
 /* Cell k of the band: update, gravity, U -> W; mx receives a + |u|, a + |v|. */
@@ -252,6 +331,24 @@ __device__ __forceinline__ void staged_update(const Fm &f, const Mh2dArgs<double
         gh[q] = fy[ymap[q] * b.plane];
         Un[q] = Uin[q][idx];
     }
+    /* the first ghost layer receives its one-sided update (here, so that its
+     * loads are in flight with the others) */
+    if (c == a.g) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx - 1] = f.sub(Uin[q][idx - 1], fl[q]);
+    }
+    if (c == a.g + a.nx - 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx + 1] = f.add(Uin[q][idx + 1], fh[q]);
+    }
+    if (r == a.g) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx - a.pitch] = f.sub(Uin[q][idx - a.pitch], gl[q]);
+    }
+    if (r == a.g + a.ny - 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) Uout[q][idx + a.pitch] = f.add(Uin[q][idx + a.pitch], gh[q]);
+    }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         Un[q] = f.sub(f.add(f.sub(f.add(Un[q], fl[q]), fh[q]), gl[q]), gh[q]);
@@ -268,57 +365,34 @@ __device__ __forceinline__ void staged_update(const Fm &f, const Mh2dArgs<double
     const double sx = f.add(as, fabs(w[1])), sy = f.add(as, fabs(w[2]));
     if (lt(mx_x, sx)) mx_x = sx;
     if (lt(mx_y, sy)) mx_y = sy;
-    /* the first ghost layer receives its one-sided update */
-    if (c == a.g) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) Uout[q][idx - 1] = Uin[q][idx - 1] - fl[q];
-    }
-    if (c == a.g + a.nx - 1) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) Uout[q][idx + 1] = Uin[q][idx + 1] + fh[q];
-    }
-    if (r == a.g) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) Uout[q][idx - a.pitch] = Uin[q][idx - a.pitch] - gl[q];
-    }
-    if (r == a.g + a.ny - 1) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) Uout[q][idx + a.pitch] = Uin[q][idx + a.pitch] + gh[q];
-    }
 }
 
 struct UpdateShared {
-    double red[2][kStagedThreads / 32];
+    unsigned long long red[2][kStagedThreads / 32];
     int am_last;
 };
 
-/* Fold a block's maxima into the next step's words (thread 0 writes them). */
-__device__ __forceinline__ void block_maxima(HydroStepControl *ctrl, double (*red)[kStagedThreads / 32], long long n, double mx_x,
-                                             double mx_y)
+/* Fold a block's maxima into the next step's words (threads 0 and 1 write
+ * them).  The maxima are never NaN; their ordered encodings (ordered_bits)
+ * reduce on the integer pipe. */
+__device__ __forceinline__ void block_maxima(HydroStepControl *ctrl, unsigned long long (*red)[kStagedThreads / 32], long long n,
+                                             double mx_x, double mx_y)
 {
     const int tid = threadIdx.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ox = __shfl_xor_sync(0xffffffffu, mx_x, o);
-        const double oy = __shfl_xor_sync(0xffffffffu, mx_y, o);
-        if (lt(mx_x, ox)) mx_x = ox;
-        if (lt(mx_y, oy)) mx_y = oy;
-    }
+    const unsigned long long bx = warp_max(ordered_bits(mx_x)), by = warp_max(ordered_bits(mx_y));
     if ((tid & 31) == 0) {
-        red[0][tid >> 5] = mx_x;
-        red[1][tid >> 5] = mx_y;
+        red[0][tid >> 5] = bx;
+        red[1][tid >> 5] = by;
     }
     __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < kStagedThreads / 32; w++) {
-            if (lt(mx_x, red[0][w])) mx_x = red[0][w];
-            if (lt(mx_y, red[1][w])) mx_y = red[1][w];
-        }
-        unsigned long long *word = ctrl->smax[(n + 1) % 3];
-        const unsigned long long bx = ordered_bits(mx_x), by = ordered_bits(mx_y);
-        if (bx > *(volatile unsigned long long *) &word[0]) atomicMax(&word[0], bx);
-        if (by > *(volatile unsigned long long *) &word[1]) atomicMax(&word[1], by);
+    if (tid < 2) {
+        unsigned long long b = red[tid][0];
+        for (int w = 1; w < kStagedThreads / 32; w++)
+            if (red[tid][w] > b) b = red[tid][w];
+        unsigned long long *word = &ctrl->smax[(n + 1) % 3][tid];
+        if (b > *(volatile unsigned long long *) word) atomicMax(word, b);
     }
+    __syncwarp();
 }
 
 /* End of an update block: fold its maxima into the next step's words; the
@@ -388,7 +462,7 @@ staged_flux_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     long long n;
     double dt;
     if (!staged_step(a.ctrl, n, dt)) return;
-    staged_flux<TAPE>(a, b, sm, blockIdx.x * kStagedThreads + threadIdx.x, staged_face_items(a.nx, b.r1 - b.r0), dt);
+    staged_flux<TAPE, false>(a, b, sm, blockIdx.x * kStagedThreads + threadIdx.x, staged_face_items(a.nx, b.r1 - b.r0), dt);
 }
 
 template <bool GRAV>
@@ -466,7 +540,7 @@ staged_batch_flux_kernel(const StagedBatchArgs g, const int *map)
     __shared__ BatchBlock sm;
     __shared__ FluxShared fs;
     if (!batch_block(g, map, sm)) return;
-    staged_flux<false>(sm.a, sm.b.band, fs, (blockIdx.x - sm.b.first[1]) * kStagedThreads + threadIdx.x,
+    staged_flux<false, false>(sm.a, sm.b.band, fs, (blockIdx.x - sm.b.first[1]) * kStagedThreads + threadIdx.x,
                        staged_face_items(sm.a.nx, sm.b.band.r1 - sm.b.band.r0), sm.dt);
 }
 
@@ -490,10 +564,10 @@ staged_batch_update_kernel(const StagedBatchArgs g, const int *map)
 /*
  * The same three stages, many steps in one cooperative launch, for grids
  * whose step is a few microseconds of work: grid barriers between the stages
- * instead of kernel boundaries.  A step has three barriers (about 1.5 us
- * each); the three launches it replaces cost about 4 us each in gaps, ramps
+ * instead of kernel boundaries.  A step has two or three barriers (about 1.5
+ * us each); the three launches it replaces cost about 4 us each in gaps, ramps
  * and control-block reads, and 11 us of host time where no graph is
- * recorded.  Every block forms the next dt itself after the third barrier.
+ * recorded.  Every block forms the next dt itself after the last barrier.
  *
  * grid_barrier: each block counts itself in on a counter that only grows and
  * waits until it has reached `target`.  All blocks are resident (cooperative
@@ -520,14 +594,16 @@ __device__ __forceinline__ bool grid_barrier(HydroStepControl *ctrl, unsigned &t
     return *ok != 0;
 }
 
-template <int LIM, int FIRST_ORDER, bool GRAV>
+template <int LIM, int FIRST_ORDER, bool GRAV, bool FUSED>
 __global__ void __launch_bounds__(kStagedThreads, MH2D_LOOP_CTAS)
 staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
 {
     constexpr int NT = kStagedThreads;
     __shared__ FluxShared sm;
-    __shared__ double red[2][NT / 32], s_dt, s_dtA[2];
+    __shared__ unsigned long long red[2][NT / 32];
+    __shared__ double s_dt, s_dtA[2];
     __shared__ int ok, failed;
+    __shared__ double v[1][NT / 2];
     HydroStepControl *ctrl = a.ctrl;
     volatile HydroStepControl *vc = ctrl;
     const int tid = threadIdx.x;
@@ -556,11 +632,16 @@ staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
             }
             return;
         }
-        for (unsigned k = blockIdx.x * NT + tid; k < recon; k += gridDim.x * NT)
-            staged_recon<LIM, FIRST_ORDER>(a, b, k, buf, n == 0, dtA);
-        if (!grid_barrier(ctrl, target, &ok)) return;
-        for (unsigned k = blockIdx.x * NT; k < faces; k += gridDim.x * NT)
-            staged_flux<false>(a, b, sm, k + tid, faces, dt);
+        if constexpr (FUSED) {
+            for (unsigned k = blockIdx.x * (NT / 2); k < faces; k += gridDim.x * (NT / 2))
+                staged_recon_flux<LIM, FIRST_ORDER>(a, b, sm, v, k, faces, dt, buf, n == 0, dtA);
+        } else {
+            for (unsigned k = blockIdx.x * NT + tid; k < recon; k += gridDim.x * NT)
+                staged_recon<LIM, FIRST_ORDER>(a, b, k, buf, n == 0, dtA);
+            if (!grid_barrier(ctrl, target, &ok)) return;
+            for (unsigned k = blockIdx.x * NT; k < faces; k += gridDim.x * NT)
+                staged_flux<false, true>(a, b, sm, k + tid, faces, dt);
+        }
         if (!grid_barrier(ctrl, target, &ok)) return;
         double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
         for (unsigned k = blockIdx.x * NT + tid; k < cells; k += gridDim.x * NT)

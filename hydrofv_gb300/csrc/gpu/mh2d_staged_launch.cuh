@@ -43,21 +43,37 @@ cudaError_t staged_launch_batch_recon(const StagedBatchArgs &b, const StagedBatc
     return launch_pdl(staged_batch_recon_kernel<LIM, FIRST_ORDER>, g.blocks[0], s, b, g.map[0]);
 }
 
-/* Blocks of the many-step kernel that are resident at once (0: it cannot be
- * launched), and its cooperative launch. */
+/* The many-step kernel for a grid: with gravity or without, faces and their
+ * states in one phase or in two. */
+typedef void (*StagedLoop)(Mh2dArgs<double>, Mh2dBand, int);
+
 template <int LIM, int FIRST_ORDER>
-int staged_loop_resident(bool gravity, int device)
+StagedLoop staged_loop(bool gravity, bool fused)
 {
+    if (gravity) return fused ? staged_loop_kernel<LIM, FIRST_ORDER, true, true> : staged_loop_kernel<LIM, FIRST_ORDER, true, false>;
+    return fused ? staged_loop_kernel<LIM, FIRST_ORDER, false, true> : staged_loop_kernel<LIM, FIRST_ORDER, false, false>;
+}
+
+inline bool staged_fused(const Mh2dArgs<double> &a, const Mh2dBand &b) { return staged_face_items(a.nx, b.r1 - b.r0) <= kStagedFusedFaces; }
+
+/* Blocks of the many-step kernel (0: it cannot be launched): as many as it has
+ * work for or as are resident at once; and its cooperative launch. */
+template <int LIM, int FIRST_ORDER>
+unsigned staged_loop_blocks(const Mh2dArgs<double> &a, const Mh2dBand &b, int device)
+{
+    const bool fused = staged_fused(a, b);
+    const int rows = b.r1 - b.r0;
+    const unsigned blocks = fused ? staged_blocks(2 * staged_face_items(a.nx, rows)) : staged_blocks(staged_recon_items(a.nx, rows));
     int per_sm = 0, sms = 0, coop = 0;
-    const cudaError_t e = gravity
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_loop_kernel<LIM, FIRST_ORDER, true>, kStagedThreads, 0)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_loop_kernel<LIM, FIRST_ORDER, false>, kStagedThreads, 0);
-    if (e != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_loop<LIM, FIRST_ORDER>(a.gravity != 0.0, fused), kStagedThreads,
+                                                      0) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    return coop ? per_sm * sms : 0;
+    const unsigned resident = coop ? (unsigned) (per_sm * sms) : 0u;
+    return blocks < resident ? blocks : resident;
 }
 
 template <int LIM, int FIRST_ORDER>
@@ -72,8 +88,7 @@ cudaError_t staged_launch_loop(const Mh2dArgs<double> &a, const Mh2dBand &b, uns
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return a.gravity != 0.0 ? cudaLaunchKernelEx(&cfg, staged_loop_kernel<LIM, FIRST_ORDER, true>, a, b, steps)
-                            : cudaLaunchKernelEx(&cfg, staged_loop_kernel<LIM, FIRST_ORDER, false>, a, b, steps);
+    return cudaLaunchKernelEx(&cfg, staged_loop<LIM, FIRST_ORDER>(a.gravity != 0.0, staged_fused(a, b)), a, b, steps);
 }
 
 }  // namespace hydro
@@ -81,7 +96,7 @@ cudaError_t staged_launch_loop(const Mh2dArgs<double> &a, const Mh2dBand &b, uns
 #define HYDRO_STAGED_INSTANTIATE(LIM, FO) \
     template cudaError_t staged_launch_recon<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, cudaStream_t); \
     template cudaError_t staged_launch_batch_recon<LIM, FO>(const StagedBatchArgs &, const StagedBatchGroup &, cudaStream_t); \
-    template int staged_loop_resident<LIM, FO>(bool, int);                                                           \
+    template unsigned staged_loop_blocks<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, int);                  \
     template cudaError_t staged_launch_loop<LIM, FO>(const Mh2dArgs<double> &, const Mh2dBand &, unsigned, int, cudaStream_t);
 
 #endif

@@ -842,6 +842,16 @@ HD double from_ordered_bits(unsigned long long e)
     return x;
 }
 
+#if defined(__CUDACC__)
+/* The warp's maximum of an ordered encoding (ordered_bits). */
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long b)
+{
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0u);
+    return ((unsigned long long) hi << 32) | lo;
+}
+#endif
+
 /* ---------------------------------------------------------------------- */
 /* Source terms (src/source_term.c).  One cell's update each, shared by    */
 /* the step kernels and the exported host functions.                       */

@@ -126,14 +126,6 @@ struct Lanes {
     int gt, GT;
 };
 
-/* The warp's maximum of an ordered encoding (ordered_bits). */
-__device__ __forceinline__ unsigned long long warp_max(unsigned long long b)
-{
-    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32));
-    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0u);
-    return ((unsigned long long) hi << 32) | lo;
-}
-
 /* The CTA's maximum of v (not NaN), encoded, written to *part (this CTA's
  * shared memory). */
 __device__ void block_partial_max(double v, unsigned long long *red, unsigned long long *part)

@@ -284,6 +284,22 @@ FXHD void predict(const Fm &f, double dtA, double dtA_rho, double rho, double n,
     hi[3] = half_step(p, f.add(zero_minus(draa), f.mul(um, d[3])), ph);
 }
 
+/* One side of predict: the state at the cell's high face or at its low one. */
+FXHD void predict_side(const Fm &f, bool high, double dtA, double dtA_rho, double rho, double n, double t, double p, double a,
+                       const double d[4], double d_rho_vel, double o[4])
+{
+    const double cn = f.mul(dtA, n);
+    const double u = f.add(f.one, high ? -cn : cn);
+    const double dr = f.mul(dtA, rho);
+    const double draa = f.mul(f.mul(f.mul(dr, a), a), d[1]);
+    const double drv = f.mul(dr, d_rho_vel), drp = f.mul(dtA_rho, d[3]);
+    const double h = high ? -f.mh : f.mh;
+    o[0] = half_step(rho, add_zero(f.add(f.mul(u, d[0]), high ? -drv : drv)), h);
+    o[1] = half_step(n, f.add(add_zero(f.mul(u, d[1])), high ? -drp : drp), h);
+    o[2] = half_step(t, add_zero(f.mul(u, d[2])), h);
+    o[3] = half_step(p, f.add(high ? zero_minus(draa) : add_zero(draa), f.mul(u, d[3])), h);
+}
+
 /* ------------------------------------------------------------------- HLLC */
 
 SLOW_PATH int classify_slow(const GasConst<double> &c, double rho_L, double u_L, double p_L, double rho_R, double u_R,
@@ -371,15 +387,27 @@ FXHD bool both_rarefactions(const Fm &f, const GasConst<double> &c, double u_L, 
     return have >= need && fx::finite(du);
 }
 
+template <bool INL>
+FXHD double dvx(double a, double b) { return INL ? dvi(a, b) : dv(a, b); }
+template <bool INL>
+FXHD double sqx(double x) { return INL ? sqi(x) : sq(x); }
+
+template <bool INL = false>
 FXHD double face_tsrs(const Fm &f, const GasConst<double> &c, double rho_L, double u_L, double p_L, double rho_R,
                       double u_R, double p_R, double ppv, double &gL, double &gR)
 {
-    gL = sq(dv(dv(2.0, f.mul(c.gp1, rho_L)), f.add(ppv, f.mul(p_L, c.gm1_gp1))));
-    gR = sq(dv(dv(2.0, f.mul(c.gp1, rho_R)), f.add(ppv, f.mul(p_R, c.gm1_gp1))));
-    return dv(f.sub(f.add(f.mul(gL, p_L), f.mul(gR, p_R)), f.sub(u_R, u_L)), f.add(gL, gR));
+    gL = sqx<INL>(dvx<INL>(dvx<INL>(2.0, f.mul(c.gp1, rho_L)), f.add(ppv, f.mul(p_L, c.gm1_gp1))));
+    gR = sqx<INL>(dvx<INL>(dvx<INL>(2.0, f.mul(c.gp1, rho_R)), f.add(ppv, f.mul(p_R, c.gm1_gp1))));
+    return dvx<INL>(f.sub(f.add(f.mul(gL, p_L), f.mul(gR, p_R)), f.sub(u_R, u_L)), f.add(gL, gR));
 }
 
-/* hllc_finish (numerics.cuh); `plain` from face_classify. */
+/* hllc_finish (numerics.cuh); `plain` from face_classify.  INL puts the
+ * quotients and roots in line, so that independent ones overlap: faster where
+ * a warp is alone on its scheduler (the many-step kernel: 64^2 23.7 -> 22.4 us a step, 256^2
+ * 52.7 -> 50.6, with the maxima on the integer pipe), slower where
+ * the code no longer fits the instruction cache (2048^2: 2.31 ms a step
+ * against 2.24). */
+template <bool INL = false>
 FXHD int face_finish(const Fm &f, const GasConst<double> &c, bool plain, double rho_L, double u_L, double v_L, double p_L,
                      double a_L, double rho_R, double u_R, double v_R, double p_R, double a_R, double pg, double F[4],
                      double wave[3])
@@ -390,18 +418,18 @@ FXHD int face_finish(const Fm &f, const GasConst<double> &c, bool plain, double 
     double q_L = 1.0, q_R = 1.0, aq_L = a_L, aq_R = a_R;
     const fx::i64 bs = (fx::i64) fx::bits(ps);
     if (bs > (fx::i64) fx::bits(p_L)) {
-        q_L = sq(f.add(f.one, f.mul(c.q_coef, diff(f, dv(ps, p_L), 1.0))));
+        q_L = sqx<INL>(f.add(f.one, f.mul(c.q_coef, diff(f, dvx<INL>(ps, p_L), 1.0))));
         aq_L = f.mul(a_L, q_L);
     }
     if (bs > (fx::i64) fx::bits(p_R)) {
-        q_R = sq(f.add(f.one, f.mul(c.q_coef, diff(f, dv(ps, p_R), 1.0))));
+        q_R = sqx<INL>(f.add(f.one, f.mul(c.q_coef, diff(f, dvx<INL>(ps, p_R), 1.0))));
         aq_R = f.mul(a_R, q_R);
     }
     const double S_L = f.sub(u_L, aq_L), S_R = f.add(u_R, aq_R);
     const double d_L = f.sub(S_L, u_L), d_R = f.sub(S_R, u_R);
     const double m_L = f.mul(rho_L, u_L), m_R = f.mul(rho_R, u_R);
     const double rd_L = f.mul(rho_L, d_L), rd_R = f.mul(rho_R, d_R);
-    const double S_s = dv(f.sub(f.add(diff(f, p_R, p_L), f.mul(m_L, d_L)), f.mul(m_R, d_R)), f.sub(rd_L, rd_R));
+    const double S_s = dvx<INL>(f.sub(f.add(diff(f, p_R, p_L), f.mul(m_L, d_L)), f.mul(m_R, d_R)), f.sub(rd_L, rd_R));
     if (!fx::finite(S_L) || !fx::finite(S_R) || !fx::finite(S_s))
         return finish_slow(c, rho_L, u_L, v_L, p_L, a_L, rho_R, u_R, v_R, p_R, a_R, pg, F, wave);
     wave[0] = q_L;
@@ -412,14 +440,14 @@ FXHD int face_finish(const Fm &f, const GasConst<double> &c, bool plain, double 
     const bool star = left ? !beyond_L : fx::not_below_zero(S_R);
     const double rho = left ? rho_L : rho_R, u = left ? u_L : u_R, v = left ? v_L : v_R, p = left ? p_L : p_R;
     const double m = left ? m_L : m_R, S = left ? S_L : S_R, rd = left ? rd_L : rd_R;
-    const double E = f.mul(rho, fma(-f.mh, f.add(f.mul(u, u), f.mul(v, v)), dv(p, f.mul(rho, c.gm1))));
+    const double E = f.mul(rho, fma(-f.mh, f.add(f.mul(u, u), f.mul(v, v)), dvx<INL>(p, f.mul(rho, c.gm1))));
     F[0] = m;
     F[1] = f.add(f.mul(m, u), p);
     F[2] = f.mul(m, v);
     F[3] = f.mul(u, f.add(E, p));
     if (star) {
-        const double rs = dv(rd, f.sub(S, S_s));
-        const double es = f.mul(rs, f.add(dv(E, rho), f.mul(f.sub(S_s, u), f.add(S_s, dv(p, rd)))));
+        const double rs = dvx<INL>(rd, f.sub(S, S_s));
+        const double es = f.mul(rs, f.add(dvx<INL>(E, rho), f.mul(f.sub(S_s, u), f.add(S_s, dvx<INL>(p, rd)))));
         F[0] = f.add(m, f.mul(S, diff(f, rs, rho)));
         F[1] = f.add(F[1], f.mul(S, f.sub(f.mul(rs, S_s), m)));
         F[2] = f.add(F[2], f.mul(S, diff(f, f.mul(rs, v), f.mul(rho, v))));
