@@ -171,7 +171,7 @@ HD double slope_partials(double wm, double w0, double wp, double &da, double &db
 {
 #if defined(__CUDA_ARCH__)
     double s;
-    if (LIM != LIM_VAN_LEER && near_slope<LIM>(wm, w0, wp, s, code)) {
+    if (LIM != LIM_VAN_LEER && near_slope<LIM>(Fm(), wm, w0, wp, s, code)) {
         const double one = LIM == LIM_MINMOD ? 1.0 : code == 1 ? 0.5 : 2.0;
         da = (LIM == LIM_MINMOD ? code == 1 : code == 1 || code == 2) ? one : 0.0;
         db = (LIM == LIM_MINMOD ? code == 2 : code == 1 || code == 3) ? one : 0.0;

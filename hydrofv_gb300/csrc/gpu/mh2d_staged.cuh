@@ -26,9 +26,9 @@
  * gravity 282 -> 58, 401 x 250 van Leer 308 -> 113, 1024^2 blast 0.86 -> 0.65
  * ms, 2048^2 3.25 -> 3.07 ms.
  *
- * Blocks per SM (registers): flux 5 / 6 / 7 (96 / 80 / 72) takes 1.99 / 1.95 /
- * 2.00 ms a step at 2048^2; recon is the same with 5 to 8; update 5 / 6 / 8
- * takes 2.25 / 2.27 / 2.26.
+ * Blocks per SM: flux 4 / 5 / 6 / 7 takes 1.99 / 1.89 / 1.90 / 1.88 ms a step
+ * on the 2048^2 shear layer and 0.356 / 0.338 / 0.347 / 0.348 on the 1024^2
+ * blast; recon is the same with 5 to 8, update with 4 to 6.
  */
 #ifndef HYDRO_GPU_MH2D_STAGED_CUH
 #define HYDRO_GPU_MH2D_STAGED_CUH
@@ -40,7 +40,7 @@
 #define MH2D_RECON_CTAS 6
 #endif
 #ifndef MH2D_FLUX_CTAS
-#define MH2D_FLUX_CTAS 6
+#define MH2D_FLUX_CTAS 5
 #endif
 #ifndef MH2D_UPDATE_CTAS
 #define MH2D_UPDATE_CTAS 5

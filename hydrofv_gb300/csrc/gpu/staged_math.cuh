@@ -10,8 +10,10 @@
  *    a + b and a * b.  A GB300 SM retires a DFMA with three register operands
  *    every 16 cycles per warp, but a DADD, a DMUL or a DFMA with a constant
  *    or immediate operand every 19 (measured with 4 to 24 warps on one SM).
- *    The two constants are read from memory so that the compiler cannot turn
- *    the fma back into an add or a multiply.
+ *    The constants are read from memory so that the compiler cannot turn the
+ *    fma back into an add or a multiply; through the read-only path, which
+ *    keeps them in L1 (volatile loads, which go to L2, took 70.8 us a step of
+ *    316^2 where these take 65.8).
  *  - Scalings by powers of two go into an fma (x - 0.5 s as fma(-0.5, s, x):
  *    0.5 s is exact, so the one rounding is the sum's) or become an exponent
  *    step on the integer pipe.
@@ -62,9 +64,9 @@ FXHD Fm make_fm()
 {
     Fm f;
 #if defined(__CUDA_ARCH__)
-    f.one = *(volatile double *) &d_fma_const[0];
-    f.mz = *(volatile double *) &d_fma_const[1];
-    f.mh = *(volatile double *) &d_fma_const[2];
+    f.one = __ldg(&d_fma_const[0]);
+    f.mz = __ldg(&d_fma_const[1]);
+    f.mh = __ldg(&d_fma_const[2]);
 #else
     f.one = 1.0;
     f.mz = -0.0;
@@ -198,10 +200,11 @@ FXHD double slope(const Fm &f, double a, double b)
  * sum and the limited value (in half units) are exact as integers and as
  * doubles, so minmod and MC take no FP64 instruction.  recon of the 1024^2
  * shear layer, MC: 66 FP64 instructions a cell where there were 88, 160 -> 128
- * us.
+ * us.  Van Leer keeps the product, the 1e-10 and the quotient (1024^2, a whole
+ * step: 516 us, 530 with the quotient called and a + b on the FP64 pipe).
  */
 template <int LIM>
-FXHD bool near_slope(double wm, double w, double wp, double &s, int &code)
+FXHD bool near_slope(const Fm &f, double wm, double w, double wp, double &s, int &code)
 {
     const unsigned em = fx::hi(wm) >> 20, ec = fx::hi(w) >> 20, ep = fx::hi(wp) >> 20;      /* with the sign */
     const unsigned e = fx::least(fx::least(em, ec), ep), up = fx::most(fx::most(em, ec), ep);
@@ -216,9 +219,9 @@ FXHD bool near_slope(double wm, double w, double wp, double &s, int &code)
     if ((unsigned) ((fx::u64) (x | y) >> 52) != 0u) return false;
     code = 1;
     if (LIM == LIM_VAN_LEER) {
-        const Fm f = make_fm();
-        const double a = fx::scaled((fx::u64) x, e & 0x7ffu, sign), b = fx::scaled((fx::u64) y, e & 0x7ffu, sign);
-        s = dv(f.mul(fx::twice(a), b), f.add(f.add(a, b), 1e-10));
+        const unsigned q = e & 0x7ffu;
+        const double a = fx::scaled((fx::u64) x, q, sign), b = fx::scaled((fx::u64) y, q, sign);
+        s = dvi(f.mul(fx::twice(a), b), f.add(fx::scaled((fx::u64) (x + y), q, sign), 1e-10));
         return true;
     }
     const fx::i64 m = x < y ? x : y;
@@ -238,7 +241,7 @@ FXHD double slope_of(const Fm &f, double wm, double w, double wp)
 {
     double s;
     int code;
-    if (near_slope<LIM>(wm, w, wp, s, code)) return s;
+    if (near_slope<LIM>(f, wm, w, wp, s, code)) return s;
     /* gas at rest beside gas at rest */
     if ((fx::bits(w) == fx::bits(wm) || fx::bits(w) == fx::bits(wp)) && fx::finite(wm) && fx::finite(wp)) return 0.0;
     return slope<LIM>(f, f.sub(w, wm), f.sub(wp, w));
