@@ -53,6 +53,24 @@ int mh2d_fp32_chunk(int slots, Items items)
     return best;
 }
 
+/* Launch with programmatic stream serialization: the launch is processed
+ * while the kernel before it in the stream runs; the step kernels wait for that
+ * kernel's completion before they read or write (pdl_wait). */
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t s, const A &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 /* Work items of c rows of an nx x ny grid. */
 inline long long mh2d_item_count(int nx, int ny, int strip_w, int c)
 {

@@ -161,12 +161,12 @@ __device__ __forceinline__ void next_dt(const Mh2dArgs<R> &a, const HydroStepCon
 {
     const bool y = threadIdx.x & 1;
     const double S = from_ordered_bits(*(const volatile unsigned long long *) &ctrl->smax[n % 3][y]);
-    const double q = dv(S, y ? a.dy : a.dx);
+    const double q = dvi(S, y ? a.dy : a.dx);
     const double qx = __shfl_sync(0xffffffffu, q, 0), qy = __shfl_sync(0xffffffffu, q, 1);
     const double cfl = (n < a.sp.shrink_steps) ? a.sp.cfl_shrunk : a.sp.cfl;
-    dt = dv(cfl, qx + qy);
+    dt = dvi(cfl, qx + qy);
     if (t + dt > tf) dt = tf - t;
-    dtA = dv(dt * (y ? a.area_y : a.area_x), a.vol);
+    dtA = dvi(dt * (y ? a.area_y : a.area_x), a.vol);
 }
 
 template <class R>
@@ -284,7 +284,7 @@ struct Mh2dShared {
     int nT, nS;
     int item;
     int am_last;
-    double red[2][NT / 32];
+    unsigned long long red[2][NT / 32];
     /* FP64: the state each interior thread carries up its column (see
      * mh2d_item); FP32 keeps it in registers and these are unused */
     static constexpr int CQ = sizeof(R) == 8 ? 4 : 1;
@@ -812,17 +812,53 @@ __device__ __forceinline__ void advance_clock(const Mh2dArgs<R> &a, HydroStepCon
  * SMs that finish early take more work (the FP64 pipe of an SM is shared by
  * its CTAs).
  */
+/* Fold a block's maxima into the next step's words (threads 0 and 1 write
+ * them).  The maxima are never NaN; their ordered encodings (ordered_bits)
+ * reduce on the integer pipe. */
+template <int NT>
+__device__ __forceinline__ void block_maxima(HydroStepControl *ctrl, unsigned long long (*red)[NT / 32], long long n, double mx_x,
+                                             double mx_y)
+{
+    const int tid = threadIdx.x;
+    const unsigned long long bx = warp_max(ordered_bits(mx_x)), by = warp_max(ordered_bits(mx_y));
+    if ((tid & 31) == 0) {
+        red[0][tid >> 5] = bx;
+        red[1][tid >> 5] = by;
+    }
+    __syncthreads();
+    if (tid < 2) {
+        unsigned long long b = red[tid][0];
+        for (int w = 1; w < NT / 32; w++)
+            if (red[tid][w] > b) b = red[tid][w];
+        unsigned long long *word = &ctrl->smax[(n + 1) % 3][tid];
+        if (b > *(volatile unsigned long long *) word) atomicMax(word, b);
+    }
+    __syncwarp();
+}
+
+/* Programmatic dependent launch: wait for the previous kernel's results.
+ * Nothing triggers the next kernel early: blocks that became resident at the
+ * start of the kernel before theirs made a step slower (64^2 37 us against
+ * 26, 128^2 48 against 29), and without the attribute it is 27 and 30. */
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <class R, int LIM, int NT, int FIRST_ORDER, bool GRAV = false>
 __global__ void __launch_bounds__(NT, (sizeof(R) == 4 ? MH2D_CTAS_FP32 : MH2D_CTAS_FP64))
 mh2d_step_kernel(const Mh2dArgs<R> a)
 {
     static_assert(NT % 32 == 0, "NT must be a whole number of warps");
+    pdl_wait();
     HydroStepControl *ctrl = a.ctrl;
-    if (!*(volatile int *) &ctrl->active) return;
-
+    /* (plain loads: one miss per SM; volatile ones go to L2 from every warp and
+     * took 16.1 us a step of 301 x 200 where these take 13.7) */
+    const int active = ctrl->active;
     const long long n = ctrl->num_steps;
     const double t_now = ctrl->t, tf = ctrl->tf, dt = ctrl->step_dt;
     const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
+    if (!active) return;
     if (dt == 0.0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             ctrl->dt = dt;
@@ -838,39 +874,21 @@ mh2d_step_kernel(const Mh2dArgs<R> a)
     double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
     int err = DEV_OK;
 
-    for (;;) {
-        if (tid == 0) sm.item = atomicAdd(&ctrl->work_next, 1);
-        __syncthreads();
-        const int item = sm.item;
-        __syncthreads();
-        if (item >= n_items) break;
+    /* the first item by the CTA's index, the others from the queue */
+    for (int item = (int) blockIdx.x; item < n_items;) {
         mh2d_item<R, LIM, NT, FIRST_ORDER, GRAV>(a, sm, item, n, dt, dtA, mx_x, mx_y, err);
+        if (n_items <= (int) gridDim.x) break;
+        if (tid == 0) sm.item = (int) gridDim.x + atomicAdd(&ctrl->work_next, 1);
+        __syncthreads();
+        item = sm.item;
+        __syncthreads();
     }
 
     if (err) record_error(ctrl, err, (int) blockIdx.x);
 
     /* ---- CTA maxima -> device maxima for the next step's dt ---- */
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ox = __shfl_xor_sync(0xffffffffu, mx_x, o);
-        const double oy = __shfl_xor_sync(0xffffffffu, mx_y, o);
-        if (ox > mx_x) mx_x = ox;
-        if (oy > mx_y) mx_y = oy;
-    }
-    if ((tid & 31) == 0) {
-        sm.red[0][tid >> 5] = mx_x;
-        sm.red[1][tid >> 5] = mx_y;
-    }
-    __syncthreads();
+    block_maxima<NT>(ctrl, sm.red, n, mx_x, mx_y);
     if (tid == 0) {
-        double bx = sm.red[0][0], by = sm.red[1][0];
-        for (int w = 1; w < NT / 32; w++) {
-            if (sm.red[0][w] > bx) bx = sm.red[0][w];
-            if (sm.red[1][w] > by) by = sm.red[1][w];
-        }
-        const int nxt = (int) ((n + 1) % 3);
-        atomicMax(&ctrl->smax[nxt][0], ordered_bits(bx));
-        atomicMax(&ctrl->smax[nxt][1], ordered_bits(by));
         __threadfence();
         sm.am_last = (atomicAdd(&ctrl->blocks_done, 1u) == gridDim.x - 1);
     }
@@ -918,6 +936,7 @@ template <class R, int LIM, int NT, int FIRST_ORDER>
 __global__ void __launch_bounds__(NT, (sizeof(R) == 4 ? MH2D_CTAS_FP32 : MH2D_CTAS_FP64))
 mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
 {
+    pdl_wait();
     __shared__ Mh2dShared<R, NT> sm;
     __shared__ int s_inst, s_local, s_go, s_last;
     __shared__ long long s_n;
@@ -964,28 +983,9 @@ mh2d_batch_step_kernel(const Mh2dBatchArgs<R> b)
         int err = DEV_OK;
         mh2d_item<R, LIM, NT, FIRST_ORDER>(a, sm, local, n, dt, dtA, mx_x, mx_y, err);
         if (err) record_error(a.ctrl, err, inst);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ox = __shfl_xor_sync(0xffffffffu, mx_x, o);
-            const double oy = __shfl_xor_sync(0xffffffffu, mx_y, o);
-            if (ox > mx_x) mx_x = ox;
-            if (oy > mx_y) mx_y = oy;
-        }
-        if ((tid & 31) == 0) {
-            sm.red[0][tid >> 5] = mx_x;
-            sm.red[1][tid >> 5] = mx_y;
-        }
-        __syncthreads();
+        block_maxima<NT>(a.ctrl, sm.red, n, mx_x, mx_y);
         if (tid == 0) {
-            double bx = sm.red[0][0], by = sm.red[1][0];
-            for (int w = 1; w < NT / 32; w++) {
-                if (sm.red[0][w] > bx) bx = sm.red[0][w];
-                if (sm.red[1][w] > by) by = sm.red[1][w];
-            }
             HydroStepControl *ctrl = a.ctrl;
-            const int nxt = (int) ((n + 1) % 3);
-            atomicMax(&ctrl->smax[nxt][0], ordered_bits(bx));
-            atomicMax(&ctrl->smax[nxt][1], ordered_bits(by));
             __threadfence();
             const int n_items = b.item_off[inst + 1] - b.item_off[inst];
             s_last = (atomicAdd(&ctrl->blocks_done, 1u) == (unsigned) (n_items - 1));

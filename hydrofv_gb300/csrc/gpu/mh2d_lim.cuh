@@ -7,6 +7,7 @@
 #ifndef HYDRO_GPU_MH2D_LIM_CUH
 #define HYDRO_GPU_MH2D_LIM_CUH
 
+#include "gpu_internal.h"
 #include "mh2d_launch.cuh"
 
 namespace hydro {
@@ -14,18 +15,16 @@ namespace hydro {
 template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_step_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s)
 {
-    if (a.gravity != 0.0)
-        mh2d_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER, true><<<grid, mh2d_threads<R>(), 0, s>>>(a);
-    else
-        mh2d_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER><<<grid, mh2d_threads<R>(), 0, s>>>(a);
-    return cudaGetLastError();
+    constexpr int nt = mh2d_threads<R>();
+    return a.gravity != 0.0 ? launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, true>, grid, nt, s, a)
+                            : launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, false>, grid, nt, s, a);
 }
 
 template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_batch_lim(const Mh2dBatchArgs<R> &b, int grid, cudaStream_t s)
 {
-    mh2d_batch_step_kernel<R, LIM, mh2d_threads<R>(), FIRST_ORDER><<<grid, mh2d_threads<R>(), 0, s>>>(b);
-    return cudaGetLastError();
+    constexpr int nt = mh2d_threads<R>();
+    return launch_after(mh2d_batch_step_kernel<R, LIM, nt, FIRST_ORDER>, grid, nt, s, b);
 }
 
 template <class R, int LIM, int FIRST_ORDER>

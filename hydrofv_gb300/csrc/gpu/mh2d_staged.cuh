@@ -84,15 +84,6 @@ enum : int { WS_XLO = 0, WS_XHI = 4, WS_YLO = 8, WS_YHI = 12, WS_FIELDS = 16 };
 inline __host__ __device__ unsigned staged_recon_items(int nx, int rows) { return (unsigned) rows * (nx + 2) + (unsigned) (rows + 2) * nx; }
 inline __host__ __device__ unsigned staged_face_items(int nx, int rows) { return (unsigned) rows * (nx + 1) + (unsigned) (rows + 1) * nx; }
 
-/* Programmatic dependent launch: wait for the previous kernel's results.
- * Nothing triggers the next kernel early: blocks that became resident at the
- * start of the kernel before theirs made a step slower (64^2 37 us against
- * 26, 128^2 48 against 29), and without the attribute it is 27 and 30. */
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 /* Face states of item k of the band: first the x items (rows r0 .. r1-1,
  * columns g-1 .. g+nx), then the y items (rows r0-1 .. r1, columns g ..
  * g+nx-1). */
@@ -372,29 +363,6 @@ struct UpdateShared {
     int am_last;
 };
 
-/* Fold a block's maxima into the next step's words (threads 0 and 1 write
- * them).  The maxima are never NaN; their ordered encodings (ordered_bits)
- * reduce on the integer pipe. */
-__device__ __forceinline__ void block_maxima(HydroStepControl *ctrl, unsigned long long (*red)[kStagedThreads / 32], long long n,
-                                             double mx_x, double mx_y)
-{
-    const int tid = threadIdx.x;
-    const unsigned long long bx = warp_max(ordered_bits(mx_x)), by = warp_max(ordered_bits(mx_y));
-    if ((tid & 31) == 0) {
-        red[0][tid >> 5] = bx;
-        red[1][tid >> 5] = by;
-    }
-    __syncthreads();
-    if (tid < 2) {
-        unsigned long long b = red[tid][0];
-        for (int w = 1; w < kStagedThreads / 32; w++)
-            if (red[tid][w] > b) b = red[tid][w];
-        unsigned long long *word = &ctrl->smax[(n + 1) % 3][tid];
-        if (b > *(volatile unsigned long long *) word) atomicMax(word, b);
-    }
-    __syncwarp();
-}
-
 /* End of an update block: fold its maxima into the next step's words; the
  * last block of the grid advances the clock (src/integrator_muscl_hancock.c:
  * 1143-1154) and forms the next dt. */
@@ -403,7 +371,7 @@ __device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateS
 {
     const int tid = threadIdx.x;
     HydroStepControl *ctrl = a.ctrl;
-    block_maxima(ctrl, sm.red, n, mx_x, mx_y);
+    block_maxima<kStagedThreads>(ctrl, sm.red, n, mx_x, mx_y);
     if (tid == 0) {
         __threadfence();
         sm.am_last = atomicAdd(&ctrl->blocks_done, 1u) == blocks - 1;
@@ -418,10 +386,10 @@ __device__ __forceinline__ void staged_finish(const Mh2dArgs<double> &a, UpdateS
  * dt is zero, which the recon kernel records). */
 __device__ __forceinline__ bool staged_step(HydroStepControl *ctrl, long long &n, double &dt)
 {
-    if (!*(volatile int *) &ctrl->active) return false;
+    const int active = ctrl->active;
     n = ctrl->num_steps;
     dt = ctrl->step_dt;
-    return dt != 0.0;
+    return active && dt != 0.0;
 }
 
 /* A step that was due but has a zero dt. */
@@ -443,13 +411,13 @@ staged_recon_kernel(const Mh2dArgs<double> a, const Mh2dBand b)
     long long n;
     double dt;
     HydroStepControl *ctrl = a.ctrl;
+    const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
     if (!staged_step(ctrl, n, dt)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) record_zero_dt(ctrl);
         return;
     }
     const unsigned k = blockIdx.x * kStagedThreads + threadIdx.x;
     if (k >= staged_recon_items(a.nx, b.r1 - b.r0)) return;
-    const double dtA[2] = { ctrl->step_dtA[0], ctrl->step_dtA[1] };
     staged_recon<LIM, FIRST_ORDER>(a, b, k, (int) (n & 1), n == 0, dtA);
 }
 
@@ -646,7 +614,7 @@ staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
         double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
         for (unsigned k = blockIdx.x * NT + tid; k < cells; k += gridDim.x * NT)
             staged_update<GRAV>(f, a, b, k, buf, dt, mx_x, mx_y);
-        block_maxima(ctrl, red, n, mx_x, mx_y);
+        block_maxima<NT>(ctrl, red, n, mx_x, mx_y);
         if (!grid_barrier(ctrl, target, &ok)) return;
         /* every block: the next dt; block 0 publishes the clock */
         if (tid < 32) {

@@ -11,22 +11,10 @@
 
 namespace hydro {
 
-/* Launch with programmatic stream serialization: the launch is processed
- * while the kernel before it in the stream runs; every staged kernel waits
- * for that kernel's completion before it reads or writes (pdl_wait). */
 template <class... P, class... A>
 cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, cudaStream_t s, const A &...args)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kStagedThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return launch_after(kernel, grid, kStagedThreads, s, args...);
 }
 
 inline unsigned staged_blocks(unsigned items) { return (items + kStagedThreads - 1) / kStagedThreads; }
