@@ -22,17 +22,17 @@ namespace hydro {
  * Rows per work item of the FP32 step when the caller sets none.  The step's
  * CTAs are persistent (one per resident slot) and take (strip, row chunk)
  * items from a queue.  An item of c rows also reconstructs the rows below it
- * (0.95 of a row's work: 2048^2 takes 317 / 244 / 182 us a step with 1 / 2 /
+ * (0.95 of a row's work: 2048^2 takes 317 / 244 / 179 us a step with 1 / 2 /
  * 12 rows), and the last items run while other slots are already idle.  In
  * units of a row's work with all slots busy (5.0 us) a step is modelled as
  *     items (c + 0.95) / slots + 1.2 + 0.24 c,
  * and as no less than an item alone, 2.1 + 0.48 c.  `items` gives the number
  * of items for a height.
  * Measured on 1064 slots, this choice / the best of 1 .. 64 rows / 32 rows, us
- * a step: 64^2 12.8 (1 row) / 12.8 / 85, 301 x 200 15.2 (1) / 15.2 / 93, 512^2
- * 26.5 (3) / 26.5 / 94, 700 x 900 44.8 (4) / 40.4 / 100, 1024^2 64.0 (6) / 63.9
- * / 103, 2048^2 181 (12) / 181 / 212, 4096^2 603 (24) / 594 / 594; 28 grids of
- * side 128 to 640 258 (12) / 258 / 298, 60 of side 500 to 900 1257 (24) / 1253
+ * a step: 64^2 11.0 (1 row) / 11.0 / 86, 301 x 200 13.2 (1) / 13.2 / 94, 512^2
+ * 23.8 (3) / 23.7 / 94, 700 x 900 42.9 (4) / 37.8 / 102, 1024^2 61.7 (6) / 61.7
+ * / 103, 2048^2 179 (12) / 179 / 216, 4096^2 601 (24) / 600 / 600; 28 grids of
+ * side 128 to 640 256 (12) / 256 / 300, 60 of side 500 to 900 1251 (24) / 1251
  * / 1253.
  */
 template <class Items>
