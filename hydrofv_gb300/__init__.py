@@ -195,6 +195,7 @@ _SIGNATURES = {
     "hydro_fx_quot_le_host": (None, [C.c_longlong, _dp, _dp, _dp, C.c_void_p, C.c_void_p]),
     "hydro_gpu_pointwise_eval": (C.c_int, [C.c_int, C.c_int, C.c_longlong, _dp, C.c_double, _dp, _dp, _dp,
                                            _dp, _P(C.c_int)]),
+    "hydro_gpu_fp32_eval": (C.c_int, [C.c_int, C.c_int, C.c_longlong] + [C.c_double] * 3 + [_P(C.c_float)] * 4),
     "hydro_gpu_device_count": (C.c_int, []),
     "hydro_gpu_calibrate": (C.c_int, [C.c_int, _dp, _dp]),
     "hydro_gpu_sm_count": (C.c_int, [C.c_int]),
@@ -957,6 +958,25 @@ def gpu_pointwise_eval(name, gamma, L, R, aux=None, tol=1e-6, device=0):
     if code != 0:
         raise HydroError(code, "hydro_gpu_pointwise_eval failed (CUDA error)")
     return (out if width == 1 else out.reshape(n, width)), rc
+
+
+FP32_OPS = {"flux": 0, "primitive": 1, "slope_minmod": 2, "slope_van_leer": 3, "slope_mc": 4, "quotient": 5, "root": 6}
+
+
+def gpu_fp32_eval(name, a, b=None, gamma=1.4, tol=1e-6, vol=1.0, device=0):
+    """The FP32 step's short form and general form of the same operands on
+    the GPU (hydro_gpu_fp32_eval): two float32 arrays."""
+    op = FP32_OPS[name]
+    a = np.ascontiguousarray(a, dtype=np.float32).reshape((-1, 4) if op <= 1 else (-1,))
+    b = np.ascontiguousarray(a if b is None else b, dtype=np.float32).reshape(a.shape)
+    fast = np.empty((len(a), 5) if op <= 1 else len(a), dtype=np.float32)
+    general = np.empty_like(fast)
+    p = lambda x: x.ctypes.data_as(_P(C.c_float))
+    code = library().hydro_gpu_fp32_eval(int(device), op, len(a), float(gamma), float(tol), float(vol), p(a), p(b),
+                                         p(fast), p(general))
+    if code != 0:
+        raise HydroError(code, "hydro_gpu_fp32_eval failed (CUDA error)")
+    return fast, general
 
 
 def fx_div_seeded_host(a, b, seed_scale):

@@ -1,23 +1,24 @@
 /*
- * fast32.cuh -- the FP32 state form's quotients, square roots and powers in
- * two or three instructions.
+ * fast32.cuh -- the FP32 state form's quotients, square roots and powers for
+ * ordinary operands.
  *
  * The FP32 step is bound by instruction issue.  Its unit is compiled with
- * approximate division and square root (at most 2 ulp), but the compiler's
- * general forms also cover operands and results outside the normal range:
- * about six instructions more for each quotient, four for each root.  Fast
- * wraps a float whose quotient is a * rcp.approx.ftz(b), whose root is
- * sqrt.approx.ftz and whose power is ex2(y lg2(x)).  For normal operands and
- * divisors below 2^126 these give the bits of the general forms, so the
- * templates of numerics.cuh instantiated with Fast give those of the same
- * templates with float (tests/test_gpu_fast32.py).  A face or cell is checked
- * once, for bounds under which every divisor and root is a normal number, and
- * takes the general instantiation, out of line, where the check fails or the
- * face opens a vacuum.
+ * approximate division and square root (at most 2 ulp over the whole range of
+ * float); most of its operands are ordinary numbers, for which a quotient is
+ * two instructions and a root one.  Fast wraps a float whose quotient is
+ * a * (1 / b) with the hardware's reciprocal (the definition that the PTX ISA
+ * gives for div.approx: at most 2 ulp for a divisor of 2^-126 to 2^126), whose
+ * root is PTX's sqrt.approx.ftz and whose power is CUDA's __powf, so the
+ * templates of numerics.cuh can be instantiated with it.  A face or cell is
+ * checked once, for bounds under which every divisor and root is a normal
+ * number, and takes the general instantiation, out of line, where the check
+ * fails or the face opens a vacuum.  tests/test_gpu_fp32_forms.py holds the
+ * quotient and the root to those bounds and the faces, cells and slopes to the
+ * general forms' bits.
  *
  * Shear 2048^2, 100 steps: 0.237 ms a step with the general forms, 0.227 with
- * the slopes alone, 0.187 with slopes, faces and primitives, 0.182 with vacuum
- * faces in the out-of-line form too.
+ * the slopes alone, 0.182 with slopes, faces and primitives, vacuum faces in
+ * the out-of-line form.
  */
 #ifndef HYDRO_GPU_FAST32_CUH
 #define HYDRO_GPU_FAST32_CUH
@@ -44,9 +45,8 @@ __device__ __forceinline__ bool operator<=(Fast a, Fast b) { return a.v <= b.v; 
 __device__ __forceinline__ bool operator>(Fast a, Fast b) { return a.v > b.v; }
 __device__ __forceinline__ bool operator>=(Fast a, Fast b) { return a.v >= b.v; }
 
-/* The general quotient is one opaque instruction until the assembler expands
- * it; its last product is then contracted with a following sum where one is
- * free.  The same two instructions in one asm give the same contractions. */
+/* a / b as a * (1 / b), and the root: PTX instructions with subnormals taken
+ * as zero. */
 __device__ __forceinline__ float fast_div(float a, float b)
 {
     float q;
@@ -61,20 +61,10 @@ __device__ __forceinline__ float fast_sqrt(float x)
     return r;
 }
 
-__device__ __forceinline__ float fast_pow(float x, float y)
-{
-    float q;
-    asm("{\n\t.reg .f32 t;\n\tlg2.approx.ftz.f32 t, %1;\n\tmul.f32 t, t, %2;\n\tex2.approx.f32 %0, t;\n\t}"
-        : "=f"(q) : "f"(x), "f"(y));
-    return q;
-}
-
 __device__ __forceinline__ Fast dv(Fast a, Fast b) { return Fast(fast_div(a.v, b.v)); }
 __device__ __forceinline__ Fast sq(Fast x) { return Fast(fast_sqrt(x.v)); }
-__device__ __forceinline__ Fast pw(Fast x, Fast y) { return Fast(fast_pow(x.v, y.v)); }
-/* A product that the sum after it does not take in (hllc_finish, the energy
- * flux: the general form's quotients end the block that holds the product). */
-__device__ __forceinline__ Fast prod(Fast a, Fast b) { return Fast(__fmul_rn(a.v, b.v)); }
+__device__ __forceinline__ Fast pw(Fast x, Fast y) { return Fast(__powf(x.v, y.v)); }
+__device__ __forceinline__ Fast prod(Fast a, Fast b) { return Fast(prod(a.v, b.v)); }
 __device__ __forceinline__ Fast operator/(Fast a, Fast b) { return dv(a, b); }
 
 /* Densities and pressures in 1e-12 .. 1e8 and |u| < 1e8: a star pressure is

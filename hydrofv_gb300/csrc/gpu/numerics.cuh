@@ -423,8 +423,20 @@ HD void hllc_vacuum_flux(const GasConst<R> &c, R rho_L, R u_L, R v_L, R p_L, R a
     F[3] = s[1] * (E + s[3]);
 }
 
+/* a * b rounded by itself: a float product is not fused with the sum after it,
+ * so that the energy flux is the same in every instantiation of hllc_finish
+ * (double is compiled without contraction). */
 template <class R>
 HD R prod(R a, R b) { return a * b; }
+
+HD float prod(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
 
 /* From the (unfloored) star-pressure guess to the flux.  Returns DEV_OK or
  * DEV_ERR_HLLC_WAVE_SPEED.  wave (may be null) receives q_L, q_R and S*, the

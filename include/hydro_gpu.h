@@ -410,6 +410,19 @@ int hydro_gpu_pointwise_eval(int device, int op, long long n, const double *gamm
                              const double *L, const double *R, const double *aux, double *out,
                              int *rc);
 
+/* The FP32 step's short forms and the general forms that they stand for, as
+ * the GPU computes them (for tests).
+ *   op 0: face flux of n state pairs a, b = (rho, u_normal, u_tangential, p):
+ *         4 values and the return code
+ *   op 1: conserved a = (mass, mom_x, mom_y, energy) in the volume vol:
+ *         rho, u, v, p and the sound speed
+ *   op 2, 3, 4: limited slope (minmod, van Leer, MC) of the differences a, b
+ *   op 5, 6: a / b; sqrt(a)
+ * b is read by every op (n values, or 4 n for op 0 and 1).  Returns a
+ * cudaError_t. */
+int hydro_gpu_fp32_eval(int device, int op, long long n, double gamma, double tol, double vol, const float *a,
+                        const float *b, float *fast, float *general);
+
 /* Number of visible CUDA devices (0 when none; never fails). */
 int hydro_gpu_device_count(void);
 
