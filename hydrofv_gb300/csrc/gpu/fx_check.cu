@@ -17,7 +17,13 @@
 #include "numerics.cuh"
 #include "quad_exact.cuh"
 #include "staged_math.cuh"
+#include "step_control.h"
+#include "step_loop.cuh"
 #include "hydro_gpu.h"
+#include <atomic>
+#include <chrono>
+#include <thread>
+#include <vector>
 
 using namespace hydro;
 
@@ -291,4 +297,95 @@ extern "C" void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA,
         to_primitive(f, c, 0.37, b[0], b[1], b[2], b[3], o + 8);
         cons_to_prim_2d(c, 0.37, b[0], b[1], b[2], b[3], r + 8);
     }
+}
+
+/* The many-step launch's order (step_loop) and its barrier with host threads
+ * as blocks.  One block lags behind whenever it looks at the error word, one
+ * records an error in the faces of a step, one never arrives. */
+namespace {
+
+struct HostGrid {
+    std::atomic<unsigned> count{ 0 };
+    std::atomic<int> error{ 0 }, active{ 1 };
+    std::atomic<long long> steps{ 0 };
+    int blocks, polls, slow, bad, bad_step;
+};
+
+struct HostCount {
+    HostGrid &g;
+    unsigned arrive() { return g.count.fetch_add(1); }
+    unsigned count()
+    {
+        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        return g.count.load();
+    }
+};
+
+void host_record(HostGrid &g, int code)
+{
+    int none = 0;
+    g.error.compare_exchange_strong(none, code);
+}
+
+/* One block; `left`: 1 out of steps, 2 a failed step, 3 a wait gave up. */
+void host_block(HostGrid &g, int id, int steps, int &left, long long &n)
+{
+    unsigned target = 0;
+    int error = 0;
+    left = 1;
+    step_loop(
+        steps, [] { return true; },
+        [&] {
+            if (id == g.bad && n == g.bad_step) host_record(g, DEV_ERR_HLLC_WAVE_SPEED);
+            return true;
+        },
+        [&] {
+            target += (unsigned) g.blocks;
+            HostCount c{ g };
+            if (arrive_and_wait(c, target, g.polls)) return true;
+            host_record(g, DEV_ERR_SPIN_LIMIT);
+            g.active = 0;
+            left = 3;
+            return false;
+        },
+        [&] {
+            if (id == g.slow) std::this_thread::sleep_for(std::chrono::milliseconds(30));
+            error = g.error.load();
+        },
+        [] {},
+        [&] {
+            if (error == 0) return false;
+            left = 2;
+            if (id == 0) g.active = 0;
+            return true;
+        },
+        [&] {
+            n++;
+            if (id == 0) g.steps = n;
+            return true;
+        });
+}
+
+}  // namespace
+
+extern "C" void hydro_fx_step_loop_host(int blocks, int steps, int slow, int bad, int bad_step, int absent, int polls,
+                                        int *left, long long *done, long long out[3])
+{
+    HostGrid g;
+    g.blocks = blocks;
+    g.polls = polls;
+    g.slow = slow;
+    g.bad = bad;
+    g.bad_step = bad_step;
+    std::vector<std::thread> threads;
+    for (int id = 0; id < blocks; id++) {
+        left[id] = 0;
+        done[id] = 0;
+        if (id == absent) continue;
+        threads.emplace_back([&g, id, steps, left, done] { host_block(g, id, steps, left[id], done[id]); });
+    }
+    for (auto &t : threads) t.join();
+    out[0] = g.steps;
+    out[1] = g.error;
+    out[2] = g.active;
 }

@@ -35,6 +35,7 @@
 
 #include "gpu_internal.h"
 #include "staged_math.cuh"
+#include "step_loop.cuh"
 
 #ifndef MH2D_RECON_CTAS
 #define MH2D_RECON_CTAS 6
@@ -537,13 +538,19 @@ staged_batch_update_kernel(const StagedBatchArgs g, const int *map)
  * and control-block reads, and 11 us of host time where no graph is
  * recorded.  Every block forms the next dt itself after the last barrier.
  *
- * grid_barrier: each block counts itself in on a counter that only grows and
- * waits until it has reached `target`.  All blocks are resident (cooperative
- * launch), so every wait ends; a limit on the polls guards against an error in
- * that, after which the block records DEV_ERR_SPIN_LIMIT and leaves (and so do
- * the others).
+ * The order of the phases and barriers is step_loop's (step_loop.cuh).  All
+ * blocks are resident (cooperative launch), so every wait ends; a limit on the
+ * polls guards against an error in that, after which the block records
+ * DEV_ERR_SPIN_LIMIT, marks the run as stopped (launches behind this one leave
+ * at once) and leaves, and so do the others.
  */
 constexpr int kBarrierPolls = 1 << 22;
+
+struct BarrierCount {
+    unsigned *word;
+    __device__ __forceinline__ unsigned arrive() { return atomicAdd(word, 1u); }
+    __device__ __forceinline__ unsigned count() { return *(volatile unsigned *) word; }
+};
 
 __device__ __forceinline__ bool grid_barrier(HydroStepControl *ctrl, unsigned &target, int *ok)
 {
@@ -551,12 +558,14 @@ __device__ __forceinline__ bool grid_barrier(HydroStepControl *ctrl, unsigned &t
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        int left = kBarrierPolls;
-        if (atomicAdd(&ctrl->barrier_count, 1u) + 1u != target)
-            while (*(volatile unsigned *) &ctrl->barrier_count - target > 0x7fffffffu && --left > 0) { }
+        BarrierCount c{ &ctrl->barrier_count };
+        const bool in = arrive_and_wait(c, target, kBarrierPolls);
         __threadfence();
-        if (left == 0) record_error(ctrl, DEV_ERR_SPIN_LIMIT, -1);
-        *ok = left > 0;
+        if (!in) {
+            record_error(ctrl, DEV_ERR_SPIN_LIMIT, -1);
+            ctrl->active = 0;
+        }
+        *ok = in;
     }
     __syncthreads();
     return *ok != 0;
@@ -590,76 +599,85 @@ staged_loop_kernel(const Mh2dArgs<double> a, const Mh2dBand b, int most)
      * base on its way out, past the launch's last barrier */
     unsigned target = vc->barrier_base;
 
-    for (int it = 0; it < most; it++) {
-        const int buf = (int) (n & 1);
-        if (dt == 0.0) {
+    step_loop(
+        most,
+        [&]() {   /* a step without a dt */
+            if (dt != 0.0) return true;
             if (leader) {
                 ctrl->dt = dt;
                 record_error(ctrl, DEV_ERR_DT_ZERO, -1);
                 ctrl->active = 0;
             }
-            return;
-        }
-        if constexpr (FUSED) {
-            for (unsigned k = blockIdx.x * (NT / 2); k < faces; k += gridDim.x * (NT / 2))
-                staged_recon_flux<LIM, FIRST_ORDER>(a, b, sm, v, k, faces, dt, buf, n == 0, dtA);
-        } else {
-            for (unsigned k = blockIdx.x * NT + tid; k < recon; k += gridDim.x * NT)
-                staged_recon<LIM, FIRST_ORDER>(a, b, k, buf, n == 0, dtA);
-            if (!grid_barrier(ctrl, target, &ok)) return;
-            for (unsigned k = blockIdx.x * NT; k < faces; k += gridDim.x * NT)
-                staged_flux<false, true>(a, b, sm, k + tid, faces, dt);
-        }
-        if (!grid_barrier(ctrl, target, &ok)) return;
-        double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
-        for (unsigned k = blockIdx.x * NT + tid; k < cells; k += gridDim.x * NT)
-            staged_update<GRAV>(f, a, b, k, buf, dt, mx_x, mx_y);
-        block_maxima<NT>(ctrl, red, n, mx_x, mx_y);
-        if (!grid_barrier(ctrl, target, &ok)) return;
-        /* every block: the next dt; block 0 publishes the clock */
-        if (tid < 32) {
-            const bool bad = vc->error_code != 0;
-            const double tn = t + dt;
-            double next, w;
-            next_dt(a, ctrl, n + 1, tn, tf, next, w);
-            if (tid == 0) { failed = bad; s_dt = next; }
-            if (tid < 2) s_dtA[tid] = w;
-        }
-        __syncthreads();
-        if (failed) {
+            return false;
+        },
+        [&]() {
+            const int buf = (int) (n & 1);
+            if constexpr (FUSED) {
+                for (unsigned k = blockIdx.x * (NT / 2); k < faces; k += gridDim.x * (NT / 2))
+                    staged_recon_flux<LIM, FIRST_ORDER>(a, b, sm, v, k, faces, dt, buf, n == 0, dtA);
+            } else {
+                for (unsigned k = blockIdx.x * NT + tid; k < recon; k += gridDim.x * NT)
+                    staged_recon<LIM, FIRST_ORDER>(a, b, k, buf, n == 0, dtA);
+                if (!grid_barrier(ctrl, target, &ok)) return false;
+                for (unsigned k = blockIdx.x * NT; k < faces; k += gridDim.x * NT)
+                    staged_flux<false, true>(a, b, sm, k + tid, faces, dt);
+            }
+            return true;
+        },
+        [&]() { return grid_barrier(ctrl, target, &ok); },
+        [&]() { if (tid == 0) failed = vc->error_code != 0; },
+        [&]() {
+            const int buf = (int) (n & 1);
+            double mx_x = -CUDART_INF, mx_y = -CUDART_INF;
+            for (unsigned k = blockIdx.x * NT + tid; k < cells; k += gridDim.x * NT)
+                staged_update<GRAV>(f, a, b, k, buf, dt, mx_x, mx_y);
+            block_maxima<NT>(ctrl, red, n, mx_x, mx_y);
+        },
+        [&]() {
+            if (!failed) return false;
             if (leader) {
                 ctrl->barrier_base = target;
                 ctrl->dt = dt;
                 ctrl->active = 0;
             }
-            return;
-        }
-        n += 1;
-        t = t + dt;
-        bool act = (t < tf) && (last < 0 || n < last), due = false;
-        if (a.sp.is_storing && t >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
-            due = true;
-            act = false;
-        }
-        if (leader) {
-            if (a.dt_log) a.dt_log[n - 1] = dt;
-            ctrl->dt = dt;
-            ctrl->t = t;
-            ctrl->num_steps = n;
-            ctrl->step_dt = s_dt;
-            ctrl->step_dtA[0] = s_dtA[0];
-            ctrl->step_dtA[1] = s_dtA[1];
-            ctrl->barrier_base = target;
-            ctrl->smax[(n + 1) % 3][0] = ordered_bits(-CUDART_INF);
-            ctrl->smax[(n + 1) % 3][1] = ordered_bits(-CUDART_INF);
-            if (due) ctrl->snapshot_due = 1;
-            if (!act) ctrl->active = 0;
-        }
-        if (!act) return;
-        dt = s_dt;
-        dtA[0] = s_dtA[0];
-        dtA[1] = s_dtA[1];
-    }
+            return true;
+        },
+        [&]() {   /* every block: the next dt; block 0 publishes the clock */
+            if (tid < 32) {
+                const double tn = t + dt;
+                double next, w;
+                next_dt(a, ctrl, n + 1, tn, tf, next, w);
+                if (tid == 0) s_dt = next;
+                if (tid < 2) s_dtA[tid] = w;
+            }
+            __syncthreads();
+            n += 1;
+            t = t + dt;
+            bool act = (t < tf) && (last < 0 || n < last), due = false;
+            if (a.sp.is_storing && t >= a.sp.storing_interval * (double) (stored - a.sp.store_initial_offset + 1)) {
+                due = true;
+                act = false;
+            }
+            if (leader) {
+                if (a.dt_log) a.dt_log[n - 1] = dt;
+                ctrl->dt = dt;
+                ctrl->t = t;
+                ctrl->num_steps = n;
+                ctrl->step_dt = s_dt;
+                ctrl->step_dtA[0] = s_dtA[0];
+                ctrl->step_dtA[1] = s_dtA[1];
+                ctrl->barrier_base = target;
+                ctrl->smax[(n + 1) % 3][0] = ordered_bits(-CUDART_INF);
+                ctrl->smax[(n + 1) % 3][1] = ordered_bits(-CUDART_INF);
+                if (due) ctrl->snapshot_due = 1;
+                if (!act) ctrl->active = 0;
+            }
+            if (!act) return false;
+            dt = s_dt;
+            dtA[0] = s_dtA[0];
+            dtA[1] = s_dtA[1];
+            return true;
+        });
 }
 
 }  // namespace hydro

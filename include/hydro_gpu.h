@@ -388,6 +388,17 @@ void hydro_fx_staged_face_host(double gamma, double tol, long long n, const doub
 void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long n, const double *wm, const double *w0,
                                const double *wp, double *out, double *ref);
 
+/* The order of the many-step kernel (the template that it runs) with host
+ * threads as blocks, for tests: `steps` steps, in which block `slow` lags
+ * whenever it looks at the error word, block `bad` records an error in the
+ * faces of step bad_step, and block `absent` never arrives (-1: no such
+ * block); a wait takes at most `polls` looks of 50 us.  Per block how it left
+ * (1 out of steps, 2 a failed step, 3 a wait gave up) and the steps it
+ * finished; out: the published number of steps, the error word and whether
+ * the run still counts as active. */
+void hydro_fx_step_loop_host(int blocks, int steps, int slow, int bad, int bad_step, int absent, int polls, int *left,
+                             long long *done, long long out[3]);
+
 /* Device build of the exported pointwise numerics over n state pairs:
  * L[4k..4k+3], R[4k..4k+3] = (rho, u, v, p) (the 1D forms read rho, u, p),
  * gas constants from gamma[k] and tol.
