@@ -850,7 +850,7 @@ static int snapshot_async(HydroRun2D *run, HydroSnapshotFn snap, void *ctx, Hydr
             CK(convert_f32_to_f64(out[q], st, (long long) run->ncell, run->stream), "convert");
             src[q] = st;
         }
-        run->kernel_launches += 5;
+        run->kernel_launches += 4;
     } else {
         double *out[4];
         for (int q = 0; q < 4; q++) out[q] = static_cast<double *>(run->snap_d[q]);
