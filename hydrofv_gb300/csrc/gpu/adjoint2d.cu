@@ -811,6 +811,8 @@ struct HydroAdj2D {
     int *err_d = nullptr;
     Mh2dArgs<double> pargs{};
     std::vector<Mh2dBand> bands;       /* the staged step's bands and workspace */
+    void *ws = nullptr;
+    size_t ws_bytes = 0;
     /* face-parallel stepper (double): replay and the reverse sweep's faces */
     StateP<double> gen[2]{};
     FacesP<double> faces{};
@@ -859,9 +861,31 @@ void set_err(HydroRunOutcome *oc, cudaError_t e, const char *what)
         }                                       \
     } while (0)
 
+cudaError_t workspace_alloc(HydroAdj2D *a, void **p, size_t bytes)
+{
+    const cudaError_t e = cudaMalloc(p, bytes);
+    a->ws = e == cudaSuccess ? *p : nullptr;
+    a->ws_bytes = e == cudaSuccess ? bytes : 0;
+    a->device_bytes += (long long) a->ws_bytes;
+    return e;
+}
+
+/* What is allocated after the staged step's workspace (the tape above all)
+ * comes before it: the workspace gives way. */
 int dalloc(HydroAdj2D *a, size_t bytes, void **p, HydroRunOutcome *oc)
 {
-    CK(cudaMalloc(p, bytes), "cudaMalloc(adjoint)");
+    *p = nullptr;
+    const cudaError_t e = alloc_beside_workspace(
+        a->pargs, a->bands, p, bytes, [](void **q, size_t n) { return cudaMalloc(q, n); },
+        [&] {
+            cudaFree(a->ws);      /* (waits for the device) */
+            a->device_bytes -= (long long) a->ws_bytes;
+            a->ws = nullptr;
+            a->ws_bytes = 0;
+        },
+        [&](void **q, size_t n) { return workspace_alloc(a, q, n); });
+    if (e != cudaSuccess && *p) cudaFree(*p);
+    CK(e, "cudaMalloc(adjoint)");
     a->allocs.push_back(*p);
     a->device_bytes += (long long) bytes;
     CK(cudaMemsetAsync(*p, 0, bytes, a->stream), "cudaMemset(adjoint)");
@@ -1149,14 +1173,7 @@ extern "C" int hydro_adj2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     pa.area_y = grid->area_y;
     pa.vol = grid->vol;
     pa.first_order = 0;
-    CK(staged_alloc(pa, a->bands, [&](void **w, size_t bytes) {
-           const cudaError_t e = cudaMalloc(w, bytes);
-           if (e == cudaSuccess) {
-               a->allocs.push_back(*w);
-               a->device_bytes += (long long) bytes;
-           }
-           return e;
-       }), "cudaMalloc(adjoint)");
+    CK(staged_alloc(pa, a->bands, [&](void **w, size_t bytes) { return workspace_alloc(a, w, bytes); }), "cudaMalloc(adjoint)");
 
     /* initial state: interior W0, ghosts from the boundary rules, U0 = W->U(W0) */
     StateP<double> s0 = a->ckpt[0];
@@ -1527,6 +1544,7 @@ extern "C" void hydro_adj2d_destroy(HydroAdj2D *a)
     cudaSetDevice(a->device);
     if (a->stream) cudaStreamSynchronize(a->stream);
     for (void *p : a->allocs) cudaFree(p);
+    cudaFree(a->ws);
     if (a->ctrl_h) cudaFreeHost(a->ctrl_h);
     for (auto &e : a->ev)
         if (e) cudaEventDestroy(e);

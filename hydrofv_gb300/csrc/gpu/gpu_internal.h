@@ -225,6 +225,28 @@ cudaError_t staged_alloc(const Mh2dArgs<double> &a, std::vector<Mh2dBand> &bands
     }
 }
 
+/*
+ * Memory that a session takes after the workspace (a solver's initial state, the
+ * adjoint's tape): where the device has no room for it, the workspace gives
+ * way.  `release()` gives it back, `alloc(p, bytes)` is asked again, and
+ * `workspace(&p, bytes)` for a workspace in what is left, in more and shorter
+ * bands.  A failure leaves no bands when not even single rows fit.
+ */
+template <class Alloc, class Release, class Workspace>
+cudaError_t alloc_beside_workspace(const Mh2dArgs<double> &a, std::vector<Mh2dBand> &bands, void **p, size_t bytes, Alloc alloc,
+                                   Release release, Workspace workspace)
+{
+    cudaError_t e = alloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || bands.empty()) return e;
+    cudaGetLastError();
+    release();
+    e = alloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    const cudaError_t w = staged_alloc(a, bands, workspace);
+    if (w != cudaSuccess) bands.clear();
+    return e != cudaSuccess ? e : w;
+}
+
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s);
 /* Batches: band `band` of instance `inst`; its blocks of the recon, flux and
  * update launches start at first[0], first[1], first[2] of the group's. */

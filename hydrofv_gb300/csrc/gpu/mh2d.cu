@@ -72,6 +72,7 @@ void staged_plan(const Mh2dArgs<double> &a, size_t budget, std::vector<Mh2dBand>
 cudaError_t staged_launch_step(const Mh2dArgs<double> &a, int limiter, const std::vector<Mh2dBand> &bands, cudaStream_t s)
 {
     const int first_order = a.first_order;
+    if (bands.empty()) return cudaErrorMemoryAllocation;
     for (const Mh2dBand &b : bands) {
         cudaError_t e = STAGED_DISPATCH(staged_launch_recon, a, b, s);
         if (e != cudaSuccess) return e;

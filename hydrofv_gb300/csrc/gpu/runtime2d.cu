@@ -198,6 +198,41 @@ extern "C" int hydro_gpu_chunk_plan(int nx, int ny, int g, int slots, int *h1, i
     return n;
 }
 
+/* The workspace's rules on a device with `room` bytes for it and for `bytes`
+ * more (host only, for tests): out = workspace bytes before, after, bands
+ * after, rows that they cover. */
+extern "C" int hydro_fx_workspace_host(int nx, int ny, int g, long long room, long long bytes, long long out[4])
+{
+    Mh2dArgs<double> a{};
+    a.nx = nx;
+    a.ny = ny;
+    a.g = g;
+    a.pitch = nx + 2 * g;
+    std::vector<Mh2dBand> bands;
+    long long used = 0, ws = 0;
+    char base = 0;
+    auto take = [&](void **p, size_t n) {
+        if (used + (long long) n > room) return cudaErrorMemoryAllocation;
+        used += (long long) n;
+        *p = &base;
+        return cudaSuccess;
+    };
+    auto take_ws = [&](void **p, size_t n) {
+        const cudaError_t e = take(p, n);
+        ws = e == cudaSuccess ? (long long) n : 0;
+        return e;
+    };
+    void *p = nullptr;
+    cudaError_t e = staged_alloc(a, bands, take_ws);
+    out[0] = ws;
+    if (e == cudaSuccess) e = alloc_beside_workspace(a, bands, &p, (size_t) bytes, take, [&] { used -= ws; ws = 0; }, take_ws);
+    out[1] = ws;
+    out[2] = (long long) bands.size();
+    out[3] = 0;
+    for (const Mh2dBand &b : bands) out[3] += b.r1 - b.r0;
+    return (int) e;
+}
+
 /*
  * Device memory of the 2D runs comes from one stream-ordered pool per device
  * that keeps what a finished run freed (release threshold: no limit).  A
@@ -251,6 +286,28 @@ static cudaError_t pool_alloc(HydroRun2D *run, void **p, size_t bytes)
     const cudaError_t e = device_pool(run->device, &pool);
     if (e != cudaSuccess) return e;
     return cudaMallocFromPoolAsync(p, bytes, pool, run->stream);
+}
+
+static cudaError_t workspace_alloc(HydroRun2D *run, void **p, size_t bytes)
+{
+    const cudaError_t e = pool_alloc(run, p, bytes);
+    run->ws = e == cudaSuccess ? *p : nullptr;
+    return e;
+}
+
+/* The workspace back to the device (through the pool, which would keep it). */
+static void workspace_release(HydroRun2D *run)
+{
+    if (!run->ws) return;
+    if (run->pooled) {
+        cudaMemPool_t pool;
+        cudaFreeAsync(run->ws, run->stream);
+        cudaStreamSynchronize(run->stream);
+        if (device_pool(run->device, &pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    } else {
+        cudaFree(run->ws);
+    }
+    run->ws = nullptr;
 }
 
 /*
@@ -400,11 +457,8 @@ extern "C" int hydro_run2d_create(const HydroGrid2D *grid, const HydroGpuOptions
     } else {
         carve<double>(run, run->args);
         setup_args<double>(run, run->args, grid, opt);
-        CK(staged_alloc(run->args, run->bands, [&](void **p, size_t bytes) {
-               const cudaError_t e = pool_alloc(run, p, bytes);
-               run->ws = *p;
-               return e;
-           }), "cudaMallocFromPoolAsync(workspace)");
+        CK(staged_alloc(run->args, run->bands, [&](void **p, size_t bytes) { return workspace_alloc(run, p, bytes); }),
+           "cudaMallocFromPoolAsync(workspace)");
         run->loop_grid = staged_loop_grid(run->args, grid->limiter, run->bands, run->device);
     }
     return 0;
@@ -457,6 +511,37 @@ static int download_fields(HydroRun2D *run, void *const dev[4], double *const ho
     return 0;
 }
 
+/* Room for the initial state, once; the FP64 step's workspace gives way. */
+static int alloc_initial(HydroRun2D *run, HydroRunOutcome *oc)
+{
+    if (run->init_slab) return 0;
+    const size_t fbytes = run->ncell * run->elem;
+    const void *ws = run->ws;
+    const cudaError_t e = alloc_beside_workspace(
+        run->args, run->bands, &run->init_slab, 8 * fbytes, [&](void **p, size_t bytes) { return pool_alloc(run, p, bytes); },
+        [&] { workspace_release(run); }, [&](void **p, size_t bytes) { return workspace_alloc(run, p, bytes); });
+    if (run->ws != ws) {
+        run->loop_grid = run->bands.empty() ? 0 : staged_loop_grid(run->args, run->grid.limiter, run->bands, run->device);
+        if (run->graph) {
+            cudaGraphExecDestroy(run->graph);
+            run->graph = nullptr;
+        }
+    }
+    if (e != cudaSuccess) {
+        if (run->init_slab) {
+            if (run->pooled) cudaFreeAsync(run->init_slab, run->stream);
+            else cudaFree(run->init_slab);
+        }
+        run->init_slab = nullptr;
+    }
+    CK(e, "cudaMallocFromPoolAsync(initial state)");
+    for (int q = 0; q < 4; q++) {
+        run->init_U[q] = static_cast<char *>(run->init_slab) + q * fbytes;
+        run->init_W[q] = static_cast<char *>(run->init_slab) + (4 + q) * fbytes;
+    }
+    return 0;
+}
+
 extern "C" int hydro_run2d_upload(HydroRun2D *run, double *const W[4], double *const U[4],
                                   int keep_initial, HydroRunOutcome *oc)
 {
@@ -471,13 +556,7 @@ extern "C" int hydro_run2d_upload(HydroRun2D *run, double *const W[4], double *c
     for (int q = 0; q < 4; q++)
         CK(cudaMemcpyAsync(fieldU(run, 1, q), u0[q], fbytes, cudaMemcpyDeviceToDevice, run->stream), "D2D U");
     if (keep_initial) {
-        if (!run->init_slab) {
-            CK(pool_alloc(run, &run->init_slab, 8 * fbytes), "cudaMallocFromPoolAsync(initial state)");
-            for (int q = 0; q < 4; q++) {
-                run->init_U[q] = static_cast<char *>(run->init_slab) + q * fbytes;
-                run->init_W[q] = static_cast<char *>(run->init_slab) + (4 + q) * fbytes;
-            }
-        }
+        if (alloc_initial(run, oc)) return -1;
         for (int q = 0; q < 4; q++) {
             CK(cudaMemcpyAsync(run->init_U[q], u0[q], fbytes, cudaMemcpyDeviceToDevice, run->stream), "D2D");
             CK(cudaMemcpyAsync(run->init_W[q], w0[q], fbytes, cudaMemcpyDeviceToDevice, run->stream), "D2D");
@@ -561,13 +640,7 @@ static void set_shape(HydroRun2D *run, int chunk, int ctas)
 static int ensure_initial_copy(HydroRun2D *run, HydroRunOutcome *oc)
 {
     const size_t fbytes = run->ncell * run->elem;
-    if (!run->init_slab) {
-        CK(pool_alloc(run, &run->init_slab, 8 * fbytes), "cudaMallocFromPoolAsync(initial state)");
-        for (int q = 0; q < 4; q++) {
-            run->init_U[q] = static_cast<char *>(run->init_slab) + q * fbytes;
-            run->init_W[q] = static_cast<char *>(run->init_slab) + (4 + q) * fbytes;
-        }
-    }
+    if (alloc_initial(run, oc)) return -1;
     if (!run->have_initial) {
         for (int q = 0; q < 4; q++) {
             CK(cudaMemcpyAsync(run->init_U[q], fieldU(run, 0, q), fbytes, cudaMemcpyDeviceToDevice, run->stream), "D2D");

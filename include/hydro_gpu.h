@@ -388,6 +388,12 @@ void hydro_fx_staged_face_host(double gamma, double tol, long long n, const doub
 void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long n, const double *wm, const double *w0,
                                const double *wp, double *out, double *ref);
 
+/* The rules of the FP64 step's workspace on a device with `room` bytes for it
+ * and for `bytes` that a session asks for later (host only, for tests): out =
+ * workspace bytes before and after, bands after, rows that they cover.  Returns
+ * a cudaError_t. */
+int hydro_fx_workspace_host(int nx, int ny, int g, long long room, long long bytes, long long out[4]);
+
 /* The order of the many-step kernel (the template that it runs) with host
  * threads as blocks, for tests: `steps` steps, in which block `slow` lags
  * whenever it looks at the error word, block `bad` records an error in the
