@@ -197,13 +197,16 @@ static int staged_setup(HydroBatch2D *b, HydroRunOutcome *oc)
     const size_t band_bytes = bands.size() * sizeof(StagedBatchBand);
     const size_t ints = map[0].size() + map[1].size() + map[2].size();
     BK(cudaMalloc(&b->plan_d, band_bytes + ints * sizeof(int)), "cudaMalloc(plan)");
-    BK(cudaMemcpy(b->plan_d, bands.data(), band_bytes, cudaMemcpyHostToDevice), "H2D plan");
+    /* on the stream of the kernels that read the plan: it does not wait for
+     * the default stream */
+    BK(cudaMemcpyAsync(b->plan_d, bands.data(), band_bytes, cudaMemcpyHostToDevice, b->stream), "H2D plan");
     int *p = reinterpret_cast<int *>(static_cast<char *>(b->plan_d) + band_bytes);
     for (int s = 0; s < 3; s++) {
-        BK(cudaMemcpy(p, map[s].data(), map[s].size() * sizeof(int), cudaMemcpyHostToDevice), "H2D plan");
+        BK(cudaMemcpyAsync(p, map[s].data(), map[s].size() * sizeof(int), cudaMemcpyHostToDevice, b->stream), "H2D plan");
         for (int g = 0; g < ng; g++) b->groups[g].map[s] = p + start[s][g];
         p += map[s].size();
     }
+    BK(cudaStreamSynchronize(b->stream), "H2D plan");   /* before the vectors go */
     b->staged.inst = static_cast<const Mh2dArgs<double> *>(b->args_d);
     b->staged.bands = static_cast<const StagedBatchBand *>(b->plan_d);
     return 0;
