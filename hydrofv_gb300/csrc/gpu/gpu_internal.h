@@ -279,6 +279,32 @@ unsigned staged_loop_grid(const Mh2dArgs<double> &a, int limiter, const std::vec
 cudaError_t staged_launch_steps(const Mh2dArgs<double> &a, int limiter, const Mh2dBand &band, unsigned grid, int steps,
                                 cudaStream_t s);
 
+/*
+ * Of `k` steps as many as the many-step kernel takes, in launches of at most
+ * `most` steps by `loop(steps)`.  A launch that the driver refuses because the
+ * process may use fewer of the SMs than the device has (its blocks would not be
+ * resident together), or because it grants no cooperative launches, has done
+ * nothing: `grid` comes back 0 and the steps left in `k` go in three launches
+ * each, as on larger grids.
+ */
+template <class Loop>
+cudaError_t staged_loop_steps(unsigned &grid, long long &k, int most, Loop loop)
+{
+    while (grid && k > 0) {
+        const int steps = (int) (k < most ? k : most);
+        const cudaError_t e = loop(steps);
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorNotPermitted) {
+            cudaGetLastError();
+            grid = 0;
+        } else if (e != cudaSuccess) {
+            return e;
+        } else {
+            k -= steps;
+        }
+    }
+    return cudaSuccess;
+}
+
 template <class R>
 cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s);
 template <class R>

@@ -233,6 +233,24 @@ extern "C" int hydro_fx_workspace_host(int nx, int ny, int g, long long room, lo
     return (int) e;
 }
 
+/* staged_loop_steps with a launch that returns `code` at its call number
+ * `at` (host only, for tests): out = steps launched, steps left, grid. */
+extern "C" int hydro_fx_loop_steps_host(long long k, int most, int at, int code, long long out[3])
+{
+    unsigned grid = 7;
+    long long launched = 0;
+    int call = 0;
+    const cudaError_t e = staged_loop_steps(grid, k, most, [&](int steps) {
+        if (call++ == at) return (cudaError_t) code;
+        launched += steps;
+        return cudaSuccess;
+    });
+    out[0] = launched;
+    out[1] = k;
+    out[2] = grid;
+    return (int) e;
+}
+
 /*
  * Device memory of the 2D runs comes from one stream-ordered pool per device
  * that keeps what a finished run freed (release threshold: no limit).  A
@@ -851,17 +869,12 @@ static int apply_host_bc(HydroRun2D *run, HydroRunOutcome *oc)
 /* Enqueue `k` step kernels. */
 static int enqueue_steps(HydroRun2D *run, long long k, HydroRunOutcome *oc)
 {
-    if (run->loop_grid) {
-        while (k > 0) {
-            const int steps = (int) (k < kLoopSteps ? k : kLoopSteps);
-            CK(staged_launch_steps(run->args, run->grid.limiter, run->bands[0], run->loop_grid, steps, run->stream),
-               "step kernel");
-            k -= steps;
-            run->step_launches += 1;
-            run->kernel_launches += 1;
-        }
-        return 0;
-    }
+    CK(staged_loop_steps(run->loop_grid, k, kLoopSteps, [&](int steps) {
+           const cudaError_t e = staged_launch_steps(run->args, run->grid.limiter, run->bands[0], run->loop_grid, steps, run->stream);
+           run->step_launches += e == cudaSuccess;
+           run->kernel_launches += e == cudaSuccess;
+           return e;
+       }), "step kernel");
     const bool graphs = run->opt.use_graph && k >= kGraphSteps;
     if (graphs && !run->graph && record_graph(run, oc)) return -1;
     while (k > 0) {

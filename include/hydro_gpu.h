@@ -394,6 +394,12 @@ void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long 
  * a cudaError_t. */
 int hydro_fx_workspace_host(int nx, int ny, int g, long long room, long long bytes, long long out[4]);
 
+/* `k` steps in launches of the many-step kernel of at most `most` steps, of
+ * which number `at` returns the cudaError_t `code` (a fake launch on the host, for
+ * tests): out = steps launched, steps left for single launches, and the grid, 0
+ * after a refusal.  Returns a cudaError_t. */
+int hydro_fx_loop_steps_host(long long k, int most, int at, int code, long long out[3]);
+
 /* The order of the many-step kernel (the template that it runs) with host
  * threads as blocks, for tests: `steps` steps, in which block `slow` lags
  * whenever it looks at the error word, block `bad` records an error in the
