@@ -272,7 +272,7 @@ HD int hllc_fwd(const GasConst<double> &c, double rl, double ul, double pl, doub
 
 /* The intermediates of a non-vacuum face from the tape: sound speeds,
  * unfloored guess, regime and the finish's q_L, q_R and S* as the forward
- * pass computed them (the same values hllc_fwd_from_guess recomputes). */
+ * pass computed them. */
 HD int hllc_fwd_from_tape(const GasConst<double> &c, double rl, double ul, double pl, double rr, double ur,
                           double pr, double aL, double aR, double pg, int reg, double qL, double qR, double Ss,
                           HllcFwd &s)
@@ -356,35 +356,6 @@ HD void vacuum_fan_vjp(const GasConst<double> &c, bool right, double rho, double
     const double kb = right ? t0b : -t0b;
     ub += kb * c.gm1 / (c.gp1 * a);
     ab += -kb * k / a;
-}
-
-/* The remaining intermediates of a face from its sound speeds, unfloored
- * guess and regime (what the tape keeps): the same expressions as
- * hllc_classify / hllc_finish. */
-HD int hllc_fwd_from_guess(const GasConst<double> &c, double rl, double ul, double pl, double rr, double ur,
-                           double pr, double aL, double aR, double pg, int reg, HllcFwd &s)
-{
-    s.aL = aL;
-    s.aR = aR;
-    s.reg = reg;
-    s.region = -1;
-    s.ppv = 0.5 * (pl + pr) - 0.125 * (ur - ul) * (rl + rr) * (aL + aR);
-    s.pg = pg;
-    s.ps = s.qL = s.qR = s.SL = s.SR = s.Ss = 0.0;
-    if (reg == PREG_VACUUM) return DEV_OK;
-    s.ps = lt(s.pg, c.tol) ? c.tol : s.pg;
-    s.qL = hllc_q(c, pl, s.ps);
-    s.qR = hllc_q(c, pr, s.ps);
-    s.SL = ul - s.aL * s.qL;
-    s.SR = ur + s.aR * s.qR;
-    s.Ss = dv(pr - pl + rl * ul * (s.SL - ul) - rr * ur * (s.SR - ur),
-              rl * (s.SL - ul) - rr * (s.SR - ur));
-    if (le(0.0, s.SL)) s.region = 0;
-    else if (le(s.SL, 0.0) && le(0.0, s.Ss)) s.region = 1;
-    else if (le(s.Ss, 0.0) && le(0.0, s.SR)) s.region = 2;
-    else if (le(s.SR, 0.0)) s.region = 3;
-    else return DEV_ERR_HLLC_WAVE_SPEED;
-    return DEV_OK;
 }
 
 /* Reverse of the vacuum / vacuum-generation flux (kept out of line: rare,

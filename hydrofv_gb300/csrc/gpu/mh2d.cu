@@ -9,7 +9,6 @@
 
 namespace hydro {
 
-template int mh2d_resident_ctas<double>(int, int, int);
 template cudaError_t mh2d_launch_step<double>(const Mh2dArgs<double> &, int, cudaStream_t);
 template cudaError_t mh2d_launch_prepare<double>(const Mh2dArgs<double> &, cudaStream_t);
 template cudaError_t mh2d_launch_arm<double>(const Mh2dArgs<double> &, cudaStream_t);

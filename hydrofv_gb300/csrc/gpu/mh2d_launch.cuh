@@ -133,8 +133,9 @@ __global__ void mh2d_ghost_sound_speed_kernel(const Mh2dArgs<R> a, int buf, int 
 /*
  * Per-limiter launchers.  Their definitions (mh2d_lim.cuh) are explicitly
  * instantiated in one translation unit per (precision, limiter) --
- * mh2d_lim_{minmod,vanleer,mc}.cu for FP64, mh2d_fp32.cu for FP32 -- so that
- * the step kernels of the three limiters compile in parallel.
+ * mh2d_lim_{minmod,vanleer,mc}.cu for FP64 (the allocation-free run),
+ * mh2d_fp32.cu for FP32 -- so that the step kernels of the three limiters
+ * compile in parallel.
  */
 template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_step_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s);
@@ -148,7 +149,10 @@ cudaError_t mh2d_launch_step(const Mh2dArgs<R> &a, int limiter, cudaStream_t s)
 {
     const int n_items = mh2d_n_items(a);
     const int grid = (a.grid_ctas > 0 && a.grid_ctas < n_items) ? a.grid_ctas : n_items;
-    if (a.first_order) return mh2d_launch_step_lim<R, LIM_MINMOD, 1>(a, grid, s);
+    if (a.first_order) {
+        if constexpr (sizeof(R) == 4) return mh2d_launch_step_lim<R, LIM_MINMOD, 1>(a, grid, s);
+        return cudaErrorNotSupported;
+    }
     switch (limiter) {
     case LIM_MINMOD: return mh2d_launch_step_lim<R, LIM_MINMOD, 0>(a, grid, s);
     case LIM_VAN_LEER: return mh2d_launch_step_lim<R, LIM_VAN_LEER, 0>(a, grid, s);

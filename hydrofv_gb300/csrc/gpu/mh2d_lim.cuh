@@ -16,8 +16,9 @@ template <class R, int LIM, int FIRST_ORDER>
 cudaError_t mh2d_launch_step_lim(const Mh2dArgs<R> &a, int grid, cudaStream_t s)
 {
     constexpr int nt = mh2d_threads<R>();
-    return a.gravity != 0.0 ? launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, true>, grid, nt, s, a)
-                            : launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, false>, grid, nt, s, a);
+    if (a.gravity == 0.0) return launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, false>, grid, nt, s, a);
+    if constexpr (sizeof(R) == 4) return launch_after(mh2d_step_kernel<R, LIM, nt, FIRST_ORDER, true>, grid, nt, s, a);
+    return cudaErrorNotSupported;
 }
 
 template <class R, int LIM, int FIRST_ORDER>
@@ -36,13 +37,14 @@ cudaError_t mh2d_step_occupancy(int *per_sm)
 
 }  // namespace hydro
 
-/* Everything one (precision, limiter, first-order) combination launches:
- * the single grid, and (FP32) the batch. */
-#define HYDRO_MH2D_INSTANTIATE_GRID(R, LIM, FO)                                                            \
-    template cudaError_t mh2d_launch_step_lim<R, LIM, FO>(const Mh2dArgs<R> &, int, cudaStream_t);        \
-    template cudaError_t mh2d_step_occupancy<R, LIM, FO>(int *);
+/* Everything one (precision, limiter, first-order) combination launches: FP64
+ * (the allocation-free run: no gravity, MUSCL-Hancock) the single grid's step,
+ * FP32 the batch's and the resident blocks besides. */
+#define HYDRO_MH2D_INSTANTIATE_STEP(R, LIM, FO)                                                            \
+    template cudaError_t mh2d_launch_step_lim<R, LIM, FO>(const Mh2dArgs<R> &, int, cudaStream_t);
 #define HYDRO_MH2D_INSTANTIATE(R, LIM, FO)                                                                 \
-    HYDRO_MH2D_INSTANTIATE_GRID(R, LIM, FO)                                                               \
+    HYDRO_MH2D_INSTANTIATE_STEP(R, LIM, FO)                                                               \
+    template cudaError_t mh2d_step_occupancy<R, LIM, FO>(int *);                                          \
     template cudaError_t mh2d_launch_batch_lim<R, LIM, FO>(const Mh2dBatchArgs<R> &, int, cudaStream_t);
 
 #endif

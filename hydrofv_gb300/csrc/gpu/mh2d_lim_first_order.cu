@@ -6,12 +6,10 @@
  * Compiled with --fmad=false: the FP64 path must issue the same IEEE
  * operations as the reference CPU code, which never contracts a*b+c.
  */
-#include "mh2d_lim.cuh"
 #include "mh2d_staged_launch.cuh"
 
 namespace hydro {
 
-HYDRO_MH2D_INSTANTIATE_GRID(double, LIM_MINMOD, 1)
 HYDRO_STAGED_INSTANTIATE(LIM_MINMOD, 1)
 
 }  // namespace hydro

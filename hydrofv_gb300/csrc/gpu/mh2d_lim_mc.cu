@@ -10,7 +10,7 @@
 
 namespace hydro {
 
-HYDRO_MH2D_INSTANTIATE_GRID(double, LIM_MC, 0)
+HYDRO_MH2D_INSTANTIATE_STEP(double, LIM_MC, 0)
 HYDRO_STAGED_INSTANTIATE(LIM_MC, 0)
 
 }  // namespace hydro

@@ -143,7 +143,7 @@ static void setup_args(HydroRun2D *run, Mh2dArgs<R> &a, const HydroGrid2D *grid,
     a.area_y = grid->area_y;
     a.vol = grid->vol;
     a.first_order = (grid->integrator == INTEGRATOR_GODUNOV_FIRST_ORDER_2D) ? 1 : 0;
-    if (sizeof(R) == 4) {
+    if constexpr (sizeof(R) == 4) {
         a.grid_ctas = mh2d_resident_ctas<R>(grid->limiter, a.first_order, run->device);
         a.chunk_h = opt->chunk_rows > 0 ? opt->chunk_rows
                                         : mh2d_fp32_chunk(a.grid_ctas, [&](int c) {
@@ -634,21 +634,19 @@ static int recompute_active(HydroStepControl *c)
 
 /* ------------------------------------------------------------ autotuner */
 
-/* Work-item shape (rows per item) and persistent grid size are tuned on the
+/* FP32: work-item shape (rows per item) and persistent grid size are tuned on the
  * run's own state: each candidate runs one warm-up and two timed steps from
  * the initial state (CUDA events), the fastest is kept, the state is rewound
- * and the choice is cached for the process per (precision, limiter, order,
- * grid shape). */
+ * and the choice is cached for the process per (limiter, order, grid shape). */
 namespace {
 std::mutex g_tune_mutex;
-std::map<std::tuple<int, int, int, int, int>, std::pair<int, int>> g_tune_cache;
+std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune_cache;
 }
 
 static void set_shape(HydroRun2D *run, int chunk, int ctas)
 {
-    run->args.chunk_h = run->args32.chunk_h = chunk;
-    run->args.tail_rows = run->args32.tail_rows = 0;
-    run->args.grid_ctas = run->args32.grid_ctas = ctas;
+    run->args32.chunk_h = chunk;
+    run->args32.grid_ctas = ctas;
     if (run->graph) {
         cudaGraphExecDestroy(run->graph);
         run->graph = nullptr;
@@ -671,8 +669,7 @@ static int ensure_initial_copy(HydroRun2D *run, HydroRunOutcome *oc)
 
 static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome *oc)
 {
-    const auto key = std::make_tuple(run->fp32, run->grid.limiter, run->args.first_order + 2 * run->args32.first_order,
-                                     run->grid.nx, run->grid.ny);
+    const auto key = std::make_tuple(run->grid.limiter, run->args32.first_order, run->grid.nx, run->grid.ny);
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
@@ -682,9 +679,9 @@ static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome 
         }
     }
     if (ensure_initial_copy(run, oc)) return -1;
-    const int resident = run->fp32 ? run->args32.grid_ctas : run->args.grid_ctas;
-    const int storing = run->args.sp.is_storing;
-    run->args.sp.is_storing = run->args32.sp.is_storing = 0;
+    const int resident = run->args32.grid_ctas;
+    const int storing = run->args32.sp.is_storing;
+    run->args32.sp.is_storing = 0;
     const int chunks[] = { run->args32.chunk_h, 8, 16, 32, 64 };   /* the model's choice first */
     int best_chunk = 32, best_ctas = resident;
     float best_ms = 1e30f;
@@ -725,7 +722,7 @@ static int autotune(HydroRun2D *run, const HydroStepParams *sp, HydroRunOutcome 
         }
     }
     set_shape(run, best_chunk, best_ctas);
-    run->args.sp.is_storing = run->args32.sp.is_storing = storing;
+    run->args32.sp.is_storing = storing;
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     g_tune_cache[key] = std::make_pair(best_chunk, best_ctas);
     return 0;
