@@ -892,8 +892,9 @@ def gpu_fx_eval(op, a, b=None, device=0):
 
 
 def chunk_plan(nx, ny, g=2, slots=608):
-    """The FP64 step's work-item plan: ((h1, h2, tail), rows) with rows an
-    (n_items, 3) array of (strip, r0, r1) as the kernel decodes the items."""
+    """The guided plan of the row-marching FP64 kernel's items (which no run
+    takes any more): ((h1, h2, tail), rows) with rows an (n_items, 3) array of
+    (strip, r0, r1) as that kernel decodes the items."""
     lib = library()
     h1, h2, tail = C.c_int(), C.c_int(), C.c_int()
     n = lib.hydro_gpu_chunk_plan(nx, ny, g, slots, C.byref(h1), C.byref(h2), C.byref(tail), None, 0)

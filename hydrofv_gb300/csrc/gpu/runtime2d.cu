@@ -175,9 +175,11 @@ static cudaError_t launch_prepare(HydroRun2D *run)
 /* Kernels that launch_step launches. */
 static int launches_per_step(const HydroRun2D *run) { return run->fp32 ? 1 : 3 * (int) run->bands.size(); }
 
-/* The row-marching FP64 kernel's work-item plan for an nx x ny grid on `slots`
- * resident CTAs (guided row chunks), and each item's strip and padded rows as
- * the kernel decodes them (rows: 3 ints per item, or NULL).  Host only. */
+/* The guided plan of row chunks for an nx x ny grid on `slots` resident CTAs of
+ * the row-marching FP64 kernel, and each item's strip and padded rows as that
+ * kernel decodes them (rows: 3 ints per item, or NULL).  No run takes it: FP64
+ * steps in the staged kernels, the allocation-free run in 64-row items.  Host
+ * only. */
 extern "C" int hydro_gpu_chunk_plan(int nx, int ny, int g, int slots, int *h1, int *h2, int *tail,
                                     int *rows, int max_items)
 {
@@ -195,6 +197,24 @@ extern "C" int hydro_gpu_chunk_plan(int nx, int ny, int g, int slots, int *h1, i
         for (int i = 0; i < n && i < max_items; i++)
             mh2d_item_rows(a, i, rows[3 * i], rows[3 * i + 1], rows[3 * i + 2]);
     }
+    return n;
+}
+
+/* The FP32 step's rows per work item for an nx x ny grid on `slots` resident
+ * CTAs, and each item's strip and padded rows as the kernel decodes them (rows:
+ * 3 ints per item, or NULL).  Host only, for tests. */
+extern "C" int hydro_fx_fp32_items_host(int nx, int ny, int g, int slots, int *height, int *rows, int max_items)
+{
+    Mh2dArgs<float> a{};
+    a.nx = nx;
+    a.ny = ny;
+    a.g = g;
+    a.strip_w = mh2d_threads<float>() - 2;
+    a.chunk_h = mh2d_fp32_chunk(slots, [&](int c) { return mh2d_item_count(nx, ny, a.strip_w, c); });
+    *height = a.chunk_h;
+    const int n = mh2d_n_items(a);
+    if (rows)
+        for (int i = 0; i < n && i < max_items; i++) mh2d_item_rows(a, i, rows[3 * i], rows[3 * i + 1], rows[3 * i + 2]);
     return n;
 }
 

@@ -182,11 +182,13 @@ int hydro_gpu_calibrate(int device, double *fp64_tflops, double *fp32_tflops);
  * SM per clock) that roofline reporting uses for issue-bound kernels. */
 int hydro_gpu_sm_count(int device);
 
-/* The FP64 step's work items for an nx x ny grid (g ghost layers) on `slots`
- * resident CTAs: the guided row-chunk plan (h1-row items, then the last
- * `tail` rows in h2-row items) and, if rows is not NULL, each item's strip
- * and padded row range [r0, r1) as the kernel decodes it (3 ints per item,
- * at most max_items).  Returns the number of items.  Host only. */
+/* A guided plan of row chunks for the row-marching FP64 kernel: an nx x ny grid
+ * (g ghost layers) on `slots` resident CTAs, h1-row items and then the last
+ * `tail` rows in h2-row items, and, if rows is not NULL, each item's strip and
+ * padded row range [r0, r1) as that kernel decodes it (3 ints per item, at most
+ * max_items).  The runs no longer take it: FP64 steps in staged kernels without
+ * work items, the allocation-free run in 64-row items.  Returns the number of
+ * items.  Host only. */
 int hydro_gpu_chunk_plan(int nx, int ny, int g, int slots, int *h1, int *h2, int *tail, int *rows,
                          int max_items);
 
@@ -387,6 +389,12 @@ void hydro_fx_staged_face_host(double gamma, double tol, long long n, const doub
                                int *rc, double *ref, int *rc_ref);
 void hydro_fx_staged_cell_host(int limiter, double gamma, double dtA, long long n, const double *wm, const double *w0,
                                const double *wp, double *out, double *ref);
+
+/* The FP32 step's work items for an nx x ny grid (g ghost layers) on `slots`
+ * resident CTAs, as a run plans them: their height and, if rows is not NULL,
+ * each item's strip and padded row range [r0, r1) (3 ints per item, at most
+ * max_items).  Returns the number of items.  Host only, for tests. */
+int hydro_fx_fp32_items_host(int nx, int ny, int g, int slots, int *height, int *rows, int max_items);
 
 /* The rules of the FP64 step's workspace on a device with `room` bytes for it
  * and for `bytes` that a session asks for later (host only, for tests): out =
