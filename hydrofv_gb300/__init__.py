@@ -591,7 +591,8 @@ class Solver2D:
 
 class Batch2D:
     """Ensemble of independent 2D problems (hydro_gpu_batch_*): one launch per
-    step for all instances, each with its own dt.  `problems` are objects with
+    step for all instances (FP64: one per stage, three a step), each with its
+    own dt.  `problems` are objects with
     the fields of hydrofv_gb300.problems.Problem2D; integrator, limiter and CFL
     are taken from the first one."""
 

@@ -159,7 +159,9 @@ __device__ __forceinline__ void fast_primitive(const GasConst<float> &c, float v
     w[4] = fabsf(a2) < 1e-37f ? sqrtf(a2) : fast_sqrt(a2);
 }
 
-/* limit_slope, without branches on the signs (the same values). */
+/* limit_slope, without branches on the signs: the same values for finite
+ * operands.  (MC beside a NaN or an infinity may differ in sign; the faces of
+ * such a cell have no wave speeds and end the run either way.) */
 template <int LIM>
 __device__ __forceinline__ float fast_slope(float a, float b)
 {

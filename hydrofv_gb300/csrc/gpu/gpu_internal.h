@@ -33,7 +33,8 @@ namespace hydro {
  * 23.8 (3) / 23.7 / 94, 700 x 900 42.9 (4) / 37.8 / 102, 1024^2 61.7 (6) / 61.7
  * / 103, 2048^2 179 (12) / 179 / 216, 4096^2 601 (24) / 600 / 600; 28 grids of
  * side 128 to 640 256 (12) / 256 / 300, 60 of side 500 to 900 1251 (24) / 1251
- * / 1253.
+ * / 1253 (with the power in two instructions; a call of __powf makes 2048^2 183
+ * and 4096^2 612).
  */
 template <class Items>
 int mh2d_fp32_chunk(int slots, Items items)
@@ -179,7 +180,7 @@ inline void mh2d_guided_chunks(int nx, int ny, int strip_w, int slots, int &h1, 
 }
 
 /* The rows of a step are processed in one band as long as its workspace stays
- * below a fixed size (1 GiB in runtime2d.cu).  Bands small enough for the L2
+ * below a fixed size (kStagedWorkspaceBytes, 1 GiB).  Bands small enough for the L2
  * cache lost: 2048^2 3.07 ms with one band, 3.16 / 3.22 / 3.35 / 3.70 ms with
  * 160 / 96 / 48 / 24 MB (the launches' tails cost more than the traffic).
  *

@@ -806,12 +806,6 @@ __device__ __forceinline__ void advance_clock(const Mh2dArgs<R> &a, HydroStepCon
     ctrl->active = act;
 }
 
-/*
- * One time step of one grid.  The grid is persistent: each CTA takes
- * (strip, row chunk) items from a device counter until none are left, so
- * SMs that finish early take more work (the FP64 pipe of an SM is shared by
- * its CTAs).
- */
 /* Fold a block's maxima into the next step's words (threads 0 and 1 write
  * them).  The maxima are never NaN; their ordered encodings (ordered_bits)
  * reduce on the integer pipe. */
@@ -845,6 +839,12 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+/*
+ * One time step of one grid.  The grid is persistent: each CTA takes
+ * (strip, row chunk) items from a device counter until none are left, so
+ * SMs that finish early take more work (the FP64 pipe of an SM is shared by
+ * its CTAs).
+ */
 template <class R, int LIM, int NT, int FIRST_ORDER, bool GRAV = false>
 __global__ void __launch_bounds__(NT, (sizeof(R) == 4 ? MH2D_CTAS_FP32 : MH2D_CTAS_FP64))
 mh2d_step_kernel(const Mh2dArgs<R> a)

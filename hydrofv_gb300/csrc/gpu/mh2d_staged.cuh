@@ -75,6 +75,8 @@ constexpr unsigned kStagedLoopItems = MH2D_LOOP_ITEMS;
 #define MH2D_FUSED_FACES 35000
 #endif
 constexpr unsigned kStagedFusedFaces = MH2D_FUSED_FACES;
+/* Blocks of the update kernel: the chip's 152 SMs full (on fewer, they take
+ * turns). */
 constexpr unsigned kStagedUpdateGrid = 152 * MH2D_UPDATE_CTAS;
 
 /* Fields of the workspace: the low and high face states of each cell in x

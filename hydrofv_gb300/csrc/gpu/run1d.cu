@@ -32,8 +32,8 @@
  * its RK4 source, 8 the predictor.  Hence quotients in line where several are
  * independent, no powers that do not matter, no solve between equal states,
  * warps dealt to the CTAs in turn and two or three barriers a step: Sod 1000
- * to t = 0.2 12.5 -> 10.5 ms, 400 Sedov steps 16.2 -> 8.4 ms (the plain
- * divides before that: 15.9 and 19.0).
+ * to t = 0.2 12.5 -> 11.0 ms (device), 400 Sedov steps 16.2 -> 8.2 ms (the
+ * plain divides before that: 15.9 and 19.0).
  *
  * Per step a cluster-wide max (partials exchanged
  * through distributed shared memory) gives dt, every face flux is computed

@@ -4,10 +4,10 @@
  *
  * The reference's time loop (src/integrator_muscl_hancock.c:530-1160) needs t,
  * dt and the step count on the host every step.  Here they live in device
- * memory: every CTA of a step kernel derives the same dt from the previous
- * step's wave-speed maxima, and the last CTA to finish advances t and the
- * step count, decides whether stepping continues, and re-arms the maxima for
- * the step after next.  The host launches steps in chunks (optionally as a
+ * memory: the last CTA of a step to finish advances t and the step count,
+ * decides whether stepping continues, forms the next step's dt from the
+ * wave-speed maxima, and re-arms the maxima for the step after next (the
+ * many-step kernel's blocks each form the same dt).  The host launches steps in chunks (optionally as a
  * CUDA graph) and only reads this block between chunks.
  */
 #ifndef HYDRO_GPU_STEP_CONTROL_H
@@ -29,7 +29,7 @@ typedef struct HydroStepControl {
     int work_next;                 /* next (strip, row chunk) item of the step, reset every step */
     int store_count;               /* snapshots stored so far (StoringParam.store_count_) */
     double tf;                     /* stop once t >= tf (the dt is clipped to it) */
-    double step_dt;                /* FP64 2D: dt of the next step, formed when the step before it ends */
+    double step_dt;                /* 2D: dt of the next step, formed when the step before it ends */
     double step_dtA[2];            /* and dt A / V of its x and y faces */
     unsigned int barrier_count;    /* grid barrier of the many-step kernel: blocks that have arrived */
     unsigned int barrier_base;     /* and the count when its launch began */

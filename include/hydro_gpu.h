@@ -58,7 +58,7 @@ typedef struct HydroGpuStats
     double step_ms;         /* CUDA-event time of the stepping phase */
     double d2h_ms;          /* CUDA-event time of the final device -> host copies */
     int64 steps;            /* completed time steps */
-    int64 step_launches;    /* step kernels launched (no-op tail launches included) */
+    int64 step_launches;    /* steps enqueued (no-op tails included); small FP64 grids: launches of many steps */
     int64 kernel_launches;  /* every kernel of this library launched by the call */
     int64 h2d_bytes;
     int64 d2h_bytes;
